@@ -4,46 +4,68 @@
 //   o[s,:] = softmax_t( scale * (q[s]·k[t] + bias[b,h,s,t]) ; t < len[b,r] ) · v[t,:]   (* gate[s,:])
 // where `bias` is the triangle bias already divided by `scale` and `gate` holds sigmoid(gate logits) (the
 // prologue writes both that way).
-// The N x N x N logits never exist in memory: a CTA owns 256 queries of one (b, r, h), walks the
-// keys in tiles of 128 and keeps a reference point and a running sum per query and the output in TMEM.
 //
-// Everything that touches a score matrix element is either a tensor-core or a TMEM operation:
-//   TMA      K tile, V tile and the two 128x128 bias tiles (one per 128-query half) -> shared memory
-//   tcgen05  S  = Q·Kᵀ          (128x128x32, K-major operands in smem, accumulator in TMEM)
-//   tcgen05  S += I·Bias        (128x128x128: the identity, resident in TMEM as the A operand, times the
-//                                bias tile as MN-major B operand - the bias add costs no CUDA-core work)
-//   softmax  one thread per query row: S from TMEM -> registers, exp2 relative to the maximum of the row's
-//            first key tile, row sum; the bf16 probabilities go straight back to TMEM
-//   tcgen05  O += P·V           (128x32x128: P is the A operand from TMEM, V the MN-major B operand from
-//                                its [key][d] tile); O is only rescaled when a tile's sum would leave the
-//                                safe fp32 range
-// The two 128-query halves are handled by two softmax warpgroups that share K/V.  Each half has its own
-// score-MMA warp, which runs one key tile ahead (also across work items), so the next scores are in TMEM
-// before a warpgroup asks for them.
+// The N x N x N logits never exist in memory.  A CTA owns four units of work at a time; a unit is 128 queries of one
+// (b, r, h), belongs to one softmax warpgroup and walks the keys in tiles of 64:
+//   TMA      K and V tiles of the item's rows, bias tiles of its 128-query blocks -> shared memory (three stages)
+//   tcgen05  S = Q·Kᵀ   (128x64x32, K-major operands in smem, accumulator in TMEM)
+//   softmax  one thread per query row: S from TMEM -> registers, + bias from shared memory, exp2 relative to the
+//            row's first score, row sum; the bf16 probabilities go straight back to TMEM
+//   tcgen05  O += P·V   (128x32x64: P is the A operand from TMEM, V the MN-major B operand from its [key][d] tile);
+//            O is only rescaled when a tile's sum would leave the safe fp32 range
+//
+// The floor is the special-function unit: 16 exponentials a clock and SM, one per score, 512 clocks of a scheduler for
+// a warp's part of a tile.  Around its exponentials a warp has some 1000 clocks of hand-overs (barrier, TMEM load, P
+// store, barrier), so the unit only stays busy when other warps of the scheduler have exponentials to do meanwhile:
+// four independent units per CTA, i.e. four softmax warps on every scheduler.  Their S, P and O columns have to fit
+// the 512 of TMEM, which is why a key tile has 64 keys, and they would be one S, P and O each (128 columns a unit); but
+// scores only pass through S, while a warpgroup's four warps sit on four schedulers and finish a tile up to 1000
+// clocks apart, and the early ones may not overwrite P before the last one's P·V.  So two units share an S buffer and
+// every unit has two P buffers.
+// The four units of an item are two pair rows x two 128-query blocks (or four rows x one block) of the same head:
+// the bias does not depend on the pair row, so one bias tile in shared memory serves two (four) units, and a K/V
+// tile two.  The bias is added by the softmax threads: on the tensor core (an identity MMA) it would need 64 more
+// columns and four times the operations of Q·Kᵀ, which cost clock rate under the power cap.
+//
+// Measured (one launch, all tokens valid, before this split of two 128-key tile halves per CTA -> now): 512 tokens
+// 224 -> 206 us, 768 tokens 681 -> 640 us, 2048 tokens 12.6 -> 10.8 ms (10.9 exponentials a clock and SM; a tile of
+// four units takes some 2650 clocks, 460 instructions a warp, against 2048 at the unit's rate), an item's end and start
+// another 3500; 333 tokens with holes in the mask 190 -> 138 us.
 //
 // A pair row without a valid key takes a constant path in "uniform" mode (probabilities all 1: the output is the
 // mean of V, as the eager reference computes it) and is skipped in "zeros" mode.
 //
-// Warp roles (384 threads): warps 0-3 softmax half 0, warps 4-7 softmax half 1, warp 8 TMA producer,
-// warps 9 and 11 score-MMA issuers of the two halves (warp 9 owns TMEM), warp 10 P·V-MMA issuer.  The third warpgroup gives most
-// of its registers to the softmax warpgroups (setmaxnreg).
+// Warp roles (640 threads): warps 0-15 softmax (warpgroup w = unit w), warp 16 TMA producer, warp 17 score MMAs / TMEM
+// owner, warps 18 and 19 P·V MMAs of units 0-1 and 2-3.  The fifth warpgroup gives most of its registers to the softmax
+// warpgroups (setmaxnreg).
 #include "common.cuh"
 #include "layout.h"
 
 namespace b200ta {
 namespace {
 
-constexpr int kThreads = 384;
-constexpr int kQTile = 128;  // queries per softmax warpgroup
-constexpr int kKTile = 128;  // keys per tile
-constexpr int kStages = 2;
+constexpr int kThreads = 640;
+constexpr int kQTile = 128;  // queries per unit
+constexpr int kKTile = 64;   // keys per tile
+constexpr int kUnits = 4;
+constexpr int kStages = 3;
 constexpr float kRebaseSum = 1.2676506e30f;  // 2^100: a tile sum at or above this moves the reference point
+
+// A range of pair rows and how its units are put together: per (b, h) `pairs` x ceil(rows / rows_pair) items of two
+// query blocks, then `singles` x ceil(rows / rows_single) items of one block.  All (b, h) of group 0 come first; the
+// host chooses both in split_items().
+struct RowGroup {
+  int row0, row_end, rows_pair, rows_single;
+  int items_pair, items_bh, num_items;
+  uint32_t bh_mul, bh_shr;
+};
 
 struct AttnParams {
   int B, R, S, S_pad;
-  int q_pairs;    // ceil(S / 256)
-  uint32_t r_mul, r_shr, qp_mul, qp_shr;  // division by R and by q_pairs as multiply-high and shift
-  int num_items;  // B * 4 * q_pairs * R
+  int pairs, singles;  // query blocks of a row: 2 * pairs + singles; the first go two by two
+  uint32_t pairs_mul, pairs_shr, singles_mul, singles_shr;  // divisions as multiply-high and shift
+  RowGroup group[2];
+  int num_items;
   const int32_t* lengths;
   long long ls_b, ls_r;
   const uint32_t* key_mask;  // masked form: bit k of word [b][r][k / 32] = key k takes part (0 at and past the length)
@@ -67,120 +89,99 @@ __device__ __forceinline__ void stg256(void* p, const uint32_t* v) {
 }
 
 // shared-memory map (bytes, relative to the 1024-aligned base)
-// K and the bias tiles are only read by the score MMAs, which run a tile ahead, so their ring frees early
-// and two stages are enough to hide the load latency; V waits for the probabilities and gets a deeper ring.
-constexpr int kVStages = 4;
-constexpr int kSmQ = 0;                        // 2 item buffers x 2 halves x 8 KiB
-constexpr int kSmStage = kSmQ + 2 * 2 * 8192;  // per stage: K 8 KiB, bias half0 32 KiB, bias half1 32 KiB
-constexpr int kStageBytes = 8192 + 2 * 32768;
-constexpr int kSmV = kSmStage + kStages * kStageBytes;  // kVStages x 8 KiB
-constexpr int kSmBars = kSmV + kVStages * 8192;
-constexpr int kSmTotal = kSmBars + 256;
+constexpr int kSmQ = 0;                             // 2 item buffers x 4 units x 8 KiB
+constexpr int kSmStage = kSmQ + 2 * kUnits * 8192;  // kStages x 48 KiB, laid out by the three functions below
+constexpr int kStageBytes = 49152;
+constexpr int kSmMask = kSmStage + kStages * kStageBytes;  // masked form: 16 warps x 64 floats, 0 or -inf per key
+constexpr int kSmInfo = kSmMask + 16 * 256;  // ItemInfo of the two item buffers
+constexpr int kSmBars = kSmInfo + 2 * 80;
+constexpr int kSmTotal = kSmBars + 320;
 constexpr int kSmDynamic = kSmTotal + 1024;
 
+// A stage holds the bias tile of block 0 (16 KiB), then either the bias tile of block 1 or the K and V tiles of rows
+// 2 and 3 (4 KiB each), then the K and V tiles of rows 0 and 1.
+__device__ __forceinline__ uint32_t stage_bias(int block) { return block * 16384; }
+__device__ __forceinline__ uint32_t stage_k(int row) { return (row < 2 ? 32768 : 16384) + (row & 1) * 4096; }
+__device__ __forceinline__ uint32_t stage_v(int row) { return stage_k(row) + 8192; }
+
 enum Bar {
-  Q_FULL = 0,    // [2] item buffer
-  Q_EMPTY = 2,   // [2]
-  KB_FULL = 4,   // [kStages] K + bias
-  KB_EMPTY = 6,  // [kStages]
-  S_FULL = 8,    // [2] per half
-  S_FREE = 10,   // [2]
-  P_FULL = 12,   // [2]
-  O_FULL = 14,   // [2]
-  V_FULL = 16,   // [kVStages]
-  V_EMPTY = 20,  // [kVStages]
-  NUM_BARS = 24
+  Q_FULL = 0,     // [2] item buffer
+  Q_EMPTY = 2,    // [2]
+  KV_FULL = 4,    // [kStages] K, V and bias of a tile
+  KV_EMPTY = 7,   // [kStages]
+  S_FULL = 10,    // [4] per unit
+  S_FREE = 14,    // [2] per S buffer
+  P_FULL = 16,    // [4][2] per unit and P buffer
+  O_FULL = 24,    // [4][2]
+  NUM_BARS = 32
 };
 
-// TMEM columns: S of half w | O of half w | P (bf16 pairs) of half w | identity (bf16 pairs)
-constexpr uint32_t kTmemS = 0, kTmemO = 256, kTmemP = 320, kTmemI = 448, kTmemCols = 512;
-
-struct Item {
-  int b, r, h, q0, br;
-  int len;       // keys that take part (S for a uniform row)
-  int nkt;       // key tiles
-  int nvalid;    // 128-query halves that hold at least one query
-  bool uniform;  // no valid key and "uniform" semantics: every logit equal
-  bool skip;     // no valid key and "zeros" semantics: nothing to compute
-};
+// TMEM columns: two S buffers (units w and w + 2 take turns on buffer w % 2: scores only wait there until the
+// warpgroup reads them), two P buffers (bf16 pairs) per unit, O of each unit.
+constexpr uint32_t kTmemS = 0, kTmemP = 128, kTmemO = 384, kTmemCols = 512;
+__device__ __forceinline__ uint32_t p_column(int unit, int buffer) { return kTmemP + unit * 64 + buffer * 32; }
 
 // n / d for n < 2^31 with the constants of fast_div_constants(); mul == 0 stands for d == 1.
 __device__ __forceinline__ int fast_div(int n, uint32_t mul, uint32_t shr) {
   return mul ? int(__umulhi(uint32_t(n), mul) >> shr) : n;
 }
 
-// Row length of a work item as stored (not clamped yet).
-__device__ __forceinline__ int item_raw_length(const AttnParams& p, int item) {
-  if (p.lengths == nullptr) return p.S;
-  const int t = fast_div(item, p.qp_mul, p.qp_shr);
-  const int t2 = fast_div(t, p.r_mul, p.r_shr);
-  const int r = t - t2 * p.R;
-  const int b = t2 / kHeads;
-  return p.lengths[b * p.ls_b + r * p.ls_r];
-}
+// What the other warps need to know about an item, written by the TMA warp into the item's slot (released by Q_FULL).
+struct __align__(16) UnitInfo {
+  int br;     // b * R + r of the unit's pair row
+  int q0;     // first query
+  int len;    // keys that take part (S for a uniform row)
+  int tiles;  // key tiles; 0: no valid key and "zeros" semantics; -1: the item has no such unit
+};
+struct __align__(16) ItemInfo {
+  UnitInfo unit[kUnits];
+  int tiles;       // of the item: the longest row's
+  int two_blocks;  // unit w = row w / 2, block w % 2; otherwise unit w = row w, block 0
+  int h;
+  uint32_t uniform;  // bit per unit: no valid key and "uniform" semantics, every logit equal
+};
+static_assert(sizeof(ItemInfo) == 80, "layout of kSmInfo");
 
-__device__ __forceinline__ Item decode_item(const AttnParams& p, int item, int len) {
+struct Item {
+  int b, h, r0, rows;  // first pair row and how many (1..4)
+  int q0;
+  bool two_blocks;
+};
+
+__device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
+  // Items are ordered (b, h, row group, query blocks) with the query blocks fastest: the CTAs that run at the same
+  // time work on the query blocks of neighbouring pair rows, so a row's K and V come from HBM once (and then from
+  // L2) while the head's bias, shared by all rows, stays in L2.
   Item it;
-  // Items are ordered (b, h, r, query pair) with the query pair fastest: the CTAs that run at the same time work
-  // on the query tiles of neighbouring pair rows, so a row's K and V come from HBM once (and then from L2) while
-  // the head's bias, shared by all rows, stays in L2.
-  const int t = fast_div(item, p.qp_mul, p.qp_shr);
-  const int qp = item - t * p.q_pairs;
-  const int t2 = fast_div(t, p.r_mul, p.r_shr);
-  it.r = t - t2 * p.R;
-  it.h = t2 % kHeads;
-  it.b = t2 / kHeads;
-  it.q0 = qp * 2 * kQTile;
-  it.br = it.b * p.R + it.r;
-  len = len < 0 ? 0 : (len > p.S ? p.S : len);
-  it.uniform = len == 0 && p.empty_uniform;
-  it.skip = len == 0 && !p.empty_uniform;
-  it.len = it.uniform ? p.S : len;
-  it.nkt = (it.len + kKTile - 1) / kKTile;
-  it.nvalid = (it.q0 + kQTile < p.S) ? 2 : 1;
+  const bool second = item >= p.group[0].num_items;
+  const RowGroup& g = p.group[second];
+  if (second) item -= p.group[0].num_items;
+  const int bh = fast_div(item, g.bh_mul, g.bh_shr);
+  int idx = item - bh * g.items_bh;
+  it.h = bh % kHeads;
+  it.b = bh / kHeads;
+  it.two_blocks = idx < g.items_pair;
+  if (it.two_blocks) {
+    const int n = fast_div(idx, p.pairs_mul, p.pairs_shr);
+    it.rows = g.rows_pair;
+    it.r0 = g.row0 + n * g.rows_pair;
+    it.q0 = (idx - n * p.pairs) * 2 * kQTile;
+  } else {
+    idx -= g.items_pair;
+    const int n = fast_div(idx, p.singles_mul, p.singles_shr);
+    it.rows = g.rows_single;
+    it.r0 = g.row0 + n * g.rows_single;
+    it.q0 = (2 * p.pairs + idx - n * p.singles) * kQTile;
+  }
+  if (it.r0 + it.rows > g.row_end) it.rows = g.row_end - it.r0;
   return it;
 }
 
-// Walks the (item, key tile) sequence of one CTA in order, skipping items without work.
-struct TileCursor {
-  int i;     // index into this CTA's item list
-  int kt;    // key tile inside the item
-  int g;     // tiles before this one (ring position)
-  int qi;    // items with work before this one (Q buffer position)
-  Item it;
-  bool valid;
-};
-
-// kWarp: called by all lanes of a converged warp; the row length read from memory is broadcast from lane 0 so
-// that everything derived from it is the same in every lane by construction (warp-uniform code).
-template <bool kWarp = false>
-__device__ __forceinline__ void cursor_seek(const AttnParams& p, TileCursor& c, int my_items) {
-  // positions the cursor on the first item with work at or after c.i
-  while (c.i < my_items) {
-    int len = item_raw_length(p, blockIdx.x + c.i * gridDim.x);
-    if (kWarp) len = __shfl_sync(0xffffffffu, len, 0);
-    c.it = decode_item(p, blockIdx.x + c.i * gridDim.x, len);
-    if (!c.it.skip) {
-      c.valid = true;
-      return;
-    }
-    ++c.i;
-  }
-  c.valid = false;
-}
-template <bool kWarp = false>
-__device__ __forceinline__ void cursor_init(const AttnParams& p, TileCursor& c, int my_items) {
-  c.i = 0, c.kt = 0, c.g = 0, c.qi = 0;
-  cursor_seek<kWarp>(p, c, my_items);
-}
-template <bool kWarp = false>
-__device__ __forceinline__ void cursor_next(const AttnParams& p, TileCursor& c, int my_items) {
-  ++c.g;
-  if (++c.kt < c.it.nkt) return;
-  c.kt = 0;
-  ++c.qi;
-  ++c.i;
-  cursor_seek<kWarp>(p, c, my_items);
+// Row length as stored of the pair row of unit `lane` (clamped to the item's rows).
+__device__ __forceinline__ int raw_length(const AttnParams& p, const Item& it, int lane) {
+  if (p.lengths == nullptr) return p.S;
+  const int row = min(it.two_blocks ? (lane & 3) >> 1 : lane & 3, it.rows - 1);
+  return p.lengths[it.b * p.ls_b + (it.r0 + row) * p.ls_r];
 }
 
 template <bool kMasked>
@@ -203,404 +204,508 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     abort_flag[1] = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + (Q_FULL + i) * 8, 1);
-      mbar_init(bars + (Q_EMPTY + i) * 8, 2);   // one arrival per score-MMA warp
-      mbar_init(bars + (KB_FULL + i) * 8, 1);
-      mbar_init(bars + (KB_EMPTY + i) * 8, 2);  // one arrival per score-MMA warp
-      mbar_init(bars + (S_FULL + i) * 8, 1);
-      mbar_init(bars + (S_FREE + i) * 8, 4);
+      mbar_init(bars + (Q_EMPTY + i) * 8, 2 + 1 + 16);  // P·V warps, score warp, softmax warps (read the item's info)
+    }
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(bars + (KV_FULL + i) * 8, 1);
+      mbar_init(bars + (KV_EMPTY + i) * 8, 2);  // one arrival per P·V warp
+    }
+    for (int i = 0; i < kUnits; ++i) mbar_init(bars + (S_FULL + i) * 8, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(bars + (S_FREE + i) * 8, 4);
+    for (int i = 0; i < 2 * kUnits; ++i) {
       mbar_init(bars + (P_FULL + i) * 8, 4);
       mbar_init(bars + (O_FULL + i) * 8, 1);
     }
-    for (int i = 0; i < kVStages; ++i) {
-      mbar_init(bars + (V_FULL + i) * 8, 1);
-      mbar_init(bars + (V_EMPTY + i) * 8, 1);
-    }
     fence_mbar_init();
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+  if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // The 128x128 bf16 identity, A operand of the bias MMA: TMEM lane q, column c holds elements (q, 2c) and
-  // (q, 2c+1) as a bf16 pair, so lane q has a single 1.0 in column q/2.
-  if (warp < 4) {
-    const int q = warp * 32 + lane;
-    const uint32_t one = (q & 1) ? 0x3F800000u : 0x00003F80u;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) v[c] = (half * 32 + c == (q >> 1)) ? one : 0u;
-      tmem_st32(tmem_base + (uint32_t(warp * 32) << 16) + kTmemI + half * 32, v);
-    }
-    tmem_st_wait();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-
   const int my_items = (p.num_items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
-  // Register budget.  The CTA starts with 168 registers per thread; setmaxnreg only moves registers inside
-  // that allocation, and an increase blocks until a decrease has freed enough: the third warpgroup drops
-  // to 72 (frees 128 x 96) and the two softmax warpgroups rise to 216 (need 256 x 48, the same number).
-  if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  // Register budget: 640 threads start with 96 registers; setmaxnreg only moves registers inside that allocation,
+  // and an increase blocks until a decrease has freed enough: the fifth warpgroup drops to 64 (frees 128 x 32) and
+  // the softmax warpgroups rise to 104 (need 512 x 8, the same number).
+  if (warp >= 16) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   }
-  if (warp == 8) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 16) {
+    // ------------------------------------------------------------------ TMA producer (whole warp, one lane issues)
     if (lane == 0) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
       tma_prefetch_desc(&tm_bias);
-      TileCursor c;
-      cursor_init(p, c, my_items);
-      int issued = 0;
-      bool ok = true;
-      while (ok && c.valid) {
-        const Item& it = c.it;
-        if (c.kt == 0) {
-          const int ib = c.qi & 1;
-          ok = mbar_wait(bars + (Q_EMPTY + ib) * 8, ((c.qi >> 1) & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          mbar_expect_tx(bars + (Q_FULL + ib) * 8, it.nvalid * 8192);
-          for (int w = 0; w < it.nvalid; ++w)
-            tma_load_4d(base + kSmQ + (ib * 2 + w) * 8192, &tm_q, bars + (Q_FULL + ib) * 8, 0, it.q0 + w * kQTile,
-                        it.h, it.br);
-        }
-        // K + bias of this tile (needed first, by the score MMAs)
-        const int stage = c.g % kStages;
-        ok = mbar_wait(bars + (KB_EMPTY + stage) * 8, ((c.g / kStages) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        const uint32_t full = bars + (KB_FULL + stage) * 8;
-        const uint32_t sbase = base + kSmStage + stage * kStageBytes;
-        mbar_expect_tx(full, 8192 + (it.uniform ? 0 : it.nvalid * 32768));
-        tma_load_4d(sbase, &tm_k, full, 0, c.kt * kKTile, it.h, it.br);
-        if (!it.uniform)
-          for (int w = 0; w < it.nvalid; ++w)
-            for (int half = 0; half < 2; ++half)
-              tma_load_4d(sbase + 8192 + w * 32768 + half * 16384, &tm_bias, full, c.kt * kKTile + half * 64,
-                          it.q0 + w * kQTile, it.h, it.b);
-        // V of this tile
-        const int vs = c.g % kVStages;
-        ok = mbar_wait(bars + (V_EMPTY + vs) * 8, ((c.g / kVStages) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        mbar_expect_tx(bars + (V_FULL + vs) * 8, 8192);
-        tma_load_4d(base + kSmV + vs * 8192, &tm_v, bars + (V_FULL + vs) * 8, 0, c.kt * kKTile, it.h, it.br);
-        ++issued;
-        cursor_next(p, c, my_items);
-      }
-      // If the loop was abandoned, give copies still in flight a bounded chance to land.
-      if (*abort_flag && issued > 0) {
-        const int last = issued - 1;
-        mbar_wait(bars + (V_FULL + last % kVStages) * 8, (last / kVStages) & 1, abort_flag + 1);
-      }
     }
-  } else if (warp == 9 || warp == 11) {
-    // ------------------------------------------------------------------ score MMA issuers (S = Q·Kᵀ + I·Bias)
-    // One warp per 128-query half.  All 32 lanes run the loop with the same values and one elected lane issues
-    // (umma_*_warp): a converged warp issues its MMAs at the rate the tensor pipe retires them, a single thread
-    // inside a branch needs 45-80 clocks per MMA.  Each warp runs one key tile ahead of the softmax (also across
-    // work items): the only thing it waits for besides the loads is that its half's S buffer has been read out.
-    {
-      constexpr uint32_t idesc_s = make_idesc_bf16(kQTile, kKTile);                // Q·Kᵀ: both operands K-major
-      constexpr uint32_t idesc_b1 = make_idesc_bf16(kQTile, 128, false, true);     // I·Bias: B MN-major
-      const int w = __shfl_sync(0xffffffffu, warp == 9 ? 0 : 1, 0);
-      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
-      const uint32_t ti = tb + kTmemI;
-      const uint32_t d = tb + kTmemS + w * 128;  // S of this half
-      int n = 0;                                 // S tiles issued (phase of S_FREE)
-      bool ok = true;
-      TileCursor c;
-      cursor_init<true>(p, c, my_items);
-      while (ok && c.valid) {
-        const Item& it = c.it;
-        const int ib = c.qi & 1, stage = c.g % kStages;
-        if (c.kt == 0) ok = mbar_wait_warp(bars + (Q_FULL + ib) * 8, (c.qi >> 1) & 1, abort_flag);
-        ok = ok && mbar_wait_warp(bars + (KB_FULL + stage) * 8, (c.g / kStages) & 1, abort_flag);
-        if (!ok) break;
-        if (w < it.nvalid) {
-          // One descriptor per operand tile; the K steps only add a constant to its address field (in 16-byte
-          // units).
-          const uint32_t sbase = base + kSmStage + stage * kStageBytes;
-          const uint64_t dk = make_smem_desc(sbase, 16, 512, kLayoutSw64);
-          const uint64_t dq = make_smem_desc(base + kSmQ + ib * 16384 + w * 8192, 16, 512, kLayoutSw64);
-          // Bias tiles: [128 query rows][64 keys] blocks with 128-byte swizzle, 16 KiB apart: keys 0-63 and
-          // 64-127 of half 0, then of half 1.  As B[key][query] this is MN-major with 16 query rows (2 KiB)
-          // per K step.
-          const uint64_t db = make_smem_desc(sbase + 8192 + w * 32768, 16384, 1024, kLayoutSw128);
-          ok = mbar_wait_warp(bars + (S_FREE + w) * 8, (n & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          if (!it.uniform) {  // a row without a valid key has equal logits: the softmax warps need no scores
-            umma_ss_warp(d, dq, dk, idesc_s, 0u);
-            umma_ss_warp(d, dq + 2, dk + 2, idesc_s, 1u);  // second 16 channels: +32 bytes
-#pragma unroll
-            for (int j = 0; j < 8; ++j) umma_ts_warp(d, ti + j * 8, db + j * 128, idesc_b1, 1u);
-          }
-          umma_commit_warp(bars + (S_FULL + w) * 8);
-          ++n;
-          umma_commit_warp(bars + (KB_EMPTY + stage) * 8);  // K and bias are free once both halves' MMAs ran
-          if (c.kt == it.nkt - 1) umma_commit_warp(bars + (Q_EMPTY + ib) * 8);  // last use of this item's Q
-        } else {
-          // this half holds no query of the item: only keep the shared barriers' counts complete
-          mbar_arrive_warp(bars + (KB_EMPTY + stage) * 8);
-          if (c.kt == it.nkt - 1) mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);
-        }
-        cursor_next<true>(p, c, my_items);
-      }
-    }
-  } else if (warp == 10) {
-    // ------------------------------------------------------------------ P·V MMA issuer (warp-collective as well)
-    {
-      constexpr uint32_t idesc_o = make_idesc_bf16(kQTile, kHeadDim, false, true);  // P·V: B is MN-major
-      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
-      int n0 = 0, n1 = 0;  // P tiles consumed per half
-      bool ok = true;
-      TileCursor c;
-      cursor_init<true>(p, c, my_items);
-      while (ok && c.valid) {
-        const Item& it = c.it;
-        const int vs = c.g % kVStages;
-        ok = mbar_wait_warp(bars + (V_FULL + vs) * 8, (c.g / kVStages) & 1, abort_flag);
-        const uint64_t dv = make_smem_desc(base + kSmV + vs * 8192, 16, 512, kLayoutSw64);
-        const uint32_t acc0 = c.kt > 0 ? 1u : 0u;
-        ok = ok && mbar_wait_warp(bars + (P_FULL + 0) * 8, n0 & 1, abort_flag);
-        if (!ok) break;
-        ++n0;
-        tc_fence_after();
-        {
-          const uint32_t d = tb + kTmemO, tp = tb + kTmemP;
-          umma_ts_warp(d, tp, dv, idesc_o, acc0);
-#pragma unroll
-          for (int j = 1; j < 8; ++j) umma_ts_warp(d, tp + j * 8, dv + j * 64, idesc_o, 1u);  // 16 keys = 1 KiB per step
-          umma_commit_warp(bars + (O_FULL + 0) * 8);
-        }
-        if (it.nvalid == 2) {
-          ok = mbar_wait_warp(bars + (P_FULL + 1) * 8, n1 & 1, abort_flag);
-          if (!ok) break;
-          ++n1;
-          tc_fence_after();
-          const uint32_t d = tb + kTmemO + 32, tp = tb + kTmemP + 64;
-          umma_ts_warp(d, tp, dv, idesc_o, acc0);
-#pragma unroll
-          for (int j = 1; j < 8; ++j) umma_ts_warp(d, tp + j * 8, dv + j * 64, idesc_o, 1u);
-          umma_commit_warp(bars + (O_FULL + 1) * 8);
-        }
-        umma_commit_warp(bars + (V_EMPTY + vs) * 8);
-        cursor_next<true>(p, c, my_items);
-      }
-    }
-  } else if (warp < 8) {
-    // ------------------------------------------------------------------ softmax warpgroups
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-    const int w = warp >> 2;               // which 128-query half
-    const int m = (warp & 3) * 32 + lane;  // query row inside the half == TMEM lane
-    const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-    const uint32_t s_addr = lane_taddr + kTmemS + w * 128;
-    const uint32_t o_addr = lane_taddr + kTmemO + w * 32;
-    const uint32_t p_addr = lane_taddr + kTmemP + w * 64;
-    const float c = p.scale_log2;                 // raw score -> log2-domain logit
-    const uint64_t c2 = pack_f32x2(c, c);
-    int ct = 0;  // tiles this half has processed (phase of S_FULL / O_FULL)
+    int g = 0, i = 0;  // tiles and items loaded
     bool ok = true;
-    int next_len = item_raw_length(p, blockIdx.x);
-    for (int i = 0; ok && i < my_items; ++i) {
-      const Item it = decode_item(p, blockIdx.x + i * gridDim.x, next_len);
-      // fetch the next item's row length now: its global-memory latency hides behind this item's work
-      if (i + 1 < my_items) next_len = item_raw_length(p, blockIdx.x + (i + 1) * gridDim.x);
-      const int q = it.q0 + w * kQTile + m;  // query position
-      __nv_bfloat16* out_row = p.out + it.br * p.o_br + (long long)q * p.o_s + it.h * p.o_h;
-      if (it.skip) {
-        if (q < p.S) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(out_row)[j] = make_uint4(0, 0, 0, 0);
-          if (p.lse) p.lse[((long long)it.br * p.S + q) * kHeads + it.h] = -INFINITY;
-        }
-        continue;
+    Item it = decode_item(p, blockIdx.x);
+    int raw = raw_length(p, it, lane);
+    while (i < my_items) {
+      // lane u: unit u
+      const int blocks = it.two_blocks ? 2 : 1;
+      const int row = it.two_blocks ? (lane & 3) >> 1 : lane & 3;
+      int len = raw < 0 ? 0 : (raw > p.S ? p.S : raw);
+      const bool exists = row < it.rows;
+      const bool uni = exists && len == 0 && p.empty_uniform;
+      if (uni) len = p.S;
+      const int nt = exists ? (len + kKTile - 1) / kKTile : -1;
+      const int tiles = max(0, __reduce_max_sync(0xffffffffu, nt));
+      const uint32_t uniform = __ballot_sync(0xffffffffu, uni) & 15u;
+      const int ib = i & 1;
+      ok = mbar_wait_warp(bars + (Q_EMPTY + ib) * 8, ((i >> 1) & 1) ^ 1, abort_flag);
+      if (!ok) break;
+      ItemInfo* info = reinterpret_cast<ItemInfo*>(gen + kSmInfo) + ib;
+      const int br = it.b * p.R + it.r0;
+      if (lane < kUnits) {
+        *reinterpret_cast<int4*>(&info->unit[lane]) =
+            make_int4(br + row, it.q0 + (it.two_blocks ? lane & 1 : 0) * kQTile, len, nt);
+      } else if (lane == kUnits) {
+        *reinterpret_cast<int4*>(&info->tiles) = make_int4(tiles, it.two_blocks, it.h, int(uniform));
       }
-      if (w >= it.nvalid) continue;  // this half holds no query of the item
-      float row_max = 0.f, row_sum = 0.f;  // row_max: reference point of the exponentials, in raw score units
-      bool have_anchor = false;            // masked form: a key tile with a valid key has been seen
-      uint4 gv[4];                               // gate row, fetched during the last key tile
-#pragma unroll
-      for (int j = 0; j < 4; ++j) gv[j] = make_uint4(0, 0, 0, 0);
-
-      for (int kt = 0; kt < it.nkt; ++kt, ++ct) {
-        if (kt == it.nkt - 1 && p.gate != nullptr && q < p.S) {
-          const uint4* gp = reinterpret_cast<const uint4*>(p.gate + it.br * p.g_br + it.h * p.g_h + (long long)q * p.g_s);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) gv[j] = __ldg(gp + j);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_expect_tx(bars + (Q_FULL + ib) * 8, tiles > 0 ? it.rows * blocks * 8192 : 0);
+        if (tiles > 0)
+          for (int r = 0; r < it.rows; ++r)
+            for (int w = 0; w < blocks; ++w)
+              tma_load_4d(base + kSmQ + (ib * kUnits + r * blocks + w) * 8192, &tm_q, bars + (Q_FULL + ib) * 8, 0,
+                          it.q0 + w * kQTile, it.h, br + r);
+      }
+      __syncwarp();
+      ++i;
+      const Item cur = it;
+      if (i < my_items) {  // the next item's row lengths arrive while this item's tiles are loaded
+        it = decode_item(p, blockIdx.x + i * gridDim.x);
+        raw = raw_length(p, it, lane);
+      }
+      for (int kt = 0; kt < tiles; ++kt, ++g) {
+        const int stage = g % kStages;
+        ok = mbar_wait_warp(bars + (KV_EMPTY + stage) * 8, ((g / kStages) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        // rows with this tile (a bit per row), and those of them that need the bias
+        const bool first = !cur.two_blocks || (lane & 1) == 0;
+        const uint32_t units = __ballot_sync(0xffffffffu, lane < kUnits && kt < nt);
+        const uint32_t loads = __ballot_sync(0xffffffffu, lane < kUnits && first && kt < nt);
+        if (lane == 0) {
+          const uint32_t full = bars + (KV_FULL + stage) * 8;
+          const uint32_t sbase = base + kSmStage + stage * kStageBytes;
+          const bool with_bias = (units & ~uniform) != 0;
+          mbar_expect_tx(full, __popc(loads) * 8192 + (with_bias ? blocks * 16384 : 0));
+          if (with_bias)
+            for (int w = 0; w < blocks; ++w)
+              tma_load_4d(sbase + stage_bias(w), &tm_bias, full, kt * kKTile, cur.q0 + w * kQTile, cur.h, cur.b);
+          for (uint32_t left = loads; left; left &= left - 1) {
+            const int u = __ffs(left) - 1, r = cur.two_blocks ? u >> 1 : u;
+            tma_load_4d(sbase + stage_k(r), &tm_k, full, 0, kt * kKTile, cur.h, br + r);
+            tma_load_4d(sbase + stage_v(r), &tm_v, full, 0, kt * kKTile, cur.h, br + r);
+          }
         }
-        ok = mbar_wait(bars + (S_FULL + w) * 8, ct & 1, abort_flag);
+        __syncwarp();
+      }
+      if (!ok) break;
+    }
+    // If the loop was abandoned, give copies still in flight a bounded chance to land.
+    if (*abort_flag && lane == 0) {
+      for (int j = g > kStages ? g - kStages : 0; j < g; ++j)
+        mbar_wait(bars + (KV_FULL + j % kStages) * 8, (j / kStages) & 1, abort_flag + 1);
+      for (int j = i > 2 ? i - 2 : 0; j < i; ++j) mbar_wait(bars + (Q_FULL + (j & 1)) * 8, (j >> 1) & 1, abort_flag + 1);
+    }
+    __syncwarp();
+  } else if (warp == 17) {
+    // ------------------------------------------------------------------ score MMAs (S = Q·Kᵀ) of the four units
+    // All 32 lanes run the loop with the same values and one elected lane issues (umma_*_warp).  The warp runs a
+    // tile ahead of the softmax, also across items: all it waits for besides the loads is that a unit's S columns
+    // have been read.
+    constexpr uint32_t idesc_s = make_idesc_bf16(kQTile, kKTile);  // both operands K-major
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int stage = 0, stage_phase = 0;
+    uint32_t ns = 0;  // bit b: parity of the tiles issued into S buffer b
+    bool ok = true;
+    for (int i = 0; ok && i < my_items; ++i) {
+      const int ib = i & 1;
+      ok = mbar_wait_warp(bars + (Q_FULL + ib) * 8, (i >> 1) & 1, abort_flag);
+      if (!ok) break;
+      const ItemInfo* info = reinterpret_cast<const ItemInfo*>(gen + kSmInfo) + ib;
+      const int tiles = info->tiles, two_blocks = info->two_blocks;
+      const uint32_t uniform = info->uniform;
+      int nt[kUnits];
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u) nt[u] = info->unit[u].tiles;
+      __syncwarp();
+      mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);  // the info has been read (Q itself: see the P·V warps)
+      const uint32_t q0 = base + kSmQ + ib * (kUnits * 8192);
+      for (int kt = 0; ok && kt < tiles; ++kt) {
+        ok = mbar_wait_warp(bars + (KV_FULL + stage) * 8, stage_phase, abort_flag);
+        const uint32_t sbase = base + kSmStage + stage * kStageBytes;
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u) {
+          if (!ok || kt >= nt[u]) continue;
+          const int sb = u & 1;
+          ok = mbar_wait_warp(bars + (S_FREE + sb) * 8, ((ns >> sb) & 1u) ^ 1u, abort_flag);
+          if (!ok) continue;
+          ns ^= 1u << sb;
+          tc_fence_after();
+          if (!((uniform >> u) & 1u)) {  // a uniform row has equal logits: the softmax warps need no scores
+            const uint64_t dq = smem_desc<16, 512, kLayoutSw64>(q0 + u * 8192);
+            const uint64_t dk = smem_desc<16, 512, kLayoutSw64>(sbase + stage_k(two_blocks ? u >> 1 : u));
+            umma_ss_warp(tb + kTmemS + sb * 64, dq, dk, idesc_s, 0u);
+            umma_ss_warp(tb + kTmemS + sb * 64, dq + 2, dk + 2, idesc_s, 1u);  // second 16 channels: +32 bytes
+          }
+          umma_commit_warp(bars + (S_FULL + u) * 8);
+        }
+        if (++stage == kStages) stage = 0, stage_phase ^= 1;
+      }
+    }
+  } else if (warp == 18 || warp == 19) {
+    // ------------------------------------------------------------------ P·V MMAs of units 2j and 2j + 1
+    constexpr uint32_t idesc_o = make_idesc_bf16(kQTile, kHeadDim, false, true);  // B is MN-major
+    const int j = __shfl_sync(0xffffffffu, warp - 18, 0);
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int stage = 0, stage_phase = 0;
+    uint32_t np[2] = {0, 0};  // P tiles consumed of the two units
+    bool ok = true;
+    for (int i = 0; ok && i < my_items; ++i) {
+      const int ib = i & 1;
+      ok = mbar_wait_warp(bars + (Q_FULL + ib) * 8, (i >> 1) & 1, abort_flag);
+      if (!ok) break;
+      const ItemInfo* info = reinterpret_cast<const ItemInfo*>(gen + kSmInfo) + ib;
+      const int tiles = info->tiles, two_blocks = info->two_blocks;
+      const int row_tiles[2] = {info->unit[2 * j].tiles, info->unit[2 * j + 1].tiles};
+      const int row[2] = {two_blocks ? j : 2 * j, two_blocks ? j : 2 * j + 1};
+      for (int kt = 0; ok && kt < tiles; ++kt) {
+        ok = mbar_wait_warp(bars + (KV_FULL + stage) * 8, stage_phase, abort_flag);
+        const uint32_t sbase = base + kSmStage + stage * kStageBytes;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (!ok || kt >= row_tiles[u]) continue;
+          const int w = 2 * j + u, pb = np[u] & 1;
+          ok = mbar_wait_warp(bars + (P_FULL + 2 * w + pb) * 8, (np[u] >> 1) & 1u, abort_flag);
+          if (!ok) continue;
+          ++np[u];
+          tc_fence_after();
+          const uint32_t d = tb + kTmemO + w * 32, tp = tb + p_column(w, pb);
+          const uint64_t dv = smem_desc<16, 512, kLayoutSw64>(sbase + stage_v(row[u]));
+          umma_ts_warp(d, tp, dv, idesc_o, kt > 0 ? 1u : 0u);
+#pragma unroll
+          for (int k = 1; k < 4; ++k) umma_ts_warp(d, tp + k * 8, dv + k * 64, idesc_o, 1u);  // 16 keys = 1 KiB per step
+          umma_commit_warp(bars + (O_FULL + 2 * w + pb) * 8);
+        }
+        if (!ok) break;
+        // The probabilities these MMAs waited for say that the scores' MMAs have read K (and Q), and the
+        // warpgroups the bias: the stage, and after the last tile the Q buffer, are free once the MMAs ran.
+        umma_commit_warp(bars + (KV_EMPTY + stage) * 8);
+        if (kt == tiles - 1) umma_commit_warp(bars + (Q_EMPTY + ib) * 8);
+        if (++stage == kStages) stage = 0, stage_phase ^= 1;
+      }
+      if (tiles == 0) mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);
+    }
+  } else if (warp < 16) {
+    // ------------------------------------------------------------------ softmax warpgroups
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int w = warp >> 2;               // unit
+    const int m = (warp & 3) * 32 + lane;  // query row inside the unit == TMEM lane
+    const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    const uint32_t s_addr = lane_taddr + kTmemS + (w & 1) * 64;
+    const uint32_t o_addr = lane_taddr + kTmemO + w * 32;
+    const float c = p.scale_log2;  // raw score -> log2-domain logit
+    const uint64_t c2 = pack_f32x2(c, c);
+    int ct = 0;  // tiles this unit has processed (phase of S_FULL / O_FULL)
+    int stage = 0, stage_phase = 0;  // ring position
+    bool ok = true;
+    for (int i = 0; ok && i < my_items; ++i) {
+      const int ib = i & 1;
+      ok = mbar_wait_warp(bars + (Q_FULL + ib) * 8, (i >> 1) & 1, abort_flag);
+      if (!ok) break;
+      const ItemInfo* info = reinterpret_cast<const ItemInfo*>(gen + kSmInfo) + ib;
+      const int4 unit = *reinterpret_cast<const int4*>(&info->unit[w]);
+      const int4 common = *reinterpret_cast<const int4*>(&info->tiles);
+      __syncwarp();
+      mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);
+      const int my_tiles = unit.w, len = unit.z, h = common.z;
+      const int br = unit.x, q = unit.y + m;  // pair row, query position
+      const bool uniform = (common.w >> w) & 1;
+      const uint32_t block_off = stage_bias(common.y ? w & 1 : 0) + sw128_offset(m, 0);
+      const __nv_bfloat16* gate_row = p.gate + br * p.g_br + h * p.g_h + (long long)q * p.g_s;
+      if (p.gate != nullptr && q < p.S) asm volatile("prefetch.global.L2 [%0];" ::"l"(gate_row));  // read at the end
+      float row_max = 0.f, row_sum = 0.f;  // row_max: reference point of the exponentials, in raw score units
+      const uint32_t* mask_row = nullptr;
+      if (kMasked) {
+        const int b = br / p.R;
+        mask_row = p.key_mask + b * p.km_b + (br - b * p.R) * p.km_r;
+      }
+      bool have_anchor = false;            // masked form: a key tile with a valid key has been seen
+
+      for (int kt = 0; kt < my_tiles; ++kt) {
+        // Scores ready; K, V and bias of the tile loaded (they are, or it would have no scores: the wait makes the
+        // copies' writes visible to this thread); P·V of the tile before the previous one complete, so that this
+        // tile's P buffer may be overwritten.
+        const int pb = ct & 1;
+        ok = mbar_wait2_warp(bars + (S_FULL + w) * 8, pb, bars + (KV_FULL + stage) * 8, stage_phase, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        if (it.uniform) {
+        const uint32_t o_done = bars + (O_FULL + 2 * w + pb) * 8;
+        const uint32_t o_parity = ((ct >> 1) & 1) ^ 1;
+        const uint32_t p_addr = lane_taddr + p_column(w, pb);
+        ++ct;
+        const uint32_t bias0 = base + kSmStage + stage * kStageBytes + block_off;
+        if (++stage == kStages) stage = 0, stage_phase ^= 1;
+        const int rem = len - kt * kKTile;  // valid keys in this tile
+        if (uniform) {
           // No valid key, eager semantics: every logit is the same, so every probability of the tile is 1 (0 past
           // the last key) and the output becomes the mean of V.  No scores are read, no exponentials taken.
           __syncwarp();
-          if (lane == 0) mbar_arrive(bars + (S_FREE + w) * 8);
-          if (kt > 0) {
-            ok = mbar_wait(bars + (O_FULL + w) * 8, (ct - 1) & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-          }
-          const int rem = it.len - kt * kKTile;  // keys in this tile
+          mbar_arrive_warp(bars + (S_FREE + (w & 1)) * 8);
+          ok = mbar_wait_warp(o_done, o_parity, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
-          for (int qtr = 0; qtr < 4; ++qtr) {
+          for (int half = 0; half < 2; ++half) {
             uint32_t pk[16];
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-              const int j0 = qtr * 32 + 2 * e;
+              const int j0 = half * 32 + 2 * e;
               pk[e] = j0 + 1 < rem ? 0x3F803F80u : (j0 < rem ? 0x00003F80u : 0u);  // bf16 pairs of 1.0
             }
-            tmem_st16(p_addr + qtr * 16, pk);
+            tmem_st16(p_addr + half * 16, pk);
           }
           row_sum += float(rem < kKTile ? rem : kKTile);
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bars + (P_FULL + w) * 8);
+          mbar_arrive_warp(bars + (P_FULL + 2 * w + pb) * 8);
           continue;
         }
-        float s2[128];  // raw scores (bias included) of this row against the tile's 128 keys
-        tmem_ld32_f128<0>(s_addr, s2);
-        tmem_ld32_f128<32>(s_addr + 32, s2);
-        tmem_ld32_f128<64>(s_addr + 64, s2);
-        tmem_ld32_f128<96>(s_addr + 96, s2);
+        float s2[64];  // raw scores of this row against the tile's 64 keys
+        tmem_ld64(s_addr, s2);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + (S_FREE + w) * 8);  // the S buffer can take the next tile's scores
+        mbar_arrive_warp(bars + (S_FREE + (w & 1)) * 8);  // the S buffer can take the next tile's scores
 
-        const int rem = it.len - kt * kKTile;  // valid keys in this tile
-        if (rem < kKTile) {
-#pragma unroll
-          for (int j = 0; j < 128; ++j)
-            if (j >= rem) s2[j] = -INFINITY;
-        }
-        // The reference point of the exponentials is the maximum of the item's first key tile.  Later tiles
-        // skip the search for a maximum: fp32 sums, fp32 O and bf16 P share the fp32 exponent range, so
+        // p = 2^(c * (s + bias - row_max)); bf16 pairs go back to TMEM as the A operand of P·V.  16 keys at a time,
+        // the bias of the next 16 requested before the exponentials of these, so that its latency and unpacking
+        // hide behind the special-function unit.
+        // The reference point of the exponentials is the row's first valid score.  No maximum is searched: the
+        // largest probability is at least 1, fp32 sums, fp32 O and bf16 P share the fp32 exponent range, so
         // probabilities far above 1 lose nothing, and a tile whose sum leaves the safe range is redone below.
-        bool find_anchor = kt == 0;
-        if (kMasked) {
-          // Keys may be switched off anywhere in the row (the same bits for every query of this item).  A tile
-          // without any valid key yields zeros (the reference point stays 0 until a tile with a valid key comes).
-          const uint32_t* mrow = p.key_mask + it.b * p.km_b + it.r * p.km_r + kt * 4;
-          const int words = (p.S + 31) >> 5;
-          uint32_t mw[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) mw[j] = kt * 4 + j < words ? __ldg(mrow + j) : 0u;
-#pragma unroll
-          for (int j = 0; j < 128; ++j)
-            if (!((mw[j >> 5] >> (j & 31)) & 1u)) s2[j] = -INFINITY;
-          find_anchor = !have_anchor && (mw[0] | mw[1] | mw[2] | mw[3]) != 0u;
-          have_anchor = have_anchor || find_anchor;
-        }
-        if (kt > 0) {
-          // the previous tile's P·V must be complete before P is overwritten
-          ok = mbar_wait(bars + (O_FULL + w) * 8, (ct - 1) & 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (find_anchor) {
-          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four independent chains
-#pragma unroll
-          for (int j = 0; j < 64; ++j) mx[j & 3] = max3_f32(mx[j & 3], s2[2 * j], s2[2 * j + 1]);
-          row_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));  // finite: the tile holds a valid key
-        }
-        // p = 2^(c * (s - row_max)); bf16 pairs go back to TMEM as the A operand of P·V
-        float tile_sum;
-        {
+        const bool plain = !kMasked && rem >= kKTile;
+        uint64_t sum2[2] = {0ull, 0ull};  // independent packed partial sums
+        if (plain) {
+          uint4 x[2][2];
+          x[0][0] = lds128(bias0), x[0][1] = lds128(bias0 ^ 16);
+          if (kt == 0) row_max = s2[0] + bf16_lo(x[0][0].x);
           const float nmc = -row_max * c;
           const uint64_t nmc2 = pack_f32x2(nmc, nmc);
-          uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};  // four independent packed partial sums
 #pragma unroll
-          for (int qtr = 0; qtr < 4; ++qtr) {
-            uint32_t pk[16];
+          for (int ch = 0; ch < 4; ++ch) {
+            if (ch < 3) {
+              x[(ch + 1) & 1][0] = lds128(bias0 ^ ((2 * ch + 2) << 4));
+              x[(ch + 1) & 1][1] = lds128(bias0 ^ ((2 * ch + 3) << 4));
+            }
+            uint32_t pk[8];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int j0 = qtr * 32 + 2 * e;
-              const uint64_t d2 = fma_f32x2(pack_f32x2(s2[j0], s2[j0 + 1]), c2, nmc2);
+            for (int e = 0; e < 8; ++e) {
+              const int j0 = ch * 16 + 2 * e;
+              const uint4& xx = x[ch & 1][e >> 2];
+              const uint32_t bw = (e & 3) == 0 ? xx.x : (e & 3) == 1 ? xx.y : (e & 3) == 2 ? xx.z : xx.w;
+              const uint64_t t2 = fma_f32x2(pack_f32x2(bf16_lo(bw), bf16_hi(bw)), c2, nmc2);
               float d0, d1;
-              unpack_f32x2(d2, d0, d1);
-              const uint64_t p2 = pack_f32x2(ex2_approx(d0), ex2_approx(d1));
-              sum2[e & 3] = add_f32x2(sum2[e & 3], p2);
-              float p0, p1;
-              unpack_f32x2(p2, p0, p1);
+              unpack_f32x2(fma_f32x2(pack_f32x2(s2[j0], s2[j0 + 1]), c2, t2), d0, d1);
+              const float p0 = ex2_approx(d0), p1 = ex2_approx(d1);
+              sum2[e & 1] = add_f32x2(sum2[e & 1], pack_f32x2(p0, p1));
               pk[e] = pack_bf16x2(p0, p1);
             }
-            tmem_st16(p_addr + qtr * 16, pk);
+            if (ch == 0) {
+              ok = mbar_wait_warp(o_done, o_parity, abort_flag);
+              tc_fence_after();
+            }
+            tmem_st8(p_addr + ch * 8, pk);
           }
+        } else {
+          // last tile (keys past the row length) and masked form
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch) {
+            const uint4 x = lds128(bias0 ^ (ch << 4));
+            const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int j0 = ch * 8 + 2 * e;
+              unpack_f32x2(add_f32x2(pack_f32x2(s2[j0], s2[j0 + 1]), pack_f32x2(bf16_lo(xw[e]), bf16_hi(xw[e]))), s2[j0],
+                           s2[j0 + 1]);
+            }
+          }
+          bool find_anchor = false;
+          if (kMasked) {
+            // Keys may be switched off anywhere in the row (the same bits for every query of the unit): the warp
+            // expands the tile's bits to 0 / -inf in its own scratch and adds them.  Keys past the row length have
+            // their bit clear.  A tile without any valid key yields zeros (the reference point stays 0 until a tile
+            // with a valid key comes).
+            const uint32_t* mrow = mask_row + kt * 2;
+            const int words = (p.S + 31) >> 5;
+            const uint32_t m0 = __ldg(mrow), m1 = kt * 2 + 1 < words ? __ldg(mrow + 1) : 0u;
+            const uint32_t scratch = base + kSmMask + warp * 256;
+            {
+              const uint32_t pair = (lane < 16 ? m0 : m1) >> ((2 * lane) & 31);
+              __syncwarp();  // the previous tile's reads are done
+              asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(scratch + lane * 8),
+                           "r"((pair & 1u) ? 0u : 0xFF800000u), "r"((pair & 2u) ? 0u : 0xFF800000u)
+                           : "memory");
+              __syncwarp();
+            }
+#pragma unroll
+            for (int ch = 0; ch < 16; ++ch) {
+              const uint4 x = lds128(scratch + ch * 16);
+              unpack_f32x2(add_f32x2(pack_f32x2(s2[ch * 4], s2[ch * 4 + 1]),
+                                     pack_f32x2(__uint_as_float(x.x), __uint_as_float(x.y))), s2[ch * 4], s2[ch * 4 + 1]);
+              unpack_f32x2(add_f32x2(pack_f32x2(s2[ch * 4 + 2], s2[ch * 4 + 3]),
+                                     pack_f32x2(__uint_as_float(x.z), __uint_as_float(x.w))), s2[ch * 4 + 2], s2[ch * 4 + 3]);
+            }
+            find_anchor = !have_anchor && (m0 | m1) != 0u;
+            have_anchor = have_anchor || find_anchor;
+          }
+          if (rem < kKTile) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j)
+              if (j >= rem) s2[j] = -INFINITY;
+          }
+          if (!kMasked && kt == 0) {
+            row_max = s2[0];
+          } else if (kMasked && find_anchor) {
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four independent chains
+#pragma unroll
+            for (int j = 0; j < 32; ++j) mx[j & 3] = max3_f32(mx[j & 3], s2[2 * j], s2[2 * j + 1]);
+            row_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));  // finite: the tile holds a valid key
+          }
+          const float nmc = -row_max * c;
+          const uint64_t nmc2 = pack_f32x2(nmc, nmc);
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            uint32_t pk[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int j0 = ch * 16 + 2 * e;
+              float d0, d1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(s2[j0], s2[j0 + 1]), c2, nmc2), d0, d1);
+              const float p0 = ex2_approx(d0), p1 = ex2_approx(d1);
+              sum2[e & 1] = add_f32x2(sum2[e & 1], pack_f32x2(p0, p1));
+              pk[e] = pack_bf16x2(p0, p1);
+            }
+            if (ch == 0) {
+              ok = mbar_wait_warp(o_done, o_parity, abort_flag);
+              tc_fence_after();
+            }
+            tmem_st8(p_addr + ch * 8, pk);
+          }
+        }
+        if (!ok) break;
+        float tile_sum;
+        {
           float a0, a1;
-          unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), a0, a1);
+          unpack_f32x2(add_f32x2(sum2[0], sum2[1]), a0, a1);
           tile_sum = a0 + a1;
         }
         // Rare: some score lies so far above the reference point that the tile's sum leaves the safe range (or
         // overflowed).  Move the reference point of the affected rows to the tile's maximum, rescale what has
-        // been accumulated (the previous P·V is complete, see above) and redo the tile.
+        // been accumulated (once the previous tile's P·V is complete) and redo the tile.  The scores are gone by now
+        // (keeping them would cost the usual path 64 registers), so they are computed again from Q, K and the bias
+        // in shared memory, which the MMA warps hand back only after this tile's P·V.
         if (__any_sync(0xffffffffu, !(tile_sum < kRebaseSum))) {
-          float cm = -INFINITY;
+          // (ct counts this tile already: the previous one has number ct - 2)
+          if (ct > 1) ok = mbar_wait_warp(bars + (O_FULL + 2 * w + (ct & 1)) * 8, ((ct - 2) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          uint4 qv[4];
 #pragma unroll
-          for (int j = 0; j < 128; ++j) cm = fmaxf(cm, s2[j]);
+          for (int ch = 0; ch < 4; ++ch) qv[ch] = lds128(base + kSmQ + (ib * kUnits + w) * 8192 + sw64_offset(m, ch));
+          const uint32_t k0 = bias0 - block_off + stage_k(common.y ? w >> 1 : w);
+          auto score = [&](int key) {
+            float d = -INFINITY;
+            bool valid = key < rem;
+            if (kMasked) {
+              const int word = kt * 2 + (key >> 5);
+              valid = word < ((p.S + 31) >> 5) &&
+                      ((__ldg(mask_row + word) >> (key & 31)) & 1u);
+            }
+            if (valid) {
+              uint32_t b16;
+              asm volatile("{\n.reg .b16 h;\nld.shared.b16 h, [%1];\ncvt.u32.u16 %0, h;\n}"
+                           : "=r"(b16)
+                           : "r"((bias0 ^ ((key >> 3) << 4)) + (key & 7) * 2));
+              d = bf16_lo(b16);
+#pragma unroll
+              for (int ch = 0; ch < 4; ++ch) {
+                const uint4 kv = lds128(k0 + sw64_offset(key, ch));
+                d = fmaf(bf16_lo(qv[ch].x), bf16_lo(kv.x), fmaf(bf16_hi(qv[ch].x), bf16_hi(kv.x), d));
+                d = fmaf(bf16_lo(qv[ch].y), bf16_lo(kv.y), fmaf(bf16_hi(qv[ch].y), bf16_hi(kv.y), d));
+                d = fmaf(bf16_lo(qv[ch].z), bf16_lo(kv.z), fmaf(bf16_hi(qv[ch].z), bf16_hi(kv.z), d));
+                d = fmaf(bf16_lo(qv[ch].w), bf16_lo(kv.w), fmaf(bf16_hi(qv[ch].w), bf16_hi(kv.w), d));
+              }
+            }
+            return d;
+          };
+          float cm = -INFINITY;
+#pragma unroll 1
+          for (int key = 0; key < kKTile; ++key) cm = fmaxf(cm, score(key));
           const float new_max = (tile_sum < kRebaseSum) ? row_max : cm;
           const float alpha = ex2_approx((row_max - new_max) * c);  // 1 for rows that keep their reference point
           tmem_st_wait();
           if (kt > 0) {
-            uint32_t t[32];
-            tmem_ld32(o_addr, t);
-            tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
-            tmem_st32(o_addr, t);
+            for (int part = 0; part < 2; ++part) {
+              uint32_t t[16];
+              tmem_ld16(o_addr + part * 16, t);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
+              tmem_st16(o_addr + part * 16, t);
+            }
           }
           row_sum *= alpha;
           row_max = new_max;
-          const float nmc = -row_max * c;
           tile_sum = 0.f;
-#pragma unroll
-          for (int qtr = 0; qtr < 4; ++qtr) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int j0 = qtr * 32 + 2 * e;
-              const float p0 = ex2_approx(fmaf(s2[j0], c, nmc)), p1 = ex2_approx(fmaf(s2[j0 + 1], c, nmc));
-              tile_sum += p0 + p1;
-              pk[e] = pack_bf16x2(p0, p1);
-            }
-            tmem_st16(p_addr + qtr * 16, pk);
+#pragma unroll 1
+          for (int pair = 0; pair < kKTile / 2; ++pair) {
+            const float p0 = ex2_approx((score(2 * pair) - row_max) * c), p1 = ex2_approx((score(2 * pair + 1) - row_max) * c);
+            tile_sum += p0 + p1;
+            __syncwarp();
+            tmem_st1(p_addr + pair, pack_bf16x2(p0, p1));
           }
         }
         row_sum += tile_sum;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + (P_FULL + w) * 8);
+        mbar_arrive_warp(bars + (P_FULL + 2 * w + pb) * 8);
       }
       if (!ok) break;
-      // Output factors first (gate / row sum): they only need the gate row fetched during the last tile, and
-      // computing them here fills the time the last P·V takes.
-      float sg[32];
-      const float inv = 1.f / row_sum;
-      if (p.gate != nullptr) {
+      // tiles of the item that only longer rows have
+      for (int kt = max(my_tiles, 0); kt < common.x; ++kt)
+        if (++stage == kStages) stage = 0, stage_phase ^= 1;
+      if (my_tiles < 0) continue;  // the item has no such unit
+      __nv_bfloat16* out_row = p.out + br * p.o_br + (long long)q * p.o_s + h * p.o_h;
+      if (my_tiles == 0) {  // no valid key and "zeros" semantics
+        if (q < p.S) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t gw[4] = {gv[j].x, gv[j].y, gv[j].z, gv[j].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            sg[j * 8 + 2 * e] = bf16_lo(gw[e]) * inv;
-            sg[j * 8 + 2 * e + 1] = bf16_hi(gw[e]) * inv;
-          }
+          for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(out_row)[j] = make_uint4(0, 0, 0, 0);
+          if (p.lse) p.lse[((long long)br * p.S + q) * kHeads + h] = -INFINITY;
         }
+        continue;
+      }
+      // the unit's output: O (in TMEM) / row_sum * gate; the gate row is fetched while the last P·V runs
+      uint4 gv[4];
+      if (p.gate != nullptr && q < p.S) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gv[j] = __ldg(reinterpret_cast<const uint4*>(gate_row) + j);
       } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sg[j] = inv;
+        for (int j = 0; j < 4; ++j) gv[j] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);  // 1.0
       }
-      // the item's output: O (in TMEM) / row_sum * gate
-      ok = mbar_wait(bars + (O_FULL + w) * 8, (ct - 1) & 1, abort_flag);
+      const float inv = 1.f / row_sum;
+      ok = mbar_wait_warp(bars + (O_FULL + 2 * w + ((ct - 1) & 1)) * 8, ((ct - 1) >> 1) & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t pk[16];
@@ -609,8 +714,15 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tmem_ld32(o_addr, t);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          pk[j] = pack_bf16x2(__uint_as_float(t[2 * j]) * sg[2 * j], __uint_as_float(t[2 * j + 1]) * sg[2 * j + 1]);
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t gw[4] = {gv[j].x, gv[j].y, gv[j].z, gv[j].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int k = j * 8 + 2 * e;
+            pk[j * 4 + e] = pack_bf16x2(__uint_as_float(t[k]) * (bf16_lo(gw[e]) * inv),
+                                        __uint_as_float(t[k + 1]) * (bf16_hi(gw[e]) * inv));
+          }
+        }
       }
       tc_fence_before();
       if (q < p.S) {
@@ -623,8 +735,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             reinterpret_cast<uint4*>(out_row)[j] = make_uint4(pk[j * 4], pk[j * 4 + 1], pk[j * 4 + 2], pk[j * 4 + 3]);
         }
         if (p.lse)
-          p.lse[((long long)it.br * p.S + q) * kHeads + it.h] =
-              it.uniform ? -INFINITY : 0.6931471805599453f * (row_max * c + __log2f(row_sum));
+          p.lse[((long long)br * p.S + q) * kHeads + h] =
+              uniform ? -INFINITY : 0.6931471805599453f * (row_max * c + __log2f(row_sum));
       }
     }
   }
@@ -632,7 +744,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 17) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
@@ -656,11 +768,45 @@ void fast_div_constants(uint32_t d, uint32_t* mul, uint32_t* shr) {
   *mul = uint32_t((uint64_t(1) << (31 + l)) / d + 1);
   *shr = l - 1;
 }
-}  // namespace
-}  // namespace b200ta
 
-namespace b200ta {
-namespace {
+// How the units (128 queries of one row and head) of a (b, h) are put together into items of up to four.
+// Normally the query blocks go two by two with two rows each and an odd last block with four rows.  A problem with
+// too few units to fill the SMs that way takes fewer units per item instead: a CTA with one or two units finishes a
+// tile in some 1000 to 1600 clocks of latency, one with four in some 2700.  For the same reason, when the items come
+// to a few waves and less than half a wave, the rows of that remainder go to items of two units, which still make
+// only one wave and a shorter one (256 tokens: 3.46 waves of items, 43 us; 3 waves and one of halves: 41 us).
+void split_items(int B, int R, int S, int num_sms, AttnParams* p) {
+  const int blocks = (S + kQTile - 1) / kQTile;
+  const int64_t bh = int64_t(B) * kHeads;
+  auto fill = [&](int which, int row0, int row_end, int rows_pair, int rows_single) -> int64_t {
+    RowGroup& g = p->group[which];
+    const int rows = row_end - row0;
+    g.row0 = row0, g.row_end = row_end, g.rows_pair = rows_pair, g.rows_single = rows_single;
+    g.items_pair = p->pairs * ((rows + rows_pair - 1) / rows_pair);
+    g.items_bh = g.items_pair + p->singles * ((rows + rows_single - 1) / rows_single);
+    g.num_items = int(bh * g.items_bh);
+    fast_div_constants(uint32_t(g.items_bh), &g.bh_mul, &g.bh_shr);
+    return bh * g.items_bh;
+  };
+  auto whole = [&](int pairs, int rows_pair, int rows_single) {
+    p->pairs = pairs, p->singles = blocks - 2 * pairs;
+    fill(1, R, R, 1, 1);
+    return fill(0, 0, R, rows_pair, rows_single);
+  };
+  if (whole(0, 1, 1) > num_sms &&                                                 // one unit per item
+      (blocks == 1 ? whole(0, 1, 2) : whole(blocks / 2, 1, 2)) > num_sms) {       // two units per item
+    const int64_t items = whole(blocks / 2, R > 1 ? 2 : 1, R > 2 ? 4 : R);
+    const int64_t waves = items / num_sms, rest = items % num_sms;
+    if (waves >= 1 && waves < 12 && rest > 0 && 2 * rest <= num_sms && R >= 8) {
+      // rows that fill the whole waves, in steps of four (one item of the odd block)
+      const int64_t per_four = bh * (2 * p->pairs + p->singles);
+      const int row = int(waves * num_sms / per_four) * 4;
+      if (row > 0 && row < R) fill(0, 0, row, 2, 4), fill(1, row, R, 1, 2);
+    }
+  }
+  fast_div_constants(uint32_t(p->pairs), &p->pairs_mul, &p->pairs_shr);
+  fast_div_constants(uint32_t(p->singles), &p->singles_mul, &p->singles_shr);
+}
 
 int launch_attention(const void* q, const void* k, const void* v, const void* gate, int64_t s_br, int64_t s_h,
                      int64_t s_s, const void* bias, int64_t bs_b, int64_t bs_h, int64_t bs_q,
@@ -679,19 +825,20 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
                  "attention: out and gate must be 16-byte aligned");
   B200TA_REQUIRE(empty_row_mode == B200TA_EMPTY_ROW_ZEROS || empty_row_mode == B200TA_EMPTY_ROW_UNIFORM,
                  "attention: unknown empty_row_mode %d", empty_row_mode);
-  const int64_t q_pairs = (S + 255) / 256;
-  const int64_t items = int64_t(B) * kHeads * q_pairs * R;
-  B200TA_REQUIRE(items < (int64_t(1) << 31), "attention: too many work items");
   DeviceState* st = nullptr;
   int rc = get_device_state(&st);
   if (rc != B200TA_OK) return rc;
+  B200TA_REQUIRE(int64_t(B) * kHeads * R * ((S + kQTile - 1) / kQTile) < (int64_t(1) << 31), "attention: too many work items");
+  AttnParams p{};
+  split_items(B, R, S, st->num_sms, &p);
 
   CUtensorMap tm_q, tm_k, tm_v, tm_bias;
   {
     uint64_t dims[4] = {uint64_t(kHeadDim), uint64_t(S), uint64_t(kHeads), uint64_t(B) * R};
     uint64_t strides[3] = {uint64_t(s_s) * 2, uint64_t(s_h) * 2, B * R == 1 ? 64u : uint64_t(s_br) * 2};
-    uint32_t box[4] = {32, 128, 1, 1};
+    uint32_t box[4] = {32, kQTile, 1, 1};
     rc = encode_tensor_map(&tm_q, q, 2, 4, dims, strides, box, SWZ_64, "attention q");
+    box[1] = kKTile;
     if (rc == B200TA_OK) rc = encode_tensor_map(&tm_k, k, 2, 4, dims, strides, box, SWZ_64, "attention k");
     if (rc == B200TA_OK) rc = encode_tensor_map(&tm_v, v, 2, 4, dims, strides, box, SWZ_64, "attention v");
     if (rc != B200TA_OK) return rc;
@@ -699,17 +846,13 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
   {
     uint64_t dims[4] = {uint64_t(S_pad), uint64_t(S), uint64_t(kHeads), uint64_t(B)};
     uint64_t strides[3] = {uint64_t(bs_q) * 2, uint64_t(bs_h) * 2, B == 1 ? 64u : uint64_t(bs_b) * 2};
-    uint32_t box[4] = {64, 128, 1, 1};
+    uint32_t box[4] = {kKTile, kQTile, 1, 1};
     rc = encode_tensor_map(&tm_bias, bias, 2, 4, dims, strides, box, SWZ_128, "attention bias");
     if (rc != B200TA_OK) return rc;
   }
 
-  AttnParams p{};
   p.B = B, p.R = R, p.S = S, p.S_pad = S_pad;
-  p.q_pairs = int(q_pairs);
-  p.num_items = int(items);
-  fast_div_constants(uint32_t(R), &p.r_mul, &p.r_shr);
-  fast_div_constants(uint32_t(q_pairs), &p.qp_mul, &p.qp_shr);
+  p.num_items = p.group[0].num_items + p.group[1].num_items;
   p.lengths = lengths;
   p.ls_b = ls_b, p.ls_r = ls_r;
   p.key_mask = key_mask;

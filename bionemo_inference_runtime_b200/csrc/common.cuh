@@ -114,12 +114,33 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
-// The same wait made by all 32 lanes of a converged warp; the result is the same in every lane (a vote), so
-// the code after it stays warp-uniform.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+// The same wait made by all 32 lanes of a converged warp; every decision is a vote, so the result is the same in
+// every lane, the code after it stays warp-uniform, and a failed poll costs no divergence bookkeeping.
+__device__ __forceinline__ bool mbar_wait_warp_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  uint64_t t0 = 0;
+  for (uint32_t spins = 1;; ++spins) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((spins & 63u) == 0u) {
+      if (t0 == 0) t0 = global_timer_ns();
+      const bool late = global_timer_ns() - t0 > kWaitLimitNs;
+      if (__any_sync(0xffffffffu, late || *abort_flag)) {
+        if (late) *abort_flag = 1;
+        return false;
+      }
+    }
+  }
 }
-
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp_slow(bar, parity, abort_flag);
+}
+// Waits for two barriers at once (one vote for the usual case that both are complete already).
+__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
+                                                volatile int* abort_flag) {
+  const bool a = mbar_try_wait(bar0, parity0), b = mbar_try_wait(bar1, parity1);
+  if (__all_sync(0xffffffffu, a && b)) return true;
+  return mbar_wait_warp_slow(bar0, parity0, abort_flag) && mbar_wait_warp_slow(bar1, parity1, abort_flag);
+}
 // ---- proxies / fences --------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -221,6 +242,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
   d |= static_cast<uint64_t>(layout_type & 7u) << 61;
   return d;
 }
+// The same with lbo, sbo and layout known at compile time: only the address field is computed.
+template <uint32_t LBO, uint32_t SBO, uint32_t LAYOUT>
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
+  constexpr uint32_t hi = (SBO >> 4) | (1u << 14) | (LAYOUT << 29), lo = (LBO >> 4) << 16;
+  return (static_cast<uint64_t>(hi) << 32) | ((saddr >> 4) | lo);  // shared-memory addresses are below 2^18
+}
 constexpr uint32_t kLayoutSw128 = 2, kLayoutSw64 = 4, kLayoutSw32 = 6;
 
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulation.
@@ -308,20 +335,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
-// Same, into elements [OFF, OFF+32) of a 128-float register array.
-template <int OFF>
-__device__ __forceinline__ void tmem_ld32_f128(uint32_t taddr, float (&r)[128]) {
+// 64 columns into 64 floats.
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&r)[64]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
-      "%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=f"(r[OFF + 0]), "=f"(r[OFF + 1]), "=f"(r[OFF + 2]), "=f"(r[OFF + 3]), "=f"(r[OFF + 4]),
-        "=f"(r[OFF + 5]), "=f"(r[OFF + 6]), "=f"(r[OFF + 7]), "=f"(r[OFF + 8]), "=f"(r[OFF + 9]),
-        "=f"(r[OFF + 10]), "=f"(r[OFF + 11]), "=f"(r[OFF + 12]), "=f"(r[OFF + 13]), "=f"(r[OFF + 14]),
-        "=f"(r[OFF + 15]), "=f"(r[OFF + 16]), "=f"(r[OFF + 17]), "=f"(r[OFF + 18]), "=f"(r[OFF + 19]),
-        "=f"(r[OFF + 20]), "=f"(r[OFF + 21]), "=f"(r[OFF + 22]), "=f"(r[OFF + 23]), "=f"(r[OFF + 24]),
-        "=f"(r[OFF + 25]), "=f"(r[OFF + 26]), "=f"(r[OFF + 27]), "=f"(r[OFF + 28]), "=f"(r[OFF + 29]),
-        "=f"(r[OFF + 30]), "=f"(r[OFF + 31])
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
+      "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+      "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
+        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]), "=f"(r[16]),
+        "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), "=f"(r[24]),
+        "=f"(r[25]), "=f"(r[26]), "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31]), "=f"(r[32]),
+        "=f"(r[33]), "=f"(r[34]), "=f"(r[35]), "=f"(r[36]), "=f"(r[37]), "=f"(r[38]), "=f"(r[39]), "=f"(r[40]),
+        "=f"(r[41]), "=f"(r[42]), "=f"(r[43]), "=f"(r[44]), "=f"(r[45]), "=f"(r[46]), "=f"(r[47]), "=f"(r[48]),
+        "=f"(r[49]), "=f"(r[50]), "=f"(r[51]), "=f"(r[52]), "=f"(r[53]), "=f"(r[54]), "=f"(r[55]), "=f"(r[56]),
+        "=f"(r[57]), "=f"(r[58]), "=f"(r[59]), "=f"(r[60]), "=f"(r[61]), "=f"(r[62]), "=f"(r[63])
       : "r"(taddr)
       : "memory");
 }
@@ -360,6 +389,14 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
       "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
+}
+__device__ __forceinline__ void tmem_st1(uint32_t taddr, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(r) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
