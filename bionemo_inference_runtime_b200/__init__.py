@@ -8,7 +8,7 @@ importing the layers without the built library raises.
 
 from . import _lib
 
-_lib.load()  # fail loudly at import when the extension has not been built
+_lib.load_host()  # fail loudly at import when the library or the native host path has not been built
 
 from . import ops  # noqa: E402
 from .layers import *  # noqa: E402,F401,F403

@@ -113,6 +113,11 @@ SIGNATURES: dict[str, tuple] = {
         [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_float,
          c_int, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
     ),
+    "b200ta_trimul_output_f32": (
+        c_int,
+        [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_float,
+         c_int, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
+    ),
 }
 
 
@@ -146,6 +151,21 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def load_host():
+    """Import the native host path of the layers (``_host``, built from ``csrc/torch_host.cpp``) and hand it the entry
+    points of the library that :func:`load` opened."""
+    load()
+    if not (_PKG / "_host.so").exists():
+        raise ImportError(f"{_PKG / '_host.so'} is missing: build it with the library "
+                          "(`python -m bionemo_inference_runtime_b200.csrc.build`); this package has no fallback path.")
+    import torch  # noqa: F401  (the extension resolves PyTorch's symbols in the running process)
+
+    from . import _host
+
+    _host.bind(str(LIB_PATH), B200TAError)
+    return _host
 
 
 def last_error() -> str:

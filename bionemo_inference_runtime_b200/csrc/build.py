@@ -1,4 +1,4 @@
-"""Builds libb200ta.so (sm_100a only) next to the package with nvcc.
+"""Builds libb200ta.so (sm_100a only) and the layers' native host path (_host.so) next to the package.
 
 Usage: ``python -m bionemo_inference_runtime_b200.csrc.build [--force] [--verbose]``.
 The library is linked against the static CUDA runtime and resolves the one
@@ -18,6 +18,7 @@ from pathlib import Path
 CSRC = Path(__file__).resolve().parent
 PKG = CSRC.parent
 LIB = PKG / "libb200ta.so"
+HOST = PKG / "_host.so"
 OBJ_DIR = CSRC / "build"
 SOURCES = ["host.cu", "pack.cu", "rowgemm.cu", "attention.cu", "node.cu", "transition.cu", "trimul_project.cu",
            "trimul_contract.cu", "trimul_output.cu", "linear.cu", "pair_bias.cu"]
@@ -46,6 +47,27 @@ def _stale(target: Path, sources: list[Path]) -> bool:
     return any(s.stat().st_mtime > t for s in sources)
 
 
+def _build_host(force: bool) -> None:
+    """_host.so from torch_host.cpp against the headers of the installed PyTorch; it links none of the kernels."""
+    src = CSRC / "torch_host.cpp"
+    if not (force or _stale(HOST, [src, PKG.parent / "include" / "b200ta.h"])):
+        return
+    import sysconfig
+
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_host", "-D_GLIBCXX_USE_CXX11_ABI=1",
+           *(f"-I{p}" for p in include_paths()), f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}",
+           str(src), "-o", str(HOST), *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch_python", "-ldl"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("building _host.so failed")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ_DIR.mkdir(exist_ok=True)
@@ -63,7 +85,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 raise RuntimeError(f"nvcc failed on {src.name}")
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(8, len(sources))) as pool:
+    with ThreadPoolExecutor(max_workers=min(9, len(sources) + 1)) as pool:
+        host = pool.submit(_build_host, force)
         objs = list(pool.map(compile_one, sources))
     if force or _stale(LIB, objs):
         cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static"]
@@ -71,6 +94,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("linking libb200ta.so failed")
+    host.result()
     return LIB
 
 

@@ -1,0 +1,294 @@
+// Host path of the layers in native code: one call per layer that checks the tensors, takes outputs and workspaces from
+// PyTorch's allocator and enqueues the layer's kernels through the C ABI (include/b200ta.h).
+//
+// At small token counts a block's kernels take some 100 us of GPU time, and the same steps written with ctypes and
+// torch functions in Python took several times that on the host (about 40 us per launch: argument conversion of 20 to
+// 30 values, tensor attributes, empty(), the stream object, a getattr per parameter for the weight check); from here a
+// layer call costs its launches and a few microseconds.
+//
+// The kernels' library is not linked: bind() takes its entry points from the file that the ctypes binding loaded.
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/extension.h>
+
+#include <cstring>
+#include <string>
+
+#include "../../include/b200ta.h"
+
+namespace py = pybind11;
+
+namespace {
+
+struct Library {
+#define B200TA_ENTRY(name) decltype(&b200ta_##name) name = nullptr;
+#define B200TA_ENTRIES(X)                                                                                            \
+  X(last_error) X(node_workspace_bytes) X(node_forward) X(transition) X(transition_relu) X(trimul_project)           \
+  X(trimul_contract) X(trimul_output) X(trimul_output_f32) X(pair_bias) X(row_stats) X(linear) X(attention)
+  B200TA_ENTRIES(B200TA_ENTRY)
+#undef B200TA_ENTRY
+} lib;
+
+py::object error_type;  // _lib.B200TAError
+
+void bind(const std::string& path, py::object error) {
+  void* handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (handle == nullptr) throw py::import_error("cannot open " + path + ": " + dlerror());
+#define B200TA_LOAD(name)                                                                                    \
+  lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(handle, "b200ta_" #name));                           \
+  if (lib.name == nullptr) throw py::import_error("b200ta_" #name " is not exported by " + path);
+  B200TA_ENTRIES(B200TA_LOAD)
+#undef B200TA_LOAD
+  error_type = std::move(error);
+}
+
+// Raises what _lib.call raises for a non-zero status.
+void check(int code, const char* fn) {
+  if (code == B200TA_OK) return;
+  const std::string reason = lib.last_error();
+  if (code == B200TA_ERR_INVALID) throw py::value_error(std::string(fn) + ": " + reason);
+  PyErr_SetObject(error_type.ptr(), error_type(fn, code, reason).ptr());
+  throw py::error_already_set();
+}
+
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+std::string shape_of(const at::Tensor& t) {
+  std::string s = "(";
+  for (int64_t d : t.sizes()) s += std::to_string(d) + ", ";
+  return s + ")";
+}
+
+void require_bf16(const char* name, const at::Tensor& t) {
+  if (!t.is_cuda()) throw py::value_error(std::string(name) + " must be a CUDA tensor (this package has no CPU path)");
+  if (t.scalar_type() != at::kBFloat16) throw py::value_error(std::string(name) + " must be bfloat16");
+}
+
+// A pair tensor [B, N, N, 128] as the kernels see it; `swap` exchanges the two pair axes.
+struct Pair {
+  int B, N;
+  int64_t sb, sr, ss;
+};
+Pair pair_of(const char* name, const at::Tensor& z, bool swap) {
+  require_bf16(name, z);
+  if (z.dim() != 4 || z.size(1) != z.size(2) || z.size(3) != B200TA_C || z.stride(3) != 1)
+    throw py::value_error(std::string(name) + ": expected a square pair tensor [B, N, N, 128] with unit channel stride, got " +
+                          shape_of(z));
+  return {int(z.size(0)), int(z.size(1)), z.stride(0), z.stride(swap ? 2 : 1), z.stride(swap ? 1 : 2)};
+}
+
+at::Tensor new_bf16(const at::Tensor& like, at::IntArrayRef shape) {
+  return at::empty(shape, like.options().dtype(at::kBFloat16).memory_format(c10::MemoryFormat::Contiguous));
+}
+
+// The buffer kept in `buffers` (a dict or None) under `key`, replaced only when its shape, dtype or device changed; a
+// fresh tensor when there is no dict.
+at::Tensor buffer(const py::object& buffers, const char* key, at::IntArrayRef shape, at::ScalarType dtype,
+                  const at::Tensor& like) {
+  if (!buffers.is_none()) {
+    if (PyObject* held = PyDict_GetItemString(buffers.ptr(), key); held != nullptr && THPVariable_Check(held)) {
+      const at::Tensor& t = THPVariable_Unpack(held);
+      if (t.sizes() == shape && t.scalar_type() == dtype && t.device() == like.device()) return t;
+    }
+  }
+  at::Tensor t = at::empty(shape, like.options().dtype(dtype));
+  if (!buffers.is_none()) buffers[key] = py::cast(t);
+  return t;
+}
+
+struct Lengths {
+  const int32_t* ptr = nullptr;
+  int64_t sb = 0, sr = 0;
+};
+Lengths lengths_of(const c10::optional<at::Tensor>& lengths, int64_t B, int64_t R) {
+  if (!lengths) return {};
+  const at::Tensor& t = *lengths;
+  if (t.scalar_type() != at::kInt || !t.is_cuda() || t.numel() != B * R)
+    throw py::value_error("lengths must be a CUDA int32 tensor with B*N=" + std::to_string(B * R) + " values");
+  const at::Tensor v = t.dim() == 2 ? t : t.reshape({B, R});
+  return {v.data_ptr<int32_t>(), v.stride(0), v.stride(1)};
+}
+
+struct Mask {
+  const float* ptr = nullptr;
+  int64_t sb = 0, si = 0, sj = 0;
+};
+Mask mask_of(const c10::optional<at::Tensor>& mask, int64_t B, int64_t N, bool swap) {
+  if (!mask) return {};
+  const at::Tensor& t = *mask;
+  if (t.scalar_type() != at::kFloat || !t.is_cuda() || t.dim() != 3 || t.size(0) != B || t.size(1) != N || t.size(2) != N)
+    throw py::value_error("mask must be a CUDA float32 tensor of shape [B, N, N], got " + shape_of(t));
+  return {t.data_ptr<float>(), t.stride(0), t.stride(swap ? 2 : 1), t.stride(swap ? 1 : 2)};
+}
+
+// ---- layers ------------------------------------------------------------------------------------------------------
+
+at::Tensor node(const at::Tensor& z, const at::Tensor& packed, const c10::optional<at::Tensor>& lengths, double eps,
+                bool ending, bool residual, bool inplace, const py::object& buffers, int empty_row_mode) {
+  const Pair p = pair_of("z", z, ending);
+  const at::Tensor out = inplace ? z : new_bf16(z, z.sizes());
+  const Pair o = pair_of("out", out, ending);
+  const Lengths l = lengths_of(lengths, p.B, p.N);
+  const int64_t bytes = int64_t(lib.node_workspace_bytes(p.B, p.N));
+  const at::Tensor ws = buffer(buffers, "tri_attn_workspace", {bytes}, at::kByte, z);
+  check(lib.node_forward(z.data_ptr(), p.sb, p.sr, p.ss, packed.data_ptr(), float(eps), l.ptr, l.sb, l.sr, empty_row_mode,
+                         residual, out.data_ptr(), o.sb, o.sr, o.ss, ws.data_ptr(), size_t(bytes), p.B, p.N, stream()),
+        "b200ta_node_forward");
+  return out;
+}
+
+at::Tensor trimul(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const at::Tensor& packed, double eps,
+                  bool incoming, const c10::optional<at::Tensor>& b_scale, const py::object& buffers, bool residual,
+                  bool mask_output, bool f32) {
+  const Pair p = pair_of("z", z, false);
+  const int64_t hidden = B200TA_C, pitch = (p.N + 15) / 16 * 16;
+  const at::Tensor ab = buffer(buffers, "trimul_ab", {p.B, 2 * hidden, p.N, pitch}, at::kBFloat16, z);
+  const at::Tensor x = buffer(buffers, "trimul_contracted", {p.B, hidden, p.N, pitch}, at::kBFloat16, z);
+  const at::Tensor out = f32 ? at::empty(z.sizes(), z.options().dtype(at::kFloat).memory_format(c10::MemoryFormat::Contiguous))
+                             : new_bf16(z, z.sizes());
+  void* s = stream();
+  const Mask m = mask_of(mask, p.B, p.N, incoming);
+  check(lib.trimul_project(z.data_ptr(), p.sb, incoming ? p.ss : p.sr, incoming ? p.sr : p.ss, m.ptr, m.sb, m.si, m.sj,
+                           b_scale ? b_scale->data_ptr<float>() : nullptr, packed.data_ptr(), float(eps), ab.data_ptr(), pitch,
+                           p.B, p.N, p.N, s),
+        "b200ta_trimul_project");
+  check(lib.trimul_contract(ab.data_ptr(), x.data_ptr(), p.B, p.N, pitch, s), "b200ta_trimul_contract");
+  const Mask om = mask_output ? mask_of(mask, p.B, p.N, false) : Mask{};
+  check((f32 ? lib.trimul_output_f32 : lib.trimul_output)(z.data_ptr(), p.sb, p.sr, p.ss, x.data_ptr(), pitch, om.ptr, om.sb,
+                                                          om.si, om.sj, packed.data_ptr(), float(eps), residual,
+                                                          out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), p.B,
+                                                          p.N, s),
+        "b200ta_trimul_output");
+  return out;
+}
+
+at::Tensor transition(const at::Tensor& x, const at::Tensor& packed, const c10::optional<at::Tensor>& mask, double eps,
+                      bool residual, bool inplace, bool relu) {
+  require_bf16("x", x);
+  if (x.dim() < 1 || x.size(-1) != B200TA_C) throw py::value_error("last dimension must be 128");
+  if (!x.is_contiguous()) throw py::value_error("transition needs a contiguous input");
+  const at::Tensor out = inplace ? x : at::empty_like(x);
+  const int64_t rows = x.numel() / B200TA_C;
+  at::Tensor m;
+  if (mask) {
+    m = mask->to(at::kBFloat16).expand(x.sizes().slice(0, x.dim() - 1)).contiguous();
+    if (!m.is_cuda()) throw py::value_error("mask must be a CUDA tensor");
+  }
+  check((relu ? lib.transition_relu : lib.transition)(x.data_ptr(), B200TA_C, mask ? m.data_ptr() : nullptr, packed.data_ptr(),
+                                                      float(eps), out.data_ptr(), B200TA_C, rows, residual, stream()),
+        relu ? "b200ta_transition_relu" : "b200ta_transition");
+  return out;
+}
+
+// A transition of other widths: (row statistics,) two GEMMs.  w1 / w2 bf16, sc1 / sc2 {rowsum, const} per output column.
+at::Tensor transition_gemms(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& sc1, const at::Tensor& w2,
+                            const at::Tensor& sc2, bool normalize, double eps, bool residual, bool inplace) {
+  require_bf16("x", x);
+  if (!x.is_contiguous()) throw py::value_error("transition needs a contiguous input");
+  const int64_t K = x.size(-1), rows = x.numel() / K, hidden = w2.size(1);
+  if (K != w1.size(1)) throw py::value_error("last dimension must be " + std::to_string(w1.size(1)));
+  void* s = stream();
+  at::Tensor stats;
+  if (normalize) {
+    stats = at::empty({rows, 2}, x.options().dtype(at::kFloat));
+    check(lib.row_stats(x.data_ptr(), K, rows, int(K), float(eps), stats.data_ptr(), s), "b200ta_row_stats");
+  }
+  const at::Tensor h = new_bf16(x, {rows, hidden});
+  check(lib.linear(x.data_ptr(), rows * K, K, 128, w1.data_ptr(), sc1.data_ptr(), normalize ? stats.data_ptr() : nullptr,
+                   nullptr, 0, h.data_ptr(), hidden, 0, 2, 1, int(rows), int(K), int(2 * hidden), s),
+        "b200ta_linear");
+  const at::Tensor out = inplace ? x : at::empty_like(x);
+  check(lib.linear(h.data_ptr(), rows * hidden, hidden, 128, w2.data_ptr(), sc2.data_ptr(), nullptr,
+                   residual ? x.data_ptr() : nullptr, residual ? K : 0, out.data_ptr(), K, 0, 1, 1, int(rows), int(hidden),
+                   int(K), s),
+        "b200ta_linear");
+  return out;
+}
+
+// The single-track attention with pair bias.  `lengths` int32 [4 B]: the key count of a batch entry four times (the
+// attention kernel sees its 16 heads as four items of four).
+at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& z, const c10::optional<at::Tensor>& lengths,
+                               const at::Tensor& w_in, const at::Tensor& sc_in, const at::Tensor& w_o, const at::Tensor& sc_o,
+                               const at::Tensor& packed_z, bool normalize, double eps_s, double eps_z, double scale,
+                               const c10::optional<at::Tensor>& residual, const py::object& buffers) {
+  require_bf16("s", s16);
+  const Pair p = pair_of("z", z, false);
+  const int64_t B = p.B, N = p.N, c_s = s16.size(-1), heads = 16, dim = B200TA_HEAD_DIM, pad = (N + 7) / 8 * 8;
+  if (!s16.is_contiguous() || s16.dim() != 3 || s16.size(0) != B || s16.size(1) != N)
+    throw py::value_error("s must be a contiguous [B, N, c_s] tensor that matches z");
+  void* st = stream();
+  at::Tensor stats;
+  if (normalize) {
+    stats = at::empty({B * N, 2}, s16.options().dtype(at::kFloat));
+    check(lib.row_stats(s16.data_ptr(), c_s, B * N, int(c_s), float(eps_s), stats.data_ptr(), st), "b200ta_row_stats");
+  }
+  const at::Tensor planes = buffer(buffers, "pw_qkvg", {4, B, heads, N, dim}, at::kBFloat16, s16);
+  check(lib.linear(s16.data_ptr(), N * c_s, c_s, 128, w_in.data_ptr(), sc_in.data_ptr(), normalize ? stats.data_ptr() : nullptr,
+                   nullptr, 0, planes.data_ptr(), 0, planes.stride(0), 0, int(B), int(N), int(c_s), int(4 * heads * dim), st),
+        "b200ta_linear");
+  const at::Tensor bias = buffer(buffers, "pw_pair_bias", {B, heads, N, pad}, at::kBFloat16, s16);
+  check(lib.pair_bias(z.data_ptr(), p.sb, p.sr, p.ss, packed_z.data_ptr(), float(eps_z), bias.data_ptr(), bias.stride(0),
+                      bias.stride(1), bias.stride(2), 1, int(heads), int(B), int(N), int(N), int(pad), st),
+        "b200ta_pair_bias");
+  const at::Tensor attn = buffer(buffers, "pw_attn_output", {4 * B, 1, N, B200TA_C}, at::kBFloat16, s16);
+  const Lengths l = lengths_of(lengths, 4 * B, 1);
+  char* q = static_cast<char*>(planes.data_ptr());
+  const int64_t plane = planes.stride(0) * 2, head = N * dim;
+  check(lib.attention(q, q + plane, q + 2 * plane, q + 3 * plane, 4 * head, head, dim, bias.data_ptr(), 4 * N * pad, N * pad,
+                      pad, l.ptr, l.sb, l.sr, attn.data_ptr(), N * B200TA_C, B200TA_C, dim, nullptr, float(scale),
+                      B200TA_EMPTY_ROW_UNIFORM, int(4 * B), 1, int(N), int(pad), st),
+        "b200ta_attention");
+  const at::Tensor out = at::empty_like(s16);
+  check(lib.linear(attn.data_ptr(), 4 * N * B200TA_C, B200TA_C, N * B200TA_C, w_o.data_ptr(), sc_o.data_ptr(), nullptr,
+                   residual ? residual->data_ptr() : nullptr, residual ? c_s : 0, out.data_ptr(), c_s, 0, 1, int(B), int(N),
+                   int(heads * dim), int(c_s), st),
+        "b200ta_linear");
+  return out;
+}
+
+// ---- weight state --------------------------------------------------------------------------------------------------
+
+void add_parameters(PyObject* module, std::string& out) {
+  static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
+  static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
+  PyObject** dict = _PyObject_GetDictPtr(module);
+  if (dict == nullptr || *dict == nullptr) return;
+  PyObject *key, *value;
+  Py_ssize_t pos = 0;
+  if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
+    while (PyDict_Next(parameters, &pos, &key, &value)) {
+      if (!THPVariable_Check(value)) continue;
+      const at::Tensor& t = THPVariable_Unpack(value);
+      // address, in-place write count (inference tensors have none), device
+      const int64_t state[3] = {reinterpret_cast<int64_t>(t.data_ptr()), t.is_inference() ? -1 : int64_t(t._version()),
+                                int64_t(t.device().index()) * 256 + int64_t(t.device().type())};
+      out.append(reinterpret_cast<const char*>(state), sizeof(state));
+    }
+  }
+  pos = 0;
+  if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
+    while (PyDict_Next(modules, &pos, &key, &value))
+      if (value != Py_None) add_parameters(value, out);
+}
+
+// Address, in-place write count and device of every parameter under the modules: changes when a weight is loaded,
+// edited or replaced.
+py::bytes weight_state(const py::args& modules) {
+  std::string out;
+  for (const py::handle& m : modules) add_parameters(m.ptr(), out);
+  return py::bytes(out);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  m.doc() = "Native host path of the layers (see csrc/torch_host.cpp).";
+  m.def("bind", &bind);
+  m.def("node", &node);
+  m.def("trimul", &trimul);
+  m.def("transition", &transition);
+  m.def("transition_gemms", &transition_gemms);
+  m.def("pair_bias_attention", &pair_bias_attention);
+  m.def("weight_state", &weight_state);
+}

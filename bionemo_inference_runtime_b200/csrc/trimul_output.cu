@@ -41,7 +41,7 @@ struct OutputParams {
   int add_residual;
   const float* mask;  // [B, N, N] via strides; NULL = no output mask
   long long ms_b, ms_i, ms_j;
-  __nv_bfloat16* out;
+  void* out;  // bf16, or float in the kF32 form
   long long os_b, os_i, os_j;
   int* status;
 };
@@ -57,6 +57,7 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   return v;
 }
 
+template <bool kF32>
 __global__ void __launch_bounds__(kThreads, 1)
 trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_x,
                      const __grid_constant__ CUtensorMap tm_w, const OutputParams p) {
@@ -310,6 +311,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         }
         const uint32_t (&xg)[16] = ag[ck & 1];
         const uint32_t (&xp)[16] = ap[ck & 1];
+        const long long at = b * p.os_b + i * p.os_i + (long long)j * p.os_j + ch0;
         uint32_t packed[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -328,9 +330,14 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
           const uint32_t r = res[ck >> 1][h * 8 + c];
           float o0, o1;
           unpack_f32x2(mul_f32x2(fma_f32x2(s2, v2, pack_f32x2(bf16_lo(r), bf16_hi(r))), mval2), o0, o1);
-          packed[c] = pack_bf16x2(o0, o1);
+          if (kF32) {
+            packed[(2 * c) & 7] = __float_as_uint(o0), packed[(2 * c + 1) & 7] = __float_as_uint(o1);
+            if ((c & 3) == 3 && j < p.N) stg256(static_cast<float*>(p.out) + at + (c - 3) * 2, packed);
+          } else {
+            packed[c] = pack_bf16x2(o0, o1);
+          }
         }
-        if (j < p.N) stg256(p.out + b * p.os_b + i * p.os_i + (long long)j * p.os_j + ch0, packed);
+        if (!kF32 && j < p.N) stg256(static_cast<__nv_bfloat16*>(p.out) + at, packed);
       }
       tc_fence_before();
       __syncwarp();
@@ -351,13 +358,13 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
 }  // namespace
 }  // namespace b200ta
 
-extern "C" {
+namespace b200ta {
+namespace {
 
-int b200ta_trimul_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const void* x, int64_t pitch,
-                         const float* mask, int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps,
-                         int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
-                         void* stream) {
-  using namespace b200ta;
+template <bool kF32>
+int launch_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const void* x, int64_t pitch, const float* mask,
+                  int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps, int add_residual, void* out,
+                  int64_t os_b, int64_t os_i, int64_t os_j, int B, int N, void* stream) {
   B200TA_REQUIRE(z && x && packed && out, "trimul_output: NULL pointer");
   B200TA_REQUIRE(B > 0 && N > 0, "trimul_output: bad sizes B=%d N=%d", B, N);
   B200TA_REQUIRE(pitch >= N && pitch % 16 == 0, "trimul_output: pitch=%lld must be a multiple of 16 and >= N=%d",
@@ -409,15 +416,36 @@ int b200ta_trimul_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j
   p.add_residual = add_residual ? 1 : 0;
   p.mask = mask;
   p.ms_b = ms_b, p.ms_i = ms_i, p.ms_j = ms_j;
-  p.out = static_cast<__nv_bfloat16*>(out);
+  p.out = out;
   p.os_b = os_b, p.os_i = os_i, p.os_j = os_j;
   p.status = st->status_dev;
 
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(trimul_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
+  B200TA_CHECK_CUDA(cudaFuncSetAttribute(trimul_output_kernel<kF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  trimul_output_kernel<<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_z, tm_x, tm_w, p);
+  trimul_output_kernel<kF32><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_z, tm_x, tm_w, p);
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
+}
+
+}  // namespace
+}  // namespace b200ta
+
+extern "C" {
+
+int b200ta_trimul_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const void* x, int64_t pitch,
+                         const float* mask, int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps,
+                         int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
+                         void* stream) {
+  return b200ta::launch_output<false>(z, zs_b, zs_i, zs_j, x, pitch, mask, ms_b, ms_i, ms_j, packed, eps, add_residual, out,
+                                      os_b, os_i, os_j, B, N, stream);
+}
+
+int b200ta_trimul_output_f32(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const void* x, int64_t pitch,
+                             const float* mask, int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps,
+                             int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
+                             void* stream) {
+  return b200ta::launch_output<true>(z, zs_b, zs_i, zs_j, x, pitch, mask, ms_b, ms_i, ms_j, packed, eps, add_residual, out,
+                                     os_b, os_i, os_j, B, N, stream);
 }
 
 }  // extern "C"

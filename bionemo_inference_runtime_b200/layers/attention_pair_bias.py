@@ -22,10 +22,9 @@ import math
 import torch
 import torch.nn as nn
 
-from .. import _lib, ops
-from .buffers import ensure_buffer
+from .. import _host, ops
 from .linear import Linear, WeightMode, WeightsLoadingConfig
-from .triangle_nodes import _refold_after_load_state_dict, _weight_state
+from .triangle_nodes import _refold_after_load_state_dict
 
 _HEADS = ops.SINGLE_HEADS
 _PAD = ops.HEAD_DIM  # head width of the attention kernel
@@ -144,11 +143,11 @@ class AttentionPairBias(nn.Module):
             self._folded = self._folded_state = None
             return
         self._folded = self._fold(self.in_proj.weight.device)
-        self._folded_state = _weight_state(*self._params())
+        self._folded_state = _host.weight_state(self, *self._input_norm)
 
     @torch.no_grad()
     def _weights(self, device) -> dict:
-        state = _weight_state(*self._params())
+        state = _host.weight_state(self, *self._input_norm)
         if self._folded is None or self._folded["w_in"].device != device or state != self._folded_state:
             folded = self._fold(device)
             if not torch.cuda.is_current_stream_capturing():
@@ -182,13 +181,21 @@ class AttentionPairBias(nn.Module):
             raise ValueError(f"expected one key count per batch entry, got {lengths.numel()} for B={B}")
         return lengths.to(device)
 
+    def key_counts(self, mask: torch.Tensor | None, mask_bias: torch.Tensor | None, B: int, N: int, device) -> torch.Tensor:
+        """The key counts in the attention kernel's form: every batch entry four times (it becomes four items of four
+        heads), ``[4 B, 1]``."""
+        lengths = self._lengths(mask, mask_bias, B, N, device)
+        return lengths.reshape(1, 1).expand(4, 1) if B == 1 else lengths.repeat_interleave(4).view(4 * B, 1)
+
     def forward(self, s: torch.Tensor, z: torch.Tensor | None, mask: torch.Tensor | None,
                 single_embedding: torch.Tensor | None = None, attn_metadata=None,
                 mask_bias: torch.Tensor | None = None, mask_bias_local: torch.Tensor | None = None,
                 buffers: dict | None = None, residual: torch.Tensor | None = None,
-                output_gate_logits: torch.Tensor | None = None, adaln_conditioning=None) -> torch.Tensor:
+                output_gate_logits: torch.Tensor | None = None, adaln_conditioning=None,
+                _key_counts: torch.Tensor | None = None) -> torch.Tensor:
         """``s``: ``[B, N, c_s]``; ``z``: ``[B, N, N, 128]``; ``mask``: ``[B, N]`` (1 = valid key, left-aligned).
-        Returns the update of ``s`` (``residual + update`` when ``residual`` is given), in the dtype of ``s``."""
+        Returns the update of ``s`` (``residual + update`` when ``residual`` is given), in the dtype of ``s``.
+        ``_key_counts`` (from :meth:`key_counts`, for a stack whose layers share the mask) replaces the masks."""
         if single_embedding is not None or output_gate_logits is not None or adaln_conditioning is not None:
             raise ValueError("AdaLN conditioning and the output gate are not supported by the sm_100a single track")
         if mask_bias_local is not None or (attn_metadata is not None and getattr(attn_metadata, "query_to_keys", None) is not None):
@@ -203,20 +210,13 @@ class AttentionPairBias(nn.Module):
         out_dtype = s.dtype
         s16 = s.to(torch.bfloat16).contiguous()
         w = self._weights(s.device)
-        lengths = self._lengths(mask, mask_bias, B, N, s.device)
-
+        if _key_counts is None:
+            _key_counts = self.key_counts(mask, mask_bias, B, N, s.device)
         norm = self._norm_of_s()
-        stats = ops.row_stats(s16, norm.eps) if norm is not None else None
-        planes = ensure_buffer(buffers, "pw_qkvg", (4, B, _HEADS, N, _PAD), torch.bfloat16, s.device)
-        planes = ops.linear(s16, w["w_in"], w["sc_in"], ops.LINEAR_PLANES, B=B, rows=N, stats=stats, out=planes)
-        bias = ensure_buffer(buffers, "pw_pair_bias", (B, _HEADS, N, ops.pad8(N)), torch.bfloat16, s.device)
-        bias = self.project_pair_bias(z, bias=bias)
-        # the attention kernel handles 4 heads per item: batch entry b becomes the 4 items 4b .. 4b+3
-        attn = ensure_buffer(buffers, "pw_attn_output", (4 * B, 1, N, ops.C), torch.bfloat16, s.device)
-        attn = ops.attention(planes.view(4, 4 * B, ops.HEADS, N, _PAD), bias.view(4 * B, ops.HEADS, N, bias.shape[-1]),
-                             lengths.repeat_interleave(4), 4 * B, 1, N, out=attn, scale=1.0 / math.sqrt(self.head_dim),
-                             empty_row_mode=_lib.EMPTY_ROW_UNIFORM)
+        if z.dtype != torch.bfloat16:
+            z = z.to(torch.bfloat16)
         res16 = None if residual is None else residual.to(torch.bfloat16).contiguous()
-        out = ops.linear(attn, w["w_o"], w["sc_o"], ops.LINEAR_ROWS, B=B, rows=N,
-                         a_strides=(4 * N * ops.C, ops.C, N * ops.C), residual=res16)
+        out = _host.pair_bias_attention(s16, z, _key_counts, w["w_in"], w["sc_in"], w["w_o"], w["sc_o"], w["packed_z"],
+                                        norm is not None, self.eps if norm is None else norm.eps, self.eps,
+                                        1.0 / math.sqrt(self.head_dim), res16, buffers)
         return out if out.dtype == out_dtype else out.to(out_dtype)

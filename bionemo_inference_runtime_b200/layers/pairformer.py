@@ -19,6 +19,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from .. import _host
 from .attention_backend import (AttentionMetadata, PrecomputedPairMasks, precompute_pair_masks,
                                 precompute_single_masks)
 from .attention_pair_bias import AttentionPairBias
@@ -27,7 +28,7 @@ from .buffers import PreallocatedBuffers
 from .transition import Transition
 from .triangle_multiplication import (TriangleMultiplicationMetadata, TriangleMultiplicationNode,
                                       TriangleMultiplicationNodeType, precompute_trimul_metadata)
-from .triangle_nodes import TriangleAttentionEndingNode, TriangleAttentionStartingNode, _weight_state
+from .triangle_nodes import TriangleAttentionEndingNode, TriangleAttentionStartingNode
 
 
 class PairformerLayerV1(nn.Module):
@@ -84,9 +85,11 @@ class PairformerLayerV1(nn.Module):
                      precomputed_masks: PrecomputedPairMasks | None = None,
                      buffers: PreallocatedBuffers | None = None, inplace_safe: bool = False) -> torch.Tensor:
         can_update_inplace = inplace_safe and not torch.cuda.is_current_stream_capturing()
-        z = self.tri_mul_out(z, mask=pair_mask, trimul_metadata=trimul_metadata, residual=True, buffers=buffers)
-        z = self.tri_mul_in(z, mask=pair_mask, trimul_metadata=trimul_metadata, residual=True, buffers=buffers)
-        if self.dtype is not None:
+        # every step reads bfloat16: fp32 results of the triangle multiplications would only be converted back
+        keep = self.dtype == torch.bfloat16
+        z = self.tri_mul_out(z, mask=pair_mask, trimul_metadata=trimul_metadata, residual=True, buffers=buffers, _keep_bf16=keep)
+        z = self.tri_mul_in(z, mask=pair_mask, trimul_metadata=trimul_metadata, residual=True, buffers=buffers, _keep_bf16=keep)
+        if self.dtype is not None and z.dtype != self.dtype:
             z = z.to(self.dtype)
         tri_attn_metadata = (attn_metadatas or {}).get("triangle_attn")
         if precomputed_masks is not None:
@@ -111,7 +114,7 @@ class PairformerLayerV1(nn.Module):
             # attention(..., residual=s) is the reference's ``s + attention(s, z, mask)`` with the add in the
             # output-projection kernel; the result is a fresh tensor, so the transition updates it in place
             s = self.attention(s, z, mask, attn_metadata=(attn_metadatas or {}).get("pairwise_attn"),
-                               mask_bias=mask_bias, buffers=buffers, residual=s)
+                               mask_bias=mask_bias, buffers=buffers, residual=s, _key_counts=kwargs.get("_key_counts"))
             s = self.transition_s(s.to(torch.bfloat16), residual=True, inplace=True).to(s_dtype)
         return s, z
 
@@ -143,7 +146,7 @@ class PairformerLayerV2(PairformerLayerV1):
         s_in = s16 if self._pre_norm_folded else self.pre_norm_s(s16)
         s16 = self.attention(s_in, z, mask, attn_metadata=(attn_metadatas or {}).get("pairwise_attn"),
                              mask_bias=getattr(precomputed_single_masks, "mask_bias", None), buffers=buffers,
-                             residual=s16)
+                             residual=s16, _key_counts=kwargs.get("_key_counts"))
         s16 = self.transition_s(s16, residual=True, inplace=True)
         if self.post_norm_s is not None:
             s16 = self.post_norm_s(s16)
@@ -213,7 +216,7 @@ class PairformerModule(nn.Module):
         inputs = (s, z, mask, pair_mask)
         # the recorded kernels hold the addresses of the layers' packed weights: a reload or an in-place edit of
         # any parameter must record a new graph
-        key = (*((tuple(t.shape), t.dtype, t.device) for t in inputs), _weight_state(*self.parameters()))
+        key = (*((t.shape, t.dtype, t.device) for t in inputs), _host.weight_state(self))
         if self._graph is None or key != self._graph_key:
             static = [t.clone() for t in inputs]
             graph_buffers: dict = {}
@@ -245,6 +248,9 @@ class PairformerModule(nn.Module):
         # the key mask of the single track, reduced once for all layers (reference: pairformer.py:472-476)
         precomputed_single = None if first.no_update_s else precompute_single_masks(
             first.pairwise_attn_backend, mask, inf=first.attention.inf)
+        if precomputed_single is not None:
+            kwargs["_key_counts"] = first.attention.key_counts(mask, precomputed_single.mask_bias, s.shape[0], s.shape[1],
+                                                               s.device)
         for layer in self.layers:
             s, z = layer(s, z, mask, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed,
                          precomputed_single_masks=precomputed_single, buffers=buffers, **kwargs)
@@ -290,7 +296,7 @@ class PairformerNoSeqModule(nn.Module):
             return self._run(z, pair_mask, attn_metadatas, buffers, **kwargs)
         # the recorded kernels hold the addresses of the layers' packed weights: a reload or an in-place edit of
         # any parameter must record a new graph
-        key = (tuple(z.shape), z.dtype, z.device, tuple(pair_mask.shape), pair_mask.dtype, _weight_state(*self.parameters()))
+        key = (z.shape, z.dtype, z.device, pair_mask.shape, pair_mask.dtype, _host.weight_state(self))
         if self._graph is None or key != self._graph_key:
             self._graph_in, self._graph_mask = z.clone(), pair_mask.clone()
             graph_buffers: dict = {}

@@ -16,10 +16,10 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from .. import ops
+from .. import _host, ops
 from .auto_chunk import ChunkPolicy
 from .linear import Linear, WeightMode, WeightsLoadingConfig
-from .triangle_nodes import _refold_after_load_state_dict, _weight_state
+from .triangle_nodes import _refold_after_load_state_dict
 
 
 def _row_mask(x: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
@@ -79,7 +79,7 @@ class Transition(nn.Module):
             self._pack = self._pack_state = None
             return
         self._pack = self._fold(self.fc3.weight.device)
-        self._pack_state = _weight_state(*self._params())
+        self._pack_state = _host.weight_state(self)
 
     @torch.no_grad()
     def _fold(self, device):
@@ -96,7 +96,7 @@ class Transition(nn.Module):
         return {"w1": w1_f, "sc1": sc1, "w2": w2_f, "sc2": sc2}
 
     def _packed(self, device) -> torch.Tensor:
-        state = _weight_state(*self._params())
+        state = _host.weight_state(self)
         held = self._pack["w1"] if isinstance(self._pack, dict) else self._pack
         if held is None or held.device != device or state != self._pack_state:
             pack = self._fold(device)
@@ -129,29 +129,18 @@ class Transition(nn.Module):
             mask_p = None if mask is None else _row_mask(x, mask).permute(order[:-1])
             y = self.forward(x.permute(order), mask_p, residual=residual, inplace=inplace)
             return x if (residual and inplace) else y.permute(inverse)
-        xc = x
         if not self._fused:
-            return self._forward_gemms(x, xc, mask, residual, inplace)
-        out = xc if (residual and inplace) else None
-        row_mask = None if mask is None else _row_mask(xc, mask)
-        return ops.transition(xc, self._packed(x.device), row_mask, self.eps if self.norm is None else self.norm.eps,
-                              residual=residual, out=out)
+            if mask is not None:
+                raise ValueError("a row mask is only supported by the fused pair transition (dim 128, hidden 512)")
+            w = self._packed(x.device)
+            return _host.transition_gemms(x, w["w1"], w["sc1"], w["w2"], w["sc2"], self.norm is not None, self._norm_eps(),
+                                          residual, residual and inplace)
+        row_mask = None if mask is None else _row_mask(x, mask)
+        return _host.transition(x, self._packed(x.device), row_mask, self._norm_eps(), residual, residual and inplace, False)
 
-    def _forward_gemms(self, x, xc, mask, residual: bool, inplace: bool) -> torch.Tensor:
-        if mask is not None:
-            raise ValueError("a row mask is only supported by the fused pair transition (dim 128, hidden 512)")
-        w = self._packed(x.device)
-        rows = xc.numel() // self.dim
-        eps = self.eps if self.norm is None else self.norm.eps
-        stats = ops.row_stats(xc, eps) if self.norm is not None else None
-        h = ops.linear(xc, w["w1"], w["sc1"], ops.LINEAR_SWIGLU, B=1, rows=rows, stats=stats)
-        x3 = xc.view(1, rows, self.dim)
-        y = ops.linear(h, w["w2"], w["sc2"], ops.LINEAR_ROWS, B=1, rows=rows, residual=x3 if residual else None,
-                       out=x3 if (residual and inplace) else None).view(xc.shape)
-        if residual and inplace and xc is not x:
-            x.copy_(y)
-            return x
-        return y
+    def _norm_eps(self) -> float:
+        norm = self.norm
+        return self.eps if norm is None else norm.eps
 
 
 class PairTransition(nn.Module):
@@ -190,10 +179,10 @@ class PairTransition(nn.Module):
             return
         device = self.linear_2.weight.device  # LayerNorm's parameters may still sit on the host at load time
         self._pack = ops.pack_relu_transition_weights(*[t.to(device) for t in self._params()])
-        self._pack_state = _weight_state(*self._params())
+        self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _weight_state(*self._params())
+        state = _host.weight_state(self)
         if self._pack is None or self._pack.device != device or state != self._pack_state:
             pack = ops.pack_relu_transition_weights(*[t.to(device) for t in self._params()])
             if not torch.cuda.is_current_stream_capturing():
@@ -218,4 +207,4 @@ class PairTransition(nn.Module):
             mask_p = None if mask is None else _row_mask(z, mask).permute(order[:-1])
             return self.forward(z.permute(order), mask_p, residual=residual).permute(inverse)
         row_mask = None if mask is None else _row_mask(z, mask)
-        return ops.transition(z, self._packed(z.device), row_mask, self.layer_norm.eps, residual=residual, relu=True)
+        return _host.transition(z, self._packed(z.device), row_mask, self.layer_norm.eps, residual, False, True)

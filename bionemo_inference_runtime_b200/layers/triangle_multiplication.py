@@ -16,10 +16,9 @@ from enum import IntEnum
 import torch
 import torch.nn as nn
 
-from .. import ops
-from .buffers import ensure_buffer
+from .. import _host, ops
 from .linear import Linear, WeightMode, WeightsLoadingConfig
-from .triangle_nodes import _refold_after_load_state_dict, _weight_state
+from .triangle_nodes import _refold_after_load_state_dict
 
 _GEMM_TOKEN_ALIGN = 8
 
@@ -124,10 +123,10 @@ class TriangleMultiplicationNode(nn.Module):
             self._pack = self._pack_state = None
             return
         self._pack = self._fold(self.p_in.weight.device)
-        self._pack_state = _weight_state(*self._params())
+        self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _weight_state(*self._params())
+        state = _host.weight_state(self)
         if self._pack is None or self._pack.device != device or state != self._pack_state:
             pack = self._fold(device)
             # a fold recorded during graph capture is only filled at replay: use it for this call only
@@ -145,12 +144,13 @@ class TriangleMultiplicationNode(nn.Module):
     # ---- forward ------------------------------------------------------------------------------
     def forward(self, x: torch.Tensor, mask: torch.Tensor | None = None,
                 trimul_metadata: TriangleMultiplicationMetadata | None = None, *, residual: bool = False,
-                buffers: dict | None = None) -> torch.Tensor:
+                buffers: dict | None = None, _keep_bf16: bool = False) -> torch.Tensor:
         """``x``: pair tensor ``[B, I, J, dim]``; ``mask``: pair mask ``[B, I, J]`` (1 = valid) or ``None``.
         Returns the update, or with ``residual`` ``x + update`` - multiplied by the mask when the metadata carries
         the outgoing row lengths and the token counts are multiples of 8, which is where the reference takes its
         fused masked-residual kernel (lines 706-722).  ``buffers`` (optional dict) keeps the two channel-major
-        intermediates between calls."""
+        intermediates between calls; ``_keep_bf16`` (for the pairformer layers, whose next step takes bfloat16)
+        returns the bfloat16 result where the caller of a single node gets it in fp32."""
         if x.dim() != 4 or x.shape[-1] != self.dim or x.shape[1] != x.shape[2]:
             raise ValueError(f"expected a square pair tensor [B, N, N, {self.dim}], got {tuple(x.shape)}")
         if not x.is_cuda:
@@ -169,21 +169,17 @@ class TriangleMultiplicationNode(nn.Module):
         if self.mean_normalization:
             n_valid = mask_f[:, 0, :].sum(dim=-1) if mask_f is not None else x.new_full((B,), float(N), dtype=torch.float32)
             b_scale = (1.0 / (n_valid + 1e-3)).contiguous()
-        packed = self._packed(x.device)
-        pitch = ops.pad16(N)
-        ab = ensure_buffer(buffers, "trimul_ab", (B, 2 * self.hidden_dim, N, pitch), torch.bfloat16, x.device)
-        t = ensure_buffer(buffers, "trimul_contracted", (B, self.hidden_dim, N, pitch), torch.bfloat16, x.device)
-        ab = ops.trimul_project(x, mask_f, packed, self.eps, incoming=incoming, b_scale=b_scale, ab=ab)
-        t = ops.trimul_contract(ab, N, x=t)
-        metadata = trimul_metadata if trimul_metadata is not None else TriangleMultiplicationMetadata()
-        fuse_mask = (residual and mask_f is not None and metadata.outgoing_actual_seqlen is not None
-                     and self.can_fuse_residual(x))
-        out = ops.trimul_output(x, t, packed, self.eps, residual=residual, mask=mask_f if fuse_mask else None)
-        if self.high_precision:
-            out = out.to(torch.float32)
-        elif residual and residual_pair.dtype != out.dtype:
-            out = out.to(torch.promote_types(residual_pair.dtype, out.dtype))
-        return out
+        fuse_mask = (residual and mask_f is not None and trimul_metadata is not None
+                     and trimul_metadata.outgoing_actual_seqlen is not None and self.can_fuse_residual(x))
+        if _keep_bf16:
+            out_dtype = torch.bfloat16
+        elif self.high_precision:
+            out_dtype = torch.float32
+        else:
+            out_dtype = torch.promote_types(residual_pair.dtype, torch.bfloat16) if residual else torch.bfloat16
+        out = _host.trimul(x, mask_f, self._packed(x.device), self.eps, incoming, b_scale, buffers, residual, fuse_mask,
+                           out_dtype == torch.float32)  # written as fp32 by the output kernel, not converted after it
+        return out if out.dtype == out_dtype else out.to(out_dtype)
 
 
 def set_trimul_token_padding(module: nn.Module, enabled: bool) -> None:

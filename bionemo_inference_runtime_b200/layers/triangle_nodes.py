@@ -15,7 +15,7 @@ from enum import IntEnum
 import torch
 import torch.nn as nn
 
-from .. import _lib, ops
+from .. import _host, _lib, ops
 from .attention_backend import (AttentionMetadata, AttentionType, create_attention, mask_to_lengths,
                                 triangle_bias_pad_multiple)
 from .auto_chunk import CHUNK_REGISTRY, TRIANGLE_ATTENTION, ChunkPolicy, iter_chunks
@@ -28,14 +28,6 @@ _EMPTY_ROW_MODES = {"uniform": _lib.EMPTY_ROW_UNIFORM, "zeros": _lib.EMPTY_ROW_Z
 class TriangleAttentionNodeType(IntEnum):
     STARTING = 0
     ENDING = 1
-
-
-def _weight_state(*params) -> tuple | None:
-    """(address, in-place write count) of every parameter; changes when a weight is loaded or edited."""
-    try:
-        return tuple((p.data_ptr(), p._version, p.device) for p in params if p is not None)
-    except RuntimeError:
-        return None
 
 
 def _refold_after_load_state_dict(module, *args) -> None:
@@ -90,7 +82,7 @@ class TriangleAttention(nn.Module):
 
     def _packed(self, device) -> torch.Tensor:
         """Packed weights for the stand-alone path (no LayerNorm, zero triangle-bias rows)."""
-        state = _weight_state(self.in_proj.weight, self.in_proj.bias, self.o_proj.weight, self.o_proj.bias)
+        state = _host.weight_state(self)
         if self._pack is None or self._pack.device != device or state != self._pack_state:
             zero_bias_rows = torch.zeros((ops.HEADS, ops.C), dtype=self.in_proj.weight.dtype, device=device)
             pack = ops.pack_node_weights(None, None, self.in_proj.weight, self.in_proj.bias, zero_bias_rows,
@@ -191,10 +183,10 @@ class TriangleAttentionNode(nn.Module):
             return
         dev = params[2].device
         self._pack = ops.pack_node_weights(*[None if p is None else p.to(dev) for p in params])
-        self._pack_state = _weight_state(*params)
+        self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _weight_state(*self._params())
+        state = _host.weight_state(self)
         if self._pack is None or self._pack.device != device or state != self._pack_state:
             pack = ops.pack_node_weights(*[None if p is None else p.to(device) for p in self._params()])
             # a fold recorded during graph capture is only filled at replay: use it for this call only
@@ -242,22 +234,23 @@ class TriangleAttentionNode(nn.Module):
             else:
                 m = mask.transpose(1, 2) if ending else mask
                 lengths = (m > 0.5).sum(dim=-1).to(torch.int32).contiguous()
+        elif mask_bias.dtype == torch.int32 and mask_bias.numel() == B * R:
+            lengths = mask_bias
         else:
             lengths = mask_to_lengths(mask_bias, B, R).contiguous()
         packed = self._packed(x.device)
         eps = self.layer_norm.eps
+        mode = _EMPTY_ROW_MODES[self.empty_row_mode]
+        policy = self.mha.chunk_policy
+        chunked = policy is not None and policy.chunk_size < R and policy.should_chunk(x)
+        if not chunked and not self.transposed_bias and key_mask is None:
+            # common case: one native call for the whole node, intermediates in one workspace
+            return _host.node(x, packed, lengths, eps, ending, residual, residual and inplace_residual, buffers, mode)
+        if lengths is not None:
+            lengths = lengths.reshape(B, R)
         out = x if (residual and inplace_residual) else torch.empty_like(x, memory_format=torch.contiguous_format)
         xk = x.transpose(1, 2) if ending else x      # kernel-order views [B, R, S, c]
         outk = out.transpose(1, 2) if ending else out
-        mode = _EMPTY_ROW_MODES[self.empty_row_mode]
-
-        policy = self.mha.chunk_policy
-        chunked = policy is not None and policy.should_chunk(xk) and policy.chunk_size < R
-        if not chunked and not self.transposed_bias and key_mask is None:
-            # common case: one library call for the whole node, intermediates in one workspace
-            ws = ensure_buffer(buffers, "tri_attn_workspace", (ops.node_workspace_bytes(B, N),), torch.uint8, x.device)
-            return ops.node_forward(x, packed, lengths, eps, ending=ending, residual=residual, out=out, workspace=ws,
-                                    empty_row_mode=mode)
         bias = ensure_buffer(buffers, "tri_attn_bias", (B, ops.HEADS, S, ops.pad8(S)), torch.bfloat16, x.device)
         if self.transposed_bias and bias is None:
             bias = torch.zeros((B, ops.HEADS, S, ops.pad8(S)), dtype=torch.bfloat16, device=x.device)

@@ -388,6 +388,11 @@ int b200ta_trimul_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j
                          const float* mask, int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps,
                          int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
                          void* stream);
+/* The same with a float result (out strides in float elements). */
+int b200ta_trimul_output_f32(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const void* x, int64_t pitch,
+                             const float* mask, int64_t ms_b, int64_t ms_i, int64_t ms_j, const void* packed, float eps,
+                             int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
+                             void* stream);
 
 #ifdef __cplusplus
 }
