@@ -118,6 +118,8 @@ SIGNATURES: dict[str, tuple] = {
         [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_float,
          c_int, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
     ),
+    "b200ta_mask_lengths": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "b200ta_mask_bits": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
 }
 
 

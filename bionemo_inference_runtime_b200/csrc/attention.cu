@@ -199,6 +199,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -219,6 +220,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     fence_mbar_init();
   }
   if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -870,14 +872,11 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
   const int grid = p.num_items < st->num_sms ? p.num_items : st->num_sms;
   if (key_mask != nullptr) {
     B200TA_REQUIRE(lengths != nullptr, "attention: the masked form needs the row lengths (last valid key + 1) as well");
-    B200TA_CHECK_CUDA(cudaFuncSetAttribute(attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
-    attention_kernel<true><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_q, tm_k, tm_v, tm_bias, p);
-  } else {
-    B200TA_CHECK_CUDA(cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
-    attention_kernel<false><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_q, tm_k, tm_v, tm_bias, p);
+    return launch_kernel(st, kKernelAttentionMasked, attention_kernel<true>, dim3(grid), kThreads, kSmDynamic, stream, tm_q,
+                         tm_k, tm_v, tm_bias, p);
   }
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelAttention, attention_kernel<false>, dim3(grid), kThreads, kSmDynamic, stream, tm_q, tm_k,
+                       tm_v, tm_bias, p);
 }
 
 }  // namespace

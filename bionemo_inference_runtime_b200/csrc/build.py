@@ -21,7 +21,7 @@ LIB = PKG / "libb200ta.so"
 HOST = PKG / "_host.so"
 OBJ_DIR = CSRC / "build"
 SOURCES = ["host.cu", "pack.cu", "rowgemm.cu", "attention.cu", "node.cu", "transition.cu", "trimul_project.cu",
-           "trimul_contract.cu", "trimul_output.cu", "linear.cu", "pair_bias.cu"]
+           "trimul_contract.cu", "trimul_output.cu", "linear.cu", "pair_bias.cu", "masks.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo", "--use_fast_math",

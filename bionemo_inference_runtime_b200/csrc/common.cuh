@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/b200ta.h"
 
 namespace b200ta {
@@ -42,8 +44,41 @@ struct DeviceState {
   int device = -1;
   int num_sms = 0;
   int* status_dev = nullptr;  // device word kernels write when they abandon a bounded wait
+  std::atomic<uint32_t> configured{0};  // bit per KernelId: its shared-memory limit has been raised on this device
+};
+enum KernelId {
+  kKernelPrologue, kKernelEpilogue, kKernelAttention, kKernelAttentionMasked, kKernelTransition, kKernelTransitionRelu,
+  kKernelProject, kKernelContract, kKernelOutput, kKernelOutputF32, kKernelLinear, kKernelPairBias, kKernelRowStats,
+  kKernelMaskRows
 };
 int get_device_state(DeviceState** out);
+
+#ifdef __CUDACC__
+// Launches a kernel that begins with pdl_wait(): the stream may start its blocks while the last blocks of the kernel
+// before it still run (programmatic dependent launch), so that barrier and tensor-memory set-up and the launch latency
+// itself hide behind them.  A block's set-up takes 2-3 us of the 5-12 us a kernel needs at small token counts.
+template <typename... P, typename... A>
+int launch_kernel(DeviceState* st, KernelId id, void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, void* stream,
+                  A&&... args) {
+  const uint32_t bit = 1u << id;
+  if (smem_bytes > 0 && !(st->configured.load(std::memory_order_relaxed) & bit)) {
+    B200TA_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+    st->configured.fetch_or(bit, std::memory_order_relaxed);
+  }
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(unsigned(threads));
+  config.dynamicSmemBytes = size_t(smem_bytes);
+  config.stream = static_cast<cudaStream_t>(stream);
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  B200TA_CHECK_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...));
+  return B200TA_OK;
+}
+#endif
 
 // Encodes a tiled bf16/fp32 tensor map. `dims`, `strides_bytes` (rank-1 entries,
 // for dims 1..rank-1) and `box` are innermost first.
@@ -70,6 +105,13 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
+
+// ---- programmatic dependent launch -------------------------------------------
+// At the top of a kernel: lets the stream's next kernel start its blocks as soon as there is room for them.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Returns once the kernels before this one in the stream are complete and their writes visible.  Every thread calls it
+// before its first access to global memory (reads of weights included: a fold may be the kernel before).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- mbarrier --------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -78,6 +78,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
   const int n0 = blockIdx.y * kTile;
   const int steps = p.K / kStepK;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -88,8 +89,9 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
     mbar_init(bars + ACC_FULL * 8, 1);
     fence_mbar_init();
   }
-  if (threadIdx.x < kTile) reinterpret_cast<float2*>(gen + kSmSc)[threadIdx.x] = p.sc[n0 + threadIdx.x];
   if (warp == 5) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 128);
+  pdl_wait();
+  if (threadIdx.x < kTile) reinterpret_cast<float2*>(gen + kSmSc)[threadIdx.x] = p.sc[n0 + threadIdx.x];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -214,6 +216,8 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
 // {rstd, -mean * rstd} of every row: one warp per row, the row held in registers between the two passes.
 __global__ void row_stats_kernel(const __nv_bfloat16* x, long long row_stride, long long rows, int K, float eps,
                                  float2* stats) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -255,11 +259,12 @@ int b200ta_row_stats(const void* x, int64_t row_stride, int64_t rows, int K, flo
   B200TA_REQUIRE(rows > 0 && K > 0 && K <= 2048 && K % 2 == 0 && row_stride % 2 == 0,
                  "row_stats: need an even K <= 2048 and an even row stride (K=%d)", K);
   B200TA_REQUIRE((reinterpret_cast<uintptr_t>(x) & 3u) == 0, "row_stats: x must be 4-byte aligned");
+  DeviceState* st = nullptr;
+  const int rc = get_device_state(&st);
+  if (rc != B200TA_OK) return rc;
   const int warps = 4;
-  row_stats_kernel<<<unsigned((rows + warps - 1) / warps), warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), row_stride, rows, K, eps, static_cast<float2*>(stats));
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelRowStats, row_stats_kernel, dim3(unsigned((rows + warps - 1) / warps)), warps * 32, 0, stream,
+                       static_cast<const __nv_bfloat16*>(x), row_stride, rows, K, eps, static_cast<float2*>(stats));
 }
 
 int b200ta_linear(const void* a, int64_t as_b, int64_t as_row, int64_t as_chunk, const void* w, const void* sc,
@@ -308,11 +313,8 @@ int b200ta_linear(const void* a, int64_t as_b, int64_t as_row, int64_t as_chunk,
   p.os_row = os_row, p.rs_row = rs_row, p.plane_stride = plane_stride;
   p.mode = mode;
   p.status = st->status_dev;
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const dim3 grid(unsigned(B * p.tiles_m), unsigned(N / kTile));
-  linear_kernel<<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_a, tm_w, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelLinear, linear_kernel, grid, kThreads, kSmDynamic, stream, tm_a, tm_w, p);
 }
 
 }  // extern "C"

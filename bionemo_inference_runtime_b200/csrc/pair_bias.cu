@@ -58,6 +58,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -72,11 +73,12 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
     }
     fence_mbar_init();
   }
+  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 32);
+  pdl_wait();
   if (threadIdx.x < kMaxHeads / 2) {
     const float2 a = p.sc[kFirstRow + 2 * threadIdx.x], b = p.sc[kFirstRow + 2 * threadIdx.x + 1];
     reinterpret_cast<float4*>(gen + kSmSc)[threadIdx.x] = make_float4(a.x, b.x, a.y, b.y);
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 32);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -254,11 +256,8 @@ int b200ta_pair_bias(const void* z, int64_t zs_b, int64_t zs_q, int64_t zs_k, co
   p.bias = static_cast<__nv_bfloat16*>(bias);
   p.bs_b = bs_b, p.bs_h = bs_h, p.bs_q = bs_q, p.bs_k = bs_k;
   p.status = st->status_dev;
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(pair_bias_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  pair_bias_kernel<<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_z, tm_w, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelPairBias, pair_bias_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_w, p);
 }
 
 }  // extern "C"

@@ -105,6 +105,7 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   const int u_begin = (MODE == kPrologue && !p.want_qkvg) ? 2 : 0;
   const int u_end = MODE == kPrologue ? 3 : 1;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;  // scratch flag for the producer's drain wait
@@ -117,6 +118,8 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     }
     fence_mbar_init();
   }
+  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  pdl_wait();
   // stage the per-column vectors
   if (MODE == kPrologue) {
     float4* dst = reinterpret_cast<float4*>(gen + L::kVec);
@@ -128,7 +131,6 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     float* dst = reinterpret_cast<float*>(gen + L::kVec);
     for (int i = threadIdx.x; i < kC; i += kThreads) dst[i] = p.bo[i];
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -433,12 +435,9 @@ int launch_epilogue(const void* og, int64_t gs_b, int64_t gs_r, int64_t gs_s, co
   p.has_residual = residual ? 1 : 0;
   p.status = st->status_dev;
 
-  auto kern = rowgemm_kernel<kEpilogue>;
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<kEpilogue>::kDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  kern<<<grid, kThreads, Smem<kEpilogue>::kDynamic, static_cast<cudaStream_t>(stream)>>>(tm_a, tm_w, tm_res, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelEpilogue, rowgemm_kernel<kEpilogue>, dim3(grid), kThreads, Smem<kEpilogue>::kDynamic, stream,
+                       tm_a, tm_w, tm_res, p);
 }
 
 }  // namespace
@@ -496,12 +495,9 @@ int b200ta_prologue(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_s, con
                  qs_h % 16 == 0 && qs_s % 16 == 0;
   p.status = st->status_dev;
 
-  auto kern = rowgemm_kernel<kPrologue>;
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<kPrologue>::kDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  kern<<<grid, kThreads, Smem<kPrologue>::kDynamic, static_cast<cudaStream_t>(stream)>>>(tm_a, tm_w, tm_a, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelPrologue, rowgemm_kernel<kPrologue>, dim3(grid), kThreads, Smem<kPrologue>::kDynamic, stream,
+                       tm_a, tm_w, tm_a, p);
 }
 
 int b200ta_epilogue(const void* og, int64_t gs_b, int64_t gs_r, int64_t gs_s, const void* packed,

@@ -25,7 +25,8 @@ struct Library {
 #define B200TA_ENTRY(name) decltype(&b200ta_##name) name = nullptr;
 #define B200TA_ENTRIES(X)                                                                                            \
   X(last_error) X(node_workspace_bytes) X(node_forward) X(transition) X(transition_relu) X(trimul_project)           \
-  X(trimul_contract) X(trimul_output) X(trimul_output_f32) X(pair_bias) X(row_stats) X(linear) X(attention)
+  X(trimul_contract) X(trimul_output) X(trimul_output_f32) X(pair_bias) X(row_stats) X(linear) X(attention)            \
+  X(attention_masked) X(prologue) X(epilogue) X(mask_lengths) X(mask_bits)
   B200TA_ENTRIES(B200TA_ENTRY)
 #undef B200TA_ENTRY
 } lib;
@@ -138,6 +139,36 @@ at::Tensor node(const at::Tensor& z, const at::Tensor& packed, const c10::option
   return out;
 }
 
+// The node with one bit per key beside the row lengths (masks that are not left-aligned), from prologue to epilogue.
+at::Tensor node_masked(const at::Tensor& z, const at::Tensor& packed, const at::Tensor& lengths, const at::Tensor& bits,
+                       double eps, bool ending, bool residual, bool inplace, const py::object& buffers, int empty_row_mode) {
+  const Pair p = pair_of("z", z, ending);
+  const int64_t B = p.B, N = p.N, dim = B200TA_HEAD_DIM, heads = B200TA_HEADS, pad = (N + 7) / 8 * 8, words = (N + 31) / 32;
+  if (bits.scalar_type() != at::kInt || !bits.is_cuda() || !bits.is_contiguous() || bits.numel() != B * N * words)
+    throw py::value_error("key bits must be a contiguous CUDA int32 tensor [B, N, ceil(N / 32)]");
+  const at::Tensor out = inplace ? z : new_bf16(z, z.sizes());
+  const Pair o = pair_of("out", out, ending);
+  const Lengths l = lengths_of(lengths, B, N);
+  const at::Tensor bias = buffer(buffers, "tri_attn_bias", {B, heads, N, pad}, at::kBFloat16, z);
+  const at::Tensor qkvg = buffer(buffers, "tri_attn_qkvg", {4, B * N, heads, N, dim}, at::kBFloat16, z);
+  const at::Tensor og = buffer(buffers, "tri_attn_output", {B * N, N, heads, dim}, at::kBFloat16, z);
+  void* s = stream();
+  const int64_t head = N * dim, row = heads * head, plane = B * N * row;
+  check(lib.prologue(z.data_ptr(), p.sb, p.sr, p.ss, packed.data_ptr(), float(eps), qkvg.data_ptr(), plane, row, head, dim, 1,
+                     bias.data_ptr(), heads * N * pad, N * pad, pad, 1, p.B, p.N, p.N, int(pad), s),
+        "b200ta_prologue");
+  char* q = static_cast<char*>(qkvg.data_ptr());
+  check(lib.attention_masked(q, q + 2 * plane, q + 4 * plane, q + 6 * plane, row, head, dim, bias.data_ptr(), heads * N * pad,
+                             N * pad, pad, l.ptr, l.sb, l.sr, reinterpret_cast<const uint32_t*>(bits.data_ptr<int32_t>()),
+                             N * words, words, og.data_ptr(), N * B200TA_C, B200TA_C, dim, nullptr, 0.17677669529663687f,
+                             empty_row_mode, p.B, p.N, p.N, int(pad), s),
+        "b200ta_attention_masked");
+  check(lib.epilogue(og.data_ptr(), N * N * B200TA_C, N * B200TA_C, B200TA_C, packed.data_ptr(),
+                     residual ? z.data_ptr() : nullptr, p.sb, p.sr, p.ss, out.data_ptr(), o.sb, o.sr, o.ss, p.B, p.N, p.N, s),
+        "b200ta_epilogue");
+  return out;
+}
+
 at::Tensor trimul(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const at::Tensor& packed, double eps,
                   bool incoming, const c10::optional<at::Tensor>& b_scale, const py::object& buffers, bool residual,
                   bool mask_output, bool f32) {
@@ -247,6 +278,30 @@ at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& z, const
   return out;
 }
 
+// ---- masks -----------------------------------------------------------------------------------------------------------
+
+at::Tensor new_int32(const at::Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kInt)); }
+
+// Keys with mask > 0.5 per row of a float [B, I, J] mask and per row of its transpose.
+std::pair<at::Tensor, at::Tensor> mask_lengths(const at::Tensor& mask) {
+  const int B = int(mask.size(0)), I = int(mask.size(1)), J = int(mask.size(2));
+  const at::Tensor rows = new_int32(mask, {B, I}), cols = new_int32(mask, {B, J});
+  check(lib.mask_lengths(mask.data_ptr<float>(), mask.stride(0), mask.stride(1), mask.stride(2), rows.data_ptr<int32_t>(),
+                         cols.data_ptr<int32_t>(), B, I, J, stream()),
+        "b200ta_mask_lengths");
+  return {rows, cols};
+}
+
+// Row lengths (last valid key + 1) and key bits of a float [B, R, S] mask; valid: > 0.5, or >= 0 in the additive form.
+std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additive) {
+  const int B = int(mask.size(0)), R = int(mask.size(1)), S = int(mask.size(2));
+  const at::Tensor lengths = new_int32(mask, {B, R}), bits = new_int32(mask, {B, R, (S + 31) / 32});
+  check(lib.mask_bits(mask.data_ptr<float>(), mask.stride(0), mask.stride(1), mask.stride(2), additive,
+                      lengths.data_ptr<int32_t>(), reinterpret_cast<uint32_t*>(bits.data_ptr<int32_t>()), B, R, S, stream()),
+        "b200ta_mask_bits");
+  return {lengths, bits};
+}
+
 // ---- weight state --------------------------------------------------------------------------------------------------
 
 void add_parameters(PyObject* module, std::string& out) {
@@ -286,9 +341,12 @@ PYBIND11_MODULE(_host, m) {
   m.doc() = "Native host path of the layers (see csrc/torch_host.cpp).";
   m.def("bind", &bind);
   m.def("node", &node);
+  m.def("node_masked", &node_masked);
   m.def("trimul", &trimul);
   m.def("transition", &transition);
   m.def("transition_gemms", &transition_gemms);
   m.def("pair_bias_attention", &pair_bias_attention);
+  m.def("mask_lengths", &mask_lengths);
+  m.def("mask_bits", &mask_bits);
   m.def("weight_state", &weight_state);
 }

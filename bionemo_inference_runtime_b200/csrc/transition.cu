@@ -168,6 +168,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -191,13 +192,14 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     mbar_init(bars + XN_EMPTY * 8, 4);
     fence_mbar_init();
   }
+  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+  pdl_wait();
   // stage the constants: LayerNorm gamma | beta, and for the ReLU form the two linears' biases
   if (threadIdx.x < 2 * kC) reinterpret_cast<float*>(gen + kSmLn)[threadIdx.x] = p.ln[threadIdx.x];
   if (kRelu) {
     for (int q = threadIdx.x; q < kHidden; q += kThreads) reinterpret_cast<float*>(gen + kSmSc)[q] = p.sc[q].y;
     if (threadIdx.x < kC) reinterpret_cast<float*>(gen + kSmSc + 4096)[threadIdx.x] = p.b2[threadIdx.x];
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -566,9 +568,12 @@ int launch_transition(const void* x, int64_t xs, const void* mask, const void* p
     uint64_t ostrides[1] = {uint64_t(os) * 2};
     uint32_t obox[2] = {32, 32};
     for (int k = 0; k < kMaxPeers; ++k) {
-      const int src = k < num_outs ? k : 0;
-      B200TA_REQUIRE(outs[src], "transition: NULL output pointer");
-      rc = encode_tensor_map(&tm_outs.m[k], outs[src], 2, 2, dims, ostrides, obox, SWZ_64, "transition out");
+      if (k >= num_outs) {
+        tm_outs.m[k] = tm_outs.m[0];
+        continue;
+      }
+      B200TA_REQUIRE(outs[k], "transition: NULL output pointer");
+      rc = encode_tensor_map(&tm_outs.m[k], outs[k], 2, 2, dims, ostrides, obox, SWZ_64, "transition out");
       if (rc != B200TA_OK) return rc;
     }
   }
@@ -602,14 +607,11 @@ int launch_transition(const void* x, int64_t xs, const void* mask, const void* p
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
   if (relu) {
-    B200TA_CHECK_CUDA(cudaFuncSetAttribute(transition_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
-    transition_kernel<true><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_x, tm_w1, tm_w2, tm_outs, p);
-  } else {
-    B200TA_CHECK_CUDA(cudaFuncSetAttribute(transition_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
-    transition_kernel<false><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_x, tm_w1, tm_w2, tm_outs, p);
+    return launch_kernel(st, kKernelTransitionRelu, transition_kernel<true>, dim3(grid), kThreads, kSmDynamic, stream, tm_x,
+                         tm_w1, tm_w2, tm_outs, p);
   }
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelTransition, transition_kernel<false>, dim3(grid), kThreads, kSmDynamic, stream, tm_x, tm_w1,
+                       tm_w2, tm_outs, p);
 }
 
 }  // namespace

@@ -68,6 +68,7 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const Contract
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kSmBars + NUM_BARS * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     for (int i = 0; i < kStages; ++i) {
@@ -81,6 +82,7 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const Contract
     fence_mbar_init();
   }
   if (warp == 5) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -224,11 +226,8 @@ int b200ta_trimul_contract(const void* ab, void* x, int B, int N, int64_t pitch,
   p.x_row = pitch, p.x_plane = pitch * N;
   p.status = st->status_dev;
 
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(trimul_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  trimul_contract_kernel<<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_ab, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelContract, trimul_contract_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_ab, p);
 }
 
 }  // extern "C"

@@ -69,6 +69,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kSmBars + NUM_BARS * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     mbar_init(bars + W_FULL * 8, 1);
@@ -84,6 +85,8 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     }
     fence_mbar_init();
   }
+  if (warp == 13) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  pdl_wait();
   // per-channel constants of the epilogue
   if (threadIdx.x < kC / 2) {
     const int c = 2 * threadIdx.x;
@@ -91,7 +94,6 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     reinterpret_cast<float4*>(gen + kSmConst)[threadIdx.x] = make_float4(g0.y, g1.y, g0.x, g1.x);
     reinterpret_cast<float4*>(gen + kSmConst + 1024)[threadIdx.x] = make_float4(q0.y, q1.y, q0.x, q1.x);
   }
-  if (warp == 13) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -420,11 +422,8 @@ int launch_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const
   p.os_b = os_b, p.os_i = os_i, p.os_j = os_j;
   p.status = st->status_dev;
 
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(trimul_output_kernel<kF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  trimul_output_kernel<kF32><<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_z, tm_x, tm_w, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kF32 ? kKernelOutputF32 : kKernelOutput, trimul_output_kernel<kF32>, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_x, tm_w, p);
 }
 
 }  // namespace

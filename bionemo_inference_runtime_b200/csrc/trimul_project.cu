@@ -65,6 +65,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kSmBars + NUM_BARS * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     mbar_init(bars + W_FULL * 8, 1);
@@ -80,6 +81,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     fence_mbar_init();
   }
   if (warp == 21) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -321,11 +323,8 @@ int b200ta_trimul_project(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_
   p.pitch = pitch;
   p.status = st->status_dev;
 
-  B200TA_CHECK_CUDA(cudaFuncSetAttribute(trimul_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmDynamic));
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  trimul_project_kernel<<<grid, kThreads, kSmDynamic, static_cast<cudaStream_t>(stream)>>>(tm_z, tm_w, p);
-  B200TA_CHECK_CUDA(cudaGetLastError());
-  return B200TA_OK;
+  return launch_kernel(st, kKernelProject, trimul_project_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_w, p);
 }
 
 }  // extern "C"

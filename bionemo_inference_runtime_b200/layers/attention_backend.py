@@ -22,7 +22,7 @@ from dataclasses import dataclass
 
 import torch
 
-from .. import _lib, ops
+from .. import _host, _lib, ops
 
 DEBUG_ASSERTS = os.environ.get("B200TA_DEBUG_ASSERTS", os.environ.get("BIOIR_DEBUG_ASSERTS", "0")) == "1"
 
@@ -205,6 +205,10 @@ def _additive_precompute(pair_mask, inf=1e9, dtype=None):
 
 def _length_precompute(pair_mask, inf=1e9, dtype=None):
     del inf, dtype
+    if (pair_mask.is_cuda and pair_mask.dtype == torch.float32 and pair_mask.dim() == 3 and pair_mask.numel() > 0
+            and not DEBUG_ASSERTS):
+        rows, columns = _host.mask_lengths(pair_mask)  # both directions in one pass
+        return PrecomputedPairMasks(pair_mask=pair_mask, mask_bias=rows, mask_bias_transposed=columns)
     mb = pair_mask > 0.5
     if DEBUG_ASSERTS and not torch.cuda.is_current_stream_capturing():
         if not (bool(torch.all(mb[..., :-1] >= mb[..., 1:])) and bool(torch.all(mb[..., :-1, :] >= mb[..., 1:, :]))):

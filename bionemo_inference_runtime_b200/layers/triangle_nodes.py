@@ -218,22 +218,29 @@ class TriangleAttentionNode(nn.Module):
         key_mask = None
         if not self.pair_mask_left_aligned and (mask is not None or mask_bias is not None):
             # keys may be switched off anywhere in a row: the kernel takes one bit per key beside the row lengths
-            if mask_bias is None:
-                valid = (mask.transpose(1, 2) if ending else mask) > 0.5
+            additive = mask_bias is not None
+            if not additive:
+                source = mask.transpose(1, 2) if ending else mask
             elif mask_bias.dtype == torch.int32:
                 raise ValueError("a node built with pair_mask_left_aligned=False takes the pair mask or its additive "
                                  "form ([B, R, 1, 1, S]); int32 row lengths describe left-aligned masks only")
             else:
-                valid = (mask_bias[:, :, 0, 0, :] if mask_bias.dim() == 5 else mask_bias) >= 0
-            if tuple(valid.shape) != (B, R, S):
-                raise ValueError(f"mask of shape {tuple(valid.shape)} does not match the pair tensor [B={B}, {R}, {S}]")
-            lengths, key_mask = ops.key_mask_bits(valid)
+                source = mask_bias[:, :, 0, 0, :] if mask_bias.dim() == 5 else mask_bias
+            if tuple(source.shape) != (B, R, S):
+                raise ValueError(f"mask of shape {tuple(source.shape)} does not match the pair tensor [B={B}, {R}, {S}]")
+            if source.is_cuda and source.dtype == torch.float32:
+                lengths, key_mask = _host.mask_bits(source, additive)
+            else:
+                lengths, key_mask = ops.key_mask_bits(source >= 0 if additive else source > 0.5)
         elif mask_bias is None:
             if mask is None:
                 lengths = None
             else:
-                m = mask.transpose(1, 2) if ending else mask
-                lengths = (m > 0.5).sum(dim=-1).to(torch.int32).contiguous()
+                if mask.is_cuda and mask.dtype == torch.float32 and mask.dim() == 3:
+                    lengths = _host.mask_lengths(mask)[ending]
+                else:
+                    m = mask.transpose(1, 2) if ending else mask
+                    lengths = (m > 0.5).sum(dim=-1).to(torch.int32).contiguous()
         elif mask_bias.dtype == torch.int32 and mask_bias.numel() == B * R:
             lengths = mask_bias
         else:
@@ -243,7 +250,10 @@ class TriangleAttentionNode(nn.Module):
         mode = _EMPTY_ROW_MODES[self.empty_row_mode]
         policy = self.mha.chunk_policy
         chunked = policy is not None and policy.chunk_size < R and policy.should_chunk(x)
-        if not chunked and not self.transposed_bias and key_mask is None:
+        if not chunked and not self.transposed_bias and key_mask is not None:
+            return _host.node_masked(x, packed, lengths, key_mask, eps, ending, residual, residual and inplace_residual,
+                                     buffers, mode)
+        if not chunked and not self.transposed_bias:
             # common case: one native call for the whole node, intermediates in one workspace
             return _host.node(x, packed, lengths, eps, ending, residual, residual and inplace_residual, buffers, mode)
         if lengths is not None:

@@ -394,6 +394,17 @@ int b200ta_trimul_output_f32(const void* z, int64_t zs_b, int64_t zs_i, int64_t 
                              int add_residual, void* out, int64_t os_b, int64_t os_i, int64_t os_j, int B, int N,
                              void* stream);
 
+/*
+ * Row payloads of a float mask [B,R,S] (element strides s_*).  b200ta_mask_lengths: keys with mask > 0.5 per row, and with
+ * lengths_t also per row of the transposed mask (the left-aligned form; bionemo_ir/_torch/attention_backend/utils.py:201-391).
+ * b200ta_mask_bits: last valid key + 1 and one bit per key, [B][R][ceil(S/32)] words (the form of b200ta_attention_masked);
+ * valid means mask > 0.5, or with `additive` mask >= 0.
+ */
+int b200ta_mask_lengths(const float* mask, int64_t s_b, int64_t s_r, int64_t s_s, int32_t* lengths, int32_t* lengths_t,
+                        int B, int R, int S, void* stream);
+int b200ta_mask_bits(const float* mask, int64_t s_b, int64_t s_r, int64_t s_s, int additive, int32_t* lengths,
+                     uint32_t* bits, int B, int R, int S, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
