@@ -110,7 +110,9 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // At the top of a kernel: lets the stream's next kernel start its blocks as soon as there is room for them.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Returns once the kernels before this one in the stream are complete and their writes visible.  Every thread calls it
-// before its first access to global memory (reads of weights included: a fold may be the kernel before).
+// before its first access to global memory, except for reads of packed weights: the pack entry points end with an
+// ordinary launch, behind which no kernel can start before the weights are complete.  Loading them early takes the
+// 32-135 KB a block needs off the critical path of a small call.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- mbarrier --------------------------------------------------------------

@@ -72,6 +72,10 @@ __global__ void convert_kernel(const void* src, int dtype, size_t n, __nv_bfloat
 
 __global__ void set_flag_kernel(int* flags, int value) { flags[0] = value; }
 
+// Last launch of every pack: an ordinary one, so it starts when the folds before it are complete and visible, and a kernel
+// launched behind it may read the weights without waiting for its predecessors (see pdl_wait in common.cuh).
+__global__ void weights_complete_kernel() {}
+
 // The transition's LayerNorm vectors as floats (gamma | beta) and its "apply the LayerNorm" flag.
 void pack_transition_layernorm(const void* ln_w, const void* ln_b, int dtype, char* base, cudaStream_t s) {
   float* ln = reinterpret_cast<float*>(base + kTransLnOff);
@@ -114,6 +118,7 @@ int b200ta_pack_node_weights(const void* ln_w, const void* ln_b, const void* w_i
   convert_kernel<<<(kC * kC + 255) / 256, 256, 0, s>>>(w_out, weight_dtype, size_t(kC) * kC,
                                                        reinterpret_cast<__nv_bfloat16*>(base + kNodeWoOff), nullptr);
   convert_kernel<<<1, kC, 0, s>>>(b_out, weight_dtype, kC, nullptr, reinterpret_cast<float*>(base + kNodeBoOff));
+  weights_complete_kernel<<<1, 1, 0, s>>>();
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
 }
@@ -136,6 +141,7 @@ int b200ta_pack_pair_bias_weights(const void* ln_w, const void* ln_b, const void
       nullptr, kFirst, w_z, num_heads, nullptr, ln_w, ln_b, weight_dtype, kFirst, kFirst + num_heads, bias_scale,
       reinterpret_cast<__nv_bfloat16*>(base + kNodeWOff), reinterpret_cast<float2*>(base + kNodeScOff),
       reinterpret_cast<int*>(base + kNodeFlagsOff));
+  weights_complete_kernel<<<1, 1, 0, s>>>();
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
 }
@@ -177,6 +183,7 @@ int b200ta_pack_trimul_weights(const void* ln_in_w, const void* ln_in_b, const v
                                      wp + size_t(kTriInRows) * kC, sc + kTriInRows, flags);
   fold_rows_kernel<<<kC, kC, 0, s>>>(w_p_out, kC, nullptr, 0, b_p_out, ln_out_w, ln_out_b, weight_dtype, 0, 0, 1.f,
                                      wp + size_t(kTriInRows + kC) * kC, sc + kTriInRows + kC, flags);
+  weights_complete_kernel<<<1, 1, 0, s>>>();
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
 }
@@ -202,6 +209,7 @@ int b200ta_pack_transition_weights(const void* ln_w, const void* ln_b, const voi
   convert_kernel<<<(kC * kHidden + 255) / 256, 256, 0, s>>>(w2, weight_dtype, size_t(kC) * kHidden,
                                                             reinterpret_cast<__nv_bfloat16*>(base + kTransW2Off), nullptr);
   convert_kernel<<<1, kC, 0, s>>>(nullptr, weight_dtype, kC, nullptr, reinterpret_cast<float*>(base + kTransB2Off));
+  weights_complete_kernel<<<1, 1, 0, s>>>();
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
 }
@@ -227,6 +235,7 @@ int b200ta_pack_relu_transition_weights(const void* ln_w, const void* ln_b, cons
   convert_kernel<<<(kC * kHidden + 255) / 256, 256, 0, s>>>(w2, weight_dtype, size_t(kC) * kHidden,
                                                             reinterpret_cast<__nv_bfloat16*>(base + kTransW2Off), nullptr);
   convert_kernel<<<1, kC, 0, s>>>(b2, weight_dtype, kC, nullptr, reinterpret_cast<float*>(base + kTransB2Off));
+  weights_complete_kernel<<<1, 1, 0, s>>>();
   B200TA_CHECK_CUDA(cudaGetLastError());
   return B200TA_OK;
 }

@@ -74,7 +74,6 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
     fence_mbar_init();
   }
   if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 32);
-  pdl_wait();
   if (threadIdx.x < kMaxHeads / 2) {
     const float2 a = p.sc[kFirstRow + 2 * threadIdx.x], b = p.sc[kFirstRow + 2 * threadIdx.x + 1];
     reinterpret_cast<float4*>(gen + kSmSc)[threadIdx.x] = make_float4(a.x, b.x, a.y, b.y);
@@ -92,6 +91,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
       mbar_expect_tx(bars + W_FULL * 8, 2 * kMaxHeads * 128);
       for (int kh = 0; kh < 2; ++kh)
         tma_load_2d(base + kSmW + kh * kMaxHeads * 128, &tm_w, bars + W_FULL * 8, kh * 64, kFirstRow);
+      pdl_wait();
       int issued = 0;
       for (int i = 0; i < my_tiles; ++i) {
         const int tile = blockIdx.x + i * gridDim.x;
@@ -131,6 +131,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
       }
     }
   } else {
+    pdl_wait();
     const int wg = warp >> 2;               // this warpgroup takes the tiles i with i % 2 == wg
     const int m = (warp & 3) * 32 + lane;  // row of the tile == TMEM lane
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);

@@ -119,7 +119,6 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     fence_mbar_init();
   }
   if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
-  pdl_wait();
   // stage the per-column vectors
   if (MODE == kPrologue) {
     float4* dst = reinterpret_cast<float4*>(gen + L::kVec);
@@ -149,6 +148,7 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         for (int j = 0; j < L::kWRows / kBoxRows; ++j)
           tma_load_2d(base + L::kW + kh * L::kWHalf + j * kBoxRows * 128, &tm_w, bars + W_FULL * 8, kh * 64,
                       j * kBoxRows);
+      pdl_wait();
       int issued = 0;
       for (int i = 0; i < my_tiles; ++i) {
         const int tile = blockIdx.x + i * gridDim.x;
@@ -206,6 +206,7 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     }
   } else {
     // ------------------------------------------------------------- epilogue warps
+    pdl_wait();
     const int e = warp >> 2;               // which alternate column groups this warpgroup takes
     const int m = (warp & 3) * 32 + lane;  // row of the tile == TMEM lane
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);

@@ -193,7 +193,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     fence_mbar_init();
   }
   if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
-  pdl_wait();
   // stage the constants: LayerNorm gamma | beta, and for the ReLU form the two linears' biases
   if (threadIdx.x < 2 * kC) reinterpret_cast<float*>(gen + kSmLn)[threadIdx.x] = p.ln[threadIdx.x];
   if (kRelu) {
@@ -221,6 +220,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     // start) — the x ring's slots, which only feed the residual now, free too late for that.  It layer-normalises the
     // rows in place and, once GEMM1 has finished with the previous tile, copies them into tensor memory as the A
     // operand of GEMM1.  Only the copy sits on the tile switch's critical path.
+    pdl_wait();
     const int m = (warp & 3) * 32 + lane;
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
     const bool normalize = __ldg(p.flags) != 0;
@@ -280,7 +280,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         tma_load_2d(base + kSmX + xs * 32768 + 16384, &tm_x, bars + (X_FULL + xs) * 8, 64, tile * kTileM);
         return true;
       };
-      ok = load_x(0);
       for (int i = 0; ok && i < my_tiles; ++i) {
         for (int j = 0; j < kChunks; ++j, ++c) {
           const int st = c & 1;
@@ -292,6 +291,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
             const uint32_t dst = base + kSmW1 + st * 32768 + kh * 16384;
             tma_load_2d(dst, &tm_w1, f1, kh * 64, j * kChunk);                  // value rows
             tma_load_2d(dst + 8192, &tm_w1, f1, kh * 64, kHidden + j * kChunk);  // gate rows
+          }
+          if (c == 1) {  // the first two chunks do not depend on the kernels before this one
+            pdl_wait();
+            ok = load_x(0);
+            if (!ok) break;
           }
           // the next tile's rows, early enough for the SwiGLU warpgroups to normalise them during this tile
           if (j == 2 && i + 1 < my_tiles) {
@@ -389,6 +393,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   } else if (warp < 8) {
     // ------------------------------------------------------------------ SwiGLU / output warpgroups
     asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
+    pdl_wait();
     const int e = warp >> 2;               // chunk parity and output column half this warpgroup owns
     const int m = (warp & 3) * 32 + lane;  // row inside the tile == TMEM lane
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);

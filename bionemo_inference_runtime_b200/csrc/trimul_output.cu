@@ -86,7 +86,6 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     fence_mbar_init();
   }
   if (warp == 13) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
-  pdl_wait();
   // per-channel constants of the epilogue
   if (threadIdx.x < kC / 2) {
     const int c = 2 * threadIdx.x;
@@ -110,6 +109,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       for (int mat = 0; mat < 2; ++mat)
         for (int kh = 0; kh < 2; ++kh)
           tma_load_2d(base + kSmW + mat * 32768 + kh * 16384, &tm_w, bars + W_FULL * 8, kh * 64, kTriInRows + mat * kC);
+      pdl_wait();
       int issued = 0;
       for (int it = 0; it < my_tiles; ++it) {
         const int tile = blockIdx.x + it * gridDim.x;
@@ -163,6 +163,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     }
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ normaliser
+    pdl_wait();
     const int t = (warp - 8) * 32 + lane;
     bool ok = true;
     for (int it = 0; ok && it < my_tiles; ++it) {
@@ -255,6 +256,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps: one thread per position
+    pdl_wait();
     const int e = warp >> 2;
     const int m = (warp & 3) * 32 + lane;
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);

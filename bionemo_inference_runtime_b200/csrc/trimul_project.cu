@@ -81,7 +81,6 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     fence_mbar_init();
   }
   if (warp == 21) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
-  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -97,6 +96,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
       for (int kh = 0; kh < 2; ++kh)
         for (int j = 0; j < kTriInRows / 128; ++j)
           tma_load_2d(base + kSmW + kh * kWHalf + j * 128 * 128, &tm_w, bars + W_FULL * 8, kh * 64, j * 128);
+      pdl_wait();
       int issued = 0;
       for (int i = 0; i < my_tiles; ++i) {
         const int tile = blockIdx.x + i * gridDim.x;
@@ -146,6 +146,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     }
   } else if (warp >= 16 && warp < 20) {
     // ------------------------------------------------------------------ statistics: one thread per position
+    pdl_wait();
     const int m = (warp - 16) * 32 + lane;
     bool ok = true;
     for (int i = 0; ok && i < my_tiles; ++i) {
@@ -199,6 +200,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     }
   } else if (warp < 16) {
     // ------------------------------------------------------------------ epilogue warps: one thread per channel
+    pdl_wait();
     const int wg = warp >> 3;        // 0: a channels, 1: b channels
     const int half = (warp >> 2) & 1;  // which 64 positions of the tile
     const int ch = (warp & 3) * 32 + lane;  // channel inside the 128 == TMEM lane
