@@ -61,7 +61,7 @@ def _build_host(force: bool) -> None:
            "-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_host", "-D_GLIBCXX_USE_CXX11_ABI=1",
            *(f"-I{p}" for p in include_paths()), f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}",
            str(src), "-o", str(HOST), *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
-           "-ltorch_python", "-ldl"]
+           "-ltorch_python", f"-L{cuda / 'lib64'}", "-lcudart", "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)

@@ -7,7 +7,9 @@
 // layer call costs its launches and a few microseconds.
 //
 // The kernels' library is not linked: bind() takes its entry points from the file that the ctypes binding loaded.
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
@@ -125,17 +127,25 @@ Mask mask_of(const c10::optional<at::Tensor>& mask, int64_t B, int64_t N, bool s
 
 // ---- layers ------------------------------------------------------------------------------------------------------
 
-at::Tensor node(const at::Tensor& z, const at::Tensor& packed, const c10::optional<at::Tensor>& lengths, double eps,
-                bool ending, bool residual, bool inplace, const py::object& buffers, int empty_row_mode) {
+at::Tensor node_workspace(const py::object& buffers, const at::Tensor& z) {
+  return buffer(buffers, "tri_attn_workspace", {int64_t(lib.node_workspace_bytes(int(z.size(0)), int(z.size(1))))}, at::kByte, z);
+}
+
+void node_into(const at::Tensor& z, const at::Tensor& packed, const c10::optional<at::Tensor>& lengths, double eps, bool ending,
+               bool residual, const at::Tensor& out, const at::Tensor& ws, int empty_row_mode) {
   const Pair p = pair_of("z", z, ending);
-  const at::Tensor out = inplace ? z : new_bf16(z, z.sizes());
   const Pair o = pair_of("out", out, ending);
   const Lengths l = lengths_of(lengths, p.B, p.N);
-  const int64_t bytes = int64_t(lib.node_workspace_bytes(p.B, p.N));
-  const at::Tensor ws = buffer(buffers, "tri_attn_workspace", {bytes}, at::kByte, z);
   check(lib.node_forward(z.data_ptr(), p.sb, p.sr, p.ss, packed.data_ptr(), float(eps), l.ptr, l.sb, l.sr, empty_row_mode,
-                         residual, out.data_ptr(), o.sb, o.sr, o.ss, ws.data_ptr(), size_t(bytes), p.B, p.N, stream()),
+                         residual, out.data_ptr(), o.sb, o.sr, o.ss, ws.data_ptr(), size_t(ws.numel()), p.B, p.N, stream()),
         "b200ta_node_forward");
+}
+
+at::Tensor node(const at::Tensor& z, const at::Tensor& packed, const c10::optional<at::Tensor>& lengths, double eps,
+                bool ending, bool residual, bool inplace, const py::object& buffers, int empty_row_mode) {
+  pair_of("z", z, ending);
+  const at::Tensor out = inplace ? z : new_bf16(z, z.sizes());
+  node_into(z, packed, lengths, eps, ending, residual, out, node_workspace(buffers, z), empty_row_mode);
   return out;
 }
 
@@ -169,15 +179,12 @@ at::Tensor node_masked(const at::Tensor& z, const at::Tensor& packed, const at::
   return out;
 }
 
-at::Tensor trimul(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const at::Tensor& packed, double eps,
-                  bool incoming, const c10::optional<at::Tensor>& b_scale, const py::object& buffers, bool residual,
-                  bool mask_output, bool f32) {
+void trimul_into(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const at::Tensor& packed, double eps, bool incoming,
+                 const c10::optional<at::Tensor>& b_scale, const at::Tensor& ab, const at::Tensor& x, const at::Tensor& out,
+                 bool residual, bool mask_output) {
   const Pair p = pair_of("z", z, false);
-  const int64_t hidden = B200TA_C, pitch = (p.N + 15) / 16 * 16;
-  const at::Tensor ab = buffer(buffers, "trimul_ab", {p.B, 2 * hidden, p.N, pitch}, at::kBFloat16, z);
-  const at::Tensor x = buffer(buffers, "trimul_contracted", {p.B, hidden, p.N, pitch}, at::kBFloat16, z);
-  const at::Tensor out = f32 ? at::empty(z.sizes(), z.options().dtype(at::kFloat).memory_format(c10::MemoryFormat::Contiguous))
-                             : new_bf16(z, z.sizes());
+  const int64_t pitch = ab.size(3);
+  const bool f32 = out.scalar_type() == at::kFloat;
   void* s = stream();
   const Mask m = mask_of(mask, p.B, p.N, incoming);
   check(lib.trimul_project(z.data_ptr(), p.sb, incoming ? p.ss : p.sr, incoming ? p.sr : p.ss, m.ptr, m.sb, m.si, m.sj,
@@ -191,6 +198,25 @@ at::Tensor trimul(const at::Tensor& z, const c10::optional<at::Tensor>& mask, co
                                                           out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), p.B,
                                                           p.N, s),
         "b200ta_trimul_output");
+}
+
+struct TrimulBuffers {
+  at::Tensor ab, x;
+};
+TrimulBuffers trimul_buffers(const py::object& buffers, const at::Tensor& z) {
+  const int64_t B = z.size(0), N = z.size(1), pitch = (N + 15) / 16 * 16;
+  return {buffer(buffers, "trimul_ab", {B, 2 * B200TA_C, N, pitch}, at::kBFloat16, z),
+          buffer(buffers, "trimul_contracted", {B, B200TA_C, N, pitch}, at::kBFloat16, z)};
+}
+
+at::Tensor trimul(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const at::Tensor& packed, double eps,
+                  bool incoming, const c10::optional<at::Tensor>& b_scale, const py::object& buffers, bool residual,
+                  bool mask_output, bool f32) {
+  pair_of("z", z, false);
+  const TrimulBuffers t = trimul_buffers(buffers, z);
+  const at::Tensor out = at::empty(z.sizes(), z.options().dtype(f32 ? at::kFloat : at::kBFloat16)
+                                                  .memory_format(c10::MemoryFormat::Contiguous));
+  trimul_into(z, mask, packed, eps, incoming, b_scale, t.ab, t.x, out, residual, mask_output);
   return out;
 }
 
@@ -237,15 +263,26 @@ at::Tensor transition_gemms(const at::Tensor& x, const at::Tensor& w1, const at:
   return out;
 }
 
-// The single-track attention with pair bias.  `lengths` int32 [4 B]: the key count of a batch entry four times (the
-// attention kernel sees its 16 heads as four items of four).
-at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& z, const c10::optional<at::Tensor>& lengths,
-                               const at::Tensor& w_in, const at::Tensor& sc_in, const at::Tensor& w_o, const at::Tensor& sc_o,
-                               const at::Tensor& packed_z, bool normalize, double eps_s, double eps_z, double scale,
-                               const c10::optional<at::Tensor>& residual, const py::object& buffers) {
-  require_bf16("s", s16);
+// bias[b, h, q, k] of the single-track attention, [B, 16, N, ceil8(N)], kept in `buffers` under `key`.
+at::Tensor pair_bias(const at::Tensor& z, const at::Tensor& packed_z, double eps_z, const py::object& buffers,
+                     const char* key) {
   const Pair p = pair_of("z", z, false);
-  const int64_t B = p.B, N = p.N, c_s = s16.size(-1), heads = 16, dim = B200TA_HEAD_DIM, pad = (N + 7) / 8 * 8;
+  const int64_t heads = 16, pad = (p.N + 7) / 8 * 8;
+  const at::Tensor bias = buffer(buffers, key, {p.B, heads, p.N, pad}, at::kBFloat16, z);
+  check(lib.pair_bias(z.data_ptr(), p.sb, p.sr, p.ss, packed_z.data_ptr(), float(eps_z), bias.data_ptr(), bias.stride(0),
+                      bias.stride(1), bias.stride(2), 1, int(heads), p.B, p.N, p.N, int(pad), stream()),
+        "b200ta_pair_bias");
+  return bias;
+}
+
+// The single-track attention with the bias that pair_bias() wrote.  `lengths` int32 [4 B]: the key count of a batch entry four times (the
+// attention kernel sees its 16 heads as four items of four).
+at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& bias, const c10::optional<at::Tensor>& lengths,
+                               const at::Tensor& w_in, const at::Tensor& sc_in, const at::Tensor& w_o, const at::Tensor& sc_o,
+                               bool normalize, double eps_s, double scale, const c10::optional<at::Tensor>& residual,
+                               const py::object& buffers) {
+  require_bf16("s", s16);
+  const int64_t B = bias.size(0), N = bias.size(2), c_s = s16.size(-1), heads = 16, dim = B200TA_HEAD_DIM, pad = bias.size(3);
   if (!s16.is_contiguous() || s16.dim() != 3 || s16.size(0) != B || s16.size(1) != N)
     throw py::value_error("s must be a contiguous [B, N, c_s] tensor that matches z");
   void* st = stream();
@@ -258,10 +295,6 @@ at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& z, const
   check(lib.linear(s16.data_ptr(), N * c_s, c_s, 128, w_in.data_ptr(), sc_in.data_ptr(), normalize ? stats.data_ptr() : nullptr,
                    nullptr, 0, planes.data_ptr(), 0, planes.stride(0), 0, int(B), int(N), int(c_s), int(4 * heads * dim), st),
         "b200ta_linear");
-  const at::Tensor bias = buffer(buffers, "pw_pair_bias", {B, heads, N, pad}, at::kBFloat16, s16);
-  check(lib.pair_bias(z.data_ptr(), p.sb, p.sr, p.ss, packed_z.data_ptr(), float(eps_z), bias.data_ptr(), bias.stride(0),
-                      bias.stride(1), bias.stride(2), 1, int(heads), int(B), int(N), int(N), int(pad), st),
-        "b200ta_pair_bias");
   const at::Tensor attn = buffer(buffers, "pw_attn_output", {4 * B, 1, N, B200TA_C}, at::kBFloat16, s16);
   const Lengths l = lengths_of(lengths, 4 * B, 1);
   char* q = static_cast<char*>(planes.data_ptr());
@@ -277,6 +310,149 @@ at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& z, const
         "b200ta_linear");
   return out;
 }
+
+// ---- a second stream for the single track -------------------------------------------------------------------------
+
+// In a block the single track needs the pair tensor's bias, but nothing of the next block's pair track needs the single
+// track: a stack enqueues it on a stream of its own.  Its kernels have one row per token (a few to 144 blocks, 2-13 us
+// each, bound by latency), and run beside the pair track's instead of between them.
+// The stream is of high priority, so that the few blocks start at the next kernel boundary of the pair track.
+class SideTrack {
+ public:
+  SideTrack() : side_(c10::cuda::getStreamFromPool(/*isHighPriority=*/true)), main_(c10::cuda::getCurrentCUDAStream()) {
+    for (cudaEvent_t* e : {&ready_, &done_[0], &done_[1]}) cuda(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
+  SideTrack(const SideTrack&) = delete;
+  ~SideTrack() {
+    for (cudaEvent_t e : {ready_, done_[0], done_[1]}) cudaEventDestroy(e);
+  }
+  // The side stream continues from what the main stream has been given so far.
+  void fork() {
+    cuda(cudaEventRecord(ready_, main_.stream()));
+    cuda(cudaStreamWaitEvent(side_.stream(), ready_, 0));
+  }
+  void enter() { c10::cuda::setCurrentCUDAStream(side_); }
+  void leave() { c10::cuda::setCurrentCUDAStream(main_); }
+  // `slot` (0 or 1): what the side stream has been given so far is the last use of the slot's bias buffer ...
+  void done(int slot) { cuda(cudaEventRecord(done_[slot & 1], side_.stream())); }
+  // ... which the main stream may overwrite after this.
+  void wait(int slot) { cuda(cudaStreamWaitEvent(main_.stream(), done_[slot & 1], 0)); }
+  // `result` was allocated on the side stream and goes to a user of the main stream.
+  void hand_over(const at::Tensor& result) {
+    c10::cuda::CUDACachingAllocator::recordStream(result.storage().data_ptr(), main_);
+  }
+
+ private:
+  static void cuda(cudaError_t e) {
+    if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA: ") + cudaGetErrorString(e));
+  }
+  c10::cuda::CUDAStream side_, main_;
+  cudaEvent_t ready_ = nullptr, done_[2] = {nullptr, nullptr};
+};
+
+// ---- a whole stack ---------------------------------------------------------------------------------------------------
+
+// The blocks of a pairformer stack with their packed weights, enqueued by one call: the Python of seven layers per block
+// took some 100 us of host time, as much as a block's kernels need at 120 tokens.  The pair tensor alternates between two
+// buffers (the attention nodes and the transition work in place); the single track runs on the side stream.
+class Stack {
+ public:
+  struct Weights {
+    at::Tensor packed;
+    double eps;
+  };
+  struct Node {
+    at::Tensor packed;
+    double eps;
+    int empty_row_mode;
+  };
+  struct Single {
+    at::Tensor w_in, sc_in, w_o, sc_o, packed_z, w1, sc1, w2, sc2;
+    bool norm, norm_t;
+    double eps, eps_z, scale, eps_t;
+  };
+  void add(const at::Tensor& tri_out, double eps_out, const at::Tensor& tri_in, double eps_in, const at::Tensor& start,
+           double eps_start, int mode_start, const at::Tensor& end, double eps_end, int mode_end, const at::Tensor& transition,
+           double eps_transition) {
+    blocks_.push_back({{tri_out, eps_out}, {tri_in, eps_in}, {start, eps_start, mode_start}, {end, eps_end, mode_end},
+                       {transition, eps_transition}});
+  }
+  void add_single(const at::Tensor& w_in, const at::Tensor& sc_in, const at::Tensor& w_o, const at::Tensor& sc_o,
+                  const at::Tensor& packed_z, bool norm, double eps, double eps_z, double scale, const at::Tensor& w1,
+                  const at::Tensor& sc1, const at::Tensor& w2, const at::Tensor& sc2, bool norm_t, double eps_t) {
+    singles_.push_back({w_in, sc_in, w_o, sc_o, packed_z, w1, sc1, w2, sc2, norm, norm_t, eps, eps_z, scale, eps_t});
+  }
+
+  // z bf16 [B, N, N, 128] (left as it is), mask fp32 [B, N, N] or None, row lengths of the mask and of its transpose.
+  at::Tensor run_pair(const at::Tensor& z, const c10::optional<at::Tensor>& mask, const c10::optional<at::Tensor>& lengths,
+                      const c10::optional<at::Tensor>& lengths_t, bool mask_output, const py::object& buffers) {
+    return run(c10::nullopt, z, mask, lengths, lengths_t, mask_output, c10::nullopt, buffers, nullptr).second;
+  }
+  std::pair<at::Tensor, at::Tensor> run_both(const at::Tensor& s, const at::Tensor& z, const c10::optional<at::Tensor>& mask,
+                                             const c10::optional<at::Tensor>& lengths,
+                                             const c10::optional<at::Tensor>& lengths_t, bool mask_output,
+                                             const at::Tensor& key_counts, const py::object& buffers, SideTrack& track) {
+    return run(s, z, mask, lengths, lengths_t, mask_output, key_counts, buffers, &track);
+  }
+
+ private:
+  struct Block {
+    Weights tri_out, tri_in;
+    Node start, end;
+    Weights transition;
+  };
+  std::pair<at::Tensor, at::Tensor> run(c10::optional<at::Tensor> s, at::Tensor z, const c10::optional<at::Tensor>& mask,
+                                        const c10::optional<at::Tensor>& lengths, const c10::optional<at::Tensor>& lengths_t,
+                                        bool mask_output, const c10::optional<at::Tensor>& key_counts,
+                                        const py::object& buffers, SideTrack* track) {
+    pair_of("z", z, false);
+    const at::Tensor ws = node_workspace(buffers, z);
+    const TrimulBuffers t = trimul_buffers(buffers, z);
+    const at::Tensor a = new_bf16(z, z.sizes()), out = new_bf16(z, z.sizes());
+    const py::object none = py::none();
+    at::Tensor s16;
+    if (s) {
+      s16 = *s;
+      const int64_t B = z.size(0), N = z.size(1);
+      // used on the side stream, but allocated on the caller's, which has joined it when they are freed
+      buffer(buffers, "pw_qkvg", {4, B, 16, N, B200TA_HEAD_DIM}, at::kBFloat16, z);
+      buffer(buffers, "pw_attn_output", {4 * B, 1, N, B200TA_C}, at::kBFloat16, z);
+    }
+    for (size_t i = 0; i < blocks_.size(); ++i) {
+      const Block& b = blocks_[i];
+      trimul_into(z, mask, b.tri_out.packed, b.tri_out.eps, false, c10::nullopt, t.ab, t.x, a, true, mask_output);
+      trimul_into(a, mask, b.tri_in.packed, b.tri_in.eps, true, c10::nullopt, t.ab, t.x, out, true, mask_output);
+      z = out;
+      node_into(z, b.start.packed, lengths, b.start.eps, false, true, z, ws, b.start.empty_row_mode);
+      node_into(z, b.end.packed, lengths_t, b.end.eps, true, true, z, ws, b.end.empty_row_mode);
+      transition(z, b.transition.packed, c10::nullopt, b.transition.eps, true, true, false);
+      if (!s) continue;
+      const Single& w = singles_[i];
+      if (i >= 2) track->wait(int(i));
+      const at::Tensor bias = pair_bias(z, w.packed_z, w.eps_z, buffers, (i & 1) ? "pw_pair_bias_1" : "pw_pair_bias_0");
+      track->fork();
+      track->enter();
+      try {
+        s16 = pair_bias_attention(s16, bias, key_counts, w.w_in, w.sc_in, w.w_o, w.sc_o, w.norm, w.eps, w.scale, s16, buffers);
+        transition_gemms(s16, w.w1, w.sc1, w.w2, w.sc2, w.norm_t, w.eps_t, true, true);
+        track->done(int(i));
+      } catch (...) {
+        track->leave();
+        throw;
+      }
+      track->leave();
+    }
+    if (s) {
+      track->wait(int(blocks_.size()) - 1);
+      track->hand_over(s16);
+    }
+    return {s16, z};
+  }
+  std::vector<Block> blocks_;
+  std::vector<Single> singles_;
+};
+
+int64_t current_stream() { return reinterpret_cast<int64_t>(stream()); }
 
 // ---- masks -----------------------------------------------------------------------------------------------------------
 
@@ -304,11 +480,31 @@ std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additiv
 
 // ---- weight state --------------------------------------------------------------------------------------------------
 
-void add_parameters(PyObject* module, std::string& out) {
+// With `strict` the modules themselves belong to the state as well, and false means that one of them has a forward hook.
+bool add_parameters(PyObject* module, std::string& out, bool strict) {
   static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
   static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
   PyObject** dict = _PyObject_GetDictPtr(module);
-  if (dict == nullptr || *dict == nullptr) return;
+  if (dict == nullptr || *dict == nullptr) return true;
+  if (strict) {
+    static PyObject* const k_hooks = PyUnicode_InternFromString("_forward_hooks");
+    static PyObject* const k_pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks");
+    for (PyObject* k : {k_hooks, k_pre_hooks})
+      if (PyObject* hooks = PyDict_GetItem(*dict, k); hooks != nullptr && PyDict_Check(hooks) && PyDict_Size(hooks) > 0) return false;
+    // the module's attributes by identity (flags, eps, policies, ...), without the caches of its packed weights
+    static PyObject* const k_caches[] = {
+        PyUnicode_InternFromString("_pack"), PyUnicode_InternFromString("_pack_state"), PyUnicode_InternFromString("_folded"),
+        PyUnicode_InternFromString("_folded_state"), PyUnicode_InternFromString("_zero_bias")};
+    uint64_t mix = reinterpret_cast<uint64_t>(module);
+    PyObject *key, *value;
+    Py_ssize_t pos = 0;
+    while (PyDict_Next(*dict, &pos, &key, &value)) {
+      bool cache = false;
+      for (PyObject* k : k_caches) cache = cache || k == key;
+      if (!cache) mix = (mix ^ reinterpret_cast<uint64_t>(value)) * 0x9E3779B97F4A7C15ull, mix ^= mix >> 29;
+    }
+    out.append(reinterpret_cast<const char*>(&mix), sizeof(mix));
+  }
   PyObject *key, *value;
   Py_ssize_t pos = 0;
   if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
@@ -324,14 +520,23 @@ void add_parameters(PyObject* module, std::string& out) {
   pos = 0;
   if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
     while (PyDict_Next(modules, &pos, &key, &value))
-      if (value != Py_None) add_parameters(value, out);
+      if (value != Py_None && !add_parameters(value, out, strict)) return false;
+  return true;
 }
 
 // Address, in-place write count and device of every parameter under the modules: changes when a weight is loaded,
 // edited or replaced.
 py::bytes weight_state(const py::args& modules) {
   std::string out;
-  for (const py::handle& m : modules) add_parameters(m.ptr(), out);
+  for (const py::handle& m : modules) add_parameters(m.ptr(), out, false);
+  return py::bytes(out);
+}
+
+// The same with the identity of every module under `module` and of its attributes (a hash of the addresses); None if one
+// of the modules has a forward hook.
+py::object stack_state(const py::handle& module) {
+  std::string out;
+  if (!add_parameters(module.ptr(), out, true)) return py::none();
   return py::bytes(out);
 }
 
@@ -345,7 +550,24 @@ PYBIND11_MODULE(_host, m) {
   m.def("trimul", &trimul);
   m.def("transition", &transition);
   m.def("transition_gemms", &transition_gemms);
+  m.def("pair_bias", &pair_bias);
   m.def("pair_bias_attention", &pair_bias_attention);
+  m.def("current_stream", &current_stream);
+  py::class_<SideTrack>(m, "SideTrack")
+      .def(py::init<>())
+      .def("fork", &SideTrack::fork)
+      .def("enter", &SideTrack::enter)
+      .def("leave", &SideTrack::leave)
+      .def("done", &SideTrack::done)
+      .def("wait", &SideTrack::wait)
+      .def("hand_over", &SideTrack::hand_over);
+  py::class_<Stack>(m, "Stack")
+      .def(py::init<>())
+      .def("add", &Stack::add)
+      .def("add_single", &Stack::add_single)
+      .def("run_pair", &Stack::run_pair)
+      .def("run_both", &Stack::run_both);
+  m.def("stack_state", &stack_state);
   m.def("mask_lengths", &mask_lengths);
   m.def("mask_bits", &mask_bits);
   m.def("weight_state", &weight_state);

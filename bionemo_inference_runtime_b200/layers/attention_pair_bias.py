@@ -215,8 +215,9 @@ class AttentionPairBias(nn.Module):
         norm = self._norm_of_s()
         if z.dtype != torch.bfloat16:
             z = z.to(torch.bfloat16)
+        bias = _host.pair_bias(z, w["packed_z"], self.eps, buffers, "pw_pair_bias")
         res16 = None if residual is None else residual.to(torch.bfloat16).contiguous()
-        out = _host.pair_bias_attention(s16, z, _key_counts, w["w_in"], w["sc_in"], w["w_o"], w["sc_o"], w["packed_z"],
-                                        norm is not None, self.eps if norm is None else norm.eps, self.eps,
+        out = _host.pair_bias_attention(s16, bias, _key_counts, w["w_in"], w["sc_in"], w["w_o"], w["sc_o"],
+                                        norm is not None, self.eps if norm is None else norm.eps,
                                         1.0 / math.sqrt(self.head_dim), res16, buffers)
         return out if out.dtype == out_dtype else out.to(out_dtype)

@@ -20,7 +20,7 @@ import torch
 import torch.nn as nn
 
 from .. import _host
-from .attention_backend import (AttentionMetadata, PrecomputedPairMasks, precompute_pair_masks,
+from .attention_backend import (AttentionMetadata, PrecomputedPairMasks, mask_to_lengths, precompute_pair_masks,
                                 precompute_single_masks)
 from .attention_pair_bias import AttentionPairBias
 from .auto_chunk import CHUNK_REGISTRY, PAIR_TRANSITION
@@ -28,7 +28,91 @@ from .buffers import PreallocatedBuffers
 from .transition import Transition
 from .triangle_multiplication import (TriangleMultiplicationMetadata, TriangleMultiplicationNode,
                                       TriangleMultiplicationNodeType, precompute_trimul_metadata)
-from .triangle_nodes import TriangleAttentionEndingNode, TriangleAttentionStartingNode
+from .triangle_nodes import _EMPTY_ROW_MODES, TriangleAttentionEndingNode, TriangleAttentionStartingNode
+
+# caller's stream -> the stream and events of the single track beside it; taken out while a call uses it
+_side_tracks: dict[int, "_host.SideTrack"] = {}
+
+
+class _NativeStack:
+    """The packed weights of a stack in the form of ``_host.Stack``, valid for one state of its modules; not copied or
+    pickled with the module."""
+
+    def __init__(self, state: bytes, stack, chunk_policies):
+        self.state, self.stack, self.chunk_policies = state, stack, chunk_policies
+
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
+def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
+    """The native form of ``module.layers`` for this call, or None when a layer has to be called itself: it is hooked or
+    of another class, its options need the general path, or its rows are chunked at this size."""
+    state = None if nn.modules.module._has_any_global_hook() else _host.stack_state(module.layers)
+    held = module.__dict__.get("_native")
+    if state is None or (held is not None and held.state == state):
+        native = held if state is not None else None
+    elif torch.cuda.is_current_stream_capturing():
+        return None  # folding weights now would only fill them at replay
+    else:
+        stack = _build_native_stack(module.layers, z.device)
+        policies = {} if stack is None else {
+            id(p): p for layer in module.layers
+            for p in (layer.tri_attn_start.mha.chunk_policy, layer.tri_attn_end.mha.chunk_policy) if p is not None}
+        # a stack that has no native form is remembered as well
+        native = module._native = _NativeStack(state, stack, list(policies.values()))
+    if native is None or native.stack is None:
+        return None
+    chunked = any(p.chunk_size < z.shape[1] and p.should_chunk(z) for p in native.chunk_policies)
+    return None if chunked else native
+
+
+def _build_native_stack(layers, device):
+    bf16 = torch.bfloat16
+    stack = _host.Stack()
+    for layer in layers:
+        if type(layer) not in (PairformerLayerV1, PairformerLayerV2, PairformerNoSeqLayer) or layer.dtype != bf16:
+            return None
+        tri, nodes, trans = (layer.tri_mul_out, layer.tri_mul_in), (layer.tri_attn_start, layer.tri_attn_end), layer.transition_z
+        if (any(type(t) is not TriangleMultiplicationNode or t.mean_normalization for t in tri)
+                or [int(t.multiplication_type) for t in tri] != [0, 1]
+                or [type(n) for n in nodes] != [TriangleAttentionStartingNode, TriangleAttentionEndingNode]
+                or [int(n.node_type) for n in nodes] != [0, 1]
+                or any(n.dtype != bf16 or n.transposed_bias or not n.pair_mask_left_aligned for n in nodes)
+                or type(trans) is not Transition or trans.dtype != bf16 or not trans._fused):
+            return None
+        args = []
+        for t in tri:
+            args += [t._packed(device), t.eps]
+        for n in nodes:
+            args += [n._packed(device), n.layer_norm.eps, _EMPTY_ROW_MODES[n.empty_row_mode]]
+        stack.add(*args, trans._packed(device), trans._norm_eps())
+        if layer.no_update_s:
+            continue
+        attn, trans = layer.attention, layer.transition_s
+        if (type(attn) is not AttentionPairBias or type(trans) is not Transition or trans.dtype != bf16 or trans._fused
+                or (isinstance(layer, PairformerLayerV2) and (not layer._pre_norm_folded or layer.post_norm_s is not None))):
+            return None
+        w, t, norm = attn._weights(device), trans._packed(device), attn._norm_of_s()
+        stack.add_single(w["w_in"], w["sc_in"], w["w_o"], w["sc_o"], w["packed_z"], norm is not None,
+                         attn.eps if norm is None else norm.eps, attn.eps, attn.head_dim**-0.5, t["w1"], t["sc1"], t["w2"],
+                         t["sc2"], trans.norm is not None, trans._norm_eps())
+    return stack
+
+
+def _native_pair_inputs(first, z: torch.Tensor, pair_mask: torch.Tensor, precomputed: PrecomputedPairMasks,
+                        metadata: TriangleMultiplicationMetadata) -> tuple:
+    """The pair track's inputs as the native stack takes them; the same conversions and rules as in the layers."""
+    if tuple(pair_mask.shape) != tuple(z.shape[:3]):
+        raise ValueError(f"mask must have shape {tuple(z.shape[:3])}, got {tuple(pair_mask.shape)}")
+    z = z.to(torch.bfloat16)
+    lengths = [m if m.dtype == torch.int32 else mask_to_lengths(m, z.shape[0], z.shape[1]).contiguous()
+               for m in (precomputed.mask_bias, precomputed.mask_bias_transposed)]
+    mask_output = metadata.outgoing_actual_seqlen is not None and first.tri_mul_out.can_fuse_residual(z)
+    return z, pair_mask.to(torch.float32), *lengths, mask_output
 
 
 class PairformerLayerV1(nn.Module):
@@ -109,14 +193,20 @@ class PairformerLayerV1(nn.Module):
         z = self._transform_z(z, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed_masks,
                               buffers=buffers, inplace_safe=bool(kwargs.get("inplace_safe", False)))
         if not self.no_update_s:
-            mask_bias = getattr(precomputed_single_masks, "mask_bias", None)
-            s_dtype = s.dtype
-            # attention(..., residual=s) is the reference's ``s + attention(s, z, mask)`` with the add in the
-            # output-projection kernel; the result is a fresh tensor, so the transition updates it in place
-            s = self.attention(s, z, mask, attn_metadata=(attn_metadatas or {}).get("pairwise_attn"),
-                               mask_bias=mask_bias, buffers=buffers, residual=s, _key_counts=kwargs.get("_key_counts"))
-            s = self.transition_s(s.to(torch.bfloat16), residual=True, inplace=True).to(s_dtype)
+            s = self._transform_s(s, z, mask, attn_metadatas, getattr(precomputed_single_masks, "mask_bias", None), buffers,
+                                  _key_counts=kwargs.get("_key_counts"))
         return s, z
+
+    def _transform_s(self, s: torch.Tensor, z: torch.Tensor | None, mask: torch.Tensor,
+                     attn_metadatas: dict[str, AttentionMetadata] | None, mask_bias: torch.Tensor | None,
+                     buffers: PreallocatedBuffers | None, **shared) -> torch.Tensor:
+        """The block's single track on the updated pair tensor (``shared``: what a stack has computed already)."""
+        s_dtype = s.dtype
+        # attention(..., residual=s) is the reference's ``s + attention(s, z, mask)`` with the add in the
+        # output-projection kernel; the result is a fresh tensor, so the transition updates it in place
+        s = self.attention(s, z, mask, attn_metadata=(attn_metadatas or {}).get("pairwise_attn"),
+                           mask_bias=mask_bias, buffers=buffers, residual=s, **shared)
+        return self.transition_s(s.to(torch.bfloat16), residual=True, inplace=True).to(s_dtype)
 
 
 class PairformerLayerV2(PairformerLayerV1):
@@ -134,23 +224,18 @@ class PairformerLayerV2(PairformerLayerV1):
         if self._pre_norm_folded:
             self.attention.set_input_norm(self.pre_norm_s)
 
-    def forward(self, s: torch.Tensor, z: torch.Tensor, mask: torch.Tensor, pair_mask: torch.Tensor,
-                trimul_metadata: TriangleMultiplicationMetadata,
-                attn_metadatas: dict[str, AttentionMetadata] | None = None,
-                precomputed_masks: PrecomputedPairMasks | None = None, precomputed_single_masks=None,
-                buffers: PreallocatedBuffers | None = None, **kwargs) -> tuple[torch.Tensor, torch.Tensor]:
-        z = self._transform_z(z, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed_masks,
-                              buffers=buffers, inplace_safe=bool(kwargs.get("inplace_safe", False)))
+    def _transform_s(self, s: torch.Tensor, z: torch.Tensor | None, mask: torch.Tensor,
+                     attn_metadatas: dict[str, AttentionMetadata] | None, mask_bias: torch.Tensor | None,
+                     buffers: PreallocatedBuffers | None, **shared) -> torch.Tensor:
         s_dtype = s.dtype
         s16 = s.to(torch.bfloat16)
         s_in = s16 if self._pre_norm_folded else self.pre_norm_s(s16)
         s16 = self.attention(s_in, z, mask, attn_metadata=(attn_metadatas or {}).get("pairwise_attn"),
-                             mask_bias=getattr(precomputed_single_masks, "mask_bias", None), buffers=buffers,
-                             residual=s16, _key_counts=kwargs.get("_key_counts"))
+                             mask_bias=mask_bias, buffers=buffers, residual=s16, **shared)
         s16 = self.transition_s(s16, residual=True, inplace=True)
         if self.post_norm_s is not None:
             s16 = self.post_norm_s(s16)
-        return s16.to(s_dtype), z
+        return s16.to(s_dtype)
 
 
 class PairformerNoSeqLayer(PairformerLayerV1):
@@ -251,6 +336,17 @@ class PairformerModule(nn.Module):
         if precomputed_single is not None:
             kwargs["_key_counts"] = first.attention.key_counts(mask, precomputed_single.mask_bias, s.shape[0], s.shape[1],
                                                                s.device)
+            native = None if attn_metadatas or first.no_update_s else _native_stack(self, z)
+            if native is not None:
+                stream = _host.current_stream()
+                track = _side_tracks.pop(stream, None) or _host.SideTrack()
+                s_out, z = native.stack.run_both(s.to(torch.bfloat16).contiguous(),
+                                                 *_native_pair_inputs(first, z, pair_mask, precomputed, trimul_metadata),
+                                                 kwargs["_key_counts"], buffers, track)
+                while len(_side_tracks) >= 8:  # programs use a few streams; a bounded number is kept
+                    _side_tracks.pop(next(iter(_side_tracks)), None)
+                _side_tracks[stream] = track
+                return s_out.to(s.dtype), z
         for layer in self.layers:
             s, z = layer(s, z, mask, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed,
                          precomputed_single_masks=precomputed_single, buffers=buffers, **kwargs)
@@ -282,6 +378,9 @@ class PairformerNoSeqModule(nn.Module):
         trimul_metadata = precompute_trimul_metadata(
             z, precomputed.mask_bias if int_lengths else None,
             precomputed.mask_bias_transposed if int_lengths else None, enabled=self.pair_mask_left_aligned)
+        native = _native_stack(self, z)
+        if native is not None:
+            return native.stack.run_pair(*_native_pair_inputs(first, z, pair_mask, precomputed, trimul_metadata), buffers)
         for layer in self.layers:
             z = layer(z, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed, buffers=buffers,
                       **kwargs)

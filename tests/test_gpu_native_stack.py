@@ -1,0 +1,63 @@
+"""The native form of a stack (one call, single track on a second stream) against the same layers called one by one."""
+
+import pytest
+import torch
+
+import bionemo_inference_runtime_b200 as b200
+from bionemo_inference_runtime_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _randomise(module):
+    g = torch.Generator(device=DEV).manual_seed(1)
+    for name, p in module.named_parameters():
+        p.data.copy_(torch.randn(p.shape, generator=g, device=DEV) * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1)
+                     + (1.0 if p.dim() == 1 and not name.endswith("bias") else 0.0))
+    return module
+
+
+@pytest.mark.parametrize("version,f32,backend", [("v1", False, "Heuristic"), ("v1", True, "VANILLA"), ("v2", False, "Heuristic")])
+@pytest.mark.parametrize("B,N", [(1, 33), (3, 72)])
+def test_native_stack_equals_the_layers(version, f32, backend, B, N):
+    stack = _randomise(b200.PairformerModule(num_blocks=3, dtype=torch.bfloat16, version=version, trimul_high_precision=f32,
+                                             triangle_attn_backend=backend, attention_initial_norm=version == "v1").to(DEV))
+    g = torch.Generator(device=DEV).manual_seed(2)
+    s = torch.randn(B, N, 384, generator=g, device=DEV).bfloat16()
+    z = torch.randn(B, N, N, 128, generator=g, device=DEV).bfloat16()
+    mask = (torch.arange(N, device=DEV)[None] < torch.tensor([N, N - 5, 7][:B], device=DEV)[:, None]).float()
+    pair = mask[:, :, None] * mask[:, None, :]
+    z0 = z.clone()
+    got = stack(s, z, mask, pair)
+    assert stack._native.stack is not None and torch.equal(z, z0)
+    again = stack(s, z, mask, pair)
+    handle = stack.layers[1].register_forward_hook(lambda *args: None)  # a hooked layer is called itself
+    want = stack(s, z, mask, pair)
+    handle.remove()
+    for a, b, c in zip(got, again, want):
+        assert torch.equal(a, b) and torch.equal(a, c)
+    # an edited option takes effect: the ending node's bias written transposed has no native form
+    stack.layers[0].tri_attn_end.transposed_bias = True
+    stack(s, z, mask, pair)
+    assert stack._native.stack is None
+    stack.layers[0].tri_attn_end.transposed_bias = False
+    # ... and so does an edited weight
+    with torch.no_grad():
+        stack.layers[2].transition_s.fc3.weight.mul_(2.0)
+    assert not torch.equal(stack(s, z, mask, pair)[0], got[0])
+    assert _lib.device_status() == 0
+
+
+def test_masks_in_one_launch_equal_the_torch_operations():
+    g = torch.Generator(device=DEV).manual_seed(3)
+    from bionemo_inference_runtime_b200 import _host, ops
+
+    for B, N in ((1, 1), (2, 31), (1, 96), (3, 130)):
+        mask = (torch.rand(B, N, N, generator=g, device=DEV) > 0.4).float()
+        rows, columns = _host.mask_lengths(mask)
+        assert torch.equal(rows, (mask > 0.5).sum(-1).int()) and torch.equal(columns, (mask > 0.5).sum(-2).int())
+        for source, additive in ((mask.transpose(1, 2), False), ((mask - 1) * 1e9, True)):
+            valid = source >= 0 if additive else source > 0.5
+            for a, b in zip(_host.mask_bits(source, additive), ops.key_mask_bits(valid)):
+                assert torch.equal(a, b)
