@@ -232,6 +232,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t src,
                "r"(src), "r"(c0), "r"(c1)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(m), "r"(src),
+               "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, uint32_t src, int c0, int c1,
                                              int c2, int c3) {
   asm volatile(
@@ -523,6 +528,34 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z),
                "r"(v.w)
                : "memory");
+}
+
+// LayerNorm statistics {rstd, -mean * rstd} of a row of 128 bf16 channels in shared memory (two 64-channel halves of
+// 128-byte swizzled rows, 16 KiB apart).  One pass over the row in packed fp32 pairs: sums of (x - k) and (x - k)^2 with k
+// the row's first channel.  (k - mean)^2 is at most 127 variances, so the variance formula E[d^2] - E[d]^2 loses no more
+// than 1e-5 of it.
+__device__ __forceinline__ float2 row_stats_128(uint32_t tile, int row, float eps) {
+  const float k = bf16_lo(lds128(tile + sw128_offset(row, 0)).x);
+  const uint64_t nk2 = pack_f32x2(-k, -k);
+  uint64_t sa[4] = {0ull, 0ull, 0ull, 0ull}, sq[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll 8
+  for (int c = 0; c < 16; ++c) {
+    const uint4 x = lds128(tile + (c >> 3) * 16384 + sw128_offset(row, c & 7));
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint64_t d = add_f32x2(pack_f32x2(bf16_lo(w[e]), bf16_hi(w[e])), nk2);
+      sa[e] = add_f32x2(sa[e], d);
+      sq[e] = fma_f32x2(d, d, sq[e]);
+    }
+  }
+  float a0, a1, q0, q1;
+  unpack_f32x2(add_f32x2(add_f32x2(sa[0], sa[1]), add_f32x2(sa[2], sa[3])), a0, a1);
+  unpack_f32x2(add_f32x2(add_f32x2(sq[0], sq[1]), add_f32x2(sq[2], sq[3])), q0, q1);
+  const float md = (a0 + a1) * (1.f / 128);  // mean of x - k
+  const float var = fmaxf((q0 + q1) * (1.f / 128) - md * md, 0.f);
+  const float rstd = rsqrtf(var + eps);
+  return make_float2(rstd, -(md + k) * rstd);
 }
 
 #endif  // __CUDACC__

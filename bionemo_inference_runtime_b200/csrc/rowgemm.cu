@@ -11,8 +11,11 @@
 //              as sigmoid(g)) and 4 triangle-bias heads.
 //   kEpilogue: og tile -> og · W_oᵀ + b_o + residual.
 //
-// Warp roles (320 threads): warps 0-7 epilogue (TMEM lanes 32(w%4)..+31), warp 8 TMA producer, warp 9 MMA
-// issuer / TMEM owner.
+// Warp roles: warps 0-7 epilogue (TMEM lanes 32(w%4)..+31), warp 8 TMA producer, warp 9 MMA issuer / TMEM owner, and in
+// the prologue warps 10-13 LayerNorm statistics (one thread per row, a tile ahead of the epilogue).
+//
+// The prologue is bound by its writes (1032 of 1288 bytes per position).  Its epilogue warps used to compute the
+// statistics themselves, in both warpgroups: 15.9 thousand warp instructions a tile, a third of them for that.
 #include "common.cuh"
 #include "layout.h"
 
@@ -20,11 +23,12 @@ namespace b200ta {
 namespace {
 
 constexpr int kTileM = 128;
-constexpr int kThreads = 320;
 constexpr int kSlotCols = 256;  // TMEM columns per accumulator slot (2 slots)
 
 enum Mode { kPrologue = 0, kEpilogue = 1 };
 constexpr int kMaxPeers = 8;
+template <int MODE>
+constexpr int kThreads = MODE == kPrologue ? 448 : 320;
 
 struct RowGemmParams {
   int B, R, S, S_pad;
@@ -59,13 +63,15 @@ struct Smem {
   static constexpr int kVec = kRes + (MODE == kEpilogue ? 2 * 32768 : 0);
   // prologue: per column pair {rowsum0, rowsum1, const0, const1}; epilogue: b_o
   static constexpr int kVecBytes = MODE == kPrologue ? (kNodeRows / 2) * 16 : kC * 4;
-  static constexpr int kBars = kVec + kVecBytes;
+  // prologue: {rstd, -mean*rstd} of the rows, 4 slots (tile i uses slot i & 3)
+  static constexpr int kStats = kVec + kVecBytes;
+  static constexpr int kBars = kStats + (MODE == kPrologue ? 4 * 1024 : 0);
   static constexpr int kTotal = kBars + 128;
   static constexpr int kDynamic = kTotal + 1024;  // slack for manual 1024-byte alignment
 };
 
 // barrier slots inside the kBars block (8 bytes each)
-enum Bar { W_FULL = 0, A_FULL = 1, A_EMPTY = 3, ACC_FULL = 5, ACC_EMPTY = 7, NUM_BARS = 9 };
+enum Bar { W_FULL = 0, A_FULL = 1, A_EMPTY = 3, ACC_FULL = 5, ACC_EMPTY = 7, STATS = 9, NUM_BARS = 13 };
 
 __device__ __forceinline__ void stg128(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   *reinterpret_cast<uint4*>(p) = make_uint4(a, b, c, d);
@@ -89,7 +95,7 @@ __device__ __forceinline__ void store_row64(__nv_bfloat16* dst, const uint32_t (
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads<MODE>, 1)
 rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                const __grid_constant__ CUtensorMap tm_res, const RowGemmParams p) {
   using L = Smem<MODE>;
@@ -112,23 +118,25 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     mbar_init(bars + W_FULL * 8, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + (A_FULL + i) * 8, 1);
-      mbar_init(bars + (A_EMPTY + i) * 8, 9);  // 8 epilogue warps + the MMA commit
+      mbar_init(bars + (A_EMPTY + i) * 8, MODE == kPrologue ? 5 : 9);  // statistics (residual) readers + the MMA commit
       mbar_init(bars + (ACC_FULL + i) * 8, 1);
       mbar_init(bars + (ACC_EMPTY + i) * 8, 8);
     }
+    if (MODE == kPrologue)
+      for (int i = 0; i < 4; ++i) mbar_init(bars + (STATS + i) * 8, 4);
     fence_mbar_init();
   }
   if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   // stage the per-column vectors
   if (MODE == kPrologue) {
     float4* dst = reinterpret_cast<float4*>(gen + L::kVec);
-    for (int i = threadIdx.x; i < kNodeRows / 2; i += kThreads) {
+    for (int i = threadIdx.x; i < kNodeRows / 2; i += kThreads<MODE>) {
       const float2 a = p.sc[2 * i], b = p.sc[2 * i + 1];
       dst[i] = make_float4(a.x, b.x, a.y, b.y);
     }
   } else {
     float* dst = reinterpret_cast<float*>(gen + L::kVec);
-    for (int i = threadIdx.x; i < kC; i += kThreads) dst[i] = p.bo[i];
+    for (int i = threadIdx.x; i < kC; i += kThreads<MODE>) dst[i] = p.bo[i];
   }
   tc_fence_before();
   __syncthreads();
@@ -204,13 +212,31 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         umma_commit(bars + (A_EMPTY + stage) * 8);
       }
     }
+  } else if (warp >= 10) {
+    // ------------------------------------------------------------- LayerNorm statistics (prologue only)
+    pdl_wait();
+    const int m = (warp - 10) * 32 + lane;
+    const bool normalize = __ldg(p.flags) != 0;
+    for (int i = 0; i < my_tiles; ++i) {
+      const int stage = i & 1;
+      if (!mbar_wait(bars + (A_FULL + stage) * 8, (i >> 1) & 1, abort_flag)) break;
+      // Four slots: the epilogue of a tile reads its slot while the statistics of the next two tiles are written.  A
+      // slot is rewritten four tiles later, when that epilogue is long done (the MMAs of tile t + 2 wait for the
+      // accumulators of tile t, the loads of tile t + 4 for those MMAs).
+      reinterpret_cast<float2*>(gen + L::kStats + (i & 3) * 1024)[m] =
+          normalize ? row_stats_128(base + L::kA + stage * 32768, m, p.eps) : make_float2(1.f, 0.f);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bars + (STATS + (i & 3)) * 8);
+        mbar_arrive(bars + (A_EMPTY + stage) * 8);  // done reading the tile
+      }
+    }
   } else {
     // ------------------------------------------------------------- epilogue warps
     pdl_wait();
     const int e = warp >> 2;               // which alternate column groups this warpgroup takes
     const int m = (warp & 3) * 32 + lane;  // row of the tile == TMEM lane
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-    const bool normalize = MODE == kPrologue && __ldg(p.flags) != 0;
     int uc = 0;
     bool ok = true;
     for (int i = 0; ok && i < my_tiles; ++i) {
@@ -220,35 +246,15 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       const int r = br % p.R, b = br / p.R;
       const int stage = i & 1;
       const int s = st * kTileM + m;  // this thread's position along the sequence axis
-      ok = mbar_wait(bars + (A_FULL + stage) * 8, (i >> 1) & 1, abort_flag);
-      if (!ok) break;
       float rstd = 1.f, nmr = 0.f;
-      if (normalize) {
-        // LayerNorm statistics of row m from the swizzled smem copy of the z tile.
-        uint32_t v[64];
-        const uint32_t a0 = base + L::kA + stage * 32768;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          uint4 x = lds128(a0 + (c >> 3) * 16384 + sw128_offset(m, c & 7));
-          v[c * 4 + 0] = x.x, v[c * 4 + 1] = x.y, v[c * 4 + 2] = x.z, v[c * 4 + 3] = x.w;
-        }
-        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 64; ++j) sum4[j & 3] += bf16_lo(v[j]) + bf16_hi(v[j]);
-        const float mu = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) * (1.f / kC);
-        float var4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          const float d0 = bf16_lo(v[j]) - mu, d1 = bf16_hi(v[j]) - mu;
-          var4[j & 3] = fmaf(d0, d0, var4[j & 3]);
-          var4[j & 3] = fmaf(d1, d1, var4[j & 3]);
-        }
-        rstd = rsqrtf(((var4[0] + var4[1]) + (var4[2] + var4[3])) * (1.f / kC) + p.eps);
-        nmr = -mu * rstd;
-      }
       if (MODE == kPrologue) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bars + (A_EMPTY + stage) * 8);  // done reading the z tile
+        ok = mbar_wait(bars + (STATS + (i & 3)) * 8, (i >> 2) & 1, abort_flag);
+        if (!ok) break;
+        const float2 st = reinterpret_cast<const float2*>(gen + L::kStats + (i & 3) * 1024)[m];
+        rstd = st.x, nmr = st.y;
+      } else {
+        ok = mbar_wait(bars + (A_FULL + stage) * 8, (i >> 1) & 1, abort_flag);  // the residual tile
+        if (!ok) break;
       }
       const uint64_t rstd2 = pack_f32x2(rstd, rstd), nmr2 = pack_f32x2(nmr, nmr);
       for (int u = u_begin; ok && u < u_end; ++u, ++uc) {
@@ -437,7 +443,7 @@ int launch_epilogue(const void* og, int64_t gs_b, int64_t gs_r, int64_t gs_s, co
   p.status = st->status_dev;
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  return launch_kernel(st, kKernelEpilogue, rowgemm_kernel<kEpilogue>, dim3(grid), kThreads, Smem<kEpilogue>::kDynamic, stream,
+  return launch_kernel(st, kKernelEpilogue, rowgemm_kernel<kEpilogue>, dim3(grid), kThreads<kEpilogue>, Smem<kEpilogue>::kDynamic, stream,
                        tm_a, tm_w, tm_res, p);
 }
 
@@ -497,7 +503,7 @@ int b200ta_prologue(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_s, con
   p.status = st->status_dev;
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  return launch_kernel(st, kKernelPrologue, rowgemm_kernel<kPrologue>, dim3(grid), kThreads, Smem<kPrologue>::kDynamic, stream,
+  return launch_kernel(st, kKernelPrologue, rowgemm_kernel<kPrologue>, dim3(grid), kThreads<kPrologue>, Smem<kPrologue>::kDynamic, stream,
                        tm_a, tm_w, tm_a, p);
 }
 

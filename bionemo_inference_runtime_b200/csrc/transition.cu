@@ -88,29 +88,8 @@ __device__ __forceinline__ void prepare_row(uint32_t x0, int m, bool normalize, 
                                             uint32_t stage0) {
   float rstd = 1.f, nmr = 0.f;
   if (normalize) {
-    // One pass: sums of (x - k) and (x - k)^2 with k = the row's first channel (a shift keeps the variance
-    // formula E[d^2] - E[d]^2 free of cancellation when the row has a large common offset).
-    const float k = bf16_lo(lds128(x0 + sw128_offset(m, 0)).x);
-    const uint64_t nk2 = pack_f32x2(-k, -k);
-    uint64_t sa[4] = {0ull, 0ull, 0ull, 0ull}, sq[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll 8
-    for (int c = 0; c < 16; ++c) {
-      const uint4 x = lds128(x0 + (c >> 3) * 16384 + sw128_offset(m, c & 7));
-      const uint64_t d0 = add_f32x2(pack_f32x2(bf16_lo(x.x), bf16_hi(x.x)), nk2);
-      const uint64_t d1 = add_f32x2(pack_f32x2(bf16_lo(x.y), bf16_hi(x.y)), nk2);
-      const uint64_t d2 = add_f32x2(pack_f32x2(bf16_lo(x.z), bf16_hi(x.z)), nk2);
-      const uint64_t d3 = add_f32x2(pack_f32x2(bf16_lo(x.w), bf16_hi(x.w)), nk2);
-      sa[0] = add_f32x2(sa[0], d0), sa[1] = add_f32x2(sa[1], d1), sa[2] = add_f32x2(sa[2], d2), sa[3] = add_f32x2(sa[3], d3);
-      sq[0] = fma_f32x2(d0, d0, sq[0]), sq[1] = fma_f32x2(d1, d1, sq[1]);
-      sq[2] = fma_f32x2(d2, d2, sq[2]), sq[3] = fma_f32x2(d3, d3, sq[3]);
-    }
-    float a0, a1, q0, q1;
-    unpack_f32x2(add_f32x2(add_f32x2(sa[0], sa[1]), add_f32x2(sa[2], sa[3])), a0, a1);
-    unpack_f32x2(add_f32x2(add_f32x2(sq[0], sq[1]), add_f32x2(sq[2], sq[3])), q0, q1);
-    const float md = (a0 + a1) * (1.f / kC);  // mean of x - k
-    const float var = fmaxf((q0 + q1) * (1.f / kC) - md * md, 0.f);
-    rstd = rsqrtf(var + eps);
-    nmr = -(md + k) * rstd;
+    const float2 st = row_stats_128(x0, m, eps);
+    rstd = st.x, nmr = st.y;
   }
   const uint64_t rstd2 = pack_f32x2(rstd, rstd), nmr2 = pack_f32x2(nmr, nmr);
 #pragma unroll 4

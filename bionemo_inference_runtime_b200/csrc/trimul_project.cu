@@ -4,19 +4,27 @@
 // written channel-major, ab[b][ch][r][s], so that the contraction kernel finds the index it sums over (s)
 // contiguous.  The incoming node calls this with the pair strides swapped (rows r = pair columns).
 //
-// The GEMM is computed transposed, D[channel, position] = W'[channel, :] · x̂[position, :]ᵀ: the folded weight
-// rows are the A operand (M = 128 channels), the normalised tile of 128 positions the B operand (N = 128), so a
-// TMEM lane is a channel and every epilogue thread owns one channel of 128 consecutive positions - exactly one
-// contiguous 256-byte run of the channel-major output.  Per tile four such products: gate and value of the a
-// channels (warpgroup 0 finishes them) and of the b channels (warpgroup 1).
+// The GEMM is computed transposed, D[channel, position] = W'[channel, :] · z[position, :]ᵀ: a TMEM lane is a channel, so
+// that every epilogue thread owns one channel of consecutive positions - one contiguous run of the channel-major output.
+// The folded weight rows (four blocks of 128: gate and value of the a and of the b channels) stay in tensor memory as the
+// A operand for the whole kernel (256 columns), the raw tile of 128 positions is the B operand.
+//
+// Bound: the writes, 512 of 768 bytes per position (a plain fill of this memory reaches 3.95 TB/s).  The weights used to
+// be A operands in shared memory (128 KiB, read again for every tile) with four accumulators of 128 positions in all of
+// tensor memory: the MMAs of a tile waited for the epilogue of the one before, and with two 32 KiB stages left, so did
+// the loads (131 us at 768 tokens, 3.4 TB/s).  With the weights in tensor memory an MMA takes 36 instead of 69 clocks for
+// half the positions, so accumulators of 64 positions cost nothing, and two of them (a, b) are in turn filled and read;
+// shared memory is a ring of four tiles.  What took the time then was the load-store unit: a 32-byte store of 32 lanes to
+// 32 channels' runs occupies it for some 56 clocks.  Each warp now stages its 32 channels x 32 positions in shared memory
+// and hands them to a TMA store.
 //
 // LayerNorm is folded into the weights (rows centred, per-row sum kept; gamma, beta and the biases included): the
 // MMAs run on the raw tile as soon as it has landed, four statistics warps (one thread per position) compute mean
 // and rstd of every position meanwhile, and the epilogue applies rstd[pos]·(D − mean[pos]·rowsum[ch]) + const[ch].
 //
-// Warp roles (704 threads): warps 0-15 epilogue - warpgroup g finishes the a (g < 2) or b (g >= 2) channels for
-// the first (g even) or second (g odd) 64 positions of the tile -, warps 16-19 statistics, warp 20 TMA producer,
-// warp 21 MMA issuer / TMEM owner.
+// Warp roles (704 threads): warps 0-15 epilogue - warps 0-7 finish the a, 8-15 the b channels; of each eight, two warps
+// share a quarter of the channels, for 32 of the accumulator's 64 positions each -, warps 16-19 statistics, warp 20 TMA
+// producer, warp 21 MMA issuer / TMEM owner.
 #include "common.cuh"
 #include "layout.h"
 
@@ -25,15 +33,19 @@ namespace {
 
 constexpr int kThreads = 704;
 constexpr int kTileM = 128;                 // positions per tile
-constexpr int kSmW = 0;                     // folded rows: 2 halves (64 channels of K each) x 512 rows x 128 B
-constexpr int kWHalf = kTriInRows * 128;    // 64 KiB
-constexpr int kSmZ = kSmW + 2 * kWHalf;     // 2 stages x 32 KiB
-constexpr int kSmStats = kSmZ + 2 * 32768;  // 4 slots (tile i uses slot i & 3) x 3 x 128 floats: rstd, -mean*rstd, mask/2
-constexpr int kStatsSlot = 3 * 512;
-constexpr int kSmBars = kSmStats + 4 * kStatsSlot;
-enum Bar { W_FULL = 0, Z_FULL = 1, STATS_READY = 3, Z_EMPTY = 7, ACC_FULL = 9, ACC_EMPTY = 11, NUM_BARS = 13 };
+constexpr int kHalf = 64;                   // positions per accumulator
+constexpr int kStages = 4;                  // tiles in flight (at first: the four weight blocks)
+constexpr int kSmZ = 0;                     // kStages x 32 KiB
+constexpr int kSmStats = kSmZ + kStages * 32768;  // 8 slots (tile i uses slot i & 7) x 4 x 128 floats
+constexpr int kStatsSlot = 4 * 512;         // rstd, -mean*rstd, mask/2, mask/2 * b_scale
+constexpr int kSmOut = kSmStats + 8 * kStatsSlot;  // 16 warps x 2 slabs x 2 KiB: 32 channels x 32 positions
+constexpr int kSmBars = kSmOut + 16 * 2 * 2048;
+enum Bar { W_FULL = 0, W_READY = 1, Z_FULL = 2, Z_EMPTY = Z_FULL + kStages, STATS_READY = Z_EMPTY + kStages, ACC_FULL = STATS_READY + 8,
+           ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2 };
 constexpr int kSmTotal = kSmBars + 256;
 constexpr int kSmDynamic = kSmTotal + 1024;
+// TMEM: the two accumulators (gate 64 | value 64 columns each), then the four weight blocks (64 columns each)
+constexpr uint32_t kTmemW = 256;
 
 struct ProjectParams {
   int B, R, S;
@@ -43,20 +55,12 @@ struct ProjectParams {
   const float* mask;  // may be NULL
   long long ms_b, ms_r, ms_s;
   const float* b_scale;  // per batch item, multiplies the b channels; may be NULL
-  __nv_bfloat16* ab;
-  long long pitch;  // elements between rows of a plane
   int* status;
 };
 
-__device__ __forceinline__ void stg256(void* p, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_w,
-                      const ProjectParams p) {
+                      const __grid_constant__ CUtensorMap tm_ab, const ProjectParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -69,15 +73,16 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     mbar_init(bars + W_FULL * 8, 1);
-    for (int i = 0; i < 2; ++i) {
+    mbar_init(bars + W_READY * 8, 16);
+    for (int i = 0; i < kStages; ++i) {
       mbar_init(bars + (Z_FULL + i) * 8, 1);
-      mbar_init(bars + (Z_EMPTY + i) * 8, 5);   // the MMA commit + the four statistics warps have read the tile
-      mbar_init(bars + (ACC_FULL + i) * 8, 1);  // per warpgroup
-      mbar_init(bars + (ACC_EMPTY + i) * 8, 8);  // two warpgroups read each accumulator pair
+      mbar_init(bars + (Z_EMPTY + i) * 8, 5);  // the MMA commit + the four statistics warps have read the tile
     }
-    // statistics of a tile written (the four statistics warps): one barrier per statistics slot, because the
-    // statistics of tile t + 2 may be complete before the epilogue of tile t has looked at its barrier
-    for (int i = 0; i < 4; ++i) mbar_init(bars + (STATS_READY + i) * 8, 4);
+    for (int i = 0; i < 8; ++i) mbar_init(bars + (STATS_READY + i) * 8, 4);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bars + (ACC_FULL + i) * 8, 1);
+      mbar_init(bars + (ACC_EMPTY + i) * 8, 8);
+    }
     fence_mbar_init();
   }
   if (warp == 21) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
@@ -91,175 +96,182 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_z);
-      tma_prefetch_desc(&tm_w);
-      mbar_expect_tx(bars + W_FULL * 8, 2 * kWHalf);
-      for (int kh = 0; kh < 2; ++kh)
-        for (int j = 0; j < kTriInRows / 128; ++j)
-          tma_load_2d(base + kSmW + kh * kWHalf + j * 128 * 128, &tm_w, bars + W_FULL * 8, kh * 64, j * 128);
+      // the weights pass through the ring on their way to tensor memory: block k in stage k
+      mbar_expect_tx(bars + W_FULL * 8, kStages * 32768);
+      for (int k = 0; k < kStages; ++k)
+        for (int kh = 0; kh < 2; ++kh)
+          tma_load_2d(base + kSmZ + k * 32768 + kh * 16384, &tm_w, bars + W_FULL * 8, kh * 64, k * 128);
+      mbar_wait(bars + W_READY * 8, 0, abort_flag);
       pdl_wait();
       int issued = 0;
-      for (int i = 0; i < my_tiles; ++i) {
+      for (int i = 0, stage = 0, phase = 1; i < my_tiles; ++i) {
         const int tile = blockIdx.x + i * gridDim.x;
         const int st = tile % p.tiles_s, br = tile / p.tiles_s;
         const int r = br % p.R, b = br / p.R;
-        const int stage = i & 1;
-        if (!mbar_wait(bars + (Z_EMPTY + stage) * 8, ((i >> 1) & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait(bars + (Z_EMPTY + stage) * 8, phase, abort_flag)) break;
         const uint32_t full = bars + (Z_FULL + stage) * 8;
         mbar_expect_tx(full, 32768);
         tma_load_4d(base + kSmZ + stage * 32768, &tm_z, full, 0, st * kTileM, r, b);
         tma_load_4d(base + kSmZ + stage * 32768 + 16384, &tm_z, full, 64, st * kTileM, r, b);
         ++issued;
+        if (++stage == kStages) stage = 0, phase ^= 1;
       }
-      if (*abort_flag && issued > 0) {
-        const int last = issued - 1;
-        mbar_wait(bars + (Z_FULL + (last & 1)) * 8, (last >> 1) & 1, abort_flag + 1);
-      }
+      // If the loop was abandoned, give copies still in flight a bounded chance to land.
+      if (*abort_flag)
+        for (int j = issued > kStages ? issued - kStages : 0; j < issued; ++j)
+          mbar_wait(bars + (Z_FULL + j % kStages) * 8, (j / kStages) & 1, abort_flag + 1);
     }
   } else if (warp == 21) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(128, kTileM);
-      bool ok = mbar_wait(bars + W_FULL * 8, 0, abort_flag);
-      for (int i = 0; ok && i < my_tiles; ++i) {
-        const int stage = i & 1;
-        ok = mbar_wait(bars + (Z_FULL + stage) * 8, (i >> 1) & 1, abort_flag);
-        if (!ok) break;
-        const uint64_t dz = make_smem_desc(base + kSmZ + stage * 32768, 16, 1024, kLayoutSw128);
-        for (int wg = 0; ok && wg < 2; ++wg) {
-          ok = mbar_wait(bars + (ACC_EMPTY + wg) * 8, (i & 1) ^ 1, abort_flag);
+    // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
+    constexpr uint32_t idesc = make_idesc_bf16(128, kHalf);
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = mbar_wait_warp(bars + W_READY * 8, 0, abort_flag);
+    uint32_t uses = 0;  // accumulators filled, of each kind
+    for (int i = 0, stage = 0, phase = 0; ok && i < my_tiles; ++i) {
+      ok = mbar_wait_warp(bars + (Z_FULL + stage) * 8, phase, abort_flag);
+      const uint64_t dz = smem_desc<16, 1024, kLayoutSw128>(base + kSmZ + stage * 32768);
+      for (int half = 0; ok && half < 2; ++half, ++uses) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {  // a channels, b channels
+          if (!ok) break;
+          ok = mbar_wait_warp(bars + (ACC_EMPTY + g) * 8, (uses & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
-          for (int acc = 0; acc < 2; ++acc) {  // gate rows, then value rows of this warpgroup's channels
-            const uint32_t d = tmem_base + (wg * 2 + acc) * 128;
-            const uint64_t dw = make_smem_desc(base + kSmW + (wg * 2 + acc) * 128 * 128, 16, 1024, kLayoutSw128);
+          for (int acc = 0; acc < 2; ++acc) {  // gate rows, then value rows
+            const uint32_t d = tb + g * 128 + acc * 64, w = tb + kTmemW + (g * 2 + acc) * 64;
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              umma_ss(d, dw + ((k >> 2) * (kWHalf >> 4) + (k & 3) * 2), dz + ((k >> 2) * (16384 >> 4) + (k & 3) * 2), idesc,
-                      k > 0 ? 1u : 0u);
+              umma_ts_warp(d, w + k * 8, dz + (half * (8192 >> 4) + (k >> 2) * (16384 >> 4) + (k & 3) * 2), idesc,
+                           k > 0 ? 1u : 0u);
           }
-          umma_commit(bars + (ACC_FULL + wg) * 8);
+          umma_commit_warp(bars + (ACC_FULL + g) * 8);
         }
-        if (!ok) break;
-        umma_commit(bars + (Z_EMPTY + stage) * 8);
       }
+      if (!ok) break;
+      umma_commit_warp(bars + (Z_EMPTY + stage) * 8);
+      if (++stage == kStages) stage = 0, phase ^= 1;
     }
-  } else if (warp >= 16 && warp < 20) {
+  } else if (warp >= 16) {
     // ------------------------------------------------------------------ statistics: one thread per position
     pdl_wait();
     const int m = (warp - 16) * 32 + lane;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; ++i) {
+    for (int i = 0, stage = 0, phase = 0; i < my_tiles; ++i) {
       const int tile = blockIdx.x + i * gridDim.x;
       const int st = tile % p.tiles_s, br = tile / p.tiles_s;
       const int r = br % p.R, b = br / p.R;
-      const int stage = i & 1;
       const int s = st * kTileM + m;
       float mval = 0.f;
       if (s < p.S) mval = p.mask ? __ldg(p.mask + b * p.ms_b + r * p.ms_r + (long long)s * p.ms_s) : 1.f;
-      ok = mbar_wait(bars + (Z_FULL + stage) * 8, (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      const uint32_t z0 = base + kSmZ + stage * 32768;
-      // two passes over the 256-byte row in shared memory (mean, then squared deviations), eight 16-byte loads in
-      // flight at a time; the reads are conflict-free and nothing is written back
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int c = 0; c < 16; ++c) {
-        const uint4 x = lds128(z0 + (c >> 3) * 16384 + sw128_offset(m, c & 7));
-        sum4[0] += bf16_lo(x.x) + bf16_hi(x.x);
-        sum4[1] += bf16_lo(x.y) + bf16_hi(x.y);
-        sum4[2] += bf16_lo(x.z) + bf16_hi(x.z);
-        sum4[3] += bf16_lo(x.w) + bf16_hi(x.w);
-      }
-      const float mu = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) * (1.f / kC);
-      float var4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int c = 0; c < 16; ++c) {
-        const uint4 x = lds128(z0 + (c >> 3) * 16384 + sw128_offset(m, c & 7));
-        const uint32_t w4[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float d0 = bf16_lo(w4[e]) - mu, d1 = bf16_hi(w4[e]) - mu;
-          var4[e] = fmaf(d0, d0, var4[e]);
-          var4[e] = fmaf(d1, d1, var4[e]);
-        }
-      }
-      const float rstd = rsqrtf(((var4[0] + var4[1]) + (var4[2] + var4[3])) * (1.f / kC) + p.eps);
-      // Statistics and mask go to one of four slots: the epilogue of a tile reads its slot while the statistics of
-      // the next two tiles are written.  A slot is rewritten four tiles later, when that epilogue is long done
-      // (the MMAs of tile t + 1 wait for the accumulators of tile t, the loads of tile t + 3 for those MMAs).
-      float* slot = reinterpret_cast<float*>(gen + kSmStats + (i & 3) * kStatsSlot);
-      slot[m] = rstd;
-      slot[128 + m] = -mu * rstd;
+      const float scale = p.b_scale ? __ldg(p.b_scale + b) : 1.f;
+      if (!mbar_wait(bars + (Z_FULL + stage) * 8, phase, abort_flag)) break;
+      const float2 v = row_stats_128(base + kSmZ + stage * 32768, m, p.eps);
+      // Eight slots: a slot is rewritten eight tiles later, after the MMAs of the tile two later, whose accumulators the
+      // epilogue has handed back only after it was done with this tile.
+      float* slot = reinterpret_cast<float*>(gen + kSmStats + (i & 7) * kStatsSlot);
+      slot[m] = v.x;
+      slot[128 + m] = v.y;
       slot[256 + m] = 0.5f * mval;  // sigmoid(g) * v * mask = tanh(g/2) * h + h with h = v * mask / 2
+      slot[384 + m] = 0.5f * mval * scale;
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(bars + (STATS_READY + (i & 3)) * 8);
+        mbar_arrive(bars + (STATS_READY + (i & 7)) * 8);
         mbar_arrive(bars + (Z_EMPTY + stage) * 8);  // done reading the tile
       }
+      if (++stage == kStages) stage = 0, phase ^= 1;
     }
-  } else if (warp < 16) {
+  } else {
     // ------------------------------------------------------------------ epilogue warps: one thread per channel
-    pdl_wait();
-    const int wg = warp >> 3;        // 0: a channels, 1: b channels
-    const int half = (warp >> 2) & 1;  // which 64 positions of the tile
+    const int g = warp >> 3;           // 0: a channels, 1: b channels
+    const int part = (warp >> 2) & 1;  // which 32 positions of the accumulator
     const int ch = (warp & 3) * 32 + lane;  // channel inside the 128 == TMEM lane
-    // gate columns of these 64 positions; the value columns lie 128 further
-    const uint32_t acc = tmem_base + (uint32_t((warp & 3) * 32) << 16) + wg * 256 + half * 64;
-    const float2 kg = p.sc[wg * 256 + ch], kp = p.sc[wg * 256 + 128 + ch];  // {rowsum, const} of the gate / value row
+    const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    {
+      // this warp's 32 rows of weight block 2 g + part, as bf16 pairs
+      mbar_wait_warp(bars + W_FULL * 8, 0, abort_flag);
+      const uint32_t src = base + kSmZ + (g * 2 + part) * 32768;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t v[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 x = lds128(src + (k >> 1) * 16384 + sw128_offset(ch, (k & 1) * 4 + j));
+          v[j * 4] = x.x, v[j * 4 + 1] = x.y, v[j * 4 + 2] = x.z, v[j * 4 + 3] = x.w;
+        }
+        tmem_st16(lane_taddr + kTmemW + (g * 2 + part) * 64 + k * 16, v);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      mbar_arrive_warp(bars + W_READY * 8);
+    }
+    const uint32_t acc = lane_taddr + g * 128 + part * 32;  // the value columns lie 64 further
+    const float2 kg = p.sc[g * 256 + ch], kp = p.sc[g * 256 + 128 + ch];  // {rowsum, const} of the gate / value row
     const uint64_t cg2 = pack_f32x2(kg.y, kg.y), cp2 = pack_f32x2(kp.y, kp.y);
     const uint64_t rg2 = pack_f32x2(kg.x, kg.x), rp2 = pack_f32x2(kp.x, kp.x);
+    pdl_wait();
     bool ok = true;
+    uint32_t uses = 0;
     for (int i = 0; ok && i < my_tiles; ++i) {
       const int tile = blockIdx.x + i * gridDim.x;
       const int st = tile % p.tiles_s, br = tile / p.tiles_s;
       const int r = br % p.R, b = br / p.R;
-      const float bscale = (wg == 1 && p.b_scale) ? __ldg(p.b_scale + b) : 1.f;
-      const uint64_t hs2 = pack_f32x2(bscale, bscale);
-      // per position: rstd, -mean*rstd, mask/2, as pairs of neighbouring positions
-      const float2* stats = reinterpret_cast<const float2*>(gen + kSmStats + (i & 3) * kStatsSlot) + half * 32;
-      __nv_bfloat16* dst = p.ab + ((long long)(b * 2 + wg) * kTriHidden + ch) * p.R * p.pitch + (long long)r * p.pitch +
-                           st * kTileM + half * 64;
-      ok = mbar_wait(bars + (STATS_READY + (i & 3)) * 8, (i >> 2) & 1, abort_flag) &&
-           mbar_wait(bars + (ACC_FULL + wg) * 8, i & 1, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      // 8 positions at a time; the TMEM loads of the next chunk are in flight while this one is computed
-      uint32_t g[2][8], v[2][8];
-      tmem_ld8(acc, g[0]);
-      tmem_ld8(acc + 128, v[0]);
-      uint32_t packed[8];
+      const uint32_t stats = base + kSmStats + (i & 7) * kStatsSlot;
+      for (int half = 0; half < 2; ++half, ++uses) {
+        ok = mbar_wait2_warp(bars + (STATS_READY + (i & 7)) * 8, (i >> 3) & 1, bars + (ACC_FULL + g) * 8, uses & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const int pos = half * kHalf + part * 32;
+        const uint32_t slab = base + kSmOut + (warp * 2 + (uses & 1)) * 2048;
+        if (lane == 0) tma_store_wait_read<1>();  // the store before the previous one has read this slab
+        __syncwarp();
 #pragma unroll
-      for (int part = 0; part < 8; ++part) {
-        tmem_ld_wait();
-        if (part + 1 < 8) {
-          tmem_ld8(acc + (part + 1) * 8, g[(part + 1) & 1]);
-          tmem_ld8(acc + 128 + (part + 1) * 8, v[(part + 1) & 1]);
-        }
-        const uint32_t (&gg)[8] = g[part & 1];
-        const uint32_t (&vv)[8] = v[part & 1];
+        for (int q = 0; q < 2; ++q) {
+          uint32_t gg[16], vv[16];
+          tmem_ld16(acc + q * 16, gg);
+          tmem_ld16(acc + 64 + q * 16, vv);
+          tmem_ld_wait();
+          if (q == 1) {  // the accumulator is in registers: the next MMAs may have it
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_warp(bars + (ACC_EMPTY + g) * 8);
+          }
+          uint32_t packed[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // packed fp32x2 math on two positions: LayerNorm finished per position, gate rows are pre-halved
-          const float2 rs = stats[part * 4 + j], nm = stats[64 + part * 4 + j], mh = stats[128 + part * 4 + j];
-          const uint64_t rs2 = pack_f32x2(rs.x, rs.y), nm2 = pack_f32x2(nm.x, nm.y);
-          float a0, a1;
-          unpack_f32x2(fma_f32x2(rs2, pack_f32x2(__uint_as_float(gg[2 * j]), __uint_as_float(gg[2 * j + 1])),
-                                 fma_f32x2(nm2, rg2, cg2)), a0, a1);
-          const uint64_t val2 = fma_f32x2(rs2, pack_f32x2(__uint_as_float(vv[2 * j]), __uint_as_float(vv[2 * j + 1])),
-                                          fma_f32x2(nm2, rp2, cp2));
-          // sigmoid(g) * v * mask = tanh(g/2) * h + h with h = v * mask / 2
-          const uint64_t h2 = mul_f32x2(val2, mul_f32x2(pack_f32x2(mh.x, mh.y), hs2));
-          float o0, o1;
-          unpack_f32x2(fma_f32x2(pack_f32x2(tanh_approx(a0), tanh_approx(a1)), h2, h2), o0, o1);
-          packed[(part & 1) * 4 + j] = pack_bf16x2(o0, o1);
+          for (int e = 0; e < 4; ++e) {  // four positions, as two packed pairs
+            const uint32_t at = stats + (pos + q * 16 + e * 4) * 4;
+            const uint4 rs = lds128(at), nm = lds128(at + 512), mh = lds128(at + 1024 + g * 512);
+            const uint32_t rs4[4] = {rs.x, rs.y, rs.z, rs.w}, nm4[4] = {nm.x, nm.y, nm.z, nm.w}, mh4[4] = {mh.x, mh.y, mh.z, mh.w};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int j = e * 4 + h * 2;
+              const uint64_t rs2 = pack_f32x2(__uint_as_float(rs4[2 * h]), __uint_as_float(rs4[2 * h + 1]));
+              const uint64_t nm2 = pack_f32x2(__uint_as_float(nm4[2 * h]), __uint_as_float(nm4[2 * h + 1]));
+              float a0, a1;
+              unpack_f32x2(fma_f32x2(rs2, pack_f32x2(__uint_as_float(gg[j]), __uint_as_float(gg[j + 1])),
+                                     fma_f32x2(nm2, rg2, cg2)), a0, a1);
+              const uint64_t val2 = fma_f32x2(rs2, pack_f32x2(__uint_as_float(vv[j]), __uint_as_float(vv[j + 1])),
+                                              fma_f32x2(nm2, rp2, cp2));
+              const uint64_t h2 = mul_f32x2(val2, pack_f32x2(__uint_as_float(mh4[2 * h]), __uint_as_float(mh4[2 * h + 1])));
+              float o0, o1;  // gate rows are pre-halved
+              unpack_f32x2(fma_f32x2(pack_f32x2(tanh_approx(a0), tanh_approx(a1)), h2, h2), o0, o1);
+              packed[e * 2 + h] = pack_bf16x2(o0, o1);
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            sts128(slab + sw64_offset(lane, q * 2 + c), make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]));
         }
-        if ((part & 1) && st * kTileM + half * 64 + (part - 1) * 8 + 16 <= p.pitch) stg256(dst + (part - 1) * 8, packed);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          // (positions past the row pitch are not written; between the token count and the pitch they are zero)
+          tma_store_3d(&tm_ab, slab, st * kTileM + pos, r, (b * 2 + g) * kTriHidden + (warp & 3) * 32);
+          tma_store_commit();
+        }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + (ACC_EMPTY + wg) * 8);
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   __syncwarp();
@@ -294,7 +306,7 @@ int b200ta_trimul_project(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_
   int rc = get_device_state(&st);
   if (rc != B200TA_OK) return rc;
 
-  CUtensorMap tm_z, tm_w;
+  CUtensorMap tm_z, tm_w, tm_ab;
   {
     // (c, s, r, b); a size-1 dimension may carry any stride: give it a valid one
     auto fix = [](int64_t stride, int extent) -> uint64_t { return extent == 1 ? 256u : uint64_t(stride) * 2u; };
@@ -312,6 +324,14 @@ int b200ta_trimul_project(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_
     rc = encode_tensor_map(&tm_w, pk + kTriWOff, 2, 2, dims, strides, box, SWZ_128, "trimul_project weights");
     if (rc != B200TA_OK) return rc;
   }
+  {
+    // (position, row, plane): a warp's slab of 32 channels
+    uint64_t dims[3] = {uint64_t(pitch), uint64_t(R), uint64_t(B) * 2 * kTriHidden};
+    uint64_t strides[2] = {uint64_t(pitch) * 2, uint64_t(pitch) * R * 2};
+    uint32_t box[3] = {32, 1, 32};
+    rc = encode_tensor_map(&tm_ab, ab, 2, 3, dims, strides, box, SWZ_64, "trimul_project ab");
+    if (rc != B200TA_OK) return rc;
+  }
   ProjectParams p{};
   p.B = B, p.R = R, p.S = S;
   p.tiles_s = (S + kTileM - 1) / kTileM;
@@ -321,12 +341,10 @@ int b200ta_trimul_project(const void* z, int64_t zs_b, int64_t zs_r, int64_t zs_
   p.mask = mask;
   p.ms_b = ms_b, p.ms_r = ms_r, p.ms_s = ms_s;
   p.b_scale = b_scale;
-  p.ab = static_cast<__nv_bfloat16*>(ab);
-  p.pitch = pitch;
   p.status = st->status_dev;
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  return launch_kernel(st, kKernelProject, trimul_project_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_w, p);
+  return launch_kernel(st, kKernelProject, trimul_project_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_w, tm_ab, p);
 }
 
 }  // extern "C"
