@@ -8,16 +8,22 @@
 // position, applies rstd·(D − mean·rowsum) + const with the statistics the statistics warps computed from the two
 // tiles while the MMAs ran - neither tile is rewritten and the MMAs wait for nothing but the loads.
 //
-// Warp roles (448 threads): warps 0-7 epilogue (thread = position; the two warpgroups take alternate groups of 32
+// The residual is read from the z tile in shared memory, and the result takes its place there, from where TMA stores it:
+// with a thread per position, 32-byte global accesses of a warp go to 32 rows and occupy the load-store unit for some 56
+// clocks each, which bounded the kernel (148 us at 768 tokens, 3.1 TB/s of the 768 bytes per position).  The fp32 form
+// stores its 64 KiB tile from the places of both input tiles.
+//
+// Warp roles (480 threads): warps 0-7 epilogue (thread = position; the two warpgroups take alternate groups of 32
 // output channels), warps 8-11 statistics (z rows: one thread per position; x columns: a thread takes two
-// neighbouring positions over half of the channels), warp 12 TMA producer, warp 13 MMA issuer / TMEM owner.
+// neighbouring positions over half of the channels), warp 12 TMA producer, warp 13 MMA issuer / TMEM owner, warp 14
+// TMA stores.
 #include "common.cuh"
 #include "layout.h"
 
 namespace b200ta {
 namespace {
 
-constexpr int kThreads = 448;
+constexpr int kThreads = 480;
 constexpr int kTileM = 128;
 constexpr int kSmW = 0;                      // W_go' and W_po': 2 matrices x 2 K-halves x 128 rows x 128 B
 constexpr int kSmZ = kSmW + 65536;           // 2 stages x 32 KiB
@@ -27,7 +33,7 @@ constexpr int kSmStats = kSmConst + 2048;    // 4 slots (tile i uses slot i & 3)
 constexpr int kStatsSlot = 2048 + 512;
 constexpr int kSmXch = kSmStats + 4 * kStatsSlot;  // 2 x float4 [128] partial x statistics (alternating per tile)
 constexpr int kSmBars = kSmXch + 2 * 2048;
-enum Bar { W_FULL = 0, IN_FULL = 1, READY = 3, IN_EMPTY = 7, ACC_FULL = 9, ACC_EMPTY = 11, XCH = 13, NUM_BARS = 14 };
+enum Bar { W_FULL = 0, IN_FULL = 1, READY = 3, IN_EMPTY = 7, ACC_FULL = 9, ACC_EMPTY = 11, XCH = 13, OUT_FULL = 14, NUM_BARS = 16 };
 constexpr int kSmTotal = kSmBars + 256;
 constexpr int kSmDynamic = kSmTotal + 1024;
 
@@ -36,21 +42,12 @@ struct OutputParams {
   int tiles_j, num_tiles;
   const float2* sc;  // folded {rowsum, const} of the output gate rows, then of the output projection rows
   float eps;
-  const __nv_bfloat16* z;  // residual source (same tensor the z tiles are loaded from)
-  long long zs_b, zs_i, zs_j;
   int add_residual;
   const float* mask;  // [B, N, N] via strides; NULL = no output mask
   long long ms_b, ms_i, ms_j;
-  void* out;  // bf16, or float in the kF32 form
-  long long os_b, os_i, os_j;
   int* status;
 };
 
-__device__ __forceinline__ void stg256(void* p, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -60,7 +57,8 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 template <bool kF32>
 __global__ void __launch_bounds__(kThreads, 1)
 trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_x,
-                     const __grid_constant__ CUtensorMap tm_w, const OutputParams p) {
+                     const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_out,
+                     const OutputParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -79,7 +77,9 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     for (int i = 0; i < 4; ++i) mbar_init(bars + (READY + i) * 8, 4);
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + (IN_FULL + i) * 8, 1);
-      mbar_init(bars + (IN_EMPTY + i) * 8, 5);  // the MMA commit + the four statistics warps have read the tiles
+      // MMA commit and statistics warps (have read the tiles), store warp (has read the result in their place)
+      mbar_init(bars + (IN_EMPTY + i) * 8, 6);
+      mbar_init(bars + (OUT_FULL + i) * 8, 8);
       mbar_init(bars + (ACC_FULL + i) * 8, 1);
       mbar_init(bars + (ACC_EMPTY + i) * 8, 8);
     }
@@ -131,35 +131,58 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       }
     }
   } else if (warp == 13) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_g = make_idesc_bf16(kTileM, kC);              // both operands K-major
-      constexpr uint32_t idesc_p = make_idesc_bf16(kTileM, kC, true, false);  // A (the x tile) MN-major
-      bool ok = mbar_wait(bars + W_FULL * 8, 0, abort_flag);
-      for (int it = 0; ok && it < my_tiles; ++it) {
-        const int stage = it & 1, slot = it & 1;
-        ok = mbar_wait(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, abort_flag);
-        ok = ok && mbar_wait(bars + (ACC_EMPTY + slot) * 8, ((it >> 1) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + slot * 256;
-        const uint64_t dz = make_smem_desc(base + kSmZ + stage * 32768, 16, 1024, kLayoutSw128);
-        const uint64_t dwg = make_smem_desc(base + kSmW, 16, 1024, kLayoutSw128);
-        const uint64_t dwp = make_smem_desc(base + kSmW + 32768, 16, 1024, kLayoutSw128);
-        // x tile: [128 d][64 j] blocks of 128-byte rows, the two 64-position blocks 16 KiB apart; as A[pos][d] this
-        // is MN-major, a K step of 16 channels is 16 rows = 2 KiB
-        const uint64_t dx = make_smem_desc(base + kSmX + stage * 32768, 16384, 1024, kLayoutSw128);
+    // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
+    constexpr uint32_t idesc_g = make_idesc_bf16(kTileM, kC);               // both operands K-major
+    constexpr uint32_t idesc_p = make_idesc_bf16(kTileM, kC, true, false);  // A (the x tile) MN-major
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = mbar_wait_warp(bars + W_FULL * 8, 0, abort_flag);
+    for (int it = 0; ok && it < my_tiles; ++it) {
+      const int stage = it & 1, slot = it & 1;
+      ok = mbar_wait2_warp(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, bars + (ACC_EMPTY + slot) * 8, ((it >> 1) & 1) ^ 1,
+                           abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tb + slot * 256;
+      const uint64_t dz = smem_desc<16, 1024, kLayoutSw128>(base + kSmZ + stage * 32768);
+      const uint64_t dwg = smem_desc<16, 1024, kLayoutSw128>(base + kSmW);
+      const uint64_t dwp = smem_desc<16, 1024, kLayoutSw128>(base + kSmW + 32768);
+      // x tile: [128 d][64 j] blocks of 128-byte rows, the two 64-position blocks 16 KiB apart; as A[pos][d] this
+      // is MN-major, a K step of 16 channels is 16 rows = 2 KiB
+      const uint64_t dx = smem_desc<16384, 1024, kLayoutSw128>(base + kSmX + stage * 32768);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t koff = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
-          umma_ss(d, dz + koff, dwg + koff, idesc_g, k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_ss(d + 128, dx + k * 128, dwp + ((k >> 2) * (16384 >> 4) + (k & 3) * 2), idesc_p, k > 0 ? 1u : 0u);
-        umma_commit(bars + (ACC_FULL + slot) * 8);
-        umma_commit(bars + (IN_EMPTY + stage) * 8);
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t koff = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
+        umma_ss_warp(d, dz + koff, dwg + koff, idesc_g, k > 0 ? 1u : 0u);
       }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        umma_ss_warp(d + 128, dx + k * 128, dwp + ((k >> 2) * (16384 >> 4) + (k & 3) * 2), idesc_p, k > 0 ? 1u : 0u);
+      umma_commit_warp(bars + (ACC_FULL + slot) * 8);
+      umma_commit_warp(bars + (IN_EMPTY + stage) * 8);
+    }
+  } else if (warp == 14) {
+    // ------------------------------------------------------------------ TMA stores
+    if (lane == 0) {
+      tma_prefetch_desc(&tm_out);
+      pdl_wait();
+      for (int it = 0; it < my_tiles; ++it) {
+        const int tile = blockIdx.x + it * gridDim.x;
+        const int jt = tile % p.tiles_j, bi = tile / p.tiles_j;
+        const int i = bi % p.N, b = bi / p.N;
+        const int stage = it & 1;
+        if (!mbar_wait(bars + (OUT_FULL + stage) * 8, (it >> 1) & 1, abort_flag)) break;
+        if (kF32) {  // four blocks of 32 channels: two in the place of the z tile, two in that of the x tile
+          for (int g = 0; g < 4; ++g)
+            tma_store_4d(&tm_out, base + (g < 2 ? kSmZ : kSmX) + stage * 32768 + (g & 1) * 16384, g * 32, jt * kTileM, i, b);
+        } else {
+          for (int h = 0; h < 2; ++h)
+            tma_store_4d(&tm_out, base + kSmZ + stage * 32768 + h * 16384, h * 64, jt * kTileM, i, b);
+        }
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(bars + (IN_EMPTY + stage) * 8);
+      }
+      tma_store_wait_all();
     }
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ normaliser
@@ -176,58 +199,33 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       if (p.mask != nullptr) mval = j < p.N ? __ldg(p.mask + b * p.ms_b + i * p.ms_i + (long long)j * p.ms_j) : 0.f;
       ok = mbar_wait(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, abort_flag);
       if (!ok) break;
-      // ---- z row t: mean and variance (two passes over the row in shared memory; nothing is written back)
-      float rstd_i, nmr_i;
-      {
-        const uint32_t z0 = base + kSmZ + stage * 32768;
-        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int c = 0; c < 16; ++c) {
-          const uint4 x = lds128(z0 + (c >> 3) * 16384 + sw128_offset(t, c & 7));
-          sum4[0] += bf16_lo(x.x) + bf16_hi(x.x);
-          sum4[1] += bf16_lo(x.y) + bf16_hi(x.y);
-          sum4[2] += bf16_lo(x.z) + bf16_hi(x.z);
-          sum4[3] += bf16_lo(x.w) + bf16_hi(x.w);
-        }
-        const float mu = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) * (1.f / kC);
-        float var4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int c = 0; c < 16; ++c) {
-          const uint4 x = lds128(z0 + (c >> 3) * 16384 + sw128_offset(t, c & 7));
-          const uint32_t w4[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float d0 = bf16_lo(w4[e]) - mu, d1 = bf16_hi(w4[e]) - mu;
-            var4[e] = fmaf(d0, d0, var4[e]);
-            var4[e] = fmaf(d1, d1, var4[e]);
-          }
-        }
-        rstd_i = rsqrtf(((var4[0] + var4[1]) + (var4[2] + var4[3])) * (1.f / kC) + p.eps);
-        nmr_i = -mu * rstd_i;
-      }
-      // ---- x columns: this thread takes positions 2q, 2q+1 over channels [64 h, 64 h + 64)
+      // ---- z row t (nothing is written back)
+      const float2 zi = row_stats_128(base + kSmZ + stage * 32768, t, p.eps);
+      // ---- x columns: this thread takes positions 2q, 2q+1 over channels [64 h, 64 h + 64), in one pass of packed sums
+      // shifted by the first channel (as row_stats_128)
       {
         const int q = t & 63, h = t >> 6;
         const int jj = (2 * q) & 63;
-        const uint32_t x0 = base + kSmX + stage * 32768 + ((2 * q) >> 6) * 16384 + (jj & 7) * 2;
+        const uint32_t x0 = base + kSmX + stage * 32768 + ((2 * q) >> 6) * 16384 + h * 8192 + (jj & 7) * 2;
         const uint32_t chunk = uint32_t(jj >> 3);
-        uint32_t w[64];
-#pragma unroll
+        const uint32_t first = lds32(x0 + (chunk << 4));
+        const float k0 = bf16_lo(first), k1 = bf16_hi(first);
+        const uint64_t nk2 = pack_f32x2(-k0, -k1);
+        uint64_t sa[2] = {0ull, 0ull}, sq[2] = {0ull, 0ull};
+#pragma unroll 16
         for (int d = 0; d < 64; ++d) {
-          const uint32_t row = uint32_t(h * 64 + d);
-          w[d] = lds32(x0 + row * 128 + ((chunk ^ (row & 7)) << 4));
+          const uint32_t w = lds32(x0 + d * 128 + ((chunk ^ (d & 7)) << 4));
+          const uint64_t v = add_f32x2(pack_f32x2(bf16_lo(w), bf16_hi(w)), nk2);
+          sa[d & 1] = add_f32x2(sa[d & 1], v);
+          sq[d & 1] = fma_f32x2(v, v, sq[d & 1]);
         }
-        float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-        for (int d = 0; d < 64; ++d) s0 += bf16_lo(w[d]), s1 += bf16_hi(w[d]);
-        const float m0 = s0 * (1.f / 64), m1 = s1 * (1.f / 64);
-        float q0 = 0.f, q1 = 0.f;
-#pragma unroll
-        for (int d = 0; d < 64; ++d) {
-          const float d0 = bf16_lo(w[d]) - m0, d1 = bf16_hi(w[d]) - m1;
-          q0 = fmaf(d0, d0, q0), q1 = fmaf(d1, d1, q1);
-        }
-        reinterpret_cast<float4*>(gen + kSmXch + (it & 1) * 2048)[t] = make_float4(m0, q0, m1, q1);
+        float s0, s1, q0, q1;
+        unpack_f32x2(add_f32x2(sa[0], sa[1]), s0, s1);
+        unpack_f32x2(add_f32x2(sq[0], sq[1]), q0, q1);
+        // mean and sum of squared deviations of the 64 channels
+        reinterpret_cast<float4*>(gen + kSmXch + (it & 1) * 2048)[t] =
+            make_float4(s0 * (1.f / 64) + k0, fmaxf(q0 - s0 * s0 * (1.f / 64), 0.f), s1 * (1.f / 64) + k1,
+                        fmaxf(q1 - s1 * s1 * (1.f / 64), 0.f));
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + XCH * 8);
@@ -245,7 +243,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         // Statistics and mask go to one of four slots: the epilogue of a tile may still read its slot while the
         // next two tiles' statistics are written (the stage itself is handed back below, before the epilogue ran).
         uint8_t* slot = gen + kSmStats + (it & 3) * kStatsSlot;
-        reinterpret_cast<float4*>(slot)[t] = make_float4(rstd, -mean * rstd, rstd_i, nmr_i);
+        reinterpret_cast<float4*>(slot)[t] = make_float4(rstd, -mean * rstd, zi.x, zi.y);
         reinterpret_cast<float*>(slot + 2048)[t] = mval;
       }
       __syncwarp();
@@ -264,33 +262,24 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     const float4* c4b = reinterpret_cast<const float4*>(gen + kSmConst + 1024);  // per channel pair
     bool ok = true;
     for (int it = 0; ok && it < my_tiles; ++it) {
-      const int tile = blockIdx.x + it * gridDim.x;
-      const int jt = tile % p.tiles_j, bi = tile / p.tiles_j;
-      const int i = bi % p.N, b = bi / p.N;
       const int slot = it & 1;
-      const int j = jt * kTileM + m;
-      // The residual values do not depend on the accumulators: fetch this thread's 2 x 32 channels (they were just
-      // loaded as part of the z tile, so they come from L2) before waiting for the MMAs.
-      uint32_t res[2][16];
-#pragma unroll
-      for (int gi = 0; gi < 2; ++gi) {
-        if (p.add_residual && j < p.N) {
-          const uint4* rp = reinterpret_cast<const uint4*>(p.z + b * p.zs_b + i * p.zs_i + (long long)j * p.zs_j +
-                                                           (e + 2 * gi) * 32);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 x = __ldg(rp + c);
-            res[gi][c * 4 + 0] = x.x, res[gi][c * 4 + 1] = x.y, res[gi][c * 4 + 2] = x.z, res[gi][c * 4 + 3] = x.w;
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < 16; ++c) res[gi][c] = 0u;
-        }
-      }
-      ok = mbar_wait(bars + (READY + (it & 3)) * 8, (it >> 2) & 1, abort_flag) &&
-           mbar_wait(bars + (ACC_FULL + slot) * 8, (it >> 1) & 1, abort_flag);
+      // (IN_FULL is complete, or there would be no statistics: it makes the copies' writes visible to this thread)
+      ok = mbar_wait2_warp(bars + (READY + (it & 3)) * 8, (it >> 2) & 1, bars + (ACC_FULL + slot) * 8, (it >> 1) & 1, abort_flag) &&
+           mbar_wait_warp(bars + (IN_FULL + slot) * 8, (it >> 1) & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
+      const uint32_t row = base + kSmZ + slot * 32768 + sw128_offset(m, 0);  // chunk c of a row lies at chunk c ^ (row % 8)
+      uint32_t res[2][16];
+      if (kF32) {  // the result needs the room of the residuals of both warpgroups: read them first
+#pragma unroll
+        for (int gi = 0; gi < 2; ++gi)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint4 x = lds128((row + gi * 16384) ^ ((e * 4 + c) << 4));
+            res[gi][c * 4 + 0] = x.x, res[gi][c * 4 + 1] = x.y, res[gi][c * 4 + 2] = x.z, res[gi][c * 4 + 3] = x.w;
+          }
+        named_bar_sync(1 + (warp & 3), 64);  // the two warps of these 32 rows
+      }
       const uint8_t* stats = gen + kSmStats + (it & 3) * kStatsSlot;
       const float4 stv = reinterpret_cast<const float4*>(stats)[m];
       const float mval = reinterpret_cast<const float*>(stats + 2048)[m];
@@ -315,7 +304,15 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         }
         const uint32_t (&xg)[16] = ag[ck & 1];
         const uint32_t (&xp)[16] = ap[ck & 1];
-        const long long at = b * p.os_b + i * p.os_i + (long long)j * p.os_j + ch0;
+        // 16 channels of the residual: two 16-byte chunks of this row, whose place the bf16 result takes
+        const uint32_t place = row + (g >> 1) * 16384;
+        if (!kF32) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const uint4 x = lds128(place ^ (((g & 1) * 4 + h * 2 + c) << 4));
+            res[0][c * 4 + 0] = x.x, res[0][c * 4 + 1] = x.y, res[0][c * 4 + 2] = x.z, res[0][c * 4 + 3] = x.w;
+          }
+        }
         uint32_t packed[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -331,21 +328,32 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
           const uint64_t s2 = fma_f32x2(pack_f32x2(tanh_approx(a0), tanh_approx(a1)), half2, half2);
           const uint64_t v2 = fma_f32x2(rstd2, pack_f32x2(__uint_as_float(xp[2 * c]), __uint_as_float(xp[2 * c + 1])),
                                         fma_f32x2(nmr2, pack_f32x2(kb.z, kb.w), pack_f32x2(kb.x, kb.y)));
-          const uint32_t r = res[ck >> 1][h * 8 + c];
+          const uint32_t r = !p.add_residual ? 0u : kF32 ? res[ck >> 1][h * 8 + c] : res[0][c];
           float o0, o1;
           unpack_f32x2(mul_f32x2(fma_f32x2(s2, v2, pack_f32x2(bf16_lo(r), bf16_hi(r))), mval2), o0, o1);
           if (kF32) {
             packed[(2 * c) & 7] = __float_as_uint(o0), packed[(2 * c + 1) & 7] = __float_as_uint(o1);
-            if ((c & 3) == 3 && j < p.N) stg256(static_cast<float*>(p.out) + at + (c - 3) * 2, packed);
+            if ((c & 3) == 3) {
+              const uint32_t dst = base + (g < 2 ? kSmZ : kSmX) + slot * 32768 + (g & 1) * 16384 + sw128_offset(m, 0);
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+                sts128(dst ^ ((h * 4 + (c - 3) / 2 + q) << 4), make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]));
+            }
           } else {
             packed[c] = pack_bf16x2(o0, o1);
           }
         }
-        if (!kF32 && j < p.N) stg256(static_cast<__nv_bfloat16*>(p.out) + at, packed);
+        if (!kF32) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            sts128(place ^ (((g & 1) * 4 + h * 2 + c) << 4), make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]));
+        }
       }
       tc_fence_before();
+      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars + (ACC_EMPTY + slot) * 8);
+      mbar_arrive_warp(bars + (ACC_EMPTY + slot) * 8);
+      mbar_arrive_warp(bars + (OUT_FULL + slot) * 8);
     }
   }
 
@@ -384,13 +392,19 @@ int launch_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const
   int rc = get_device_state(&st);
   if (rc != B200TA_OK) return rc;
 
-  CUtensorMap tm_z, tm_x, tm_w;
+  CUtensorMap tm_z, tm_x, tm_w, tm_out;
   {
     auto fix = [](int64_t stride, int extent) -> uint64_t { return extent == 1 ? 256u : uint64_t(stride) * 2u; };
     uint64_t dims[4] = {uint64_t(kC), uint64_t(N), uint64_t(N), uint64_t(B)};
     uint64_t strides[3] = {fix(zs_j, N), fix(zs_i, N), fix(zs_b, B)};
     uint32_t box[4] = {64, kTileM, 1, 1};
     rc = encode_tensor_map(&tm_z, z, 2, 4, dims, strides, box, SWZ_128, "trimul_output z");
+    if (rc != B200TA_OK) return rc;
+    constexpr int kBytes = kF32 ? 4 : 2;
+    auto fix_out = [](int64_t stride, int extent) -> uint64_t { return uint64_t(extent == 1 ? 128 : stride) * kBytes; };
+    uint64_t ostrides[3] = {fix_out(os_j, N), fix_out(os_i, N), fix_out(os_b, B)};
+    box[0] = 128 / kBytes;
+    rc = encode_tensor_map(&tm_out, out, kBytes, 4, dims, ostrides, box, SWZ_128, "trimul_output out");
     if (rc != B200TA_OK) return rc;
   }
   {
@@ -415,17 +429,13 @@ int launch_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const
   p.num_tiles = B * N * p.tiles_j;
   p.sc = reinterpret_cast<const float2*>(pk + kTriScOff) + kTriInRows;
   p.eps = eps;
-  p.z = static_cast<const __nv_bfloat16*>(z);
-  p.zs_b = zs_b, p.zs_i = zs_i, p.zs_j = zs_j;
   p.add_residual = add_residual ? 1 : 0;
   p.mask = mask;
   p.ms_b = ms_b, p.ms_i = ms_i, p.ms_j = ms_j;
-  p.out = out;
-  p.os_b = os_b, p.os_i = os_i, p.os_j = os_j;
   p.status = st->status_dev;
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  return launch_kernel(st, kF32 ? kKernelOutputF32 : kKernelOutput, trimul_output_kernel<kF32>, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_x, tm_w, p);
+  return launch_kernel(st, kF32 ? kKernelOutputF32 : kKernelOutput, trimul_output_kernel<kF32>, dim3(grid), kThreads, kSmDynamic, stream, tm_z, tm_x, tm_w, tm_out, p);
 }
 
 }  // namespace

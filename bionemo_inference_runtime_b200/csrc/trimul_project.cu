@@ -240,19 +240,20 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
 #pragma unroll
           for (int e = 0; e < 4; ++e) {  // four positions, as two packed pairs
             const uint32_t at = stats + (pos + q * 16 + e * 4) * 4;
-            const uint4 rs = lds128(at), nm = lds128(at + 512), mh = lds128(at + 1024 + g * 512);
-            const uint32_t rs4[4] = {rs.x, rs.y, rs.z, rs.w}, nm4[4] = {nm.x, nm.y, nm.z, nm.w}, mh4[4] = {mh.x, mh.y, mh.z, mh.w};
+            uint64_t rs[2], nm[2], mh[2];
+            lds_f32x2(at, rs[0], rs[1]);
+            lds_f32x2(at + 512, nm[0], nm[1]);
+            lds_f32x2(at + 1024 + g * 512, mh[0], mh[1]);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               const int j = e * 4 + h * 2;
-              const uint64_t rs2 = pack_f32x2(__uint_as_float(rs4[2 * h]), __uint_as_float(rs4[2 * h + 1]));
-              const uint64_t nm2 = pack_f32x2(__uint_as_float(nm4[2 * h]), __uint_as_float(nm4[2 * h + 1]));
+              const uint64_t rs2 = rs[h], nm2 = nm[h];
               float a0, a1;
               unpack_f32x2(fma_f32x2(rs2, pack_f32x2(__uint_as_float(gg[j]), __uint_as_float(gg[j + 1])),
                                      fma_f32x2(nm2, rg2, cg2)), a0, a1);
               const uint64_t val2 = fma_f32x2(rs2, pack_f32x2(__uint_as_float(vv[j]), __uint_as_float(vv[j + 1])),
                                               fma_f32x2(nm2, rp2, cp2));
-              const uint64_t h2 = mul_f32x2(val2, pack_f32x2(__uint_as_float(mh4[2 * h]), __uint_as_float(mh4[2 * h + 1])));
+              const uint64_t h2 = mul_f32x2(val2, mh[h]);
               float o0, o1;  // gate rows are pre-halved
               unpack_f32x2(fma_f32x2(pack_f32x2(tanh_approx(a0), tanh_approx(a1)), h2, h2), o0, o1);
               packed[e * 2 + h] = pack_bf16x2(o0, o1);
