@@ -337,8 +337,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       int nt[kUnits];
 #pragma unroll
       for (int u = 0; u < kUnits; ++u) nt[u] = info->unit[u].tiles;
-      __syncwarp();
-      mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);  // the info has been read (Q itself: see the P·V warps)
+      mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);  // the info has been read (Q itself: see the P·V warps)
       const uint32_t q0 = base + kSmQ + ib * (kUnits * 8192);
       for (int kt = 0; ok && kt < tiles; ++kt) {
         ok = mbar_wait_warp(bars + (KV_FULL + stage) * 8, stage_phase, abort_flag);
@@ -425,8 +424,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const ItemInfo* info = reinterpret_cast<const ItemInfo*>(gen + kSmInfo) + ib;
       const int4 unit = *reinterpret_cast<const int4*>(&info->unit[w]);
       const int4 common = *reinterpret_cast<const int4*>(&info->tiles);
-      __syncwarp();
-      mbar_arrive_warp(bars + (Q_EMPTY + ib) * 8);
+      mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);
       const int my_tiles = unit.w, len = unit.z, h = common.z;
       const int br = unit.x, q = unit.y + m;  // pair row, query position
       const bool uniform = (common.w >> w) & 1;

@@ -362,6 +362,13 @@ __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
       "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(bar)
       : "memory");
 }
+// An arrival that hands shared memory back right after it was read, before the values have been used: the fence makes
+// the loads complete first (without it the next TMA write overtook them now and then).
+__device__ __forceinline__ void mbar_arrive_warp_after_reads(uint32_t bar) {
+  __threadfence_block();
+  __syncwarp();
+  mbar_arrive_warp(bar);
+}
 // Arrives on `bar` once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(

@@ -8,22 +8,22 @@
 // position, applies rstd·(D − mean·rowsum) + const with the statistics the statistics warps computed from the two
 // tiles while the MMAs ran - neither tile is rewritten and the MMAs wait for nothing but the loads.
 //
-// The residual is read from the z tile in shared memory, and the result takes its place there, from where TMA stores it:
-// with a thread per position, 32-byte global accesses of a warp go to 32 rows and occupy the load-store unit for some 56
-// clocks each, which bounded the kernel (148 us at 768 tokens, 3.1 TB/s of the 768 bytes per position).  The fp32 form
-// stores its 64 KiB tile from the places of both input tiles.
+// The residual is read from the z tile in shared memory, and the result leaves through a slab per warp (32 positions of
+// 64 bytes) and TMA: with a thread per position, 32-byte global accesses of a warp go to 32 rows and occupy the load-store
+// unit for some 56 clocks each, which bounded the kernel (148 us at 768 tokens, 3.1 TB/s of the 768 bytes per position).
+// What bounds it now is the time from a tile's load to the reuse of its stage, with room for two (the weights take 64
+// KiB): some 3600 clocks of latency, 1900 of statistics, then the epilogue copies the residual and hands the stage back.
 //
-// Warp roles (480 threads): warps 0-7 epilogue (thread = position; the two warpgroups take alternate groups of 32
-// output channels), warps 8-11 statistics (z rows: one thread per position; x columns: a thread takes two
-// neighbouring positions over half of the channels), warp 12 TMA producer, warp 13 MMA issuer / TMEM owner, warp 14
-// TMA stores.
+// Warp roles (576 threads): warps 0-7 epilogue (thread = position; the two warpgroups take alternate groups of 32
+// output channels), warps 8-11 statistics of the z rows (one thread per position), warps 12-15 of the x columns (a thread
+// takes two neighbouring positions over half of the channels), warp 16 TMA producer, warp 17 MMA issuer / TMEM owner.
 #include "common.cuh"
 #include "layout.h"
 
 namespace b200ta {
 namespace {
 
-constexpr int kThreads = 480;
+constexpr int kThreads = 576;
 constexpr int kTileM = 128;
 constexpr int kSmW = 0;                      // W_go' and W_po': 2 matrices x 2 K-halves x 128 rows x 128 B
 constexpr int kSmZ = kSmW + 65536;           // 2 stages x 32 KiB
@@ -31,9 +31,9 @@ constexpr int kSmX = kSmZ + 2 * 32768;       // 2 stages x 32 KiB
 constexpr int kSmConst = kSmX + 2 * 32768;   // per channel pair: float4 [64] {c_gate0, c_gate1, rowsum_g0, rowsum_g1}, float4 [64] {c_p0, c_p1, rowsum_p0, rowsum_p1}
 constexpr int kSmStats = kSmConst + 2048;    // 4 slots (tile i uses slot i & 3) x { float4 [128] {rstd_o, -mean_o*rstd_o, rstd_i, -mean_i*rstd_i}, float [128] mask }
 constexpr int kStatsSlot = 2048 + 512;
-constexpr int kSmXch = kSmStats + 4 * kStatsSlot;  // 2 x float4 [128] partial x statistics (alternating per tile)
-constexpr int kSmBars = kSmXch + 2 * 2048;
-enum Bar { W_FULL = 0, IN_FULL = 1, READY = 3, IN_EMPTY = 7, ACC_FULL = 9, ACC_EMPTY = 11, XCH = 13, OUT_FULL = 14, NUM_BARS = 16 };
+constexpr int kSmOut = kSmStats + 4 * kStatsSlot;  // 8 warps x 2 KiB: 32 positions x 64 bytes
+constexpr int kSmBars = kSmOut + 8 * 2048;
+enum Bar { W_FULL = 0, IN_FULL = 1, READY = 3, IN_EMPTY = 7, ACC_FULL = 9, ACC_EMPTY = 11, NUM_BARS = 13 };
 constexpr int kSmTotal = kSmBars + 256;
 constexpr int kSmDynamic = kSmTotal + 1024;
 
@@ -71,21 +71,18 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     mbar_init(bars + W_FULL * 8, 1);
-    mbar_init(bars + XCH * 8, 4);
     // statistics written (the four statistics warps): one barrier per statistics slot, because the statistics of
     // tile t + 2 may be complete before the epilogue of tile t has looked at its barrier
-    for (int i = 0; i < 4; ++i) mbar_init(bars + (READY + i) * 8, 4);
+    for (int i = 0; i < 4; ++i) mbar_init(bars + (READY + i) * 8, 8);
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + (IN_FULL + i) * 8, 1);
-      // MMA commit and statistics warps (have read the tiles), store warp (has read the result in their place)
-      mbar_init(bars + (IN_EMPTY + i) * 8, 6);
-      mbar_init(bars + (OUT_FULL + i) * 8, 8);
+      mbar_init(bars + (IN_EMPTY + i) * 8, 1 + 8 + 8);  // MMA commit, statistics, epilogue (residual) have read the tiles
       mbar_init(bars + (ACC_FULL + i) * 8, 1);
       mbar_init(bars + (ACC_EMPTY + i) * 8, 8);
     }
     fence_mbar_init();
   }
-  if (warp == 13) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   // per-channel constants of the epilogue
   if (threadIdx.x < kC / 2) {
     const int c = 2 * threadIdx.x;
@@ -99,7 +96,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
-  if (warp == 12) {
+  if (warp == 16) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_z);
@@ -130,7 +127,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         mbar_wait(bars + (IN_FULL + (last & 1)) * 8, (last >> 1) & 1, abort_flag + 1);
       }
     }
-  } else if (warp == 13) {
+  } else if (warp == 17) {
     // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
     constexpr uint32_t idesc_g = make_idesc_bf16(kTileM, kC);               // both operands K-major
     constexpr uint32_t idesc_p = make_idesc_bf16(kTileM, kC, true, false);  // A (the x tile) MN-major
@@ -160,36 +157,11 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       umma_commit_warp(bars + (ACC_FULL + slot) * 8);
       umma_commit_warp(bars + (IN_EMPTY + stage) * 8);
     }
-  } else if (warp == 14) {
-    // ------------------------------------------------------------------ TMA stores
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_out);
-      pdl_wait();
-      for (int it = 0; it < my_tiles; ++it) {
-        const int tile = blockIdx.x + it * gridDim.x;
-        const int jt = tile % p.tiles_j, bi = tile / p.tiles_j;
-        const int i = bi % p.N, b = bi / p.N;
-        const int stage = it & 1;
-        if (!mbar_wait(bars + (OUT_FULL + stage) * 8, (it >> 1) & 1, abort_flag)) break;
-        if (kF32) {  // four blocks of 32 channels: two in the place of the z tile, two in that of the x tile
-          for (int g = 0; g < 4; ++g)
-            tma_store_4d(&tm_out, base + (g < 2 ? kSmZ : kSmX) + stage * 32768 + (g & 1) * 16384, g * 32, jt * kTileM, i, b);
-        } else {
-          for (int h = 0; h < 2; ++h)
-            tma_store_4d(&tm_out, base + kSmZ + stage * 32768 + h * 16384, h * 64, jt * kTileM, i, b);
-        }
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(bars + (IN_EMPTY + stage) * 8);
-      }
-      tma_store_wait_all();
-    }
-  } else if (warp >= 8) {
-    // ------------------------------------------------------------------ normaliser
+  } else if (warp >= 8 && warp < 12) {
+    // ------------------------------------------------------------------ statistics of the z rows
     pdl_wait();
     const int t = (warp - 8) * 32 + lane;
-    bool ok = true;
-    for (int it = 0; ok && it < my_tiles; ++it) {
+    for (int it = 0; it < my_tiles; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       const int jt = tile % p.tiles_j, bi = tile / p.tiles_j;
       const int i = bi % p.N, b = bi / p.N;
@@ -197,14 +169,29 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       const int j = jt * kTileM + t;
       float mval = 1.f;
       if (p.mask != nullptr) mval = j < p.N ? __ldg(p.mask + b * p.ms_b + i * p.ms_i + (long long)j * p.ms_j) : 0.f;
-      ok = mbar_wait(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, abort_flag);
-      if (!ok) break;
-      // ---- z row t (nothing is written back)
-      const float2 zi = row_stats_128(base + kSmZ + stage * 32768, t, p.eps);
+      if (!mbar_wait(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, abort_flag)) break;
+      const float2 v = row_stats_128(base + kSmZ + stage * 32768, t, p.eps);
+      // Statistics and mask go to one of four slots: the epilogue of a tile may still read its slot while the
+      // next two tiles' statistics are written.
+      uint8_t* slot = gen + kSmStats + (it & 3) * kStatsSlot;
+      reinterpret_cast<float2*>(slot)[2 * t + 1] = v;
+      reinterpret_cast<float*>(slot + 2048)[t] = mval;
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bars + (READY + (it & 3)) * 8);
+        mbar_arrive(bars + (IN_EMPTY + stage) * 8);  // done reading the tile
+      }
+    }
+  } else if (warp >= 12 && warp < 16) {
+    // ------------------------------------------------------------------ statistics of the x columns
+    pdl_wait();
+    for (int it = 0; it < my_tiles; ++it) {
+      const int stage = it & 1;
+      if (!mbar_wait(bars + (IN_FULL + stage) * 8, (it >> 1) & 1, abort_flag)) break;
       // ---- x columns: this thread takes positions 2q, 2q+1 over channels [64 h, 64 h + 64), in one pass of packed sums
       // shifted by the first channel (as row_stats_128)
       {
-        const int q = t & 63, h = t >> 6;
+        const int q = (warp - 12) * 16 + (lane & 15), h = lane >> 4;
         const int jj = (2 * q) & 63;
         const uint32_t x0 = base + kSmX + stage * 32768 + ((2 * q) >> 6) * 16384 + h * 8192 + (jj & 7) * 2;
         const uint32_t chunk = uint32_t(jj >> 3);
@@ -222,37 +209,24 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         float s0, s1, q0, q1;
         unpack_f32x2(add_f32x2(sa[0], sa[1]), s0, s1);
         unpack_f32x2(add_f32x2(sq[0], sq[1]), q0, q1);
-        // mean and sum of squared deviations of the 64 channels
-        reinterpret_cast<float4*>(gen + kSmXch + (it & 1) * 2048)[t] =
-            make_float4(s0 * (1.f / 64) + k0, fmaxf(q0 - s0 * s0 * (1.f / 64), 0.f), s1 * (1.f / 64) + k1,
-                        fmaxf(q1 - s1 * s1 * (1.f / 64), 0.f));
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + XCH * 8);
-      ok = mbar_wait(bars + XCH * 8, it & 1, abort_flag);
-      if (!ok) break;
-      {
-        // position t = 2q + e: combine the two channel halves (means m, sums of squared deviations Q of 64 each)
-        const int q = t >> 1, e = t & 1;
-        const float4 a = reinterpret_cast<const float4*>(gen + kSmXch + (it & 1) * 2048)[q];
-        const float4 c = reinterpret_cast<const float4*>(gen + kSmXch + (it & 1) * 2048)[64 + q];
-        const float ma = e ? a.z : a.x, qa = e ? a.w : a.y, mc = e ? c.z : c.x, qc = e ? c.w : c.y;
-        const float mean = 0.5f * (ma + mc);
-        const float var = (qa + qc + (ma - mc) * (ma - mc) * 32.f) * (1.f / kTriHidden);
+        // Mean and sum of squared deviations of the 64 channels, combined with those of the other half of the channels
+        // in lane ^ 16; lanes 0-15 write position 2q, lanes 16-31 position 2q + 1.
+        const float m0 = s0 * (1.f / 64) + k0, m1 = s1 * (1.f / 64) + k1;
+        const float d0 = fmaxf(q0 - s0 * s0 * (1.f / 64), 0.f), d1 = fmaxf(q1 - s1 * s1 * (1.f / 64), 0.f);
+        const float mo = __shfl_xor_sync(0xffffffffu, h ? m0 : m1, 16), qo = __shfl_xor_sync(0xffffffffu, h ? d0 : d1, 16);
+        const float mm = h ? m1 : m0, qm = h ? d1 : d0;
+        const float mean = 0.5f * (mm + mo);
+        const float var = (qm + qo + (mm - mo) * (mm - mo) * 32.f) * (1.f / kTriHidden);
         const float rstd = rsqrtf(var + p.eps);
-        // Statistics and mask go to one of four slots: the epilogue of a tile may still read its slot while the
-        // next two tiles' statistics are written (the stage itself is handed back below, before the epilogue ran).
-        uint8_t* slot = gen + kSmStats + (it & 3) * kStatsSlot;
-        reinterpret_cast<float4*>(slot)[t] = make_float4(rstd, -mean * rstd, zi.x, zi.y);
-        reinterpret_cast<float*>(slot + 2048)[t] = mval;
+        reinterpret_cast<float2*>(gen + kSmStats + (it & 3) * kStatsSlot)[2 * (2 * q + h)] = make_float2(rstd, -mean * rstd);
       }
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(bars + (READY + (it & 3)) * 8);
-        mbar_arrive(bars + (IN_EMPTY + stage) * 8);  // done reading the two tiles
+        mbar_arrive(bars + (IN_EMPTY + stage) * 8);  // done reading the tile
       }
     }
-  } else {
+  } else if (warp < 8) {
     // ------------------------------------------------------------------ epilogue warps: one thread per position
     pdl_wait();
     const int e = warp >> 2;
@@ -260,8 +234,13 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
     const float4* c4 = reinterpret_cast<const float4*>(gen + kSmConst);         // per channel pair
     const float4* c4b = reinterpret_cast<const float4*>(gen + kSmConst + 1024);  // per channel pair
+    const uint32_t slab = base + kSmOut + warp * 2048;
     bool ok = true;
     for (int it = 0; ok && it < my_tiles; ++it) {
+      const int tile = blockIdx.x + it * gridDim.x;
+      const int jt = tile % p.tiles_j, bi = tile / p.tiles_j;
+      const int i = bi % p.N, b = bi / p.N;
+      const int j0 = jt * kTileM + (warp & 3) * 32;  // the warp's first position
       const int slot = it & 1;
       // (IN_FULL is complete, or there would be no statistics: it makes the copies' writes visible to this thread)
       ok = mbar_wait2_warp(bars + (READY + (it & 3)) * 8, (it >> 2) & 1, bars + (ACC_FULL + slot) * 8, (it >> 1) & 1, abort_flag) &&
@@ -269,49 +248,35 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
       if (!ok) break;
       tc_fence_after();
       const uint32_t row = base + kSmZ + slot * 32768 + sw128_offset(m, 0);  // chunk c of a row lies at chunk c ^ (row % 8)
-      uint32_t res[2][16];
-      if (kF32) {  // the result needs the room of the residuals of both warpgroups: read them first
+      uint32_t res[2][16];  // the residual of this thread's channel groups e and e + 2
 #pragma unroll
-        for (int gi = 0; gi < 2; ++gi)
+      for (int gi = 0; gi < 2; ++gi)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 x = lds128((row + gi * 16384) ^ ((e * 4 + c) << 4));
-            res[gi][c * 4 + 0] = x.x, res[gi][c * 4 + 1] = x.y, res[gi][c * 4 + 2] = x.z, res[gi][c * 4 + 3] = x.w;
-          }
-        named_bar_sync(1 + (warp & 3), 64);  // the two warps of these 32 rows
-      }
+        for (int c = 0; c < 4; ++c) {
+          const uint4 x = lds128((row + gi * 16384) ^ ((e * 4 + c) << 4));
+          res[gi][c * 4 + 0] = x.x, res[gi][c * 4 + 1] = x.y, res[gi][c * 4 + 2] = x.z, res[gi][c * 4 + 3] = x.w;
+        }
+      mbar_arrive_warp_after_reads(bars + (IN_EMPTY + slot) * 8);
       const uint8_t* stats = gen + kSmStats + (it & 3) * kStatsSlot;
       const float4 stv = reinterpret_cast<const float4*>(stats)[m];
       const float mval = reinterpret_cast<const float*>(stats + 2048)[m];
       const uint64_t rstd2 = pack_f32x2(stv.x, stv.x), nmr2 = pack_f32x2(stv.y, stv.y), mval2 = pack_f32x2(mval, mval);
       const uint64_t rstdg2 = pack_f32x2(stv.z, stv.z), nmrg2 = pack_f32x2(stv.w, stv.w);
       const uint64_t half2 = pack_f32x2(0.5f, 0.5f);
-      // four chunks of 16 output channels: [32 g + 16 h, +16) for this warpgroup's groups g = e, e + 2; the TMEM
-      // loads of the next chunk are in flight while this one is computed
-      uint32_t ag[2][16], ap[2][16];
+      // four chunks of 16 output channels: [32 g + 16 h, +16) for this warpgroup's groups g = e, e + 2
       const uint32_t acc = lane_taddr + slot * 256;
-      tmem_ld16(acc + e * 32, ag[0]);
-      tmem_ld16(acc + 128 + e * 32, ap[0]);
 #pragma unroll
       for (int ck = 0; ck < 4; ++ck) {
         const int g = e + 2 * (ck >> 1), h = ck & 1;
         const int ch0 = g * 32 + h * 16;
+        uint32_t xg[16], xp[16];
+        tmem_ld16(acc + ch0, xg);
+        tmem_ld16(acc + 128 + ch0, xp);
         tmem_ld_wait();
-        if (ck + 1 < 4) {
-          const int gn = e + 2 * ((ck + 1) >> 1), hn = (ck + 1) & 1;
-          tmem_ld16(acc + gn * 32 + hn * 16, ag[(ck + 1) & 1]);
-          tmem_ld16(acc + 128 + gn * 32 + hn * 16, ap[(ck + 1) & 1]);
-        }
-        const uint32_t (&xg)[16] = ag[ck & 1];
-        const uint32_t (&xp)[16] = ap[ck & 1];
-        // 16 channels of the residual: two 16-byte chunks of this row, whose place the bf16 result takes
-        const uint32_t place = row + (g >> 1) * 16384;
-        if (!kF32) {
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const uint4 x = lds128(place ^ (((g & 1) * 4 + h * 2 + c) << 4));
-            res[0][c * 4 + 0] = x.x, res[0][c * 4 + 1] = x.y, res[0][c * 4 + 2] = x.z, res[0][c * 4 + 3] = x.w;
-          }
+        // a slab holds 32 bf16 or 16 float channels of the warp's 32 positions
+        if (kF32 || h == 0) {
+          if (lane == 0) tma_store_wait_read<0>();
+          __syncwarp();
         }
         uint32_t packed[8];
 #pragma unroll
@@ -328,16 +293,15 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
           const uint64_t s2 = fma_f32x2(pack_f32x2(tanh_approx(a0), tanh_approx(a1)), half2, half2);
           const uint64_t v2 = fma_f32x2(rstd2, pack_f32x2(__uint_as_float(xp[2 * c]), __uint_as_float(xp[2 * c + 1])),
                                         fma_f32x2(nmr2, pack_f32x2(kb.z, kb.w), pack_f32x2(kb.x, kb.y)));
-          const uint32_t r = !p.add_residual ? 0u : kF32 ? res[ck >> 1][h * 8 + c] : res[0][c];
+          const uint32_t r = p.add_residual ? res[ck >> 1][h * 8 + c] : 0u;
           float o0, o1;
           unpack_f32x2(mul_f32x2(fma_f32x2(s2, v2, pack_f32x2(bf16_lo(r), bf16_hi(r))), mval2), o0, o1);
           if (kF32) {
             packed[(2 * c) & 7] = __float_as_uint(o0), packed[(2 * c + 1) & 7] = __float_as_uint(o1);
             if ((c & 3) == 3) {
-              const uint32_t dst = base + (g < 2 ? kSmZ : kSmX) + slot * 32768 + (g & 1) * 16384 + sw128_offset(m, 0);
 #pragma unroll
               for (int q = 0; q < 2; ++q)
-                sts128(dst ^ ((h * 4 + (c - 3) / 2 + q) << 4), make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]));
+                sts128(slab + sw64_offset(lane, (c - 3) / 2 + q), make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]));
             }
           } else {
             packed[c] = pack_bf16x2(o0, o1);
@@ -346,21 +310,28 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
         if (!kF32) {
 #pragma unroll
           for (int c = 0; c < 2; ++c)
-            sts128(place ^ (((g & 1) * 4 + h * 2 + c) << 4), make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]));
+            sts128(slab + sw64_offset(lane, h * 2 + c), make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]));
+        }
+        if (kF32 || h == 1) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && j0 < p.N) {
+            tma_store_4d(&tm_out, slab, kF32 ? ch0 : g * 32, j0, i, b);
+            tma_store_commit();
+          }
         }
       }
       tc_fence_before();
-      fence_proxy_async_smem();
       __syncwarp();
       mbar_arrive_warp(bars + (ACC_EMPTY + slot) * 8);
-      mbar_arrive_warp(bars + (OUT_FULL + slot) * 8);
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 13) {
+  if (warp == 17) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -403,8 +374,8 @@ int launch_output(const void* z, int64_t zs_b, int64_t zs_i, int64_t zs_j, const
     constexpr int kBytes = kF32 ? 4 : 2;
     auto fix_out = [](int64_t stride, int extent) -> uint64_t { return uint64_t(extent == 1 ? 128 : stride) * kBytes; };
     uint64_t ostrides[3] = {fix_out(os_j, N), fix_out(os_i, N), fix_out(os_b, B)};
-    box[0] = 128 / kBytes;
-    rc = encode_tensor_map(&tm_out, out, kBytes, 4, dims, ostrides, box, SWZ_128, "trimul_output out");
+    uint32_t obox[4] = {64 / kBytes, 32, 1, 1};
+    rc = encode_tensor_map(&tm_out, out, kBytes, 4, dims, ostrides, obox, SWZ_64, "trimul_output out");
     if (rc != B200TA_OK) return rc;
   }
   {
