@@ -4,25 +4,33 @@
 // writes a and b channel-major with the contraction index k contiguous (for the incoming node it walks the pair
 // tensor through swapped strides, so the same layout serves both directions), so both operands are K-major.
 //
-// One CTA computes [128 x 256] output tiles: TMA loads [128 x 64] / [256 x 64] operand tiles into a four-stage
-// ring, one thread issues tcgen05.mma (M 128, N 256, K 16) into one of two TMEM accumulators, and four epilogue
-// warps (TMEM lane = output row) convert the finished accumulator to bf16 and write 512 contiguous bytes per
-// thread while the next tile's MMAs run.
+// Bound: the operand tiles' way from L2 (12.8 TB/s reached).  With [128 x 256] output tiles and two accumulators of them
+// (the epilogue of one beside the MMAs of the other) every 64-wide K step of 548 clocks of MMAs asked for 48 KiB, which L2
+// does not deliver: 106 us at 768 tokens, half of the tensor cores' rate.  A CTA now computes [256 x 256] tiles, two
+// accumulators of 128 rows side by side in all of tensor memory: 64 KiB per step and twice the MMAs.  The epilogue is no
+// longer hidden behind MMAs, but behind the next tile's loads.  Column tiles are as wide as the token count needs (a
+// multiple of 32), a lower half without rows is left out.  768 tokens 106 -> 98 us; at 512 tokens (46 us) and 64 x 256
+// (522 us) the bytes from HBM bound it as before.
 //
-// Warp roles (192 threads): warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer / TMEM owner.
+// TMA loads [256 x 64] operand tiles into a three-stage ring, one warp issues tcgen05.mma (M 128, N up to 256, K 16), and
+// eight epilogue warps (TMEM lane = output row) convert the finished accumulators to bf16, stage 32 rows of 64 bytes each
+// and store them by TMA (a lane's own 32-byte stores of 32 rows occupy the load-store unit for some 56 clocks).
+//
+// Warp roles (320 threads): warps 0-7 epilogue, warp 8 TMA producer, warp 9 MMA issuer / TMEM owner.
 #include "common.cuh"
 #include "layout.h"
 
 namespace b200ta {
 namespace {
 
-constexpr int kThreads = 192;
-constexpr int kBM = 128, kBN = 256, kBK = 64;
-constexpr int kStages = 4;
-constexpr int kStageBytes = (kBM + kBN) * kBK * 2;  // 48 KiB
-constexpr int kSmBars = kStages * kStageBytes;
+constexpr int kThreads = 320;
+constexpr int kBM = 256, kBN = 256, kBK = 64;
+constexpr int kStages = 3;
+constexpr int kStageBytes = (kBM + kBN) * kBK * 2;  // 64 KiB
+constexpr int kSmOut = kStages * kStageBytes;       // 8 warps x 2 slabs x 2 KiB: 32 rows of 64 bytes
+constexpr int kSmBars = kSmOut + 8 * 2 * 2048;
 enum Bar { FULL = 0, EMPTY = kStages, ACC_FULL = 2 * kStages, ACC_EMPTY = 2 * kStages + 2, NUM_BARS = 2 * kStages + 4 };
-constexpr int kSmTotal = kSmBars + 256;
+constexpr int kSmTotal = kSmBars + 128;
 constexpr int kSmDynamic = kSmTotal + 1024;
 
 struct ContractParams {
@@ -30,8 +38,7 @@ struct ContractParams {
   int planes;     // B * hidden
   int hidden;     // channels per batch item (a planes first, b planes next)
   int tiles_m, tiles_n, num_tiles;
-  __nv_bfloat16* x;
-  long long x_plane, x_row;  // element strides of x[plane][i][j]
+  int width;  // columns of a tile, a multiple of 32
   int* status;
 };
 
@@ -47,19 +54,13 @@ __device__ __forceinline__ Tile decode_tile(const ContractParams& p, int t) {
   const int b = r.plane / p.hidden, d = r.plane - b * p.hidden;
   r.a_plane = b * 2 * p.hidden + d;
   r.b_plane = r.a_plane + p.hidden;
-  r.m0 = mt * kBM, r.n0 = nt * kBN;
+  r.m0 = mt * kBM, r.n0 = nt * p.width;
   return r;
 }
 
-// 32-byte store; the address must be 32-byte aligned.
-__device__ __forceinline__ void stg256(void* p, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
-trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const ContractParams p) {
+trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_constant__ CUtensorMap tm_x,
+                       const ContractParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -81,7 +82,7 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const Contract
     }
     fence_mbar_init();
   }
-  if (warp == 5) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   pdl_wait();
   tc_fence_before();
   __syncthreads();
@@ -91,98 +92,122 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const Contract
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
   const int ksteps = (p.N + kBK - 1) / kBK;
 
-  if (warp == 4) {
+  if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_ab);
       int g = 0;  // ring position
       bool ok = true;
+      const bool wide = p.width > 128;
       for (int i = 0; ok && i < my_tiles; ++i) {
         const Tile t = decode_tile(p, blockIdx.x + i * gridDim.x);
+        const bool lower = t.m0 + 128 < p.N;
         for (int ks = 0; ks < ksteps; ++ks, ++g) {
           const int stage = g % kStages;
           ok = mbar_wait(bars + (EMPTY + stage) * 8, ((g / kStages) & 1) ^ 1, abort_flag);
           if (!ok) break;
           const uint32_t full = bars + (FULL + stage) * 8;
-          const uint32_t sa = base + stage * kStageBytes;
-          mbar_expect_tx(full, kStageBytes);
+          const uint32_t sa = base + stage * kStageBytes, sb = sa + kBM * kBK * 2;
+          mbar_expect_tx(full, (2 + lower + wide) * 128 * kBK * 2);
           tma_load_3d(sa, &tm_ab, full, ks * kBK, t.m0, t.a_plane);
-          tma_load_3d(sa + kBM * kBK * 2, &tm_ab, full, ks * kBK, t.n0, t.b_plane);
-          tma_load_3d(sa + kBM * kBK * 2 + 128 * kBK * 2, &tm_ab, full, ks * kBK, t.n0 + 128, t.b_plane);
+          if (lower) tma_load_3d(sa + 128 * kBK * 2, &tm_ab, full, ks * kBK, t.m0 + 128, t.a_plane);
+          tma_load_3d(sb, &tm_ab, full, ks * kBK, t.n0, t.b_plane);
+          if (wide) tma_load_3d(sb + 128 * kBK * 2, &tm_ab, full, ks * kBK, t.n0 + 128, t.b_plane);
         }
       }
       // If the loop was abandoned, give copies still in flight a bounded chance to land.
-      if (*abort_flag && g > 0) mbar_wait(bars + (FULL + (g - 1) % kStages) * 8, ((g - 1) / kStages) & 1, abort_flag + 1);
+      if (*abort_flag)
+        for (int j = g > kStages ? g - kStages : 0; j < g; ++j)
+          mbar_wait(bars + (FULL + j % kStages) * 8, (j / kStages) & 1, abort_flag + 1);
     }
-  } else if (warp == 5) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kBM, kBN);
-      int g = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; ++i) {
-        const int slot = i & 1;
-        ok = mbar_wait(bars + (ACC_EMPTY + slot) * 8, ((i >> 1) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + slot * kBN;
-        for (int ks = 0; ks < ksteps; ++ks, ++g) {
-          const int stage = g % kStages;
-          ok = mbar_wait(bars + (FULL + stage) * 8, (g / kStages) & 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t sa = base + stage * kStageBytes;
-          // [rows][64 k] tiles with 128-byte swizzle: 8-row groups 1 KiB apart; a K step of 16 = 32 bytes
-          const uint64_t da = make_smem_desc(sa, 16, 1024, kLayoutSw128);
-          const uint64_t db = make_smem_desc(sa + kBM * kBK * 2, 16, 1024, kLayoutSw128);
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) umma_ss(d, da + k * 2, db + k * 2, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-          umma_commit(bars + (EMPTY + stage) * 8);  // the stage is free once these MMAs have read it
-        }
-        if (!ok) break;
-        umma_commit(bars + (ACC_FULL + slot) * 8);
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ epilogue warps
-    const int m = warp * 32 + lane;  // output row inside the tile == TMEM lane
-    const uint32_t lane_taddr = tmem_base + (uint32_t(warp * 32) << 16);
+  } else if (warp == 9) {
+    // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
+    const uint32_t idesc = make_idesc_bf16(128, p.width);
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int g = 0;
     bool ok = true;
     for (int i = 0; ok && i < my_tiles; ++i) {
       const Tile t = decode_tile(p, blockIdx.x + i * gridDim.x);
-      const int slot = i & 1;
-      ok = mbar_wait(bars + (ACC_FULL + slot) * 8, (i >> 1) & 1, abort_flag);
+      const bool lower = t.m0 + 128 < p.N;
+      for (int ks = 0; ks < ksteps; ++ks, ++g) {
+        const int stage = g % kStages;
+        ok = mbar_wait_warp(bars + (FULL + stage) * 8, (g / kStages) & 1, abort_flag);
+        // each accumulator is handed over on its own, so that a tile's first half starts while the second half of the
+        // tile before is still being stored (both are handed over each tile, also when the lower half was left out)
+        if (ok && ks == 0) ok = mbar_wait_warp(bars + ACC_EMPTY * 8, (i & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sa = base + stage * kStageBytes;
+        // [rows][64 k] tiles with 128-byte swizzle: 8-row groups 1 KiB apart; a K step of 16 = 32 bytes
+        const uint64_t da = smem_desc<16, 1024, kLayoutSw128>(sa);
+        const uint64_t db = smem_desc<16, 1024, kLayoutSw128>(sa + kBM * kBK * 2);
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k) umma_ss_warp(tb, da + k * 2, db + k * 2, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+        if (ks == ksteps - 1) umma_commit_warp(bars + ACC_FULL * 8);
+        if (ks == 0) {
+          ok = mbar_wait_warp(bars + (ACC_EMPTY + 1) * 8, (i & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        if (lower) {
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_ss_warp(tb + kBN, da + (16384 >> 4) + k * 2, db + k * 2, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit_warp(bars + (EMPTY + stage) * 8);  // the stage is free once these MMAs have read it
+      }
+      if (!ok) break;
+      umma_commit_warp(bars + (ACC_FULL + 1) * 8);
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue warps
+    const int half = warp >> 2;             // which accumulator
+    const int m = (warp & 3) * 32;          // first output row of the warp == TMEM lane
+    const uint32_t acc = tmem_base + (uint32_t(m) << 16) + half * kBN;
+    const uint32_t slab0 = base + kSmOut + warp * 4096;
+    bool ok = true;
+    for (int i = 0; ok && i < my_tiles; ++i) {
+      const Tile t = decode_tile(p, blockIdx.x + i * gridDim.x);
+      ok = mbar_wait_warp(bars + (ACC_FULL + half) * 8, i & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      const int row = t.m0 + m;
-      __nv_bfloat16* dst = p.x + t.plane * p.x_plane + (long long)row * p.x_row + t.n0;
-      uint32_t acc[2][32];
-      tmem_ld32(lane_taddr + slot * kBN, acc[0]);
+      const int row0 = t.m0 + half * 128 + m;
+      if (row0 < p.N) {
+        const int columns = p.width < p.N - t.n0 ? p.width : p.N - t.n0;
+        for (int c = 0; c < columns; c += 32) {
+          uint32_t a[32];
+          tmem_ld32(acc + c, a);
+          const uint32_t slab = slab0 + ((c >> 5) & 1) * 2048;
+          if (lane == 0) tma_store_wait_read<1>();  // the store before the previous one has read this slab
+          __syncwarp();
+          tmem_ld_wait();
+          uint32_t packed[16];
 #pragma unroll
-      for (int g = 0; g < kBN / 32; ++g) {
-        tmem_ld_wait();
-        if (g + 1 < kBN / 32) tmem_ld32(lane_taddr + slot * kBN + (g + 1) * 32, acc[(g + 1) & 1]);
-        const uint32_t (&a)[32] = acc[g & 1];
-        uint32_t packed[16];
+          for (int j = 0; j < 16; ++j) packed[j] = pack_bf16x2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
 #pragma unroll
-        for (int j = 0; j < 16; ++j) packed[j] = pack_bf16x2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
-        // columns past the row pitch are never written; columns between N and the pitch receive zeros (the
-        // operand rows past N are zero-filled by the TMA loads)
-        if (row < p.N) {
-          if (t.n0 + g * 32 + 16 <= p.x_row) stg256(dst + g * 32, packed);
-          if (t.n0 + g * 32 + 32 <= p.x_row) stg256(dst + g * 32 + 16, packed + 8);
+          for (int j = 0; j < 4; ++j)
+            sts128(slab + sw64_offset(lane, j), make_uint4(packed[j * 4], packed[j * 4 + 1], packed[j * 4 + 2], packed[j * 4 + 3]));
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            // rows past the token count and columns past the row pitch are not written; columns between the token count
+            // and the pitch receive zeros (the operand rows past the token count are zero-filled by the loads)
+            tma_store_3d(&tm_x, slab, t.n0 + c, row0, t.plane);
+            tma_store_commit();
+          }
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars + (ACC_EMPTY + slot) * 8);
+      mbar_arrive_warp(bars + (ACC_EMPTY + half) * 8);
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) {
+  if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -216,18 +241,26 @@ int b200ta_trimul_contract(const void* ab, void* x, int B, int N, int64_t pitch,
     rc = encode_tensor_map(&tm_ab, ab, 2, 3, dims, strides, box, SWZ_128, "trimul a/b planes");
     if (rc != B200TA_OK) return rc;
   }
+  CUtensorMap tm_x;
+  {
+    // (column, row, plane): an epilogue warp's slab
+    uint64_t dims[3] = {uint64_t(pitch), uint64_t(N), uint64_t(B) * kHidden};
+    uint64_t strides[2] = {uint64_t(pitch) * 2, uint64_t(pitch) * N * 2};
+    uint32_t box[3] = {32, 32, 1};
+    rc = encode_tensor_map(&tm_x, x, 2, 3, dims, strides, box, SWZ_64, "trimul x planes");
+    if (rc != B200TA_OK) return rc;
+  }
   ContractParams p{};
   p.N = N, p.planes = B * kHidden, p.hidden = kHidden;
   p.tiles_m = (N + kBM - 1) / kBM, p.tiles_n = (N + kBN - 1) / kBN;
   const int64_t tiles = int64_t(p.planes) * p.tiles_m * p.tiles_n;
   B200TA_REQUIRE(tiles < (int64_t(1) << 31), "trimul_contract: too many tiles");
   p.num_tiles = int(tiles);
-  p.x = static_cast<__nv_bfloat16*>(x);
-  p.x_row = pitch, p.x_plane = pitch * N;
+  p.width = ((N + p.tiles_n - 1) / p.tiles_n + 31) / 32 * 32;
   p.status = st->status_dev;
 
   const int grid = p.num_tiles < st->num_sms ? p.num_tiles : st->num_sms;
-  return launch_kernel(st, kKernelContract, trimul_contract_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_ab, p);
+  return launch_kernel(st, kKernelContract, trimul_contract_kernel, dim3(grid), kThreads, kSmDynamic, stream, tm_ab, tm_x, p);
 }
 
 }  // extern "C"
