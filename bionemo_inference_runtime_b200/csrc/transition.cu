@@ -1,7 +1,9 @@
 // Pair transition for sm_100a: out = [x +] mask * ( (silu(gate) * value) · W2ᵀ ),
 // [value|gate] = LayerNorm(x) · W1ᵀ, hidden 512, one kernel, hidden kept on chip.
 // The ReLU form (kRelu) computes out = [x +] mask * ( relu(LayerNorm(x) · W1ᵀ + b1) · W2ᵀ + b2 ) with the same
-// pipeline: its 512 hidden rows sit in the value half of the packed first linear, the gate half is zero.
+// pipeline: its 512 hidden rows sit in the value half of the packed first linear.  It has no gates, so that an accumulator
+// of GEMM1 holds 128 hidden units: four of them per tile, each in two H tiles.  (With 64 values and 64 zero gates, as
+// the SwiGLU form, it had twice the hand-overs and half again the operations: 640 x 640 rows 168 us, now 163.)
 //
 // A persistent CTA per SM walks 128-row tiles of x.  The hidden dimension is cut in
 // 8 chunks of 64 units; for each chunk
@@ -27,6 +29,9 @@ constexpr int kThreads = 512;
 constexpr int kTileM = 128;
 constexpr int kChunk = 64;                 // hidden units per chunk
 constexpr int kChunks = kHidden / kChunk;  // 8
+// GEMM1 accumulators per tile: 64 value and 64 gate columns, or 128 hidden units of the ReLU form
+template <bool kRelu>
+constexpr int kSteps = kRelu ? kChunks / 2 : kChunks;
 
 struct TransParams {
   long long rows;
@@ -67,8 +72,10 @@ constexpr int kSmDynamic = kSmTotal + 1024;
 
 enum Bar {
   X_FULL = 0, X_EMPTY = 2, W1_FULL = 4, W1_EMPTY = 6, W2_FULL = 8, W2_EMPTY = 10,
-  ACC1_FULL = 12, ACC1_FREE = 14, H_FULL = 16, H_FREE = 18, ACC2_FULL = 20, ACC2_FREE = 21, XH_FULL = 22, XH_FREE = 23,
-  XN_FULL = 24, XN_EMPTY = 25, NUM_BARS = 26
+  ACC1_FULL = 12, ACC1_FREE = 14, H_FULL = 16, ACC2_FULL = 18, ACC2_FREE = 19, XH_FULL = 20, XH_FREE = 21,
+  XN_FULL = 22, XN_EMPTY = 23,
+  H_FREE = 24,  // per H buffer; ReLU form: per warpgroup that filled it and buffer
+  NUM_BARS = 28
 };
 
 // Tensor memory: two GEMM1 accumulators (64 value + 64 gate columns each), the tile's output accumulator, the
@@ -161,8 +168,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       mbar_init(bars + (ACC1_FULL + i) * 8, 1);
       mbar_init(bars + (ACC1_FREE + i) * 8, 4);
       mbar_init(bars + (H_FULL + i) * 8, 4);
-      mbar_init(bars + (H_FREE + i) * 8, 1);
     }
+    for (int i = 0; i < 4; ++i) mbar_init(bars + (H_FREE + i) * 8, 1);
     mbar_init(bars + ACC2_FULL * 8, 1);
     mbar_init(bars + ACC2_FREE * 8, 8);
     mbar_init(bars + XH_FULL * 8, 4);
@@ -260,7 +267,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         return true;
       };
       for (int i = 0; ok && i < my_tiles; ++i) {
-        for (int j = 0; j < kChunks; ++j, ++c) {
+        for (int j = 0; j < kSteps<kRelu>; ++j, ++c) {
           const int st = c & 1;
           ok = mbar_wait(bars + (W1_EMPTY + st) * 8, ((c >> 1) & 1) ^ 1, abort_flag);
           if (!ok) break;
@@ -268,8 +275,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           mbar_expect_tx(f1, 32768);
           for (int kh = 0; kh < 2; ++kh) {
             const uint32_t dst = base + kSmW1 + st * 32768 + kh * 16384;
-            tma_load_2d(dst, &tm_w1, f1, kh * 64, j * kChunk);                  // value rows
-            tma_load_2d(dst + 8192, &tm_w1, f1, kh * 64, kHidden + j * kChunk);  // gate rows
+            // 64 value rows and their gate rows, or 128 rows
+            tma_load_2d(dst, &tm_w1, f1, kh * 64, (kRelu ? 2 * j : j) * kChunk);
+            tma_load_2d(dst + 8192, &tm_w1, f1, kh * 64, kRelu ? (2 * j + 1) * kChunk : kHidden + j * kChunk);
           }
           if (c == 1) {  // the first two chunks do not depend on the kernels before this one
             pdl_wait();
@@ -321,7 +329,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       for (int i = 0; ok && i < my_tiles; ++i) {
         ok = mbar_wait_warp(bars + XH_FULL * 8, i & 1, abort_flag);  // the tile's rows are in tensor memory
         if (!ok) break;
-        for (int j = 0; ok && j < kChunks; ++j, ++c1) {
+        for (int j = 0; ok && j < kSteps<kRelu>; ++j, ++c1) {
           const int e = c1 & 1;
           const uint32_t par = (c1 >> 1) & 1;
           ok = mbar_wait_warp(bars + (W1_FULL + e) * 8, par, abort_flag) &&
@@ -338,7 +346,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           }
           umma_commit_warp(bars + (ACC1_FULL + e) * 8);
           umma_commit_warp(bars + (W1_EMPTY + e) * 8);
-          if (j == kChunks - 1) umma_commit_warp(bars + XH_FREE * 8);  // the next tile's rows may replace this tile's
+          if (j == kSteps<kRelu> - 1) umma_commit_warp(bars + XH_FREE * 8);  // the next tile's rows may replace this tile's
         }
       }
     }
@@ -364,7 +372,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 #pragma unroll
           for (int k = 1; k < 4; ++k) umma_ts_warp(d2, th + k * 8, dw + k * 2, idesc, 1u);
           umma_commit_warp(bars + (W2_EMPTY + e) * 8);
-          umma_commit_warp(bars + (H_FREE + e) * 8);
+          umma_commit_warp(bars + (H_FREE + (kRelu ? (c2 & 2) + e : e)) * 8);
           if (jj == kChunks - 1) umma_commit_warp(bars + ACC2_FULL * 8);
         }
       }
@@ -384,7 +392,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       const int xs = i & 1;
       const long long row = (long long)tile * kTileM + m;
       const uint32_t x0 = base + kSmX + xs * 32768;
-      for (int j = e; ok && j < kChunks; j += 2, ++n) {
+      for (int j = e; ok && j < kSteps<kRelu>; j += 2, ++n) {
         ok = mbar_wait(bars + (ACC1_FULL + e) * 8, n & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
@@ -394,14 +402,41 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         const uint32_t acc1 = lane_taddr + kTmemAcc1 + e * 128;
         tmem_ld32(acc1, reinterpret_cast<uint32_t(&)[32]>(xv[0]));
         tmem_ld32(acc1 + 32, reinterpret_cast<uint32_t(&)[32]>(xv[32]));
-        if (!kRelu) {
-          tmem_ld32(acc1 + 64, reinterpret_cast<uint32_t(&)[32]>(xg[0]));
-          tmem_ld32(acc1 + 96, reinterpret_cast<uint32_t(&)[32]>(xg[32]));
-        }
+        tmem_ld32(acc1 + 64, reinterpret_cast<uint32_t(&)[32]>(xg[0]));
+        tmem_ld32(acc1 + 96, reinterpret_cast<uint32_t(&)[32]>(xg[32]));
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bars + (ACC1_FREE + e) * 8);
+        if (kRelu) {
+          // 64 hidden units each in the two H buffers, whose previous use, the other warpgroup's, GEMM2 must have consumed.
+          // Each warpgroup's uses have barriers of their own: with one barrier for both, this warpgroup's previous use,
+          // still open, would look the same as the one waited for.
+#pragma unroll
+          for (int piece = 0; piece < 2; ++piece) {
+            ok = ok && mbar_wait(bars + (H_FREE + 2 * (e ^ 1) + piece) * 8, (n & 1) ^ e ^ 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t (&x)[64] = piece ? xg : xv;
+            const float2* b1s = reinterpret_cast<const float2*>(gen + kSmSc) + j * kChunk + piece * (kChunk / 2);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              uint32_t pk[16];
+#pragma unroll
+              for (int t = 0; t < 16; ++t) {
+                const float2 b = b1s[half * 16 + t];
+                const int u = half * 32 + 2 * t;
+                pk[t] = pack_bf16x2(fmaxf(__uint_as_float(x[u]) + b.x, 0.f), fmaxf(__uint_as_float(x[u + 1]) + b.y, 0.f));
+              }
+              tmem_st16(lane_taddr + kTmemH + piece * 32 + half * 16, pk);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + (H_FULL + piece) * 8);
+          }
+          continue;
+        }
         // the H buffer's previous use (two chunks back) must have been consumed by its GEMM2 (long done as a rule)
         ok = mbar_wait(bars + (H_FREE + e) * 8, (n & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -409,15 +444,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 #pragma unroll
         for (int half = 0; half < 2; ++half) {  // 32 hidden units at a time -> 16 columns of the A operand of GEMM2
           uint32_t pk[16];
-          if (kRelu) {
-            const float2* b1s = reinterpret_cast<const float2*>(gen + kSmSc) + j * (kChunk / 2) + half * 16;
-#pragma unroll
-            for (int t = 0; t < 16; ++t) {
-              const float2 b = b1s[t];
-              const int u = half * 32 + 2 * t;
-              pk[t] = pack_bf16x2(fmaxf(__uint_as_float(xv[u]) + b.x, 0.f), fmaxf(__uint_as_float(xv[u + 1]) + b.y, 0.f));
-            }
-          } else {
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
               // two hidden units at a time, packed fp32x2 math; the gate rows of W1 are halved when they are
@@ -431,7 +457,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
               unpack_f32x2(hid2, o0, o1);
               pk[t] = pack_bf16x2(o0, o1);
             }
-          }
           tmem_st16(lane_taddr + kTmemH + e * 32 + half * 16, pk);
         }
         tmem_st_wait();
