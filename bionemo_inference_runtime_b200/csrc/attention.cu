@@ -28,9 +28,9 @@
 // columns and four times the operations of Q·Kᵀ, which cost clock rate under the power cap.
 //
 // Measured (one launch, all tokens valid, before this split of two 128-key tile halves per CTA -> now): 512 tokens
-// 224 -> 206 us, 768 tokens 681 -> 640 us, 2048 tokens 12.6 -> 10.8 ms (10.9 exponentials a clock and SM; a tile of
-// four units takes some 2650 clocks, 460 instructions a warp, against 2048 at the unit's rate), an item's end and start
-// another 3500; 333 tokens with holes in the mask 190 -> 138 us.
+// 224 -> 199 us, 1024 tokens 1.41 ms, 2048 tokens 12.6 -> 10.7 ms (11.1 exponentials a clock and SM; a tile of four units
+// takes some 2600 clocks against 2048 at the unit's rate), an item's end and start another 3500; the masked form at 333
+// tokens 190 -> 110 us.
 //
 // A pair row without a valid key takes a constant path in "uniform" mode (probabilities all 1: the output is the
 // mean of V, as the eager reference computes it) and is skipped in "zeros" mode.
@@ -407,9 +407,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else if (warp < 16) {
     // ------------------------------------------------------------------ softmax warpgroups
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
-    const int w = warp >> 2;               // unit
-    const int m = (warp & 3) * 32 + lane;  // query row inside the unit == TMEM lane
-    const uint32_t lane_taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    // keep_in_register: the compiler otherwise derives these from the thread index again in every tile, waiting for the
+    // special register each time (2048 tokens 10.95 -> 10.66 ms)
+    const int w = keep_in_register(warp >> 2);               // unit
+    const int m = keep_in_register((warp & 3) * 32 + lane);  // query row inside the unit == TMEM lane
+    const uint32_t lane_taddr = keep_in_register(tmem_base + (uint32_t((warp & 3) * 32) << 16));
     const uint32_t s_addr = lane_taddr + kTmemS + (w & 1) * 64;
     const uint32_t o_addr = lane_taddr + kTmemO + w * 32;
     const float c = p.scale_log2;  // raw score -> log2-domain logit
@@ -424,18 +426,16 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const ItemInfo* info = reinterpret_cast<const ItemInfo*>(gen + kSmInfo) + ib;
       const int4 unit = *reinterpret_cast<const int4*>(&info->unit[w]);
       const int4 common = *reinterpret_cast<const int4*>(&info->tiles);
-      mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);
-      const int my_tiles = unit.w, len = unit.z, h = common.z;
-      const int br = unit.x, q = unit.y + m;  // pair row, query position
+      const int my_tiles = unit.w, len = unit.z;
       const bool uniform = (common.w >> w) & 1;
       const uint32_t block_off = stage_bias(common.y ? w & 1 : 0) + sw128_offset(m, 0);
-      const __nv_bfloat16* gate_row = p.gate + br * p.g_br + h * p.g_h + (long long)q * p.g_s;
-      if (p.gate != nullptr && q < p.S) asm volatile("prefetch.global.L2 [%0];" ::"l"(gate_row));  // read at the end
+      if (p.gate != nullptr && unit.y + m < p.S)  // read at the end
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + unit.x * p.g_br + common.z * p.g_h + (long long)(unit.y + m) * p.g_s));
       float row_max = 0.f, row_sum = 0.f;  // row_max: reference point of the exponentials, in raw score units
       const uint32_t* mask_row = nullptr;
       if (kMasked) {
-        const int b = br / p.R;
-        mask_row = p.key_mask + b * p.km_b + (br - b * p.R) * p.km_r;
+        const int b = unit.x / p.R;
+        mask_row = p.key_mask + b * p.km_b + (unit.x - b * p.R) * p.km_r;
       }
       bool have_anchor = false;            // masked form: a key tile with a valid key has been seen
 
@@ -621,7 +621,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           uint4 qv[4];
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) qv[ch] = lds128(base + kSmQ + (ib * kUnits + w) * 8192 + sw64_offset(m, ch));
-          const uint32_t k0 = bias0 - block_off + stage_k(common.y ? w >> 1 : w);
+          const uint32_t k0 = bias0 - block_off + stage_k(info->two_blocks ? w >> 1 : w);
           auto score = [&](int key) {
             float d = -INFINITY;
             bool valid = key < rem;
@@ -683,8 +683,12 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       if (!ok) break;
       // tiles of the item that only longer rows have
-      for (int kt = max(my_tiles, 0); kt < common.x; ++kt)
+      for (int kt = max(my_tiles, 0), all = info->tiles; kt < all; ++kt)
         if (++stage == kStages) stage = 0, stage_phase ^= 1;
+      // The info is read again here: kept over the tiles it cost registers that the tile loop spilled (512 tokens 204 ->
+      // 199 us, the masked form at 333 tokens 138 -> 110).
+      const int br = info->unit[w].br, q = info->unit[w].q0 + m, h = info->h;  // pair row, query position
+      mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);
       if (my_tiles < 0) continue;  // the item has no such unit
       __nv_bfloat16* out_row = p.out + br * p.o_br + (long long)q * p.o_s + h * p.o_h;
       if (my_tiles == 0) {  // no valid key and "zeros" semantics
@@ -695,6 +699,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         continue;
       }
+      const __nv_bfloat16* gate_row = p.gate + br * p.g_br + h * p.g_h + (long long)q * p.g_s;
       // the unit's output: O (in TMEM) / row_sum * gate; the gate row is fetched while the last P·V runs
       uint4 gv[4];
       if (p.gate != nullptr && q < p.S) {

@@ -115,6 +115,15 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // 32-135 KB a block needs off the critical path of a small call.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The value in a register of its own, which the compiler cannot compute again from where it came from.
+template <typename T>
+__device__ __forceinline__ T keep_in_register(T v) {
+  static_assert(sizeof(T) == 4, "one register");
+  T out;
+  asm volatile("mov.b32 %0, %1;" : "=r"(out) : "r"(v));
+  return out;
+}
+
 // ---- mbarrier --------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
