@@ -220,7 +220,6 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     fence_mbar_init();
   }
   if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
-  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -245,6 +244,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int g = 0, i = 0;  // tiles and items loaded
     bool ok = true;
     Item it = decode_item(p, blockIdx.x);
+    pdl_wait();  // (the MMA warps touch no global memory)
     int raw = raw_length(p, it, lane);
     while (i < my_items) {
       // lane u: unit u
@@ -407,6 +407,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else if (warp < 16) {
     // ------------------------------------------------------------------ softmax warpgroups
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    pdl_wait();
     // keep_in_register: the compiler otherwise derives these from the thread index again in every tile, waiting for the
     // special register each time (2048 tokens 10.95 -> 10.66 ms)
     const int w = keep_in_register(warp >> 2);               // unit
