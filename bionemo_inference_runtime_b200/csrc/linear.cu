@@ -90,8 +90,6 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
     fence_mbar_init();
   }
   if (warp == 5) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 128);
-  pdl_wait();
-  if (threadIdx.x < kTile) reinterpret_cast<float2*>(gen + kSmSc)[threadIdx.x] = p.sc[n0 + threadIdx.x];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -101,6 +99,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
     if (lane == 0) {
       tma_prefetch_desc(&tm_a);
       tma_prefetch_desc(&tm_w);
+      pdl_wait();
       int issued = 0;
       for (int kk = 0; kk < steps; ++kk) {
         const int stage = kk % kStages;
@@ -137,6 +136,9 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
       if (ok) umma_commit(bars + ACC_FULL * 8);
     }
   } else {
+    pdl_wait();
+    reinterpret_cast<float2*>(gen + kSmSc)[threadIdx.x] = p.sc[n0 + threadIdx.x];
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // the four warps of this branch
     const int m = warp * 32 + lane;
     const int row = row0 + m;
     const bool valid = row < p.rows;

@@ -83,7 +83,6 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_c
     fence_mbar_init();
   }
   if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
-  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -96,6 +95,7 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_c
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_ab);
+      pdl_wait();  // (for the whole block: the epilogue stores only what came of these loads)
       int g = 0;  // ring position
       bool ok = true;
       const bool wide = p.width > 128;
