@@ -30,7 +30,7 @@
 // Measured (one launch, all tokens valid, before this split of two 128-key tile halves per CTA -> now): 512 tokens
 // 224 -> 199 us, 1024 tokens 1.41 ms, 2048 tokens 12.6 -> 10.7 ms (11.1 exponentials a clock and SM; a tile of four units
 // takes some 2600 clocks against 2048 at the unit's rate), an item's end and start another 3500; the masked form at 333
-// tokens 190 -> 110 us.
+// tokens 190 -> 106 us.
 //
 // A pair row without a valid key takes a constant path in "uniform" mode (probabilities all 1: the output is the
 // mean of V, as the eager reference computes it) and is skipped in "zeros" mode.
@@ -687,7 +687,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int kt = max(my_tiles, 0), all = info->tiles; kt < all; ++kt)
         if (++stage == kStages) stage = 0, stage_phase ^= 1;
       // The info is read again here: kept over the tiles it cost registers that the tile loop spilled (512 tokens 204 ->
-      // 199 us, the masked form at 333 tokens 138 -> 110).
+      // 199 us, the masked form at 333 tokens 136 -> 106).
       const int br = info->unit[w].br, q = info->unit[w].q0 + m, h = info->h;  // pair row, query position
       mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);
       if (my_tiles < 0) continue;  // the item has no such unit
