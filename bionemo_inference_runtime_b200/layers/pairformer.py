@@ -30,8 +30,9 @@ from .triangle_multiplication import (TriangleMultiplicationMetadata, TriangleMu
                                       TriangleMultiplicationNodeType, precompute_trimul_metadata)
 from .triangle_nodes import _EMPTY_ROW_MODES, TriangleAttentionEndingNode, TriangleAttentionStartingNode
 
-# caller's stream -> the stream and events of the single track beside it; taken out while a call uses it
-_side_tracks: dict[int, "_host.SideTrack"] = {}
+# (device, caller's stream) -> the stream and events of the single track beside it; taken out while a call uses it.  The
+# device is part of the key because stream handles are per device: the default stream's is 0 on every one.
+_side_tracks: dict[tuple[torch.device, int], "_host.SideTrack"] = {}
 
 
 class _NativeStack:
@@ -338,14 +339,14 @@ class PairformerModule(nn.Module):
                                                                s.device)
             native = None if attn_metadatas or first.no_update_s else _native_stack(self, z)
             if native is not None:
-                stream = _host.current_stream()
-                track = _side_tracks.pop(stream, None) or _host.SideTrack()
+                key = z.device, _host.current_stream()
+                track = _side_tracks.pop(key, None) or _host.SideTrack()
                 s_out, z = native.stack.run_both(s.to(torch.bfloat16).contiguous(),
                                                  *_native_pair_inputs(first, z, pair_mask, precomputed, trimul_metadata),
                                                  kwargs["_key_counts"], buffers, track)
                 while len(_side_tracks) >= 8:  # programs use a few streams; a bounded number is kept
                     _side_tracks.pop(next(iter(_side_tracks)), None)
-                _side_tracks[stream] = track
+                _side_tracks[key] = track
                 return s_out.to(s.dtype), z
         for layer in self.layers:
             s, z = layer(s, z, mask, pair_mask, trimul_metadata, attn_metadatas, precomputed_masks=precomputed,

@@ -1,0 +1,37 @@
+"""What the native form of a stack depends on, without a GPU: the kernels' side is replaced by recorders."""
+
+from types import SimpleNamespace
+
+import torch
+
+import bionemo_inference_runtime_b200 as b200
+from bionemo_inference_runtime_b200.layers import pairformer
+
+
+def _stack(**options):
+    return b200.PairformerModule(num_blocks=2, dtype=torch.bfloat16, triangle_attn_backend="Heuristic", **options)
+
+
+def _inputs(device, n=8):
+    return (torch.zeros(1, n, 384, device=device), torch.zeros(1, n, n, 128, device=device, dtype=torch.bfloat16),
+            torch.ones(1, n), torch.ones(1, n, n))
+
+
+def test_side_track_belongs_to_the_device_and_the_stream(monkeypatch):
+    """Two devices ("cpu" and "meta" stand for them) whose current stream has the same handle take different tracks; a
+    second call on a device takes the track of the first."""
+    used = []
+
+    def run_both(s, z, *args):
+        used.append((z.device, args[-1]))
+        return s, z
+
+    monkeypatch.setattr(pairformer, "_native_stack", lambda module, z: SimpleNamespace(stack=SimpleNamespace(run_both=run_both)))
+    monkeypatch.setattr(pairformer, "_side_tracks", {})
+    monkeypatch.setattr(pairformer._host, "current_stream", lambda: 0)
+    monkeypatch.setattr(pairformer._host, "SideTrack", object)
+    stack = _stack()
+    for device in ("cpu", "meta", "cpu", "meta"):
+        stack._run(*_inputs(device), None, None)
+    tracks = [track for _, track in used]
+    assert tracks[0] is not tracks[1] and tracks[0] is tracks[2] and tracks[1] is tracks[3]
