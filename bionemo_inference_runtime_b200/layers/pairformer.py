@@ -36,11 +36,11 @@ _side_tracks: dict[tuple[torch.device, int], "_host.SideTrack"] = {}
 
 
 class _NativeStack:
-    """The packed weights of a stack in the form of ``_host.Stack``, valid for one state of its modules; not copied or
-    pickled with the module."""
+    """The packed weights of a stack in the form of ``_host.Stack``, valid on one device and for one state of its modules;
+    not copied or pickled with the module."""
 
-    def __init__(self, state: bytes, stack, chunk_policies):
-        self.state, self.stack, self.chunk_policies = state, stack, chunk_policies
+    def __init__(self, state: bytes, device: torch.device, stack, chunk_policies):
+        self.state, self.device, self.stack, self.chunk_policies = state, device, stack, chunk_policies
 
     def __deepcopy__(self, memo):
         return None
@@ -54,7 +54,7 @@ def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
     of another class, its options need the general path, or its rows are chunked at this size."""
     state = None if nn.modules.module._has_any_global_hook() else _host.stack_state(module.layers)
     held = module.__dict__.get("_native")
-    if state is None or (held is not None and held.state == state):
+    if state is None or (held is not None and held.state == state and held.device == z.device):
         native = held if state is not None else None
     elif torch.cuda.is_current_stream_capturing():
         return None  # folding weights now would only fill them at replay
@@ -64,7 +64,7 @@ def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
             id(p): p for layer in module.layers
             for p in (layer.tri_attn_start.mha.chunk_policy, layer.tri_attn_end.mha.chunk_policy) if p is not None}
         # a stack that has no native form is remembered as well
-        native = module._native = _NativeStack(state, stack, list(policies.values()))
+        native = module._native = _NativeStack(state, z.device, stack, list(policies.values()))
     if native is None or native.stack is None:
         return None
     chunked = any(p.chunk_size < z.shape[1] and p.should_chunk(z) for p in native.chunk_policies)

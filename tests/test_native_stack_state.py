@@ -35,3 +35,13 @@ def test_side_track_belongs_to_the_device_and_the_stream(monkeypatch):
         stack._run(*_inputs(device), None, None)
     tracks = [track for _, track in used]
     assert tracks[0] is not tracks[1] and tracks[0] is tracks[2] and tracks[1] is tracks[3]
+
+
+def test_packed_weights_of_one_device_are_not_used_on_another(monkeypatch):
+    built = []
+    monkeypatch.setattr(pairformer, "_build_native_stack", lambda layers, device: built.append(device) or object())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    stack = _stack()
+    for device in ("cpu", "cpu", "meta", "meta"):
+        pairformer._native_stack(stack, _inputs(device)[1])
+    assert [d.type for d in built] == ["cpu", "meta"]
