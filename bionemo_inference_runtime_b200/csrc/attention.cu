@@ -38,6 +38,7 @@
 // Warp roles (640 threads): warps 0-15 softmax (warpgroup w = unit w), warp 16 TMA producer, warp 17 score MMAs / TMEM
 // owner, warps 18 and 19 P·V MMAs of units 0-1 and 2-3.  The fifth warpgroup gives most of its registers to the softmax
 // warpgroups (setmaxnreg).
+#include "attention_items.h"
 #include "common.cuh"
 #include "layout.h"
 
@@ -45,27 +46,13 @@ namespace b200ta {
 namespace {
 
 constexpr int kThreads = 640;
-constexpr int kQTile = 128;  // queries per unit
-constexpr int kKTile = 64;   // keys per tile
-constexpr int kUnits = 4;
+constexpr int kKTile = 64;  // keys per tile
 constexpr int kStages = 3;
 constexpr float kRebaseSum = 1.2676506e30f;  // 2^100: a tile sum at or above this moves the reference point
 
-// A range of pair rows and how its units are put together: per (b, h) `pairs` x ceil(rows / rows_pair) items of two
-// query blocks, then `singles` x ceil(rows / rows_single) items of one block.  All (b, h) of group 0 come first; the
-// host chooses both in split_items().
-struct RowGroup {
-  int row0, row_end, rows_pair, rows_single;
-  int items_pair, items_bh, num_items;
-  uint32_t bh_mul, bh_shr;
-};
-
 struct AttnParams {
   int B, R, S, S_pad;
-  int pairs, singles;  // query blocks of a row: 2 * pairs + singles; the first go two by two
-  uint32_t pairs_mul, pairs_shr, singles_mul, singles_shr;  // divisions as multiply-high and shift
-  RowGroup group[2];
-  int num_items;
+  ItemPlan plan;
   const int32_t* lengths;
   long long ls_b, ls_r;
   const uint32_t* key_mask;  // masked form: bit k of word [b][r][k / 32] = key k takes part (0 at and past the length)
@@ -121,14 +108,9 @@ enum Bar {
 constexpr uint32_t kTmemS = 0, kTmemP = 128, kTmemO = 384, kTmemCols = 512;
 __device__ __forceinline__ uint32_t p_column(int unit, int buffer) { return kTmemP + unit * 64 + buffer * 32; }
 
-// n / d for n < 2^31 with the constants of fast_div_constants(); mul == 0 stands for d == 1.
-__device__ __forceinline__ int fast_div(int n, uint32_t mul, uint32_t shr) {
-  return mul ? int(__umulhi(uint32_t(n), mul) >> shr) : n;
-}
-
 // What the other warps need to know about an item, written by the TMA warp into the item's slot (released by Q_FULL).
 struct __align__(16) UnitInfo {
-  int br;     // b * R + r of the unit's pair row
+  int br;     // b * R + r of the unit's pair row; of the item's last row where the item has no such unit
   int q0;     // first query
   int len;    // keys that take part (S for a uniform row)
   int tiles;  // key tiles; 0: no valid key and "zeros" semantics; -1: the item has no such unit
@@ -142,46 +124,10 @@ struct __align__(16) ItemInfo {
 };
 static_assert(sizeof(ItemInfo) == 80, "layout of kSmInfo");
 
-struct Item {
-  int b, h, r0, rows;  // first pair row and how many (1..4)
-  int q0;
-  bool two_blocks;
-};
-
-__device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
-  // Items are ordered (b, h, row group, query blocks) with the query blocks fastest: the CTAs that run at the same
-  // time work on the query blocks of neighbouring pair rows, so a row's K and V come from HBM once (and then from
-  // L2) while the head's bias, shared by all rows, stays in L2.
-  Item it;
-  const bool second = item >= p.group[0].num_items;
-  const RowGroup& g = p.group[second];
-  if (second) item -= p.group[0].num_items;
-  const int bh = fast_div(item, g.bh_mul, g.bh_shr);
-  int idx = item - bh * g.items_bh;
-  it.h = bh % kHeads;
-  it.b = bh / kHeads;
-  it.two_blocks = idx < g.items_pair;
-  if (it.two_blocks) {
-    const int n = fast_div(idx, p.pairs_mul, p.pairs_shr);
-    it.rows = g.rows_pair;
-    it.r0 = g.row0 + n * g.rows_pair;
-    it.q0 = (idx - n * p.pairs) * 2 * kQTile;
-  } else {
-    idx -= g.items_pair;
-    const int n = fast_div(idx, p.singles_mul, p.singles_shr);
-    it.rows = g.rows_single;
-    it.r0 = g.row0 + n * g.rows_single;
-    it.q0 = (2 * p.pairs + idx - n * p.singles) * kQTile;
-  }
-  if (it.r0 + it.rows > g.row_end) it.rows = g.row_end - it.r0;
-  return it;
-}
-
 // Row length as stored of the pair row of unit `lane` (clamped to the item's rows).
 __device__ __forceinline__ int raw_length(const AttnParams& p, const Item& it, int lane) {
   if (p.lengths == nullptr) return p.S;
-  const int row = min(it.two_blocks ? (lane & 3) >> 1 : lane & 3, it.rows - 1);
-  return p.lengths[it.b * p.ls_b + (it.r0 + row) * p.ls_r];
+  return p.lengths[it.b * p.ls_b + (it.r0 + existing_row(it, lane & 3)) * p.ls_r];
 }
 
 template <bool kMasked>
@@ -225,7 +171,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int my_items = (p.num_items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
+  const int my_items = (p.plan.num_items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
   // Register budget: 640 threads start with 96 registers; setmaxnreg only moves registers inside that allocation,
   // and an increase blocks until a decrease has freed enough: the fifth warpgroup drops to 64 (frees 128 x 32) and
@@ -243,13 +189,13 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     int g = 0, i = 0;  // tiles and items loaded
     bool ok = true;
-    Item it = decode_item(p, blockIdx.x);
+    Item it = decode_item(p.plan, blockIdx.x);
     pdl_wait();  // (the MMA warps touch no global memory)
     int raw = raw_length(p, it, lane);
     while (i < my_items) {
       // lane u: unit u
       const int blocks = it.two_blocks ? 2 : 1;
-      const int row = it.two_blocks ? (lane & 3) >> 1 : lane & 3;
+      const int row = unit_row(it, lane & 3);
       int len = raw < 0 ? 0 : (raw > p.S ? p.S : raw);
       const bool exists = row < it.rows;
       const bool uni = exists && len == 0 && p.empty_uniform;
@@ -264,7 +210,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int br = it.b * p.R + it.r0;
       if (lane < kUnits) {
         *reinterpret_cast<int4*>(&info->unit[lane]) =
-            make_int4(br + row, it.q0 + (it.two_blocks ? lane & 1 : 0) * kQTile, len, nt);
+            make_int4(br + existing_row(it, lane), it.q0 + (it.two_blocks ? lane & 1 : 0) * kQTile, len, nt);
       } else if (lane == kUnits) {
         *reinterpret_cast<int4*>(&info->tiles) = make_int4(tiles, it.two_blocks, it.h, int(uniform));
       }
@@ -281,7 +227,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       ++i;
       const Item cur = it;
       if (i < my_items) {  // the next item's row lengths arrive while this item's tiles are loaded
-        it = decode_item(p, blockIdx.x + i * gridDim.x);
+        it = decode_item(p.plan, blockIdx.x + i * gridDim.x);
         raw = raw_length(p, it, lane);
       }
       for (int kt = 0; kt < tiles; ++kt, ++g) {
@@ -430,7 +376,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int my_tiles = unit.w, len = unit.z;
       const bool uniform = (common.w >> w) & 1;
       const uint32_t block_off = stage_bias(common.y ? w & 1 : 0) + sw128_offset(m, 0);
-      if (p.gate != nullptr && unit.y + m < p.S)  // read at the end
+      if (p.gate != nullptr && my_tiles > 0 && unit.y + m < p.S)  // read at the end
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + unit.x * p.g_br + common.z * p.g_h + (long long)(unit.y + m) * p.g_s));
       float row_max = 0.f, row_sum = 0.f;  // row_max: reference point of the exponentials, in raw score units
       const uint32_t* mask_row = nullptr;
@@ -757,63 +703,6 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (threadIdx.x == 0 && *abort_flag) *p.status = B200TA_ERR_DEVICE_WAIT;
 }
 
-}  // namespace
-}  // namespace b200ta
-
-namespace b200ta {
-namespace {
-// Constants for fast_div: with l = ceil(log2 d) and mul = floor(2^(31+l) / d) + 1, floor(n / d) equals
-// (n * mul) >> (31 + l) for every n < 2^31.
-void fast_div_constants(uint32_t d, uint32_t* mul, uint32_t* shr) {
-  if (d <= 1) {
-    *mul = 0, *shr = 0;
-    return;
-  }
-  uint32_t l = 0;
-  while ((uint64_t(1) << l) < d) ++l;
-  *mul = uint32_t((uint64_t(1) << (31 + l)) / d + 1);
-  *shr = l - 1;
-}
-
-// How the units (128 queries of one row and head) of a (b, h) are put together into items of up to four.
-// Normally the query blocks go two by two with two rows each and an odd last block with four rows.  A problem with
-// too few units to fill the SMs that way takes fewer units per item instead: a CTA with one or two units finishes a
-// tile in some 1000 to 1600 clocks of latency, one with four in some 2700.  For the same reason, when the items come
-// to a few waves and less than half a wave, the rows of that remainder go to items of two units, which still make
-// only one wave and a shorter one (256 tokens: 3.46 waves of items, 43 us; 3 waves and one of halves: 41 us).
-void split_items(int B, int R, int S, int num_sms, AttnParams* p) {
-  const int blocks = (S + kQTile - 1) / kQTile;
-  const int64_t bh = int64_t(B) * kHeads;
-  auto fill = [&](int which, int row0, int row_end, int rows_pair, int rows_single) -> int64_t {
-    RowGroup& g = p->group[which];
-    const int rows = row_end - row0;
-    g.row0 = row0, g.row_end = row_end, g.rows_pair = rows_pair, g.rows_single = rows_single;
-    g.items_pair = p->pairs * ((rows + rows_pair - 1) / rows_pair);
-    g.items_bh = g.items_pair + p->singles * ((rows + rows_single - 1) / rows_single);
-    g.num_items = int(bh * g.items_bh);
-    fast_div_constants(uint32_t(g.items_bh), &g.bh_mul, &g.bh_shr);
-    return bh * g.items_bh;
-  };
-  auto whole = [&](int pairs, int rows_pair, int rows_single) {
-    p->pairs = pairs, p->singles = blocks - 2 * pairs;
-    fill(1, R, R, 1, 1);
-    return fill(0, 0, R, rows_pair, rows_single);
-  };
-  if (whole(0, 1, 1) > num_sms &&                                                 // one unit per item
-      (blocks == 1 ? whole(0, 1, 2) : whole(blocks / 2, 1, 2)) > num_sms) {       // two units per item
-    const int64_t items = whole(blocks / 2, R > 1 ? 2 : 1, R > 2 ? 4 : R);
-    const int64_t waves = items / num_sms, rest = items % num_sms;
-    if (waves >= 1 && waves < 12 && rest > 0 && 2 * rest <= num_sms && R >= 8) {
-      // rows that fill the whole waves, in steps of four (one item of the odd block)
-      const int64_t per_four = bh * (2 * p->pairs + p->singles);
-      const int row = int(waves * num_sms / per_four) * 4;
-      if (row > 0 && row < R) fill(0, 0, row, 2, 4), fill(1, row, R, 1, 2);
-    }
-  }
-  fast_div_constants(uint32_t(p->pairs), &p->pairs_mul, &p->pairs_shr);
-  fast_div_constants(uint32_t(p->singles), &p->singles_mul, &p->singles_shr);
-}
-
 int launch_attention(const void* q, const void* k, const void* v, const void* gate, int64_t s_br, int64_t s_h,
                      int64_t s_s, const void* bias, int64_t bs_b, int64_t bs_h, int64_t bs_q,
                      const int32_t* lengths, int64_t ls_b, int64_t ls_r, const uint32_t* key_mask, int64_t km_b,
@@ -836,7 +725,7 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
   if (rc != B200TA_OK) return rc;
   B200TA_REQUIRE(int64_t(B) * kHeads * R * ((S + kQTile - 1) / kQTile) < (int64_t(1) << 31), "attention: too many work items");
   AttnParams p{};
-  split_items(B, R, S, st->num_sms, &p);
+  p.plan = split_items(B, R, S, st->num_sms);
 
   CUtensorMap tm_q, tm_k, tm_v, tm_bias;
   {
@@ -858,7 +747,6 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
   }
 
   p.B = B, p.R = R, p.S = S, p.S_pad = S_pad;
-  p.num_items = p.group[0].num_items + p.group[1].num_items;
   p.lengths = lengths;
   p.ls_b = ls_b, p.ls_r = ls_r;
   p.key_mask = key_mask;
@@ -873,7 +761,7 @@ int launch_attention(const void* q, const void* k, const void* v, const void* ga
   p.wide_store = (reinterpret_cast<uintptr_t>(out) & 31u) == 0 && os_br % 16 == 0 && os_s % 16 == 0 && os_h % 16 == 0;
   p.status = st->status_dev;
 
-  const int grid = p.num_items < st->num_sms ? p.num_items : st->num_sms;
+  const int grid = p.plan.num_items < st->num_sms ? p.plan.num_items : st->num_sms;
   if (key_mask != nullptr) {
     B200TA_REQUIRE(lengths != nullptr, "attention: the masked form needs the row lengths (last valid key + 1) as well");
     return launch_kernel(st, kKernelAttentionMasked, attention_kernel<true>, dim3(grid), kThreads, kSmDynamic, stream, tm_q,
