@@ -78,7 +78,6 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
   const int n0 = blockIdx.y * kTile;
   const int steps = p.K / kStepK;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -94,6 +93,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
 
   if (warp == 4) {
     if (lane == 0) {

@@ -58,7 +58,6 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -82,6 +81,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;  // blockIdx.x < num_tiles
 
   if (warp == 8) {

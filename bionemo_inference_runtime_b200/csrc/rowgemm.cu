@@ -111,7 +111,6 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   const int u_begin = (MODE == kPrologue && !p.want_qkvg) ? 2 : 0;
   const int u_end = MODE == kPrologue ? 3 : 1;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;  // scratch flag for the producer's drain wait
@@ -142,6 +141,7 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
 
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;  // blockIdx.x < num_tiles
 

@@ -154,7 +154,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -189,6 +188,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
 
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 

@@ -67,7 +67,6 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kSmBars + NUM_BARS * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     abort_flag[0] = 0, abort_flag[1] = 0;
     mbar_init(bars + W_FULL * 8, 1);
@@ -94,6 +93,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
   if (warp == 16) {
