@@ -326,13 +326,6 @@ class SideTrack {
   ~SideTrack() {
     for (cudaEvent_t e : {ready_, done_[0], done_[1]}) cudaEventDestroy(e);
   }
-  // The side stream continues from what the main stream has been given so far.
-  void fork() {
-    cuda(cudaEventRecord(ready_, main_.stream()));
-    cuda(cudaStreamWaitEvent(side_.stream(), ready_, 0));
-  }
-  void enter() { c10::cuda::setCurrentCUDAStream(side_); }
-  void leave() { c10::cuda::setCurrentCUDAStream(main_); }
   // `slot` (0 or 1): what the side stream has been given so far is the last use of the slot's bias buffer ...
   void done(int slot) { cuda(cudaEventRecord(done_[slot & 1], side_.stream())); }
   // ... which the main stream may overwrite after this.
@@ -341,6 +334,44 @@ class SideTrack {
   void hand_over(const at::Tensor& result) {
     c10::cuda::CUDACachingAllocator::recordStream(result.storage().data_ptr(), main_);
   }
+
+  // The side stream is the current one while this lives.
+  class Inside {
+   public:
+    explicit Inside(SideTrack& track) : main_(track.main_) { c10::cuda::setCurrentCUDAStream(track.side_); }
+    Inside(const Inside&) = delete;
+    ~Inside() { c10::cuda::setCurrentCUDAStream(main_); }
+
+   private:
+    c10::cuda::CUDAStream main_;
+  };
+
+  // A call's use of the side stream, which the main stream joins on every way out of the call: what was enqueued there
+  // works on tensors of the main stream's pool, which the end of the call, or an exception, hands back.
+  class Use {
+   public:
+    explicit Use(SideTrack* track) : track_(track) {}
+    Use(const Use&) = delete;
+    ~Use() {
+      if (forked_ && cudaEventRecord(track_->ready_, track_->side_.stream()) == cudaSuccess)
+        cudaStreamWaitEvent(track_->main_.stream(), track_->ready_, 0);
+    }
+    // The side stream continues from what the main stream has been given so far.
+    void fork() {
+      forked_ = true;
+      cuda(cudaEventRecord(track_->ready_, track_->main_.stream()));
+      cuda(cudaStreamWaitEvent(track_->side_.stream(), track_->ready_, 0));
+    }
+    void join() {
+      cuda(cudaEventRecord(track_->ready_, track_->side_.stream()));
+      cuda(cudaStreamWaitEvent(track_->main_.stream(), track_->ready_, 0));
+      forked_ = false;
+    }
+
+   private:
+    SideTrack* track_;
+    bool forked_ = false;
+  };
 
  private:
   static void cuda(cudaError_t e) {
@@ -404,12 +435,12 @@ class Stack {
   std::pair<at::Tensor, at::Tensor> run(c10::optional<at::Tensor> s, at::Tensor z, const c10::optional<at::Tensor>& mask,
                                         const c10::optional<at::Tensor>& lengths, const c10::optional<at::Tensor>& lengths_t,
                                         bool mask_output, const c10::optional<at::Tensor>& key_counts,
-                                        const py::object& buffers, SideTrack* track) {
+                                        const py::object& given_buffers, SideTrack* track) {
     pair_of("z", z, false);
+    const py::object buffers = given_buffers.is_none() ? py::object(py::dict()) : given_buffers;  // held until the join
     const at::Tensor ws = node_workspace(buffers, z);
     const TrimulBuffers t = trimul_buffers(buffers, z);
     const at::Tensor a = new_bf16(z, z.sizes()), out = new_bf16(z, z.sizes());
-    const py::object none = py::none();
     at::Tensor s16;
     if (s) {
       s16 = *s;
@@ -418,6 +449,7 @@ class Stack {
       buffer(buffers, "pw_qkvg", {4, B, 16, N, B200TA_HEAD_DIM}, at::kBFloat16, z);
       buffer(buffers, "pw_attn_output", {4 * B, 1, N, B200TA_C}, at::kBFloat16, z);
     }
+    SideTrack::Use use(track);  // after the tensors, so that it ends before them
     for (size_t i = 0; i < blocks_.size(); ++i) {
       const Block& b = blocks_[i];
       trimul_into(z, mask, b.tri_out.packed, b.tri_out.eps, false, c10::nullopt, t.ab, t.x, a, true, mask_output);
@@ -430,20 +462,14 @@ class Stack {
       const Single& w = singles_[i];
       if (i >= 2) track->wait(int(i));
       const at::Tensor bias = pair_bias(z, w.packed_z, w.eps_z, buffers, (i & 1) ? "pw_pair_bias_1" : "pw_pair_bias_0");
-      track->fork();
-      track->enter();
-      try {
-        s16 = pair_bias_attention(s16, bias, key_counts, w.w_in, w.sc_in, w.w_o, w.sc_o, w.norm, w.eps, w.scale, s16, buffers);
-        transition_gemms(s16, w.w1, w.sc1, w.w2, w.sc2, w.norm_t, w.eps_t, true, true);
-        track->done(int(i));
-      } catch (...) {
-        track->leave();
-        throw;
-      }
-      track->leave();
+      use.fork();
+      const SideTrack::Inside inside(*track);
+      s16 = pair_bias_attention(s16, bias, key_counts, w.w_in, w.sc_in, w.w_o, w.sc_o, w.norm, w.eps, w.scale, s16, buffers);
+      transition_gemms(s16, w.w1, w.sc1, w.w2, w.sc2, w.norm_t, w.eps_t, true, true);
+      track->done(int(i));
     }
     if (s) {
-      track->wait(int(blocks_.size()) - 1);
+      use.join();
       track->hand_over(s16);
     }
     return {s16, z};
@@ -553,14 +579,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("pair_bias", &pair_bias);
   m.def("pair_bias_attention", &pair_bias_attention);
   m.def("current_stream", &current_stream);
-  py::class_<SideTrack>(m, "SideTrack")
-      .def(py::init<>())
-      .def("fork", &SideTrack::fork)
-      .def("enter", &SideTrack::enter)
-      .def("leave", &SideTrack::leave)
-      .def("done", &SideTrack::done)
-      .def("wait", &SideTrack::wait)
-      .def("hand_over", &SideTrack::hand_over);
+  py::class_<SideTrack>(m, "SideTrack").def(py::init<>());
   py::class_<Stack>(m, "Stack")
       .def(py::init<>())
       .def("add", &Stack::add)

@@ -61,3 +61,35 @@ def test_masks_in_one_launch_equal_the_torch_operations():
             valid = source >= 0 if additive else source > 0.5
             for a, b in zip(_host.mask_bits(source, additive), ops.key_mask_bits(valid)):
                 assert torch.equal(a, b)
+
+
+def test_an_error_inside_the_single_track_joins_the_side_stream(monkeypatch):
+    """The last block's single transition is refused on the host when the blocks before it are enqueued already.  Streams
+    that are not joined again would make the capture of such a call fail at its end."""
+    from bionemo_inference_runtime_b200.layers import pairformer
+
+    class Broken(pairformer._host.Stack):
+        singles = 0
+
+        def add_single(self, *args):
+            self.singles += 1
+            args = list(args)
+            if self.singles == 2:
+                args[9] = args[9][:, :256].contiguous()  # w1 for another width
+            super().add_single(*args)
+
+    stack = _randomise(b200.PairformerModule(num_blocks=2, dtype=torch.bfloat16, triangle_attn_backend="Heuristic").to(DEV))
+    inputs = (torch.randn(1, 48, 384, device=DEV).bfloat16(), torch.randn(1, 48, 48, 128, device=DEV).bfloat16(),
+              torch.ones(1, 48, device=DEV), torch.ones(1, 48, 48, device=DEV))
+    with monkeypatch.context() as m:
+        m.setattr(pairformer._host, "Stack", Broken)
+        stream = torch.cuda.current_stream()
+        with pytest.raises(ValueError, match="last dimension"):
+            stack(*inputs)
+        assert torch.cuda.current_stream() == stream
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            with pytest.raises(ValueError, match="last dimension"):
+                stack(*inputs)
+    torch.cuda.synchronize()
+    stack._native = None
+    assert all(torch.isfinite(t).all() for t in stack(*inputs)) and _lib.device_status() == 0
