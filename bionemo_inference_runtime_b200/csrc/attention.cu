@@ -164,12 +164,14 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     fence_mbar_init();
   }
-  if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+  if (warp == 17) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+    pdl_trigger();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
 
   const int my_items = (p.plan.num_items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 

@@ -108,9 +108,10 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 
 // ---- programmatic dependent launch -------------------------------------------
 // Lets the stream's next kernel start its blocks as soon as every block of this one has come here and there is room for
-// them.  A kernel with tensor memory calls it behind the barrier that follows its allocation: tcgen05.alloc waits without
-// a limit, so a block of the next kernel that got the columns first would wait for this kernel (pdl_wait) while this
-// kernel waits for the columns.
+// them.  In a kernel with tensor memory the warp that allocates it calls this right behind the allocation: tcgen05.alloc
+// waits without a limit, so a block of the next kernel that got the columns first would wait for this kernel (pdl_wait)
+// while this kernel waits for the columns.  (Called by all threads behind the barrier that follows, a node's small
+// kernels started 0.1 us later each.)
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Returns once the kernels before this one in the stream are complete and their writes visible.  Every thread calls it
 // before its first access to global memory, except for reads of packed weights: the pack entry points end with an

@@ -88,12 +88,14 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ 
     mbar_init(bars + ACC_FULL * 8, 1);
     fence_mbar_init();
   }
-  if (warp == 5) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 128);
+  if (warp == 5) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 128);
+    pdl_trigger();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
 
   if (warp == 4) {
     if (lane == 0) {

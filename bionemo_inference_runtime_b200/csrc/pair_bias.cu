@@ -72,7 +72,10 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
     }
     fence_mbar_init();
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 32);
+  if (warp == 9) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 32);
+    pdl_trigger();
+  }
   if (threadIdx.x < kMaxHeads / 2) {
     const float2 a = p.sc[kFirstRow + 2 * threadIdx.x], b = p.sc[kFirstRow + 2 * threadIdx.x + 1];
     reinterpret_cast<float4*>(gen + kSmSc)[threadIdx.x] = make_float4(a.x, b.x, a.y, b.y);
@@ -81,7 +84,6 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;  // blockIdx.x < num_tiles
 
   if (warp == 8) {

@@ -125,7 +125,10 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       for (int i = 0; i < 4; ++i) mbar_init(bars + (STATS + i) * 8, 4);
     fence_mbar_init();
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 9) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    pdl_trigger();
+  }
   // stage the per-column vectors
   if (MODE == kPrologue) {
     float4* dst = reinterpret_cast<float4*>(gen + L::kVec);
@@ -141,7 +144,6 @@ rowgemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
 
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;  // blockIdx.x < num_tiles
 

@@ -177,7 +177,10 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     mbar_init(bars + XN_EMPTY * 8, 4);
     fence_mbar_init();
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+  if (warp == 9) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+    pdl_trigger();
+  }
   // stage the constants: LayerNorm gamma | beta, and for the ReLU form the two linears' biases
   if (threadIdx.x < 2 * kC) reinterpret_cast<float*>(gen + kSmLn)[threadIdx.x] = p.ln[threadIdx.x];
   if (kRelu) {
@@ -188,7 +191,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
 
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 

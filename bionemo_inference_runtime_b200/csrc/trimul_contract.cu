@@ -81,12 +81,14 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_c
     }
     fence_mbar_init();
   }
-  if (warp == 9) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 9) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    pdl_trigger();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
 
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
   const int ksteps = (p.N + kBK - 1) / kBK;

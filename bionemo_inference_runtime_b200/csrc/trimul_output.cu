@@ -81,7 +81,10 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
     }
     fence_mbar_init();
   }
-  if (warp == 17) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 17) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    pdl_trigger();
+  }
   // per-channel constants of the epilogue
   if (threadIdx.x < kC / 2) {
     const int c = 2 * threadIdx.x;
@@ -93,7 +96,6 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
   if (warp == 16) {

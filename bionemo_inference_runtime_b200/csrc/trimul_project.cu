@@ -84,12 +84,14 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_con
     }
     fence_mbar_init();
   }
-  if (warp == 21) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == 21) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    pdl_trigger();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
   const int my_tiles = (p.num_tiles - 1 - int(blockIdx.x)) / int(gridDim.x) + 1;
 
   if (warp == 20) {

@@ -27,5 +27,6 @@ def test_all_tensor_memory_kernels_are_seen():
 def test_next_kernel_starts_after_the_allocation_of_tensor_memory(body):
     """Otherwise a block of the next kernel can take the columns and wait for the block that waits for them."""
     alloc, trigger = body.index("tmem_alloc("), [m.start() for m in re.finditer(r"pdl_trigger\(\)", body)]
-    barrier = body.index("__syncthreads()", alloc)
-    assert trigger and all(t > barrier for t in trigger)
+    assert len(trigger) == 1 and trigger[0] > alloc
+    between = body[alloc:trigger[0]]  # the next statement of the allocating warp, or behind the block's barrier
+    assert re.fullmatch(r"tmem_alloc\(.*\);\s*", between) or "__syncthreads()" in between
