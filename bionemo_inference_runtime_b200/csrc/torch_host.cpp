@@ -506,31 +506,12 @@ std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additiv
 
 // ---- weight state --------------------------------------------------------------------------------------------------
 
-// With `strict` the modules themselves belong to the state as well, and false means that one of them has a forward hook.
-bool add_parameters(PyObject* module, std::string& out, bool strict) {
+// Address, in-place write count and device of every parameter under `module`.
+void add_parameters(PyObject* module, std::string& out) {
   static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
   static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
   PyObject** dict = _PyObject_GetDictPtr(module);
-  if (dict == nullptr || *dict == nullptr) return true;
-  if (strict) {
-    static PyObject* const k_hooks = PyUnicode_InternFromString("_forward_hooks");
-    static PyObject* const k_pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks");
-    for (PyObject* k : {k_hooks, k_pre_hooks})
-      if (PyObject* hooks = PyDict_GetItem(*dict, k); hooks != nullptr && PyDict_Check(hooks) && PyDict_Size(hooks) > 0) return false;
-    // the module's attributes by identity (flags, eps, policies, ...), without the caches of its packed weights
-    static PyObject* const k_caches[] = {
-        PyUnicode_InternFromString("_pack"), PyUnicode_InternFromString("_pack_state"), PyUnicode_InternFromString("_folded"),
-        PyUnicode_InternFromString("_folded_state"), PyUnicode_InternFromString("_zero_bias")};
-    uint64_t mix = reinterpret_cast<uint64_t>(module);
-    PyObject *key, *value;
-    Py_ssize_t pos = 0;
-    while (PyDict_Next(*dict, &pos, &key, &value)) {
-      bool cache = false;
-      for (PyObject* k : k_caches) cache = cache || k == key;
-      if (!cache) mix = (mix ^ reinterpret_cast<uint64_t>(value)) * 0x9E3779B97F4A7C15ull, mix ^= mix >> 29;
-    }
-    out.append(reinterpret_cast<const char*>(&mix), sizeof(mix));
-  }
+  if (dict == nullptr || *dict == nullptr) return;
   PyObject *key, *value;
   Py_ssize_t pos = 0;
   if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
@@ -546,24 +527,66 @@ bool add_parameters(PyObject* module, std::string& out, bool strict) {
   pos = 0;
   if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
     while (PyDict_Next(modules, &pos, &key, &value))
-      if (value != Py_None && !add_parameters(value, out, strict)) return false;
+      if (value != Py_None) add_parameters(value, out);
+}
+
+// Changes when a weight under the modules is loaded, edited or replaced.
+py::bytes weight_state(const py::args& modules) {
+  std::string out;
+  for (const py::handle& m : modules) add_parameters(m.ptr(), out);
+  return py::bytes(out);
+}
+
+// ---- module state ----------------------------------------------------------------------------------------------------
+
+// Calls visit(object) for `module`, the names and values of its attributes and its forward hooks, and the same of every
+// module under it, in an order that depends on the modules alone; stops at, and returns, the first false.  The parameters
+// and the layers' caches of packed weights are left out: weight_state() covers those.
+template <typename Visit>
+bool visit_objects(PyObject* module, const Visit& visit) {
+  static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
+  static PyObject* const k_hooks[] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks")};
+  static PyObject* const k_caches[] = {
+      PyUnicode_InternFromString("_pack"), PyUnicode_InternFromString("_pack_state"), PyUnicode_InternFromString("_folded"),
+      PyUnicode_InternFromString("_folded_state"), PyUnicode_InternFromString("_zero_bias")};
+  if (!visit(module)) return false;
+  PyObject** dict = _PyObject_GetDictPtr(module);
+  if (dict == nullptr || *dict == nullptr) return true;
+  PyObject *key, *value;
+  Py_ssize_t pos = 0;
+  while (PyDict_Next(*dict, &pos, &key, &value)) {
+    bool cache = false;
+    for (PyObject* k : k_caches) cache = cache || k == key;
+    if (!cache && !(visit(key) && visit(value))) return false;
+  }
+  for (PyObject* k : k_hooks) {
+    PyObject* hooks = PyDict_GetItem(*dict, k);
+    pos = 0;
+    if (hooks != nullptr && PyDict_Check(hooks))
+      while (PyDict_Next(hooks, &pos, &key, &value))
+        if (!visit(value)) return false;
+  }
+  pos = 0;
+  if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
+    while (PyDict_Next(modules, &pos, &key, &value))
+      if (value != Py_None && !visit_objects(value, visit)) return false;
   return true;
 }
 
-// Address, in-place write count and device of every parameter under the modules: changes when a weight is loaded,
-// edited or replaced.
-py::bytes weight_state(const py::args& modules) {
-  std::string out;
-  for (const py::handle& m : modules) add_parameters(m.ptr(), out, false);
-  return py::bytes(out);
+// What visit_objects() sees, as a tuple that holds it: an object in it cannot make room for another one at its address.
+py::tuple module_objects(const py::handle& module) {
+  py::list out;
+  visit_objects(module.ptr(), [&](PyObject* o) { return PyList_Append(out.ptr(), o) == 0; });
+  if (PyErr_Occurred()) throw py::error_already_set();
+  return py::tuple(out);
 }
 
-// The same with the identity of every module under `module` and of its attributes (a hash of the addresses); None if one
-// of the modules has a forward hook.
-py::object stack_state(const py::handle& module) {
-  std::string out;
-  if (!add_parameters(module.ptr(), out, true)) return py::none();
-  return py::bytes(out);
+// Whether visit_objects() sees the very objects of `held`: no module, option or hook has been replaced since.
+bool same_objects(const py::tuple& held, const py::handle& module) {
+  Py_ssize_t i = 0;
+  const Py_ssize_t n = PyTuple_GET_SIZE(held.ptr());
+  const bool same = visit_objects(module.ptr(), [&](PyObject* o) { return i < n && PyTuple_GET_ITEM(held.ptr(), i++) == o; });
+  return same && i == n;
 }
 
 }  // namespace
@@ -586,7 +609,8 @@ PYBIND11_MODULE(_host, m) {
       .def("add_single", &Stack::add_single)
       .def("run_pair", &Stack::run_pair)
       .def("run_both", &Stack::run_both);
-  m.def("stack_state", &stack_state);
+  m.def("module_objects", &module_objects);
+  m.def("same_objects", &same_objects);
   m.def("mask_lengths", &mask_lengths);
   m.def("mask_bits", &mask_bits);
   m.def("weight_state", &weight_state);

@@ -36,11 +36,17 @@ _side_tracks: dict[tuple[torch.device, int], "_host.SideTrack"] = {}
 
 
 class _NativeStack:
-    """The packed weights of a stack in the form of ``_host.Stack``, valid on one device and for one state of its modules;
-    not copied or pickled with the module."""
+    """The packed weights of a stack in the form of ``_host.Stack`` (None: the stack has no such form), valid on one device
+    and for one state of its modules; not copied or pickled with the module.  The objects that make up the state are held:
+    an option replaced by one at the same address would look unchanged."""
 
-    def __init__(self, state: bytes, device: torch.device, stack, chunk_policies):
-        self.state, self.device, self.stack, self.chunk_policies = state, device, stack, chunk_policies
+    def __init__(self, layers, device: torch.device, stack, chunk_policies):
+        self.objects, self.weights = _host.module_objects(layers), _host.weight_state(layers)
+        self.device, self.stack, self.chunk_policies = device, stack, chunk_policies
+
+    def fits(self, layers, device: torch.device) -> bool:
+        return (self.device == device and _host.same_objects(self.objects, layers)
+                and _host.weight_state(layers) == self.weights)
 
     def __deepcopy__(self, memo):
         return None
@@ -52,26 +58,27 @@ class _NativeStack:
 def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
     """The native form of ``module.layers`` for this call, or None when a layer has to be called itself: it is hooked or
     of another class, its options need the general path, or its rows are chunked at this size."""
-    state = None if nn.modules.module._has_any_global_hook() else _host.stack_state(module.layers)
-    held = module.__dict__.get("_native")
-    if state is None or (held is not None and held.state == state and held.device == z.device):
-        native = held if state is not None else None
-    elif torch.cuda.is_current_stream_capturing():
-        return None  # folding weights now would only fill them at replay
-    else:
+    if nn.modules.module._has_any_global_hook():
+        return None
+    native = module.__dict__.get("_native")
+    if native is None or not native.fits(module.layers, z.device):
+        if torch.cuda.is_current_stream_capturing():
+            return None  # folding weights now would only fill them at replay
         stack = _build_native_stack(module.layers, z.device)
         policies = {} if stack is None else {
             id(p): p for layer in module.layers
             for p in (layer.tri_attn_start.mha.chunk_policy, layer.tri_attn_end.mha.chunk_policy) if p is not None}
         # a stack that has no native form is remembered as well
-        native = module._native = _NativeStack(state, z.device, stack, list(policies.values()))
-    if native is None or native.stack is None:
+        native = module._native = _NativeStack(module.layers, z.device, stack, list(policies.values()))
+    if native.stack is None:
         return None
     chunked = any(p.chunk_size < z.shape[1] and p.should_chunk(z) for p in native.chunk_policies)
     return None if chunked else native
 
 
 def _build_native_stack(layers, device):
+    if any(m._forward_hooks or m._forward_pre_hooks for m in layers.modules()):
+        return None
     bf16 = torch.bfloat16
     stack = _host.Stack()
     for layer in layers:

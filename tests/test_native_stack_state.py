@@ -45,3 +45,23 @@ def test_packed_weights_of_one_device_are_not_used_on_another(monkeypatch):
     for device in ("cpu", "cpu", "meta", "meta"):
         pairformer._native_stack(stack, _inputs(device)[1])
     assert [d.type for d in built] == ["cpu", "meta"]
+
+
+def test_an_option_replaced_at_its_old_address_is_seen(monkeypatch):
+    """Two replacements between two calls: the second object may get the address of the one that was looked at."""
+    built = []
+    monkeypatch.setattr(pairformer, "_build_native_stack", lambda layers, device: built.append(1) or object())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    stack, z = _stack(), _inputs("cpu")[1]
+    node = stack.layers[1].tri_mul_in
+    node.eps = float("2e-5")
+    pairformer._native_stack(stack, z)
+    address = id(node.eps)
+    node.eps = None
+    others = []
+    while len(others) < 1000 and (not others or id(others[-1]) != address):
+        others.append(float("3e-5"))
+    node.eps = others[-1]
+    pairformer._native_stack(stack, z)
+    pairformer._native_stack(stack, z)
+    assert len(built) == 2
