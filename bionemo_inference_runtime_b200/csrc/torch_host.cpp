@@ -540,25 +540,19 @@ py::bytes weight_state(const py::args& modules) {
 // ---- module state ----------------------------------------------------------------------------------------------------
 
 // Calls visit(object) for `module`, the names and values of its attributes and its forward hooks, and the same of every
-// module under it, in an order that depends on the modules alone; stops at, and returns, the first false.  The parameters
-// and the layers' caches of packed weights are left out: weight_state() covers those.
+// module under it, in an order that depends on the modules alone; stops at, and returns, the first false.  The layers'
+// packed weights are among the attributes; the parameters are left out (weight_state() covers those).
 template <typename Visit>
 bool visit_objects(PyObject* module, const Visit& visit) {
   static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
   static PyObject* const k_hooks[] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks")};
-  static PyObject* const k_caches[] = {
-      PyUnicode_InternFromString("_pack"), PyUnicode_InternFromString("_pack_state"), PyUnicode_InternFromString("_folded"),
-      PyUnicode_InternFromString("_folded_state"), PyUnicode_InternFromString("_zero_bias")};
   if (!visit(module)) return false;
   PyObject** dict = _PyObject_GetDictPtr(module);
   if (dict == nullptr || *dict == nullptr) return true;
   PyObject *key, *value;
   Py_ssize_t pos = 0;
-  while (PyDict_Next(*dict, &pos, &key, &value)) {
-    bool cache = false;
-    for (PyObject* k : k_caches) cache = cache || k == key;
-    if (!cache && !(visit(key) && visit(value))) return false;
-  }
+  while (PyDict_Next(*dict, &pos, &key, &value))
+    if (!visit(key) || !visit(value)) return false;
   for (PyObject* k : k_hooks) {
     PyObject* hooks = PyDict_GetItem(*dict, k);
     pos = 0;

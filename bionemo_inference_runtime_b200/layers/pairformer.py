@@ -35,18 +35,16 @@ from .triangle_nodes import _EMPTY_ROW_MODES, TriangleAttentionEndingNode, Trian
 _side_tracks: dict[tuple[torch.device, int], "_host.SideTrack"] = {}
 
 
-class _NativeStack:
-    """The packed weights of a stack in the form of ``_host.Stack`` (None: the stack has no such form), valid on one device
-    and for one state of its modules; not copied or pickled with the module.  The objects that make up the state are held:
-    an option replaced by one at the same address would look unchanged."""
+class _LayersState:
+    """The state of a stack's layers: their options, hooks and packed weights, and the parameters these were folded from.
+    The objects are held, so that one replaced by another at its address does not look unchanged, and packed weights
+    whose addresses a native stack or a graph has recorded stay allocated.  Not copied or pickled with the module."""
 
-    def __init__(self, layers, device: torch.device, stack, chunk_policies):
+    def __init__(self, layers):
         self.objects, self.weights = _host.module_objects(layers), _host.weight_state(layers)
-        self.device, self.stack, self.chunk_policies = device, stack, chunk_policies
 
-    def fits(self, layers, device: torch.device) -> bool:
-        return (self.device == device and _host.same_objects(self.objects, layers)
-                and _host.weight_state(layers) == self.weights)
+    def holds(self, layers) -> bool:
+        return _host.same_objects(self.objects, layers) and _host.weight_state(layers) == self.weights
 
     def __deepcopy__(self, memo):
         return None
@@ -55,13 +53,22 @@ class _NativeStack:
         return type(None), ()
 
 
+class _NativeStack(_LayersState):
+    """The packed weights of a stack in the form of ``_host.Stack`` (None: the stack has no such form), valid on one device
+    and for the state that the layers are in now, with their weights packed."""
+
+    def __init__(self, layers, device: torch.device, stack, chunk_policies):
+        super().__init__(layers)
+        self.device, self.stack, self.chunk_policies = device, stack, chunk_policies
+
+
 def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
     """The native form of ``module.layers`` for this call, or None when a layer has to be called itself: it is hooked or
     of another class, its options need the general path, or its rows are chunked at this size."""
     if nn.modules.module._has_any_global_hook():
         return None
     native = module.__dict__.get("_native")
-    if native is None or not native.fits(module.layers, z.device):
+    if native is None or native.device != z.device or not native.holds(module.layers):
         if torch.cuda.is_current_stream_capturing():
             return None  # folding weights now would only fill them at replay
         stack = _build_native_stack(module.layers, z.device)
@@ -283,6 +290,7 @@ class PairformerModule(nn.Module):
         self.use_cuda_graph = use_cuda_graph
         self._graph = None
         self._graph_key = None
+        self._graph_state = None
         self._graph_io = None
         if config is not None:
             version = getattr(config, "version", version)
@@ -307,10 +315,10 @@ class PairformerModule(nn.Module):
         if not (self.use_cuda_graph and z.is_cuda) or torch.cuda.is_current_stream_capturing():
             return self._run(s, z, mask, pair_mask, attn_metadatas, buffers, **kwargs)
         inputs = (s, z, mask, pair_mask)
-        # the recorded kernels hold the addresses of the layers' packed weights: a reload or an in-place edit of
-        # any parameter must record a new graph
-        key = (*((t.shape, t.dtype, t.device) for t in inputs), _host.weight_state(self))
-        if self._graph is None or key != self._graph_key:
+        # the recorded kernels hold the addresses of the layers' packed weights and the values of their options: a
+        # reload, an in-place edit of a parameter or another option must record a new graph
+        key = tuple((t.shape, t.dtype, t.device) for t in inputs)
+        if self._graph is None or key != self._graph_key or not self._graph_state.holds(self.layers):
             static = [t.clone() for t in inputs]
             graph_buffers: dict = {}
             side = torch.cuda.Stream(z.device)
@@ -322,6 +330,7 @@ class PairformerModule(nn.Module):
                     outs = self._run(*static, attn_metadatas, graph_buffers, **kwargs)
             torch.cuda.current_stream(z.device).wait_stream(side)
             self._graph, self._graph_key, self._graph_io = graph, key, (static, outs, graph_buffers)
+            self._graph_state = _LayersState(self.layers)
         static, outs, _ = self._graph_io
         for dst, src in zip(static, inputs):
             dst.copy_(src)
@@ -374,6 +383,7 @@ class PairformerNoSeqModule(nn.Module):
         self.use_cuda_graph = use_cuda_graph
         self._graph = None
         self._graph_key = None
+        self._graph_state = None
         self._graph_in = self._graph_mask = self._graph_out = None
 
     def _run(self, z, pair_mask, attn_metadatas, buffers, **kwargs):
@@ -401,10 +411,9 @@ class PairformerNoSeqModule(nn.Module):
             return z
         if not (self.use_cuda_graph and z.is_cuda) or torch.cuda.is_current_stream_capturing():
             return self._run(z, pair_mask, attn_metadatas, buffers, **kwargs)
-        # the recorded kernels hold the addresses of the layers' packed weights: a reload or an in-place edit of
-        # any parameter must record a new graph
-        key = (z.shape, z.dtype, z.device, pair_mask.shape, pair_mask.dtype, _host.weight_state(self))
-        if self._graph is None or key != self._graph_key:
+        # as in PairformerModule.forward
+        key = (z.shape, z.dtype, z.device, pair_mask.shape, pair_mask.dtype)
+        if self._graph is None or key != self._graph_key or not self._graph_state.holds(self.layers):
             self._graph_in, self._graph_mask = z.clone(), pair_mask.clone()
             graph_buffers: dict = {}
             side = torch.cuda.Stream(z.device)
@@ -416,6 +425,7 @@ class PairformerNoSeqModule(nn.Module):
                     self._graph_out = self._run(self._graph_in, self._graph_mask, attn_metadatas, graph_buffers, **kwargs)
             torch.cuda.current_stream(z.device).wait_stream(side)
             self._graph, self._graph_key, self._graph_buffers = graph, key, graph_buffers
+            self._graph_state = _LayersState(self.layers)
         self._graph_in.copy_(z)
         self._graph_mask.copy_(pair_mask)
         self._graph.replay()

@@ -93,3 +93,26 @@ def test_an_error_inside_the_single_track_joins_the_side_stream(monkeypatch):
     torch.cuda.synchronize()
     stack._native = None
     assert all(torch.isfinite(t).all() for t in stack(*inputs)) and _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("seq", [False, True])
+def test_weights_refolded_by_their_layer_reach_the_stack(seq, graph):
+    """Linear.load_weights writes parameters without counting as an edit; post_load_weights() of the layer that folds them
+    is what makes it take effect, in the layer, in the native stack and in a recorded graph."""
+    cls = b200.PairformerModule if seq else b200.PairformerNoSeqModule
+    stack = _randomise(cls(num_blocks=2, dtype=torch.bfloat16, triangle_attn_backend="Heuristic", use_cuda_graph=graph).to(DEV))
+    inputs = (torch.randn(1, 40, 40, 128, device=DEV).bfloat16(), torch.ones(1, 40, 40, device=DEV))
+    if seq:
+        inputs = (torch.randn(1, 40, 384, device=DEV).bfloat16(), inputs[0], torch.ones(1, 40, device=DEV), inputs[1])
+    before = stack(*inputs)
+    transition = stack.layers[1].transition_z
+    transition.fc3.load_weights([{"weight": -transition.fc3.weight.clone()}])
+    transition.post_load_weights()
+    after = stack(*inputs)
+    handle = stack.layers[0].register_forward_hook(lambda *args: None)  # a hooked layer is called itself
+    stack.use_cuda_graph = False
+    want = stack(*inputs)
+    handle.remove()
+    z = (lambda out: out[1]) if seq else (lambda out: out)
+    assert not torch.equal(z(before), z(after)) and torch.equal(z(after), z(want))
