@@ -506,35 +506,57 @@ std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additiv
 
 // ---- weight state --------------------------------------------------------------------------------------------------
 
-// Address, in-place write count and device of every parameter under `module`.
-void add_parameters(PyObject* module, std::string& out) {
-  static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
-  static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
-  PyObject** dict = _PyObject_GetDictPtr(module);
-  if (dict == nullptr || *dict == nullptr) return;
-  PyObject *key, *value;
-  Py_ssize_t pos = 0;
-  if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
-    while (PyDict_Next(parameters, &pos, &key, &value)) {
-      if (!THPVariable_Check(value)) continue;
-      const at::Tensor& t = THPVariable_Unpack(value);
-      // address, in-place write count (inference tensors have none), device
-      const int64_t state[3] = {reinterpret_cast<int64_t>(t.data_ptr()), t.is_inference() ? -1 : int64_t(t._version()),
-                                int64_t(t.device().index()) * 256 + int64_t(t.device().type())};
-      out.append(reinterpret_cast<const char*>(state), sizeof(state));
+// The parameters under some modules as they were seen: storage, address, in-place write count, device.  The storages are
+// held weakly: their memory is free to go, but another storage cannot come to be at the address of one that was seen, so
+// that a parameter replaced twice does not look unchanged when its memory is given out again.  Not copied or pickled
+// with the layers that keep one.
+class WeightState {
+ public:
+  struct Seen {
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+    const void* data;
+    int64_t version;  // inference tensors have none
+    c10::Device device;
+  };
+  bool operator==(const WeightState& o) const {
+    if (seen.size() != o.seen.size()) return false;
+    for (size_t i = 0; i < seen.size(); ++i) {
+      const Seen &a = seen[i], &b = o.seen[i];
+      if (a.storage._unsafe_get_target() != b.storage._unsafe_get_target() || a.data != b.data || a.version != b.version ||
+          a.device != b.device)
+        return false;
     }
+    return true;
   }
-  pos = 0;
-  if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
-    while (PyDict_Next(modules, &pos, &key, &value))
-      if (value != Py_None) add_parameters(value, out);
-}
+  void add_parameters(PyObject* module) {
+    static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
+    static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
+    PyObject** dict = _PyObject_GetDictPtr(module);
+    if (dict == nullptr || *dict == nullptr) return;
+    PyObject *key, *value;
+    Py_ssize_t pos = 0;
+    if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
+      while (PyDict_Next(parameters, &pos, &key, &value)) {
+        if (!THPVariable_Check(value)) continue;
+        const at::Tensor& t = THPVariable_Unpack(value);
+        seen.push_back({t.storage().getWeakStorageImpl(), t.data_ptr(), t.is_inference() ? -1 : int64_t(t._version()), t.device()});
+      }
+    }
+    pos = 0;
+    if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
+      while (PyDict_Next(modules, &pos, &key, &value))
+        if (value != Py_None) add_parameters(value);
+  }
+
+ private:
+  std::vector<Seen> seen;
+};
 
 // Changes when a weight under the modules is loaded, edited or replaced.
-py::bytes weight_state(const py::args& modules) {
-  std::string out;
-  for (const py::handle& m : modules) add_parameters(m.ptr(), out);
-  return py::bytes(out);
+WeightState weight_state(const py::args& modules) {
+  WeightState out;
+  for (const py::handle& m : modules) out.add_parameters(m.ptr());
+  return out;
 }
 
 // ---- module state ----------------------------------------------------------------------------------------------------
@@ -607,5 +629,9 @@ PYBIND11_MODULE(_host, m) {
   m.def("same_objects", &same_objects);
   m.def("mask_lengths", &mask_lengths);
   m.def("mask_bits", &mask_bits);
+  py::class_<WeightState>(m, "WeightState")
+      .def("__eq__", [](const WeightState& a, const py::object& b) { return py::isinstance<WeightState>(b) && a == b.cast<const WeightState&>(); })
+      .def("__deepcopy__", [](const WeightState&, const py::object&) { return py::none(); })
+      .def("__reduce__", [](const WeightState&) { return py::make_tuple(py::type::of(py::none()), py::tuple()); });
   m.def("weight_state", &weight_state);
 }

@@ -1,5 +1,7 @@
 """What the native form of a stack depends on, without a GPU: the kernels' side is replaced by recorders."""
 
+import copy
+import pickle
 from types import SimpleNamespace
 
 import torch
@@ -65,3 +67,25 @@ def test_an_option_replaced_at_its_old_address_is_seen(monkeypatch):
     pairformer._native_stack(stack, z)
     pairformer._native_stack(stack, z)
     assert len(built) == 2
+
+
+def test_a_parameter_replaced_at_its_old_address_is_seen():
+    layer = b200.Transition(128, 512, dtype=torch.bfloat16).cpu()
+    weight = layer.fc3.weight
+    state, address = pairformer._host.weight_state(layer), weight.data_ptr()
+    assert state == pairformer._host.weight_state(layer) and state != None  # noqa: E711
+    weight.data = torch.empty(0, dtype=torch.bfloat16)
+    others = []
+    while len(others) < 100 and (not others or others[-1].data_ptr() != address):
+        others.append(torch.zeros(128, 512, dtype=torch.bfloat16))
+    weight.data = others[-1]
+    assert state != pairformer._host.weight_state(layer)
+
+
+def test_state_is_not_copied_with_a_layer():
+    layer = b200.Transition(128, 512, dtype=torch.bfloat16).cpu()
+    layer._pack_state = pairformer._host.weight_state(layer)
+    stack = _stack()
+    stack._native = pairformer._NativeStack(stack.layers, torch.device("cpu"), None, [])
+    assert copy.deepcopy(layer)._pack_state is None and copy.deepcopy(stack)._native is None
+    assert pickle.loads(pickle.dumps(layer))._pack_state is None and pickle.loads(pickle.dumps(stack))._native is None
