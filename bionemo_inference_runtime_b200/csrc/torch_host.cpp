@@ -275,16 +275,29 @@ at::Tensor pair_bias(const at::Tensor& z, const at::Tensor& packed_z, double eps
   return bias;
 }
 
-// The single-track attention with the bias that pair_bias() wrote.  `lengths` int32 [4 B]: the key count of a batch entry four times (the
-// attention kernel sees its 16 heads as four items of four).
+// `s` has to have the width that the in-projection's weights were folded for, and a residual the shape of `s`: the kernels
+// take both as given.
+void check_single(const at::Tensor& s, int64_t B, int64_t N, const at::Tensor& w_in) {
+  require_bf16("s", s);
+  if (!s.is_contiguous() || s.dim() != 3 || s.size(0) != B || s.size(1) != N || s.size(2) != w_in.size(1))
+    throw py::value_error("s must be a contiguous [" + std::to_string(B) + ", " + std::to_string(N) + ", " +
+                          std::to_string(w_in.size(1)) + "] tensor that matches z and the weights, got " + shape_of(s));
+}
+
+// The single-track attention with the bias that pair_bias() wrote.  `lengths` int32 [4 B]: the key count of a batch entry
+// four times (the attention kernel sees its 16 heads as four items of four).
 at::Tensor pair_bias_attention(const at::Tensor& s16, const at::Tensor& bias, const c10::optional<at::Tensor>& lengths,
                                const at::Tensor& w_in, const at::Tensor& sc_in, const at::Tensor& w_o, const at::Tensor& sc_o,
                                bool normalize, double eps_s, double scale, const c10::optional<at::Tensor>& residual,
                                const py::object& buffers) {
-  require_bf16("s", s16);
-  const int64_t B = bias.size(0), N = bias.size(2), c_s = s16.size(-1), heads = 16, dim = B200TA_HEAD_DIM, pad = bias.size(3);
-  if (!s16.is_contiguous() || s16.dim() != 3 || s16.size(0) != B || s16.size(1) != N)
-    throw py::value_error("s must be a contiguous [B, N, c_s] tensor that matches z");
+  const int64_t B = bias.size(0), N = bias.size(2), heads = 16, dim = B200TA_HEAD_DIM, pad = bias.size(3);
+  check_single(s16, B, N, w_in);
+  const int64_t c_s = s16.size(2);
+  if (residual) {
+    require_bf16("residual", *residual);
+    if (!residual->is_contiguous() || residual->sizes() != s16.sizes())
+      throw py::value_error("residual must be a contiguous tensor of the shape of s, got " + shape_of(*residual));
+  }
   void* st = stream();
   at::Tensor stats;
   if (normalize) {
@@ -437,6 +450,7 @@ class Stack {
                                         bool mask_output, const c10::optional<at::Tensor>& key_counts,
                                         const py::object& given_buffers, SideTrack* track) {
     pair_of("z", z, false);
+    if (s && !singles_.empty()) check_single(*s, z.size(0), z.size(1), singles_[0].w_in);  // before anything is enqueued
     const py::object buffers = given_buffers.is_none() ? py::object(py::dict()) : given_buffers;  // held until the join
     const at::Tensor ws = node_workspace(buffers, z);
     const TrimulBuffers t = trimul_buffers(buffers, z);

@@ -116,3 +116,17 @@ def test_weights_refolded_by_their_layer_reach_the_stack(seq, graph):
     handle.remove()
     z = (lambda out: out[1]) if seq else (lambda out: out)
     assert not torch.equal(z(before), z(after)) and torch.equal(z(after), z(want))
+
+
+def test_single_track_inputs_that_do_not_fit_are_refused():
+    """Another width of s, or a residual that would have to be broadcast, is an error on the host and not a read outside
+    the weights or the residual."""
+    stack = b200.PairformerModule(num_blocks=1, dtype=torch.bfloat16, triangle_attn_backend="Heuristic").to(DEV)
+    z, mask, pair = torch.randn(2, 24, 24, 128, device=DEV).bfloat16(), torch.ones(2, 24, device=DEV), torch.ones(2, 24, 24, device=DEV)
+    for shape in ((2, 24, 512), (2, 24, 256), (1, 24, 384), (2, 23, 384)):
+        with pytest.raises(ValueError):
+            stack(torch.zeros(shape, device=DEV).bfloat16(), z, mask, pair)
+    s = torch.zeros(2, 24, 384, device=DEV).bfloat16()
+    for residual in (s[:1], s[:, :1], s[..., :128]):
+        with pytest.raises(ValueError):
+            stack.layers[0].attention(s, z, mask, residual=residual)
