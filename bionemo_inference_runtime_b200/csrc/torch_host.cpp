@@ -103,14 +103,15 @@ at::Tensor buffer(const py::object& buffers, const char* key, at::IntArrayRef sh
 struct Lengths {
   const int32_t* ptr = nullptr;
   int64_t sb = 0, sr = 0;
+  at::Tensor held;  // as [B, R]; a copy if the values do not lie like that, so held until the launch
 };
 Lengths lengths_of(const c10::optional<at::Tensor>& lengths, int64_t B, int64_t R) {
   if (!lengths) return {};
   const at::Tensor& t = *lengths;
   if (t.scalar_type() != at::kInt || !t.is_cuda() || t.numel() != B * R)
     throw py::value_error("lengths must be a CUDA int32 tensor with B*N=" + std::to_string(B * R) + " values");
-  const at::Tensor v = t.dim() == 2 ? t : t.reshape({B, R});
-  return {v.data_ptr<int32_t>(), v.stride(0), v.stride(1)};
+  const at::Tensor v = t.reshape({B, R});
+  return {v.data_ptr<int32_t>(), v.stride(0), v.stride(1), v};
 }
 
 struct Mask {

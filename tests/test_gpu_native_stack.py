@@ -130,3 +130,15 @@ def test_single_track_inputs_that_do_not_fit_are_refused():
     for residual in (s[:1], s[:, :1], s[..., :128]):
         with pytest.raises(ValueError):
             stack.layers[0].attention(s, z, mask, residual=residual)
+
+
+def test_row_lengths_of_another_shape_mean_their_values_in_order():
+    """[B * N] and any other shape of B * N values are read as [B, N], also where that takes a copy."""
+    node = _randomise(b200.TriangleAttentionStartingNode(128, 32, 4, dtype=torch.bfloat16).to(DEV))
+    z = torch.randn(3, 20, 20, 128, device=DEV).bfloat16()
+    lengths = torch.randint(1, 21, (3, 20), device=DEV, dtype=torch.int32)
+    want = node(z, mask_bias=lengths)
+    strided = torch.zeros(20, 3, 2, device=DEV, dtype=torch.int32)
+    strided[..., 0] = lengths.reshape(20, 3)
+    for other in (lengths.reshape(-1), lengths.reshape(20, 3), strided[..., 0], lengths.t().contiguous().t()):
+        assert torch.equal(node(z, mask_bias=other), want)
