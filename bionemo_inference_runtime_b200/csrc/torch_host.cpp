@@ -85,14 +85,14 @@ at::Tensor new_bf16(const at::Tensor& like, at::IntArrayRef shape) {
   return at::empty(shape, like.options().dtype(at::kBFloat16).memory_format(c10::MemoryFormat::Contiguous));
 }
 
-// The buffer kept in `buffers` (a dict or None) under `key`, replaced only when its shape, dtype or device changed; a
-// fresh tensor when there is no dict.
+// The buffer kept in `buffers` (a dict or None) under `key`, replaced when it is not a contiguous tensor of this shape, dtype
+// and device (callers put their own in as well); a fresh tensor when there is no dict.
 at::Tensor buffer(const py::object& buffers, const char* key, at::IntArrayRef shape, at::ScalarType dtype,
                   const at::Tensor& like) {
   if (!buffers.is_none()) {
     if (PyObject* held = PyDict_GetItemString(buffers.ptr(), key); held != nullptr && THPVariable_Check(held)) {
       const at::Tensor& t = THPVariable_Unpack(held);
-      if (t.sizes() == shape && t.scalar_type() == dtype && t.device() == like.device()) return t;
+      if (t.sizes() == shape && t.scalar_type() == dtype && t.device() == like.device() && t.is_contiguous()) return t;
     }
   }
   at::Tensor t = at::empty(shape, like.options().dtype(dtype));

@@ -142,3 +142,13 @@ def test_row_lengths_of_another_shape_mean_their_values_in_order():
     strided[..., 0] = lengths.reshape(20, 3)
     for other in (lengths.reshape(-1), lengths.reshape(20, 3), strided[..., 0], lengths.t().contiguous().t()):
         assert torch.equal(node(z, mask_bias=other), want)
+
+
+def test_a_buffer_that_is_not_contiguous_is_replaced():
+    node = _randomise(b200.TriangleAttentionStartingNode(128, 32, 4, dtype=torch.bfloat16).to(DEV))
+    z = torch.randn(1, 40, 40, 128, device=DEV).bfloat16()
+    buffers = {}
+    want = node(z, buffers=buffers)
+    workspace = buffers["tri_attn_workspace"]
+    buffers["tri_attn_workspace"] = torch.zeros(1, dtype=torch.uint8, device=DEV).expand(workspace.shape)
+    assert torch.equal(node(z, buffers=buffers), want) and buffers["tri_attn_workspace"].is_contiguous()
