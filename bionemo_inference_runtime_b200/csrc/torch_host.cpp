@@ -451,6 +451,7 @@ class Stack {
                                         bool mask_output, const c10::optional<at::Tensor>& key_counts,
                                         const py::object& given_buffers, SideTrack* track) {
     pair_of("z", z, false);
+    if (s && singles_.size() != blocks_.size()) throw py::value_error("every block needs the weights of its single track");
     if (s && !singles_.empty()) check_single(*s, z.size(0), z.size(1), singles_[0].w_in);  // before anything is enqueued
     const py::object buffers = given_buffers.is_none() ? py::object(py::dict()) : given_buffers;  // held until the join
     const at::Tensor ws = node_workspace(buffers, z);

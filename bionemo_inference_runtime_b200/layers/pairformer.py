@@ -83,16 +83,26 @@ def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
     return None if chunked else native
 
 
+def _more_than_its_class(module: nn.Module) -> bool:
+    """Whether a call of ``module`` may do something else than its class's ``forward``: it is hooked or compiled, or one of
+    the class's functions is replaced in the instance."""
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._compiled_call_impl is not None
+                or any(callable(getattr(type(module), name, None)) for name in vars(module)))
+
+
 def _build_native_stack(layers, device):
-    if any(m._forward_hooks or m._forward_pre_hooks for m in layers.modules()):
+    if any(map(_more_than_its_class, layers.modules())):
         return None
     bf16 = torch.bfloat16
-    stack = _host.Stack()
+    stack, first = _host.Stack(), layers[0]
     for layer in layers:
+        if layer.no_update_s != first.no_update_s:
+            return None  # one call walks both tracks of all blocks, or the pair track alone
         if type(layer) not in (PairformerLayerV1, PairformerLayerV2, PairformerNoSeqLayer) or layer.dtype != bf16:
             return None
         tri, nodes, trans = (layer.tri_mul_out, layer.tri_mul_in), (layer.tri_attn_start, layer.tri_attn_end), layer.transition_z
-        if (any(type(t) is not TriangleMultiplicationNode or t.mean_normalization for t in tri)
+        if (any(type(t) is not TriangleMultiplicationNode or t.mean_normalization
+                or t.pair_mask_left_aligned != first.tri_mul_out.pair_mask_left_aligned for t in tri)  # masked output: all or none
                 or [int(t.multiplication_type) for t in tri] != [0, 1]
                 or [type(n) for n in nodes] != [TriangleAttentionStartingNode, TriangleAttentionEndingNode]
                 or [int(n.node_type) for n in nodes] != [0, 1]
@@ -109,7 +119,8 @@ def _build_native_stack(layers, device):
             continue
         attn, trans = layer.attention, layer.transition_s
         if (type(attn) is not AttentionPairBias or type(trans) is not Transition or trans.dtype != bf16 or trans._fused
-                or (isinstance(layer, PairformerLayerV2) and (not layer._pre_norm_folded or layer.post_norm_s is not None))):
+                or (isinstance(layer, PairformerLayerV2) and (not layer._pre_norm_folded or layer.post_norm_s is not None))
+                or any(norm is not getattr(layer, "pre_norm_s", None) for norm in attn._input_norm)):  # (not in the state)
             return None
         w, t, norm = attn._weights(device), trans._packed(device), attn._norm_of_s()
         stack.add_single(w["w_in"], w["sc_in"], w["w_o"], w["sc_o"], w["packed_z"], norm is not None,

@@ -4,6 +4,7 @@ import copy
 import pickle
 from types import SimpleNamespace
 
+import pytest
 import torch
 
 import bionemo_inference_runtime_b200 as b200
@@ -89,3 +90,36 @@ def test_state_is_not_copied_with_a_layer():
     stack._native = pairformer._NativeStack(stack.layers, torch.device("cpu"), None, [])
     assert copy.deepcopy(layer)._pack_state is None and copy.deepcopy(stack)._native is None
     assert pickle.loads(pickle.dumps(layer))._pack_state is None and pickle.loads(pickle.dumps(stack))._native is None
+
+
+def _patch_forward(layers):
+    layers[1].tri_attn_end.forward = lambda *args, **kwargs: None
+
+
+def _compile(layers):
+    layers[1].transition_z._compiled_call_impl = lambda *args, **kwargs: None
+
+
+def _one_without_single_track(layers):
+    layers[1].no_update_s = True
+
+
+def _one_without_masked_output(layers):
+    layers[1].tri_mul_in.pair_mask_left_aligned = False
+
+
+def _foreign_norm(layers):
+    layers[1].attention.set_input_norm(torch.nn.LayerNorm(384))
+
+
+@pytest.mark.parametrize("change", [_patch_forward, _compile, _one_without_single_track, _one_without_masked_output, _foreign_norm])
+def test_layers_that_differ_from_the_native_form_are_called_themselves(monkeypatch, change):
+    pack = torch.zeros(1)
+    for cls in (b200.TriangleMultiplicationNode, b200.TriangleAttentionStartingNode, b200.TriangleAttentionEndingNode):
+        monkeypatch.setattr(cls, "_packed", lambda self, device: pack)
+    monkeypatch.setattr(b200.Transition, "_packed", lambda self, device: pack if self._fused else dict.fromkeys(("w1", "sc1", "w2", "sc2"), pack))
+    monkeypatch.setattr(b200.AttentionPairBias, "_weights", lambda self, device: dict.fromkeys(("w_in", "sc_in", "w_o", "sc_o", "packed_z"), pack))
+    layers = _stack().layers
+    assert pairformer._build_native_stack(layers, "cpu") is not None
+    change(layers)
+    assert pairformer._build_native_stack(layers, "cpu") is None
