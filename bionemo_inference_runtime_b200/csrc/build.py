@@ -8,6 +8,8 @@ driver symbol it needs at run time, so it loads on machines without a GPU.
 from __future__ import annotations
 
 import argparse
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -20,6 +22,7 @@ PKG = CSRC.parent
 LIB = PKG / "libb200ta.so"
 HOST = PKG / "_host.so"
 OBJ_DIR = CSRC / "build"
+HOST_MADE_FOR = "host_made_for.txt"
 SOURCES = ["host.cu", "pack.cu", "rowgemm.cu", "attention.cu", "node.cu", "transition.cu", "trimul_project.cu",
            "trimul_contract.cu", "trimul_output.cu", "linear.cu", "pair_bias.cu", "masks.cu"]
 NVCC_FLAGS = [
@@ -47,25 +50,42 @@ def _stale(target: Path, sources: list[Path]) -> bool:
     return any(s.stat().st_mtime > t for s in sources)
 
 
+def _host_made_for() -> str:
+    """What _host.so depends on besides its sources: the installed PyTorch, whose headers and C++ ABI it is built with, the
+    interpreter and the CUDA headers."""
+    torch = importlib.util.find_spec("torch")
+    return "\n".join([f"torch {importlib.metadata.version('torch')} {Path(torch.origin).parent}", f"python {sys.version}",
+                      f"cuda {Path(_nvcc()).resolve().parent.parent}"])
+
+
+def _host_stale() -> bool:
+    """Whether _host.so is missing, older than its sources or made for another PyTorch, interpreter or toolkit."""
+    made_for = OBJ_DIR / HOST_MADE_FOR
+    return (_stale(HOST, [CSRC / "torch_host.cpp", PKG.parent / "include" / "b200ta.h"])
+            or not made_for.exists() or made_for.read_text() != _host_made_for())
+
+
 def _build_host(force: bool) -> None:
     """_host.so from torch_host.cpp against the headers of the installed PyTorch; it links none of the kernels."""
-    src = CSRC / "torch_host.cpp"
-    if not (force or _stale(HOST, [src, PKG.parent / "include" / "b200ta.h"])):
+    if not (force or _host_stale()):
         return
     import sysconfig
 
+    import torch
     from torch.utils.cpp_extension import include_paths, library_paths
 
     cuda = Path(_nvcc()).resolve().parent.parent
     cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
-           "-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_host", "-D_GLIBCXX_USE_CXX11_ABI=1",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            *(f"-I{p}" for p in include_paths()), f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}",
-           str(src), "-o", str(HOST), *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           str(CSRC / "torch_host.cpp"), "-o", str(HOST), *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch_python", f"-L{cuda / 'lib64'}", "-lcudart", "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("building _host.so failed")
+    (OBJ_DIR / HOST_MADE_FOR).write_text(_host_made_for())
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
