@@ -321,9 +321,9 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Warp-collective forms, with A in shared or tensor memory: executed by all 32 lanes of a converged warp with the same operands; one elected
-// lane issues.  A warp that stays converged lets the compiler keep descriptors and addresses in uniform
-// registers: measured on B200, a thread inside an `if (lane == 0)` branch issues one tcgen05.mma every 45-80
+// Warp-collective forms (A in shared or in tensor memory): executed by all 32 lanes of a converged warp with the same
+// operands; one elected lane issues.  A warp that stays converged lets the compiler keep descriptors and addresses in
+// uniform registers: measured on B200, a thread inside an `if (lane == 0)` branch issues one tcgen05.mma every 45-80
 // clocks whatever its size, the collective form one every 15 (N = 32) to 50 (N = 128) clocks, i.e. at the rate
 // the tensor pipe retires them.  The elected lane is the same every time (the lowest one), so a later
 // umma_commit_warp covers all MMAs of the warp.
@@ -495,6 +495,7 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+
 // Byte offset of 16-byte chunk `chunk` of row `row` inside a tile whose rows are
 // 128 bytes (128-byte swizzle) or 64 bytes (64-byte swizzle); tile base must be
 // 1024-byte (resp. 512-byte) aligned.  Matches what TMA writes and tcgen05 reads.
