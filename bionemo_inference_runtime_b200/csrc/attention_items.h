@@ -96,9 +96,12 @@ inline void fast_div_constants(uint32_t d, uint32_t* mul, uint32_t* shr) {
 // How the units (128 queries of one row and head) of a (b, h) are put together into items of up to four.
 // Normally the query blocks go two by two with two rows each and an odd last block with four rows.  A problem with
 // too few units to fill the SMs that way takes fewer units per item instead: a CTA with one or two units finishes a
-// tile in some 1000 to 1600 clocks of latency, one with four in some 2700.  For the same reason, when the items come
-// to a few waves and less than half a wave, the rows of that remainder go to items of two units, which still make
-// only one wave and a shorter one (256 tokens: 3.46 waves of items, 43 us; 3 waves and one of halves: 41 us).
+// tile in some 1000 to 1600 clocks of latency, one with four in some 2800.  For the same reason, when the last wave is at
+// most half full, the rows that do not fill whole waves go to items of two units, provided that no CTA gets more items
+// that way (with many (b, h) of few rows, rows in steps of four leave too much over: 20 x 16 rows of 384 97 us, undivided
+// 89).  What it gives goes down with the number of waves: 6-7 % at 2-3 waves (225 tokens 39.3 -> 36.9 us), 3-4 % at 7 (360
+// tokens 98.5 -> 95.6), 2 % at 11 (423 tokens 160.9 -> 157.4); at 12 to 16 it would still be 1.5 to 2.4 % (494 tokens
+// 203.5 -> 199.9), from 18 on it was between +1.7 and -2.5 %, with runs that differ by up to 2.
 inline ItemPlan split_items(int B, int R, int S, int num_sms) {
   ItemPlan p{};
   const int blocks = (S + kQTile - 1) / kQTile;
@@ -122,11 +125,12 @@ inline ItemPlan split_items(int B, int R, int S, int num_sms) {
       (blocks == 1 ? whole(0, 1, 2) : whole(blocks / 2, 1, 2)) > num_sms) {       // two units per item
     const int64_t items = whole(blocks / 2, R > 1 ? 2 : 1, R > 2 ? 4 : R);
     const int64_t waves = items / num_sms, rest = items % num_sms;
-    if (waves >= 1 && waves < 12 && rest > 0 && 2 * rest <= num_sms && R >= 8) {
+    if (waves >= 1 && waves < 12 && rest > 0 && 2 * rest <= num_sms) {
       // rows that fill the whole waves, in steps of four (one item of the odd block)
       const int64_t per_four = bh * (2 * p.pairs + p.singles);
       const int row = int(waves * num_sms / per_four) * 4;
-      if (row > 0 && row < R) fill(0, 0, row, 2, 4), fill(1, row, R, 1, 2);
+      if (row > 0 && row < R && fill(0, 0, row, 2, 4) + fill(1, row, R, 1, 2) > (waves + 1) * num_sms)
+        whole(blocks / 2, 2, 4);
     }
   }
   fast_div_constants(uint32_t(p.pairs), &p.pairs_mul, &p.pairs_shr);

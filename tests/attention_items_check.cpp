@@ -1,5 +1,6 @@
-// Walks the items of a sweep of problems: every unit (128 queries of a row and head) is in exactly one item, and the row
-// that the kernel addresses for a unit, existing or not, lies inside the tensor.
+// Walks the items of a sweep of problems: every unit (128 queries of a row and head) is in exactly one item, the row
+// that the kernel addresses for a unit, existing or not, lies inside the tensor, and rows put into smaller items for the last
+// wave do not make another wave.
 #include <cstdio>
 #include <vector>
 
@@ -22,6 +23,10 @@ static int check(int B, int R, int S, int num_sms) {
       ++seen[((size_t(it.b) * kHeads + it.h) * R + it.r0 + unit_row(it, u)) * blocks + block];
     }
   }
+  const long long bh = (long long)B * kHeads;
+  const long long undivided = bh * (blocks / 2 * ((R + 1) / 2) + blocks % 2 * ((R + 3) / 4));
+  if (plan.group[1].num_items > 0 && plan.num_items > (undivided + num_sms - 1) / num_sms * num_sms)
+    return std::printf("another wave: %d %d %d %d\n", B, R, S, num_sms);
   for (int n : seen)
     if (n != 1) return std::printf("unit %d times: %d %d %d %d\n", n, B, R, S, num_sms);
   return 0;
@@ -29,8 +34,8 @@ static int check(int B, int R, int S, int num_sms) {
 
 int main() {
   for (int num_sms : {1, 7, 148})
-    for (int B : {1, 2, 5})
-      for (int R : {1, 2, 3, 4, 5, 7, 8, 37, 63, 64, 65, 129, 201, 333})
+    for (int B : {1, 2, 5, 20})
+      for (int R : {1, 2, 3, 4, 5, 7, 8, 16, 37, 63, 64, 65, 129, 201, 333})
         for (int S : {1, 127, 128, 129, 256, 257, 385, 512, 640, 1025})
           if (check(B, R, S, num_sms) != 0) return 1;
   std::puts("ok");
