@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t p_column(int unit, int buffer) { return kTme
 // What the other warps need to know about an item, written by the TMA warp into the item's slot (released by Q_FULL).
 struct __align__(16) UnitInfo {
   int br;     // b * R + r of the unit's pair row; of the item's last row where the item has no such unit
-  int q0;     // first query
+  int q0;     // first query; S, past the last one, where the item has no such unit
   int len;    // keys that take part (S for a uniform row)
   int tiles;  // key tiles; 0: no valid key and "zeros" semantics; -1: the item has no such unit
 };
@@ -212,7 +212,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int br = it.b * p.R + it.r0;
       if (lane < kUnits) {
         *reinterpret_cast<int4*>(&info->unit[lane]) =
-            make_int4(br + existing_row(it, lane), it.q0 + (it.two_blocks ? lane & 1 : 0) * kQTile, len, nt);
+            make_int4(br + existing_row(it, lane), exists ? it.q0 + (it.two_blocks ? lane & 1 : 0) * kQTile : p.S, len, nt);
       } else if (lane == kUnits) {
         *reinterpret_cast<int4*>(&info->tiles) = make_int4(tiles, it.two_blocks, it.h, int(uniform));
       }
@@ -378,7 +378,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int my_tiles = unit.w, len = unit.z;
       const bool uniform = (common.w >> w) & 1;
       const uint32_t block_off = stage_bias(common.y ? w & 1 : 0) + sw128_offset(m, 0);
-      if (p.gate != nullptr && my_tiles > 0 && unit.y + m < p.S)  // read at the end
+      if (p.gate != nullptr && unit.y + m < p.S)  // read at the end; (a missing unit has no query below S)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + unit.x * p.g_br + common.z * p.g_h + (long long)(unit.y + m) * p.g_s));
       float row_max = 0.f, row_sum = 0.f;  // row_max: reference point of the exponentials, in raw score units
       const uint32_t* mask_row = nullptr;
