@@ -520,105 +520,172 @@ std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additiv
   return {lengths, bits};
 }
 
-// ---- weight state --------------------------------------------------------------------------------------------------
+// ---- state of modules ------------------------------------------------------------------------------------------------
 
-// The parameters under some modules as they were seen: storage, address, in-place write count, device.  The storages are
-// held weakly: their memory is free to go, but another storage cannot come to be at the address of one that was seen, so
-// that a parameter replaced twice does not look unchanged when its memory is given out again.  Not copied or pickled
-// with the layers that keep one.
-class WeightState {
- public:
-  struct Seen {
-    c10::weak_intrusive_ptr<c10::StorageImpl> storage;
-    const void* data;
-    int64_t version;  // inference tensors have none
-    c10::Device device;
-  };
-  bool operator==(const WeightState& o) const {
-    if (seen.size() != o.seen.size()) return false;
-    for (size_t i = 0; i < seen.size(); ++i) {
-      const Seen &a = seen[i], &b = o.seen[i];
-      if (a.storage._unsafe_get_target() != b.storage._unsafe_get_target() || a.data != b.data || a.version != b.version ||
-          a.device != b.device)
-        return false;
-    }
-    return true;
-  }
-  void add_parameters(PyObject* module) {
-    static PyObject* const k_parameters = PyUnicode_InternFromString("_parameters");
-    static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
-    PyObject** dict = _PyObject_GetDictPtr(module);
-    if (dict == nullptr || *dict == nullptr) return;
-    PyObject *key, *value;
-    Py_ssize_t pos = 0;
-    if (PyObject* parameters = PyDict_GetItem(*dict, k_parameters); parameters != nullptr && PyDict_Check(parameters)) {
-      while (PyDict_Next(parameters, &pos, &key, &value)) {
-        if (!THPVariable_Check(value)) continue;
-        const at::Tensor& t = THPVariable_Unpack(value);
-        seen.push_back({t.storage().getWeakStorageImpl(), t.data_ptr(), t.is_inference() ? -1 : int64_t(t._version()), t.device()});
-      }
-    }
-    pos = 0;
-    if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
-      while (PyDict_Next(modules, &pos, &key, &value))
-        if (value != Py_None) add_parameters(value);
-  }
-
- private:
-  std::vector<Seen> seen;
+// What a visit of modules looks at, in an order that depends on the modules alone.  A visitor has object(PyObject*) and
+// parameter(const at::Tensor&), which return false to end the visit.
+struct Names {
+  PyObject* const parameters = PyUnicode_InternFromString("_parameters");
+  PyObject* const modules = PyUnicode_InternFromString("_modules");
+  PyObject* const hooks = PyUnicode_InternFromString("_forward_hooks");
+  PyObject* const pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks");
+  PyObject* const compiled = PyUnicode_InternFromString("_compiled_call_impl");
 };
-
-// Changes when a weight under the modules is loaded, edited or replaced.
-WeightState weight_state(const py::args& modules) {
-  WeightState out;
-  for (const py::handle& m : modules) out.add_parameters(m.ptr());
-  return out;
+const Names& names() {
+  static const Names n;
+  return n;
 }
 
-// ---- module state ----------------------------------------------------------------------------------------------------
-
-// Calls visit(object) for `module`, the names and values of its attributes and its forward hooks, and the same of every
-// module under it, in an order that depends on the modules alone; stops at, and returns, the first false.  The layers'
-// packed weights are among the attributes; the parameters are left out (weight_state() covers those).
-template <typename Visit>
-bool visit_objects(PyObject* module, const Visit& visit) {
-  static PyObject* const k_modules = PyUnicode_InternFromString("_modules");
-  static PyObject* const k_hooks[] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks")};
-  if (!visit(module)) return false;
-  PyObject** dict = _PyObject_GetDictPtr(module);
-  if (dict == nullptr || *dict == nullptr) return true;
+template <typename Visitor>
+bool visit_parameters(PyObject* parameters, Visitor& v) {
   PyObject *key, *value;
   Py_ssize_t pos = 0;
-  while (PyDict_Next(*dict, &pos, &key, &value))
-    if (!visit(key) || !visit(value)) return false;
-  for (PyObject* k : k_hooks) {
-    PyObject* hooks = PyDict_GetItem(*dict, k);
-    pos = 0;
-    if (hooks != nullptr && PyDict_Check(hooks))
-      while (PyDict_Next(hooks, &pos, &key, &value))
-        if (!visit(value)) return false;
-  }
-  pos = 0;
-  if (PyObject* modules = PyDict_GetItem(*dict, k_modules); modules != nullptr && PyDict_Check(modules))
-    while (PyDict_Next(modules, &pos, &key, &value))
-      if (value != Py_None && !visit_objects(value, visit)) return false;
+  if (parameters != nullptr && PyDict_Check(parameters))
+    while (PyDict_Next(parameters, &pos, &key, &value))
+      if (THPVariable_Check(value) && !v.parameter(THPVariable_Unpack(value))) return false;
   return true;
 }
 
-// What visit_objects() sees, as a tuple that holds it: an object in it cannot make room for another one at its address.
-py::tuple module_objects(const py::handle& module) {
-  py::list out;
-  visit_objects(module.ptr(), [&](PyObject* o) { return PyList_Append(out.ptr(), o) == 0; });
-  if (PyErr_Occurred()) throw py::error_already_set();
-  return py::tuple(out);
+// The parameters of `module` and of every module under it.
+template <typename Visitor>
+bool visit_weights(PyObject* module, Visitor& v) {
+  PyObject** dict = _PyObject_GetDictPtr(module);
+  if (dict == nullptr || *dict == nullptr) return true;
+  if (!visit_parameters(PyDict_GetItem(*dict, names().parameters), v)) return false;
+  PyObject *key, *value;
+  Py_ssize_t pos = 0;
+  if (PyObject* modules = PyDict_GetItem(*dict, names().modules); modules != nullptr && PyDict_Check(modules))
+    while (PyDict_Next(modules, &pos, &key, &value))
+      if (value != Py_None && !visit_weights(value, v)) return false;
+  return true;
 }
 
-// Whether visit_objects() sees the very objects of `held`: no module, option or hook has been replaced since.
-bool same_objects(const py::tuple& held, const py::handle& module) {
-  Py_ssize_t i = 0;
-  const Py_ssize_t n = PyTuple_GET_SIZE(held.ptr());
-  const bool same = visit_objects(module.ptr(), [&](PyObject* o) { return i < n && PyTuple_GET_ITEM(held.ptr(), i++) == o; });
-  return same && i == n;
+// `module`, the names and values of its attributes (options, packed weights, ...), its forward hooks and its parameters,
+// and the same of every module under it.
+template <typename Visitor>
+bool visit_all(PyObject* module, Visitor& v) {
+  if (!v.object(module)) return false;
+  PyObject** dict = _PyObject_GetDictPtr(module);
+  if (dict == nullptr || *dict == nullptr) return true;
+  const Names& n = names();
+  PyObject *parameters = nullptr, *modules = nullptr, *hooks[2] = {nullptr, nullptr}, *key, *value;
+  Py_ssize_t pos = 0;
+  while (PyDict_Next(*dict, &pos, &key, &value)) {
+    if (!v.object(key) || !v.object(value)) return false;
+    if (key == n.parameters) parameters = value;
+    if (key == n.modules) modules = value;
+    if (key == n.hooks) hooks[0] = value;
+    if (key == n.pre_hooks) hooks[1] = value;
+  }
+  for (PyObject* h : hooks) {
+    pos = 0;
+    if (h != nullptr && PyDict_Check(h))
+      while (PyDict_Next(h, &pos, &key, &value))
+        if (!v.object(value)) return false;
+  }
+  if (!visit_parameters(parameters, v)) return false;
+  pos = 0;
+  if (modules != nullptr && PyDict_Check(modules))
+    while (PyDict_Next(modules, &pos, &key, &value))
+      if (value != Py_None && !visit_all(value, v)) return false;
+  return true;
+}
+
+// Parameters as they were seen: storage, address, in-place write count, device.  The storages are held weakly: their
+// memory is free to go, but another storage cannot come to be at the address of one that was seen, so that a parameter
+// replaced twice does not look unchanged when its memory is given out again.  Not copied or pickled with the layers that
+// keep one.
+class WeightState {
+ public:
+  void add(const at::Tensor& t) { seen_.push_back({t.storage().getWeakStorageImpl(), t.data_ptr(), version(t), t.device()}); }
+  bool same(size_t i, const at::Tensor& t) const {
+    return i < seen_.size() && seen_[i].storage._unsafe_get_target() == t.storage().unsafeGetStorageImpl() &&
+           seen_[i].data == t.data_ptr() && seen_[i].version == version(t) && seen_[i].device == t.device();
+  }
+  size_t size() const { return seen_.size(); }
+
+ private:
+  struct Seen {
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+    const void* data;
+    int64_t version;
+    c10::Device device;
+  };
+  static int64_t version(const at::Tensor& t) { return t.is_inference() ? -1 : int64_t(t._version()); }  // inference tensors have none
+  std::vector<Seen> seen_;
+};
+
+struct RecordAll {
+  WeightState weights;
+  std::vector<PyObject*> objects;
+  bool object(PyObject* o) { return objects.push_back(o), true; }
+  bool parameter(const at::Tensor& t) { return weights.add(t), true; }
+};
+struct CompareAll {
+  const WeightState* weights;
+  PyObject* const* objects = nullptr;
+  size_t num_objects = 0, i = 0, k = 0;
+  bool object(PyObject* o) { return i < num_objects && objects[i++] == o; }
+  bool parameter(const at::Tensor& t) { return weights->same(k++, t); }
+  bool complete() const { return i == num_objects && k == weights->size(); }
+};
+
+// The parameters under the modules, and whether they are still what `state` (None: nothing) saw: a weight that is loaded,
+// edited or replaced changes that.
+WeightState weight_state(const py::args& modules) {
+  RecordAll r;
+  for (const py::handle& m : modules) visit_weights(m.ptr(), r);
+  return std::move(r.weights);
+}
+bool same_weights(const WeightState* state, const py::args& modules) {
+  if (state == nullptr) return false;
+  CompareAll c{state};
+  for (const py::handle& m : modules)
+    if (!visit_weights(m.ptr(), c)) return false;
+  return c.complete();
+}
+
+// All that visit_all() sees of `module`: the objects in a tuple, which holds them (an object in it cannot make room for
+// another one at its address), and the parameters.
+std::pair<py::tuple, WeightState> module_state(const py::handle& module) {
+  RecordAll r;
+  visit_all(module.ptr(), r);
+  py::tuple objects(r.objects.size());
+  for (size_t i = 0; i < r.objects.size(); ++i) {
+    Py_INCREF(r.objects[i]);
+    PyTuple_SET_ITEM(objects.ptr(), i, r.objects[i]);
+  }
+  return {std::move(objects), std::move(r.weights)};
+}
+bool same_state(const py::tuple& objects, const WeightState& weights, const py::handle& module) {
+  CompareAll c{&weights, PySequence_Fast_ITEMS(objects.ptr()), objects.size()};
+  return visit_all(module.ptr(), c) && c.complete();
+}
+
+// Whether a call of `module`, or of a module under it, may do something else than its class's forward: it is hooked or
+// compiled, or one of the class's functions is replaced in the instance.
+bool more_than_its_class(PyObject* module) {
+  PyObject** dict = _PyObject_GetDictPtr(module);
+  if (dict == nullptr || *dict == nullptr) return true;
+  const Names& n = names();
+  PyObject *modules = nullptr, *key, *value;
+  Py_ssize_t pos = 0;
+  while (PyDict_Next(*dict, &pos, &key, &value)) {
+    if (key == n.modules) modules = value;
+    if ((key == n.hooks || key == n.pre_hooks) && PyDict_Check(value) && PyDict_Size(value) > 0) return true;
+    if (key == n.compiled && value != Py_None) return true;
+    if (!PyCallable_Check(value)) continue;
+    PyObject* of_class = PyObject_GetAttr(reinterpret_cast<PyObject*>(Py_TYPE(module)), key);
+    const bool replaced = of_class != nullptr && PyCallable_Check(of_class);
+    Py_XDECREF(of_class);
+    PyErr_Clear();
+    if (replaced) return true;
+  }
+  pos = 0;
+  if (modules != nullptr && PyDict_Check(modules))
+    while (PyDict_Next(modules, &pos, &key, &value))
+      if (value != Py_None && more_than_its_class(value)) return true;
+  return false;
 }
 
 }  // namespace
@@ -641,13 +708,14 @@ PYBIND11_MODULE(_host, m) {
       .def("add_single", &Stack::add_single)
       .def("run_pair", &Stack::run_pair)
       .def("run_both", &Stack::run_both);
-  m.def("module_objects", &module_objects);
-  m.def("same_objects", &same_objects);
+  m.def("more_than_its_class", [](const py::handle& module) { return more_than_its_class(module.ptr()); });
+  m.def("module_state", &module_state);
+  m.def("same_state", &same_state);
   m.def("mask_lengths", &mask_lengths);
   m.def("mask_bits", &mask_bits);
   py::class_<WeightState>(m, "WeightState")
-      .def("__eq__", [](const WeightState& a, const py::object& b) { return py::isinstance<WeightState>(b) && a == b.cast<const WeightState&>(); })
       .def("__deepcopy__", [](const WeightState&, const py::object&) { return py::none(); })
       .def("__reduce__", [](const WeightState&) { return py::make_tuple(py::type::of(py::none()), py::tuple()); });
+  m.def("same_weights", &same_weights);
   m.def("weight_state", &weight_state);
 }

@@ -147,11 +147,11 @@ class AttentionPairBias(nn.Module):
 
     @torch.no_grad()
     def _weights(self, device) -> dict:
-        state = _host.weight_state(self, *self._input_norm)
-        if self._folded is None or self._folded["w_in"].device != device or state != self._folded_state:
+        if (self._folded is None or self._folded["w_in"].device != device
+                or not _host.same_weights(self._folded_state, self, *self._input_norm)):
             folded = self._fold(device)
             if not torch.cuda.is_current_stream_capturing():
-                self._folded, self._folded_state = folded, state
+                self._folded, self._folded_state = folded, _host.weight_state(self, *self._input_norm)
             return folded
         return self._folded
 

@@ -41,10 +41,10 @@ class _LayersState:
     whose addresses a native stack or a graph has recorded stay allocated.  Not copied or pickled with the module."""
 
     def __init__(self, layers):
-        self.objects, self.weights = _host.module_objects(layers), _host.weight_state(layers)
+        self.objects, self.weights = _host.module_state(layers)
 
     def holds(self, layers) -> bool:
-        return _host.same_objects(self.objects, layers) and _host.weight_state(layers) == self.weights
+        return _host.same_state(self.objects, self.weights, layers)
 
     def __deepcopy__(self, memo):
         return None
@@ -83,15 +83,8 @@ def _native_stack(module: nn.Module, z: torch.Tensor) -> "_NativeStack | None":
     return None if chunked else native
 
 
-def _more_than_its_class(module: nn.Module) -> bool:
-    """Whether a call of ``module`` may do something else than its class's ``forward``: it is hooked or compiled, or one of
-    the class's functions is replaced in the instance."""
-    return bool(module._forward_hooks or module._forward_pre_hooks or module._compiled_call_impl is not None
-                or any(callable(getattr(type(module), name, None)) for name in vars(module)))
-
-
 def _build_native_stack(layers, device):
-    if any(map(_more_than_its_class, layers.modules())):
+    if _host.more_than_its_class(layers):  # hooked, compiled or patched
         return None
     bf16 = torch.bfloat16
     stack, first = _host.Stack(), layers[0]

@@ -96,12 +96,11 @@ class Transition(nn.Module):
         return {"w1": w1_f, "sc1": sc1, "w2": w2_f, "sc2": sc2}
 
     def _packed(self, device) -> torch.Tensor:
-        state = _host.weight_state(self)
         held = self._pack["w1"] if isinstance(self._pack, dict) else self._pack
-        if held is None or held.device != device or state != self._pack_state:
+        if held is None or held.device != device or not _host.same_weights(self._pack_state, self):
             pack = self._fold(device)
             if not torch.cuda.is_current_stream_capturing():
-                self._pack, self._pack_state = pack, state
+                self._pack, self._pack_state = pack, _host.weight_state(self)
             return pack
         return self._pack
 
@@ -182,11 +181,10 @@ class PairTransition(nn.Module):
         self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _host.weight_state(self)
-        if self._pack is None or self._pack.device != device or state != self._pack_state:
+        if self._pack is None or self._pack.device != device or not _host.same_weights(self._pack_state, self):
             pack = ops.pack_relu_transition_weights(*[t.to(device) for t in self._params()])
             if not torch.cuda.is_current_stream_capturing():
-                self._pack, self._pack_state = pack, state
+                self._pack, self._pack_state = pack, _host.weight_state(self)
             return pack
         return self._pack
 

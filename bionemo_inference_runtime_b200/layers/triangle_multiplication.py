@@ -126,12 +126,11 @@ class TriangleMultiplicationNode(nn.Module):
         self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _host.weight_state(self)
-        if self._pack is None or self._pack.device != device or state != self._pack_state:
+        if self._pack is None or self._pack.device != device or not _host.same_weights(self._pack_state, self):
             pack = self._fold(device)
             # a fold recorded during graph capture is only filled at replay: use it for this call only
             if not torch.cuda.is_current_stream_capturing():
-                self._pack, self._pack_state = pack, state
+                self._pack, self._pack_state = pack, _host.weight_state(self)
             return pack
         return self._pack
 

@@ -82,13 +82,12 @@ class TriangleAttention(nn.Module):
 
     def _packed(self, device) -> torch.Tensor:
         """Packed weights for the stand-alone path (no LayerNorm, zero triangle-bias rows)."""
-        state = _host.weight_state(self)
-        if self._pack is None or self._pack.device != device or state != self._pack_state:
+        if self._pack is None or self._pack.device != device or not _host.same_weights(self._pack_state, self):
             zero_bias_rows = torch.zeros((ops.HEADS, ops.C), dtype=self.in_proj.weight.dtype, device=device)
             pack = ops.pack_node_weights(None, None, self.in_proj.weight, self.in_proj.bias, zero_bias_rows,
                                          self.o_proj.weight, self.o_proj.bias)
             if not torch.cuda.is_current_stream_capturing():
-                self._pack, self._pack_state = pack, state
+                self._pack, self._pack_state = pack, _host.weight_state(self)
             return pack
         return self._pack
 
@@ -186,12 +185,11 @@ class TriangleAttentionNode(nn.Module):
         self._pack_state = _host.weight_state(self)
 
     def _packed(self, device) -> torch.Tensor:
-        state = _host.weight_state(self)
-        if self._pack is None or self._pack.device != device or state != self._pack_state:
+        if self._pack is None or self._pack.device != device or not _host.same_weights(self._pack_state, self):
             pack = ops.pack_node_weights(*[None if p is None else p.to(device) for p in self._params()])
             # a fold recorded during graph capture is only filled at replay: use it for this call only
             if not torch.cuda.is_current_stream_capturing():
-                self._pack, self._pack_state = pack, state
+                self._pack, self._pack_state = pack, _host.weight_state(self)
             return pack
         return self._pack
 

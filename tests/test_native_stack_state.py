@@ -74,13 +74,13 @@ def test_a_parameter_replaced_at_its_old_address_is_seen():
     layer = b200.Transition(128, 512, dtype=torch.bfloat16).cpu()
     weight = layer.fc3.weight
     state, address = pairformer._host.weight_state(layer), weight.data_ptr()
-    assert state == pairformer._host.weight_state(layer) and state != None  # noqa: E711
+    assert pairformer._host.same_weights(state, layer) and not pairformer._host.same_weights(None, layer)
     weight.data = torch.empty(0, dtype=torch.bfloat16)
     others = []
     while len(others) < 100 and (not others or others[-1].data_ptr() != address):
         others.append(torch.zeros(128, 512, dtype=torch.bfloat16))
     weight.data = others[-1]
-    assert state != pairformer._host.weight_state(layer)
+    assert not pairformer._host.same_weights(state, layer)
 
 
 def test_state_is_not_copied_with_a_layer():
