@@ -167,6 +167,7 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_c
     const int m = (warp & 3) * 32;          // first output row of the warp == TMEM lane
     const uint32_t acc = tmem_base + (uint32_t(m) << 16) + half * kBN;
     const uint32_t slab0 = base + kSmOut + warp * 4096;
+    uint32_t stores = 0;  // the slabs take turns over all stores, whatever the number of a tile's
     bool ok = true;
     for (int i = 0; ok && i < my_tiles; ++i) {
       const Tile t = decode_tile(p, blockIdx.x + i * gridDim.x);
@@ -176,10 +177,10 @@ trimul_contract_kernel(const __grid_constant__ CUtensorMap tm_ab, const __grid_c
       const int row0 = t.m0 + half * 128 + m;
       if (row0 < p.N) {
         const int columns = p.width < p.N - t.n0 ? p.width : p.N - t.n0;
-        for (int c = 0; c < columns; c += 32) {
+        for (int c = 0; c < columns; c += 32, ++stores) {
           uint32_t a[32];
           tmem_ld32(acc + c, a);
-          const uint32_t slab = slab0 + ((c >> 5) & 1) * 2048;
+          const uint32_t slab = slab0 + (stores & 1) * 2048;
           if (lane == 0) tma_store_wait_read<1>();  // the store before the previous one has read this slab
           __syncwarp();
           tmem_ld_wait();

@@ -20,3 +20,17 @@ def test_contraction_at_tile_edges(B, N):
     assert _lib.device_status() == 0
     a, b = ab[:, :128, :, :N].float(), ab[:, 128:, :, :N].float()
     torch.testing.assert_close(x[..., :N].float(), a @ b.transpose(-1, -2), rtol=1e-2, atol=1e-2 * N**0.5)
+
+
+@pytest.mark.parametrize("N", [8, 32, 70, 96, 330])
+def test_many_tiles_with_an_odd_number_of_stores(N):
+    """Tiles of 1, 1, 3, 3 and 6 + 5 column groups, a dozen tiles a block: the two slabs of a warp have to take turns over
+    the tiles as well."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    B, pitch = 16, (N + 15) // 16 * 16
+    ab = torch.randn(B, 256, N, pitch, generator=g, device="cuda").bfloat16()
+    a, b = ab[:, :128, :, :N].float(), ab[:, 128:, :, :N].float()
+    want = a @ b.transpose(-1, -2)
+    for _ in range(5):
+        torch.testing.assert_close(ops.trimul_contract(ab, N)[..., :N].float(), want, rtol=1e-2, atol=1e-2 * N**0.5)
+    assert _lib.device_status() == 0
