@@ -523,9 +523,12 @@ std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additiv
 // ---- state of modules ------------------------------------------------------------------------------------------------
 
 // What a visit of modules looks at, in an order that depends on the modules alone.  A visitor has object(PyObject*) and
-// parameter(const at::Tensor&), which return false to end the visit.
+// tensor(const at::Tensor&), which return false to end the visit.
 struct Names {
   PyObject* const parameters = PyUnicode_InternFromString("_parameters");
+  PyObject* const buffers = PyUnicode_InternFromString("_buffers");
+  PyObject* const weight = PyUnicode_InternFromString("weight");
+  PyObject* const bias = PyUnicode_InternFromString("bias");
   PyObject* const modules = PyUnicode_InternFromString("_modules");
   PyObject* const hooks = PyUnicode_InternFromString("_forward_hooks");
   PyObject* const pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks");
@@ -537,42 +540,52 @@ const Names& names() {
 }
 
 template <typename Visitor>
-bool visit_parameters(PyObject* parameters, Visitor& v) {
+bool visit_tensors(PyObject* tensors, Visitor& v) {
   PyObject *key, *value;
   Py_ssize_t pos = 0;
-  if (parameters != nullptr && PyDict_Check(parameters))
-    while (PyDict_Next(parameters, &pos, &key, &value))
-      if (THPVariable_Check(value) && !v.parameter(THPVariable_Unpack(value))) return false;
+  if (tensors != nullptr && PyDict_Check(tensors))
+    while (PyDict_Next(tensors, &pos, &key, &value))
+      if (THPVariable_Check(value) && !v.tensor(THPVariable_Unpack(value))) return false;
   return true;
 }
 
-// The parameters of `module` and of every module under it.
+// The tensors that a layer's weights are made from, in the module with this dict: its parameters and buffers, and a weight or
+// bias that is a plain attribute (replicas of a module and pruned or re-parameterised ones have such).
+template <typename Visitor>
+bool visit_own_weights(PyObject* dict, Visitor& v) {
+  const Names& n = names();
+  if (!visit_tensors(PyDict_GetItemWithError(dict, n.parameters), v) || !visit_tensors(PyDict_GetItemWithError(dict, n.buffers), v)) return false;
+  for (PyObject* k : {n.weight, n.bias})
+    if (PyObject* t = PyDict_GetItemWithError(dict, k); t != nullptr && THPVariable_Check(t) && !v.tensor(THPVariable_Unpack(t))) return false;
+  return true;
+}
+
+// The weights of `module` and of every module under it.
 template <typename Visitor>
 bool visit_weights(PyObject* module, Visitor& v) {
   PyObject** dict = _PyObject_GetDictPtr(module);
   if (dict == nullptr || *dict == nullptr) return true;
-  if (!visit_parameters(PyDict_GetItem(*dict, names().parameters), v)) return false;
+  if (!visit_own_weights(*dict, v)) return false;
   PyObject *key, *value;
   Py_ssize_t pos = 0;
-  if (PyObject* modules = PyDict_GetItem(*dict, names().modules); modules != nullptr && PyDict_Check(modules))
+  if (PyObject* modules = PyDict_GetItemWithError(*dict, names().modules); modules != nullptr && PyDict_Check(modules))
     while (PyDict_Next(modules, &pos, &key, &value))
       if (value != Py_None && !visit_weights(value, v)) return false;
   return true;
 }
 
-// `module`, the names and values of its attributes (options, packed weights, ...), its forward hooks and its parameters,
-// and the same of every module under it.
+// `module`, the names and values of its attributes (options, packed weights, ...), its forward hooks and its weights, and
+// the same of every module under it.
 template <typename Visitor>
 bool visit_all(PyObject* module, Visitor& v) {
   if (!v.object(module)) return false;
   PyObject** dict = _PyObject_GetDictPtr(module);
   if (dict == nullptr || *dict == nullptr) return true;
   const Names& n = names();
-  PyObject *parameters = nullptr, *modules = nullptr, *hooks[2] = {nullptr, nullptr}, *key, *value;
+  PyObject *modules = nullptr, *hooks[2] = {nullptr, nullptr}, *key, *value;
   Py_ssize_t pos = 0;
   while (PyDict_Next(*dict, &pos, &key, &value)) {
     if (!v.object(key) || !v.object(value)) return false;
-    if (key == n.parameters) parameters = value;
     if (key == n.modules) modules = value;
     if (key == n.hooks) hooks[0] = value;
     if (key == n.pre_hooks) hooks[1] = value;
@@ -583,7 +596,7 @@ bool visit_all(PyObject* module, Visitor& v) {
       while (PyDict_Next(h, &pos, &key, &value))
         if (!v.object(value)) return false;
   }
-  if (!visit_parameters(parameters, v)) return false;
+  if (!visit_own_weights(*dict, v)) return false;
   pos = 0;
   if (modules != nullptr && PyDict_Check(modules))
     while (PyDict_Next(modules, &pos, &key, &value))
@@ -591,8 +604,8 @@ bool visit_all(PyObject* module, Visitor& v) {
   return true;
 }
 
-// Parameters as they were seen: storage, address, in-place write count, device.  The storages are held weakly: their
-// memory is free to go, but another storage cannot come to be at the address of one that was seen, so that a parameter
+// Weights as they were seen: storage, address, in-place write count, device.  The storages are held weakly: their
+// memory is free to go, but another storage cannot come to be at the address of one that was seen, so that a weight
 // replaced twice does not look unchanged when its memory is given out again.  Not copied or pickled with the layers that
 // keep one.
 class WeightState {
@@ -619,19 +632,19 @@ struct RecordAll {
   WeightState weights;
   std::vector<PyObject*> objects;
   bool object(PyObject* o) { return objects.push_back(o), true; }
-  bool parameter(const at::Tensor& t) { return weights.add(t), true; }
+  bool tensor(const at::Tensor& t) { return weights.add(t), true; }
 };
 struct CompareAll {
   const WeightState* weights;
   PyObject* const* objects = nullptr;
   size_t num_objects = 0, i = 0, k = 0;
   bool object(PyObject* o) { return i < num_objects && objects[i++] == o; }
-  bool parameter(const at::Tensor& t) { return weights->same(k++, t); }
+  bool tensor(const at::Tensor& t) { return weights->same(k++, t); }
   bool complete() const { return i == num_objects && k == weights->size(); }
 };
 
-// The parameters under the modules, and whether they are still what `state` (None: nothing) saw: a weight that is loaded,
-// edited or replaced changes that.
+// The weights under the modules, and whether they are still what `state` (None: nothing) saw: loading, editing or replacing
+// one changes that.
 WeightState weight_state(const py::args& modules) {
   RecordAll r;
   for (const py::handle& m : modules) visit_weights(m.ptr(), r);
@@ -646,7 +659,7 @@ bool same_weights(const WeightState* state, const py::args& modules) {
 }
 
 // All that visit_all() sees of `module`: the objects in a tuple, which holds them (an object in it cannot make room for
-// another one at its address), and the parameters.
+// another one at its address), and the weights.
 std::pair<py::tuple, WeightState> module_state(const py::handle& module) {
   RecordAll r;
   visit_all(module.ptr(), r);

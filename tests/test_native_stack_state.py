@@ -123,3 +123,21 @@ def test_layers_that_differ_from_the_native_form_are_called_themselves(monkeypat
     assert pairformer._build_native_stack(layers, "cpu") is not None
     change(layers)
     assert pairformer._build_native_stack(layers, "cpu") is None
+
+
+@pytest.mark.parametrize("kind", ["parameter", "buffer", "attribute"])
+def test_an_edited_weight_is_seen_whatever_it_is(kind):
+    layer = b200.Transition(128, 512, dtype=torch.bfloat16).cpu()
+    value = layer.fc3.weight.detach().clone()
+    if kind != "parameter":
+        del layer.fc3.weight
+        if kind == "buffer":
+            layer.fc3.register_buffer("weight", value)
+        else:
+            layer.fc3.weight = value
+    state = pairformer._host.weight_state(layer)
+    objects, weights = pairformer._host.module_state(layer)
+    assert pairformer._host.same_weights(state, layer) and pairformer._host.same_state(objects, weights, layer)
+    with torch.no_grad():
+        layer.fc3.weight.zero_()
+    assert not pairformer._host.same_weights(state, layer) and not pairformer._host.same_state(objects, weights, layer)
