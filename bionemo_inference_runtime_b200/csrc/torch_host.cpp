@@ -8,6 +8,7 @@
 //
 // The kernels' library is not linked: bind() takes its entry points from the file that the ctypes binding loaded.
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
@@ -500,8 +501,11 @@ int64_t current_stream() { return reinterpret_cast<int64_t>(stream()); }
 
 at::Tensor new_int32(const at::Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kInt)); }
 
+// Masks are reduced on their own device, which need not be the current one (they may be made before a model's device is
+// entered).
 // Keys with mask > 0.5 per row of a float [B, I, J] mask and per row of its transpose.
 std::pair<at::Tensor, at::Tensor> mask_lengths(const at::Tensor& mask) {
+  const c10::cuda::CUDAGuard guard(mask.device());
   const int B = int(mask.size(0)), I = int(mask.size(1)), J = int(mask.size(2));
   const at::Tensor rows = new_int32(mask, {B, I}), cols = new_int32(mask, {B, J});
   check(lib.mask_lengths(mask.data_ptr<float>(), mask.stride(0), mask.stride(1), mask.stride(2), rows.data_ptr<int32_t>(),
@@ -512,6 +516,7 @@ std::pair<at::Tensor, at::Tensor> mask_lengths(const at::Tensor& mask) {
 
 // Row lengths (last valid key + 1) and key bits of a float [B, R, S] mask; valid: > 0.5, or >= 0 in the additive form.
 std::pair<at::Tensor, at::Tensor> mask_bits(const at::Tensor& mask, bool additive) {
+  const c10::cuda::CUDAGuard guard(mask.device());
   const int B = int(mask.size(0)), R = int(mask.size(1)), S = int(mask.size(2));
   const at::Tensor lengths = new_int32(mask, {B, R}), bits = new_int32(mask, {B, R, (S + 31) / 32});
   check(lib.mask_bits(mask.data_ptr<float>(), mask.stride(0), mask.stride(1), mask.stride(2), additive,

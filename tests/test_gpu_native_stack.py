@@ -152,3 +152,11 @@ def test_a_buffer_that_is_not_contiguous_is_replaced():
     workspace = buffers["tri_attn_workspace"]
     buffers["tri_attn_workspace"] = torch.zeros(1, dtype=torch.uint8, device=DEV).expand(workspace.shape)
     assert torch.equal(node(z, buffers=buffers), want) and buffers["tri_attn_workspace"].is_contiguous()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_masks_are_reduced_on_their_own_device():
+    mask = (torch.rand(2, 40, 40) > 0.4).float()
+    payload = b200.precompute_pair_masks("Heuristic", mask.to("cuda:1"))  # the current device is cuda:0
+    assert payload.mask_bias.device.index == 1 and torch.equal(payload.mask_bias.cpu(), (mask > 0.5).sum(-1).int())
+    assert torch.equal(payload.mask_bias_transposed.cpu(), (mask > 0.5).sum(-2).int())
