@@ -160,3 +160,36 @@ def test_masks_are_reduced_on_their_own_device():
     payload = b200.precompute_pair_masks("Heuristic", mask.to("cuda:1"))  # the current device is cuda:0
     assert payload.mask_bias.device.index == 1 and torch.equal(payload.mask_bias.cpu(), (mask > 0.5).sum(-1).int())
     assert torch.equal(payload.mask_bias_transposed.cpu(), (mask > 0.5).sum(-2).int())
+
+
+def test_native_stack_on_many_streams_and_threads():
+    """More caller's streams than side tracks are kept, and two threads on the same stream."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from bionemo_inference_runtime_b200.layers import pairformer
+
+    stack = _randomise(b200.PairformerModule(num_blocks=3, dtype=torch.bfloat16, triangle_attn_backend="Heuristic").to(DEV))
+    g = torch.Generator(device=DEV).manual_seed(5)
+    mask, pair = torch.ones(1, 56, device=DEV), torch.ones(1, 56, 56, device=DEV)
+    inputs = [(torch.randn(1, 56, 384, generator=g, device=DEV).bfloat16(),
+               torch.randn(1, 56, 56, 128, generator=g, device=DEV).bfloat16(), mask, pair) for _ in range(10)]
+    want = [stack(*i) for i in inputs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in inputs]
+
+    def call(k, repeats=3):
+        with torch.cuda.stream(streams[k]):
+            for _ in range(repeats):
+                out = stack(*inputs[k])
+        streams[k].synchronize()
+        return out
+
+    for _ in range(2):
+        for k, out in enumerate([call(k) for k in range(len(inputs))]):
+            assert all(torch.equal(a, b) for a, b in zip(out, want[k]))
+    assert len(pairformer._side_tracks) <= 8
+    streams[1] = streams[0]  # two threads, one stream
+    with ThreadPoolExecutor(2) as pool:
+        for k, out in enumerate(pool.map(lambda k: call(k, 20), (0, 1))):
+            assert all(torch.equal(a, b) for a, b in zip(out, want[k]))
+    assert _lib.device_status() == 0
