@@ -27,10 +27,17 @@
 // tile two.  The bias is added by the softmax threads: on the tensor core (an identity MMA) it would need 64 more
 // columns and four times the operations of Q·Kᵀ, which cost clock rate under the power cap.
 //
-// Measured (one launch, all tokens valid, before this split of two 128-key tile halves per CTA -> now): 512 tokens
-// 224 -> 199 us, 1024 tokens 1.41 ms, 2048 tokens 12.6 -> 10.7 ms (11.1 exponentials a clock and SM; a tile of four units
-// takes some 2600 clocks against 2048 at the unit's rate), an item's end and start another 3500; the masked form at 333
-// tokens 190 -> 106 us.
+// Measured against two halves of 256 queries x 128 keys per CTA and the bias on the tensor core (one launch, all tokens
+// valid, back to back, with the median SM clock sampled meanwhile; the clock is below 1965 MHz under the power cap):
+//   512 tokens            426 -> 383 thousand clocks    250 us at 1702 MHz -> 204 at 1875
+//   768 tokens            1.293 -> 1.220 million        775 us at 1668     -> 643 at 1897
+//   1024 tokens           2.937 -> 2.763 million        1.757 ms at 1672   -> 1.453 at 1901
+//   2048 tokens           21.48 -> 20.96 million        13.08 ms at 1642   -> 10.90 at 1924
+//   512 rows, 4096 keys   20.36 -> 20.65 million        12.45 ms at 1635   -> 10.67 at 1935
+// So short rows need fewer clocks, because the units' hand-overs fill one another and the items are smaller; long rows need
+// as many as before, and what they gain is clock rate, presumably because the bias does not go through the tensor cores.
+// A launch takes about (items per SM, rounded up) x (2790 x tiles + 5000) clocks, at 2048 tokens 11.1 of 16 exponentials a
+// clock and SM.  The masked form takes 105 us at 333 tokens, the unmasked one 84.
 //
 // A pair row without a valid key takes a constant path in "uniform" mode (probabilities all 1: the output is the
 // mean of V, as the eager reference computes it) and is skipped in "zeros" mode.
@@ -635,7 +642,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int kt = max(my_tiles, 0), all = info->tiles; kt < all; ++kt)
         if (++stage == kStages) stage = 0, stage_phase ^= 1;
       // The info is read again here: kept over the tiles it cost registers that the tile loop spilled (512 tokens 204 ->
-      // 199 us, the masked form at 333 tokens 136 -> 106).
+      // 199 us, the masked form at 333 tokens 136 -> 106; the unmasked form still spills two registers).
       const int br = info->unit[w].br, q = info->unit[w].q0 + m, h = info->h;  // pair row, query position
       mbar_arrive_warp_after_reads(bars + (Q_EMPTY + ib) * 8);
       if (my_tiles < 0) continue;  // the item has no such unit

@@ -14,8 +14,10 @@
 // Warp roles: warps 0-7 epilogue (TMEM lanes 32(w%4)..+31), warp 8 TMA producer, warp 9 MMA issuer / TMEM owner, and in
 // the prologue warps 10-13 LayerNorm statistics (one thread per row, a tile ahead of the epilogue).
 //
-// The prologue is bound by its writes (1032 of 1288 bytes per position).  Its epilogue warps used to compute the
-// statistics themselves, in both warpgroups: 15.9 thousand warp instructions a tile, a third of them for that.
+// The prologue is bound by its writes, 1032 of 1288 bytes per position: 82 us at 512 tokens and 172 at 768, where a plain
+// fill of 1032 bytes per position takes 74 and 160.  The statistics have warps of their own because both epilogue
+// warpgroups would compute them otherwise (34.4 instead of 27.7 million warp instructions at 512 tokens).
+// The epilogue kernel moves 768 bytes per position: 43 us at 512 tokens (4.7 TB/s), 80 at 768 (5.7).
 #include "common.cuh"
 #include "layout.h"
 

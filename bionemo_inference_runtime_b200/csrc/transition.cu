@@ -3,7 +3,8 @@
 // The ReLU form (kRelu) computes out = [x +] mask * ( relu(LayerNorm(x) · W1ᵀ + b1) · W2ᵀ + b2 ) with the same
 // pipeline: its 512 hidden rows sit in the value half of the packed first linear.  It has no gates, so that an accumulator
 // of GEMM1 holds 128 hidden units: four of them per tile, each in two H tiles.  (With 64 values and 64 zero gates, as
-// the SwiGLU form, it had twice the hand-overs and half again the operations: 640 x 640 rows 168 us, now 163.)
+// the SwiGLU form, it had twice the hand-overs and half again the operations: a call on 640 x 640 rows with
+// a mask 168 us instead of 164.)
 //
 // A persistent CTA per SM walks 128-row tiles of x.  The hidden dimension is cut in
 // 8 chunks of 64 units; for each chunk

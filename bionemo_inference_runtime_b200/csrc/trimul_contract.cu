@@ -4,13 +4,12 @@
 // writes a and b channel-major with the contraction index k contiguous (for the incoming node it walks the pair
 // tensor through swapped strides, so the same layout serves both directions), so both operands are K-major.
 //
-// Bound: the operand tiles' way from L2 (12.8 TB/s reached).  With [128 x 256] output tiles and two accumulators of them
-// (the epilogue of one beside the MMAs of the other) every 64-wide K step of 548 clocks of MMAs asked for 48 KiB, which L2
-// does not deliver: 106 us at 768 tokens, half of the tensor cores' rate.  A CTA now computes [256 x 256] tiles, two
-// accumulators of 128 rows side by side in all of tensor memory: 64 KiB per step and twice the MMAs.  The epilogue is no
-// longer hidden behind MMAs, but behind the next tile's loads.  Column tiles are as wide as the token count needs (a
-// multiple of 32), a lower half without rows is left out.  768 tokens 106 -> 98 us; at 512 tokens (46 us) and 64 x 256
-// (522 us) the bytes from HBM bound it as before.
+// Bound: the operand tiles' way from L2 (12.8 TB/s reached).  A CTA computes [256 x 256] tiles, two accumulators of 128 rows
+// side by side in all of tensor memory: 64 KiB per 64-wide K step of 1096 clocks of MMAs, its epilogue behind the next
+// tile's loads.  [128 x 256] tiles with two accumulators, the epilogue of one beside the MMAs of the other, ask for 48 KiB
+// per 548 clocks, which L2 does not deliver: 106 us at 768 tokens, now 98 (1180 TFLOP/s).  Column tiles are as wide as the
+// token count needs (a multiple of 32), a lower half without rows is left out.  At 512 tokens (45 us) and 64 x 256
+// (522 us) the bytes from HBM bound it.
 //
 // TMA loads [256 x 64] operand tiles into a three-stage ring, one warp issues tcgen05.mma (M 128, N up to 256, K 16), and
 // eight epilogue warps (TMEM lane = output row) convert the finished accumulators to bf16, stage 32 rows of 64 bytes each

@@ -9,14 +9,13 @@
 // The folded weight rows (four blocks of 128: gate and value of the a and of the b channels) stay in tensor memory as the
 // A operand for the whole kernel (256 columns), the raw tile of 128 positions is the B operand.
 //
-// Bound: the writes, 512 of 768 bytes per position (a plain fill of this memory reaches 3.95 TB/s).  The weights used to
-// be A operands in shared memory (128 KiB, read again for every tile) with four accumulators of 128 positions in all of
-// tensor memory: the MMAs of a tile waited for the epilogue of the one before, and with two 32 KiB stages left, so did
-// the loads (131 us at 768 tokens, 3.4 TB/s).  With the weights in tensor memory an MMA takes 36 instead of 69 clocks for
-// half the positions, so accumulators of 64 positions cost nothing, and two of them (a, b) are in turn filled and read;
-// shared memory is a ring of four tiles.  What took the time then was the load-store unit: a 32-byte store of 32 lanes to
-// 32 channels' runs occupies it for some 56 clocks.  Each warp now stages its 32 channels x 32 positions in shared memory
-// and hands them to a TMA store.
+// Bound: first the writes, 512 of 768 bytes per position: at 768 tokens the kernel takes 100 us, a plain fill of 512 bytes per
+// position 82.  No other unit is near its limit (issue slots 58 %, special functions 44 %, tensor pipe 39 % busy).
+// With the weights in tensor memory an MMA takes 36 clocks for 64 positions (as shared-memory operand 69 for 128), so that
+// accumulators of 64 positions cost nothing, two of them (a, b) are in turn filled and read, and shared memory is a ring
+// of four tiles.  A warp stages its 32 channels x 32 positions in shared memory and hands them to a TMA store, because a
+// 32-byte store of 32 lanes to 32 channels' runs occupies the load-store unit for some 56 clocks.  Without the two
+// (weights in shared memory, two tiles in flight, direct stores): 131 us.
 //
 // LayerNorm is folded into the weights (rows centred, per-row sum kept; gamma, beta and the biases included): the
 // MMAs run on the raw tile as soon as it has landed, four statistics warps (one thread per position) compute mean
