@@ -802,11 +802,11 @@ def run_sharded(args) -> dict:
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per attention launch, from the committed ncu summary of the cfg2
-# capture (profiles/attention_kernel_cfg2.md: 270.6 MB read + 53.4 MB written for 512 x 512 positions).  The traffic is
+# capture (profiles/attention_kernel_cfg2.md: 270.6 MB read + 52.5 MB written for 512 x 512 positions).  The traffic is
 # the q / k / v / gate planes read once and the output written once, i.e. proportional to the pair positions of the
 # launch, so the larger workloads scale that capture by their positions (cfg5: one rank's shard of a node).
-TRAFFIC_PER_POSITION = 324.0e6 / (512 * 512)
-TRAFFIC: dict[str, float | None] = {"cfg2": 324.0e6, "cfg3": None, "n768": TRAFFIC_PER_POSITION * 768 * 768,
+TRAFFIC_PER_POSITION = 323.1e6 / (512 * 512)
+TRAFFIC: dict[str, float | None] = {"cfg2": 323.1e6, "cfg3": None, "n768": TRAFFIC_PER_POSITION * 768 * 768,
                                     "cfg5": TRAFFIC_PER_POSITION * 4096 * 4096}
 
 
